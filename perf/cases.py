@@ -52,13 +52,13 @@ def model(kind: str, width: int, layers: int, vocab: int, batch: int, prompt: in
 def listed() -> list:
     return [
         # one token through q/k/v: the smallest call, all latency
-        linear("qkv", 2560, 1, name="linear qkv, 1 row"),
+        linear("qkv", 2560, 1, name="linear qkv 1 row"),
         # a decode batch of eleven through gate and up
-        linear("gate_up", 2560, 11, name="linear gate/up, 11 rows"),
+        linear("gate_up", 2560, 11, name="linear gate/up 11 rows"),
         # a short prompt, its length a multiple of nothing, through the long projection
-        linear("down", 2560, 333, name="linear down, 333 rows"),
+        linear("down", 2560, 333, name="linear down 333 rows"),
         # a long prompt through the largest group
-        linear("gate_up", 2560, 2048, name="linear gate/up, 2048 rows"),
+        linear("gate_up", 2560, 2048, name="linear gate/up 2048 rows"),
         # every projection of a 2B4T-shaped model, one token
         sweep(2560, 30, name="sweep of 30 layers"),
         # a chat of one user: the whole 2B4T-shaped model, 2000 tokens read, 48 written
@@ -68,9 +68,9 @@ def listed() -> list:
         # reading a document of an odd length
         model("bitnet", 2560, 8, 32000, 1, 2011, 0, name="bitnet prompt"),
         # a long conversation under a sliding window
-        model("pefolix", 2560, 4, 32000, 1, 3000, 48, window=1024, name="pefolix chat, window"),
+        model("pefolix", 2560, 4, 32000, 1, 3000, 48, window=1024, name="pefolix chat window"),
         # eight users of a model with experts
-        model("pefolix", 2560, 2, 32000, 8, 200, 32, experts=True, name="pefolix batch of 8, experts"),
+        model("pefolix", 2560, 2, 32000, 8, 200, 32, experts=True, name="pefolix batch of 8 experts"),
         # reading a document with recurrent and latent layers
         model("dugulorn", 2560, 4, 32000, 1, 2048, 0, name="dugulorn prompt"),
         # sixteen users of such a model
