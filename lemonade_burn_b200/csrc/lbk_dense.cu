@@ -2,15 +2,13 @@
 // epilogue (lbk_dense_dev.cuh: f32 rows, activated rows in the compute type, or [q; k; v] rows of which k and v
 // go straight into the cache):
 //
-//   dense_few_kernel   up to 8 tokens (decode, short portions). Bound: HBM, the weights once. 16 weight rows
-//                      are the M side of mma.sync m16n8k16, the tokens its N side; a lane's 16-byte weight load
-//                      is two MMAs' operands as it is (the contraction index may be permuted as long as both
-//                      operands are permuted alike), so weights go global -> registers -> tensor core without
-//                      shared memory or shuffles. The 16 warps of a CTA split K and meet in shared memory once per
-//                      tile. Where whole tiles would leave SMs idle in the last round, the (tile, K) stream is cut into
-//                      equal runs instead: a tile shared by several CTAs leaves partial sums in memory, and the one
-//                      that arrives last adds them up in CTA order. The norms in front of the projection run in the prologue (at one or two tokens),
-//                      while the CTA's first weight rows are on their way to L2.
+//   dense_few_kernel   up to 16 tokens (decode, short portions). Bound: HBM, the weights once. The streaming loop is
+//                      lbk_few.cuh's: TMA boxes, mma.sync, no sums across CTAs. The norms in front of the projection run in
+//                      the prologue (at one or two tokens), while the CTA's first weight rows are on their way. In a decode
+//                      step (cold weights, time until the next kernel can start), against the kernel that loaded MMA
+//                      fragments straight from global memory and cut tiles between CTAs: gate/up 2560 -> 6912 33 -> 18 us at
+//                      one token (with the norms), 31 -> 12 at eight; 6912 -> 2560 14.6 -> 7 and 53 -> 6; and against the tcgen05
+//                      kernel at 16 tokens: 2560 -> 6912 10.7 -> 7.4, 6912 -> 2560 13.7 -> 10.5, 2560 -> 10240 20 -> 12.
 //   dense_gemm_kernel  more tokens: tcgen05 (kind::f16), 128 weight rows x up to 256 tokens a tile, both operands
 //                      by TMA (SWIZZLE_128B, 64 columns a stage), two accumulators in tensor memory so that the
 //                      epilogue of one tile runs under the MMAs of the next, one persistent CTA per SM. A gated
@@ -24,8 +22,11 @@
 //                      With experts the tokens
 //                      arrive sorted and the tile list comes from the device-side counts.
 //   dense_f32_kernel   everything in 32-bit (FMA), for LBK_COMPUTE_F32.
+#include <algorithm>
+
 #include "lbk_dense.cuh"
 #include "lbk_dense_dev.cuh"
+#include "lbk_few.cuh"
 #include "lbk_ptx.cuh"
 #include "lbk_tcgen05.cuh"
 
@@ -36,33 +37,42 @@ namespace {
 using namespace tc;
 
 // ---- few tokens ---------------------------------------------------------------------------------
-constexpr int kFewThreads = 512, kFewWarps = 16;
-constexpr int kFewTokens = 8;               // up to here; 9 to 16 tokens run faster on dense_gemm_kernel (14336 -> 4096: 26 against 38 us)
+using few::kThreads;
+using few::kTiles;
+using few::kWarps;
 constexpr int kFewPreMax = 2;               // tokens whose norms run in the prologue
-constexpr size_t kFewXSmem = 96 * 1024;     // activations in shared memory up to this, else read through L1
-
-constexpr int kFewPart = 2 * 128;           // floats of a partial tile: gate and up, 8 tokens, 16 rows
-constexpr int kFewMaxTiles = 1 << 14, kFewMaxCtas = 512;
-constexpr int kFewPrefetch = 2;             // 128-byte lines a thread asks L2 for ahead of the kernel in front
+constexpr int kFewPrefetch = 8;             // boxes beyond its ring that a warp asks L2 for ahead of the kernel in front
 
 struct FewParams {
-    const uint16_t *w;
-    size_t pitch;
-    int out_rows, up_row, chunks, tiles, m;
+    alignas(64) CUtensorMap w;              // bytes [rows][pitch * 2], box [box_rows][128]
+    int out_rows, up_row, chunks, m;        // chunks of 64 columns
+    int box_rows, boxes;                    // a CTA's rows: `boxes` times box_rows
     const uint16_t *x;
     long ldx;
-    int x_smem, xs_stride;                  // bytes per token row in shared memory
-    int per;                                // 32-column chunks of the (tile, K) stream a CTA takes
-    float *parts;                           // [2 * CTAs][kFewPart] partial sums of tiles shared between CTAs
-    int *counters;                          // [tiles], zero at rest
     DenseEpi epi;
     DensePre pre;
-    int n;                                  // columns of the normed row
+    int n, xs_stride;                       // columns of the normed row; bytes between such rows in shared memory
+    int *err_word;
+};
+
+// The norms' weights, asked for before the kernel in front is known to be complete (they come from HBM: a step reads more
+// than L2 holds).
+struct FewGains {
+    float4 post[4], norm[4];
+    __device__ __forceinline__ void load(const FewParams &p) {
+        const int n4 = p.n >> 2;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = threadIdx.x + j * kThreads;
+            post[j] = p.pre.mode == kPreAddNorm && i < n4 ? __ldg(reinterpret_cast<const float4 *>(p.pre.w_post) + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+            norm[j] = p.pre.w && i < n4 ? __ldg(reinterpret_cast<const float4 *>(p.pre.w) + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        }
+    }
 };
 
 // One token's row: the norms of DensePre, the result as bf16 into shared memory (and nout). 512 threads, up to
 // four float4 each (rows of at most 8192 values).
-__device__ __forceinline__ void few_norm_row(const FewParams &p, int t, bool writer, uint16_t *dst, float *s_red) {
+__device__ __forceinline__ void few_norm_row(const FewParams &p, const FewGains &gains, int t, bool writer, uint16_t *dst, float *s_red) {
     const int n4 = p.n >> 2, tid = threadIdx.x;
     const float inv_n = 1.0f / static_cast<float>(p.n);
     const float4 *xr = reinterpret_cast<const float4 *>(p.pre.x + static_cast<size_t>(t) * p.n);
@@ -70,7 +80,7 @@ __device__ __forceinline__ void few_norm_row(const FewParams &p, int t, bool wri
     float4 v[4], u[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const int i = tid + j * kFewThreads;
+        const int i = tid + j * kThreads;
         u[j] = i < n4 ? xr[i] : zero;
     }
     if (p.pre.mode == kPreAddNorm) {
@@ -78,24 +88,24 @@ __device__ __forceinline__ void few_norm_row(const FewParams &p, int t, bool wri
         float s = 0.0f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int i = tid + j * kFewThreads;
+            const int i = tid + j * kThreads;
             v[j] = i < n4 ? yr[i] : zero;
             s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
         }
-        const float mean = p.pre.rms ? 0.0f : dense::block_sum<kFewThreads>(s, s_red) * inv_n;
+        const float mean = p.pre.rms ? 0.0f : dense::block_sum<kThreads>(s, s_red) * inv_n;
         float ss = 0.0f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int i = tid + j * kFewThreads;
+            const int i = tid + j * kThreads;
             v[j] = i < n4 ? make_float4(v[j].x - mean, v[j].y - mean, v[j].z - mean, v[j].w - mean) : zero;
             ss += (v[j].x * v[j].x + v[j].y * v[j].y) + (v[j].z * v[j].z + v[j].w * v[j].w);
         }
-        const float r = 1.0f / sqrtf(dense::block_sum<kFewThreads>(ss, s_red) * inv_n + p.pre.eps);
+        const float r = 1.0f / sqrtf(dense::block_sum<kThreads>(ss, s_red) * inv_n + p.pre.eps);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int i = tid + j * kFewThreads;
+            const int i = tid + j * kThreads;
             if (i < n4) {
-                const float4 g = __ldg(reinterpret_cast<const float4 *>(p.pre.w_post) + i);
+                const float4 g = gains.post[j];
                 u[j] = make_float4(u[j].x + v[j].x * r * g.x, u[j].y + v[j].y * r * g.y, u[j].z + v[j].z * r * g.z, u[j].w + v[j].w * r * g.w);
                 if (writer) reinterpret_cast<float4 *>(p.pre.xout + static_cast<size_t>(t) * p.n)[i] = u[j];
             }
@@ -108,24 +118,24 @@ __device__ __forceinline__ void few_norm_row(const FewParams &p, int t, bool wri
             float s = 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) s += (u[j].x + u[j].y) + (u[j].z + u[j].w);
-            mean = dense::block_sum<kFewThreads>(s, s_red) * inv_n;
+            mean = dense::block_sum<kThreads>(s, s_red) * inv_n;
         }
         float ss = 0.0f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int i = tid + j * kFewThreads;
+            const int i = tid + j * kThreads;
             u[j] = i < n4 ? make_float4(u[j].x - mean, u[j].y - mean, u[j].z - mean, u[j].w - mean) : zero;
             ss += (u[j].x * u[j].x + u[j].y * u[j].y) + (u[j].z * u[j].z + u[j].w * u[j].w);
         }
-        r = 1.0f / sqrtf(dense::block_sum<kFewThreads>(ss, s_red) * inv_n + p.pre.eps);
+        r = 1.0f / sqrtf(dense::block_sum<kThreads>(ss, s_red) * inv_n + p.pre.eps);
     }
-    const int pad4 = p.chunks * 8;          // chunks of 32 columns: zeros past the row
+    const int pad4 = p.chunks * 16;         // chunks of 64 columns: zeros past the row
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const int i = tid + j * kFewThreads;
+        const int i = tid + j * kThreads;
         uint2 o = make_uint2(0u, 0u);
         if (i < n4) {
-            const float4 g = p.pre.w ? __ldg(reinterpret_cast<const float4 *>(p.pre.w) + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+            const float4 g = gains.norm[j];
             o = make_uint2(dense::bf16_pair(u[j].x * r * g.x, u[j].y * r * g.y), dense::bf16_pair(u[j].z * r * g.z, u[j].w * r * g.w));
             if (writer && p.pre.nout) reinterpret_cast<uint2 *>(static_cast<uint16_t *>(p.pre.nout) + static_cast<size_t>(t) * p.pre.ldn)[i] = o;
         }
@@ -133,186 +143,107 @@ __device__ __forceinline__ void few_norm_row(const FewParams &p, int t, bool wri
     }
 }
 
-template <bool DUAL>
-__global__ void __launch_bounds__(kFewThreads, 1) dense_few_kernel(const __grid_constant__ FewParams p) {
-    extern __shared__ __align__(16) uint8_t few_smem[];
+// MT: tiles of 16 rows a box holds
+template <bool DUAL, int NTL, int MT>
+__global__ void __launch_bounds__(kThreads, 1) dense_few_kernel(const __grid_constant__ FewParams p) {
+    extern __shared__ uint8_t few_smem[];
     __shared__ float s_red[32];
-    constexpr int NA = DUAL ? 2 : 1;
-    constexpr int kPart = NA * 128;         // floats a warp contributes per tile
-    float *s_part = reinterpret_cast<float *>(few_smem);               // [2][16 warps][kPart]
-    uint8_t *s_x = few_smem + 2 * kFewWarps * kPart * sizeof(float);
+    constexpr int NA = DUAL ? 2 : 1, NB = kTiles / MT, TT = NB / NA;  // NB: boxes a warp carries at a time, TT: of gate and of up
+    const uint32_t raw = ptx::smem_u32(few_smem), base = (raw + 1023u) & ~1023u;
+    uint8_t *sm = few_smem + (base - raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     ptx::pdl_trigger();
-    const int s_begin = static_cast<int>(blockIdx.x) * p.per, s_end = min(p.tiles * p.chunks, s_begin + p.per);
-    // the weights are constants: the first of this CTA's rows start moving to L2 while the kernel in front finishes
-    {
-        int at = s_begin, left = kFewPrefetch * kFewThreads;
-        while (at < s_end && left > 0) {
-            const int tile = at / p.chunks, a = at - tile * p.chunks, b = min(p.chunks, a + s_end - at);
-            const int l0 = a / 2, lines = (b + 1) / 2 - l0;  // 128-byte lines of a row (pitch is a multiple of 64 columns)
-#pragma unroll
-            for (int w = 0; w < NA; ++w)
-                for (int i = tid; i < 16 * lines; i += kFewThreads) {
-                    const int r = min(tile * 16 + i / lines, p.out_rows - 1) + w * p.up_row;
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + static_cast<size_t>(r) * p.pitch + (l0 + i % lines) * 64));
-                }
-            left -= NA * 16 * lines;
-            at += b - a;
+    const int n_chunks = few::chunks_of(p.chunks, warp);                           // this warp's: warp, warp + 16, ...
+    const int row_base = static_cast<int>(blockIdx.x) * p.boxes * p.box_rows;
+    const int total = n_chunks * p.boxes * NA;                                   // its boxes
+    few::Ring ring(sm, base, warp, p.box_rows);
+    // the sequence of boxes: TT at a time, chunks within them, boxes within a chunk
+    struct Cursor {
+        int q, k, c;                        // first box, box within the chunk, chunk
+    };
+    auto step = [&](Cursor &u) {
+        if (++u.k < min(TT, p.boxes - u.q) * NA) return;
+        u.k = 0;
+        if ((u.c += kWarps) < p.chunks) return;
+        u.c = warp;
+        u.q += TT;
+    };
+    auto row_of = [&](const Cursor &u) { return row_base + (u.q + u.k / NA) * p.box_rows + (u.k % NA) * p.up_row; };
+    Cursor is{0, 0, warp};
+    auto load = [&](int slot) {
+        ring.fetch(slot, &p.w, is.c * 128, row_of(is));
+        step(is);
+    };
+    // The weights are constants: this warp's first boxes are on their way, and more of them asked into L2, while the kernel
+    // in front finishes.
+    if (lane == 0) {
+        ring.init();
+        for (int i = 0; i < min(ring.depth, total); ++i) load(i);
+        Cursor ahead = is;
+        for (int i = ring.depth; i < min(ring.depth + kFewPrefetch, total); ++i) {
+            few::prefetch_box(&p.w, ahead.c * 128, row_of(ahead));
+            step(ahead);
         }
     }
+    FewGains gains;
+    if (p.pre.mode != kPreNone) gains.load(p);
     ptx::pdl_wait();
     int pos0;
-    if (!dense::rows_fit(p.epi, p.m, pos0)) return;
+    const bool fits = dense::rows_fit(p.epi, p.m, pos0);
+    const uint8_t *xr[NTL];                 // this lane's token rows; the normed ones lie in shared memory
+    uint8_t *s_x = sm + few::rest_at(NTL);
     if (p.pre.mode != kPreNone) {
-        for (int tk = 0; tk < p.m; ++tk) few_norm_row(p, tk, blockIdx.x == 0, reinterpret_cast<uint16_t *>(s_x + tk * p.xs_stride), s_red);
-        __syncthreads();
-    } else if (p.x_smem) {
-        const int units = p.chunks * 4;     // 16-byte units per row
-        for (int i = tid; i < p.m * units; i += kFewThreads) {
-            const int tk = i / units, c = i - tk * units;
-            *reinterpret_cast<uint4 *>(s_x + tk * p.xs_stride + c * 16) = *reinterpret_cast<const uint4 *>(p.x + static_cast<size_t>(tk) * p.ldx + c * 8);
-        }
+        for (int tk = 0; tk < p.m; ++tk) few_norm_row(p, gains, tk, blockIdx.x == 0, reinterpret_cast<uint16_t *>(s_x + tk * p.xs_stride), s_red);
         __syncthreads();
     }
-    __shared__ int s_last;
-    // The CTA's run of the stream is a sequence of tile parts, a warp's share of one part a sequence of steps of U
-    // chunks. The loads of a step are issued one step ahead, across tiles too: a warp always has two steps in flight.
-    constexpr int U = DUAL ? 2 : 4;
-    struct Step {
-        int tile, k0, k1, c, c1;
+#pragma unroll
+    for (int j = 0; j < NTL; ++j)
+        xr[j] = (p.pre.mode != kPreNone ? s_x + (j * 8 + g) * p.xs_stride : reinterpret_cast<const uint8_t *>(p.x + static_cast<size_t>(j * 8 + g) * p.ldx)) + t * 32;
+    auto tokens = [&](few::Tokens<NTL> &x, int c) {
+#pragma unroll
+        for (int j = 0; j < NTL; ++j) {
+            x.lo[j] = x.hi[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (j * 8 + g < p.m) {
+                x.lo[j] = *reinterpret_cast<const uint4 *>(xr[j] + c * 128);
+                x.hi[j] = *reinterpret_cast<const uint4 *>(xr[j] + c * 128 + 16);
+            }
+        }
     };
-    int at = s_begin;
-    auto next_part = [&](Step &q) {
-        q.tile = at / p.chunks;
-        q.k0 = at - q.tile * p.chunks;
-        q.k1 = min(p.chunks, q.k0 + s_end - at);
-        at += q.k1 - q.k0;
-        const int c_per = (q.k1 - q.k0 + kFewWarps - 1) / kFewWarps;
-        q.c = min(q.k1, q.k0 + warp * c_per);
-        q.c1 = min(q.k1, q.c + c_per);
-    };
-    uint4 wl[NA][U], wh[NA][U], nl[NA][U], nh[NA][U];
-    auto load = [&](const Step &q, uint4 (&lo)[NA][U], uint4 (&hi)[NA][U]) {
-        const uint16_t *a = p.w + static_cast<size_t>(min(q.tile * 16 + g, p.out_rows - 1)) * p.pitch + t * 8;
-        const uint16_t *b = p.w + static_cast<size_t>(min(q.tile * 16 + g + 8, p.out_rows - 1)) * p.pitch + t * 8;
-        const size_t up = static_cast<size_t>(p.up_row) * p.pitch;
+    const few::Units units(lane);
+    float *red = reinterpret_cast<float *>(sm + few::red_at());
+    few::Tokens<NTL> x, x_next;
+    if (warp < p.chunks) tokens(x_next, warp);
+    int done = 0;
+    for (int q = 0; q < p.boxes; q += TT) {
+        const int boxes = min(TT, p.boxes - q);
+        float acc[kTiles][NTL][4];
+        few::zero<NTL>(acc);
+        for (int c = warp; c < p.chunks; c += kWarps) {
+            x = x_next;
+            tokens(x_next, c + kWarps < p.chunks ? c + kWarps : warp);
 #pragma unroll
-        for (int i = 0; i < U; ++i)
-            if (q.c + i < q.c1) {
-#pragma unroll
-                for (int w = 0; w < NA; ++w) {
-                    lo[w][i] = __ldcs(reinterpret_cast<const uint4 *>(a + w * up + (q.c + i) * 32));
-                    hi[w][i] = __ldcs(reinterpret_cast<const uint4 *>(b + w * up + (q.c + i) * 32));
+            for (int k = 0; k < NB; ++k)
+                if (k < boxes * NA) {
+                    few::box_mma<NTL, MT>(ring.wait(), units, x, acc + k * MT);
+                    __syncwarp();           // every lane has read the box before it is refilled
+                    if (lane == 0 && done + ring.depth < total) load(ring.s);
+                    ++done;
+                    ring.next();
                 }
-            }
-    };
-    float acc[NA][4];
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-        acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.0f;
-    int buf = 0;
-    Step cur, nxt;
-    bool more = at < s_end;
-    if (more) {
-        next_part(cur);
-        load(cur, wl, wh);
-    }
-    while (more) {
-        nxt = cur;
-        const bool part_done = cur.c + U >= cur.c1;
-        if (!part_done) {
-            nxt.c += U;
-        } else if (at < s_end) {
-            next_part(nxt);
-        } else {
-            more = false;
         }
-        if (more) load(nxt, nl, nh);
-#pragma unroll
-        for (int i = 0; i < U; ++i)
-            if (cur.c + i < cur.c1) {
-                uint4 b = make_uint4(0u, 0u, 0u, 0u);
-                if (g < p.m)
-                    b = p.x_smem ? *reinterpret_cast<const uint4 *>(s_x + g * p.xs_stride + (cur.c + i) * 64 + t * 16)
-                                 : *reinterpret_cast<const uint4 *>(p.x + static_cast<size_t>(g) * p.ldx + (cur.c + i) * 32 + t * 8);
-#pragma unroll
-                for (int a = 0; a < NA; ++a) {
-                    const uint32_t a0[4] = {wl[a][i].x, wh[a][i].x, wl[a][i].y, wh[a][i].y};
-                    const uint32_t a1[4] = {wl[a][i].z, wh[a][i].z, wl[a][i].w, wh[a][i].w};
-                    ptx::mma_bf16(acc[a], a0, b.x, b.y);
-                    ptx::mma_bf16(acc[a], a1, b.z, b.w);
-                }
-            }
-        const int tile = cur.tile, k0 = cur.k0, k1 = cur.k1;
-        cur = nxt;
-#pragma unroll
-        for (int w = 0; w < NA; ++w)
-#pragma unroll
-            for (int i = 0; i < U; ++i) {
-                wl[w][i] = nl[w][i];
-                wh[w][i] = nh[w][i];
-            }
-        if (!part_done) continue;
-        // the sixteen K ranges meet: [warp][a][token][row], then one thread per output
-        float *part = s_part + (buf * kFewWarps + warp) * kPart;
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            float *o = part + a * 128;
-            o[(2 * t) * 16 + g] = acc[a][0];
-            o[(2 * t + 1) * 16 + g] = acc[a][1];
-            o[(2 * t) * 16 + g + 8] = acc[a][2];
-            o[(2 * t + 1) * 16 + g + 8] = acc[a][3];
-            acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.0f;
-        }
-        buf ^= 1;         // the next part's sums go to the other buffer
-        __syncthreads();  // ... whose readers passed this point one part ago
-        const bool whole = k0 == 0 && k1 == p.chunks;
-        static_assert(kFewTokens == 8, "one MMA tile of tokens; 128 (token, row) pairs, a thread each");
-        const int o = tid, tk = o >> 4, r = tile * 16 + (o & 15);
-        const bool mine = o < 128 && tk < p.m && r < p.out_rows;
-        float v[NA];
-        if (mine) {
-#pragma unroll
-            for (int a = 0; a < NA; ++a) {
-                v[a] = 0.0f;
-#pragma unroll
-                for (int w = 0; w < kFewWarps; ++w) v[a] += s_part[((buf ^ 1) * kFewWarps + w) * kPart + a * 128 + o];
-            }
-        }
-        if (!whole) {
-            // a tile shared with neighbouring CTAs: a CTA's first tile has slot 2c, its last one slot 2c + 1
-            auto slot = [&](int c) { return p.parts + static_cast<size_t>(2 * c + (c * p.per / p.chunks == tile ? 0 : 1)) * kFewPart; };
-            float *own = slot(blockIdx.x);
-            if (mine) {
-#pragma unroll
-                for (int a = 0; a < NA; ++a) __stcg(own + a * 128 + o, v[a]);
-            }
-            __threadfence();
-            __syncthreads();
-            const int first = tile * p.chunks / p.per, last = ((tile + 1) * p.chunks - 1) / p.per;
-            if (tid == 0) {
-                const int before = atomicAdd(p.counters + tile, 1);
-                s_last = before == last - first;
-                if (s_last) p.counters[tile] = 0;
-            }
-            __syncthreads();
-            if (!s_last) continue;
-            __threadfence();
-            if (mine) {
-#pragma unroll
-                for (int a = 0; a < NA; ++a) v[a] = 0.0f;
-                for (int c = first; c <= last; ++c) {
-                    const float *q = slot(c);
-#pragma unroll
-                    for (int a = 0; a < NA; ++a) v[a] += __ldcg(q + a * 128 + o);
-                }
-            }
-        }
-        if (mine) {
-            const float val = DUAL ? dense::gelu_tanh<false>(v[0]) * v[NA - 1] : v[0];
-            dense::row_store<uint16_t>(p.epi, dense::row_plan<uint16_t>(p.epi, r, pos0), tk, val);
+        if (q) __syncthreads();             // the sums of the boxes before have been read
+        few::leave<NTL>(red + warp * few::red_floats(NTL), lane, boxes * NA * MT, acc);
+        __syncthreads();
+        for (int o = tid; o < boxes * MT * NTL * 128; o += kThreads) {
+            const int tile = o / (NTL * 128), f = o - tile * (NTL * 128), k = tile / MT, m = tile - k * MT;
+            const int in_box = m * 16 + few::place_row(f), tk = few::place_token(f), r = row_base + (q + k) * p.box_rows + in_box;
+            if (in_box >= p.box_rows || r >= p.out_rows || tk >= p.m || !fits) continue;
+            float v = few::collect<NTL>(red, k * NA * MT + m, f);
+            if (DUAL) v = dense::gelu_tanh<false>(v) * few::collect<NTL>(red, (k * NA + 1) * MT + m, f);
+            dense::row_store<uint16_t>(p.epi, dense::row_plan<uint16_t>(p.epi, r, pos0), tk, v);
         }
     }
+    if (!ring.ok && lane == 0) atomicExch(p.err_word, 5);
 }
 
 // ---- many tokens: tcgen05 -------------------------------------------------------------------------
@@ -714,44 +645,35 @@ __global__ void __launch_bounds__(256) dense_f32_kernel(const F32Params p) {
     }
 }
 
-int few_smem_bytes(const FewParams &p, bool dual) {
-    return 2 * kFewWarps * (dual ? 2 : 1) * 128 * static_cast<int>(sizeof(float)) + (p.x_smem ? p.m * p.xs_stride : 0);
+using FewKernel = void (*)(FewParams);
+template <bool DUAL>
+FewKernel few_kernel_of(int ntl, int mt) {
+    if (ntl == 1) return mt == 1 ? dense_few_kernel<DUAL, 1, 1> : dense_few_kernel<DUAL, 1, 2>;
+    return mt == 1 ? dense_few_kernel<DUAL, 2, 1> : dense_few_kernel<DUAL, 2, 2>;
 }
+FewKernel few_kernel(bool gated, int ntl, int mt) { return gated ? few_kernel_of<true>(ntl, mt) : few_kernel_of<false>(ntl, mt); }
 
 int launch_few(Ctx *ctx, const DenseCall &c, cudaStream_t st) {
     FewParams p{};
-    p.w = c.w.w;
-    p.pitch = c.w.pitch;
+    const int ntl = c.m > 8 ? 2 : 1;
+    const few::Deal deal = few::deal_rows(c.out_rows, ctx->sm_count);
     p.out_rows = static_cast<int>(c.out_rows);
     p.up_row = static_cast<int>(c.up_row);
-    p.chunks = static_cast<int>(c.w.pitch / 32);
-    p.tiles = static_cast<int>((c.out_rows + 15) / 16);
+    p.chunks = static_cast<int>(c.w.pitch / 64);
     p.m = static_cast<int>(c.m);
+    p.box_rows = deal.box_rows;
+    p.boxes = deal.boxes;
     p.x = static_cast<const uint16_t *>(c.x);
     p.ldx = c.ldx;
     p.epi = c.epi;
     p.pre = c.pre;
     p.n = static_cast<int>(c.w.cols);
-    p.xs_stride = static_cast<int>(c.w.pitch * 2 + 64);  // eight token rows start in different bank groups
-    p.x_smem = c.pre.mode != kPreNone || c.m * p.xs_stride <= kFewXSmem;
-    const size_t smem = static_cast<size_t>(few_smem_bytes(p, c.gated));
-    // Whole tiles, or equal runs of the (tile, K) stream when the idle SMs of the last round would cost more than the
-    // partial sums' trip through L2 (about 1.5 us; an SM streams about 40 bytes a nanosecond).
-    int grid = ctx->sm_count;
-    const int rounds = (p.tiles + grid - 1) / grid;
-    const double tile_us = static_cast<double>(p.chunks) * 1024.0 * (c.gated ? 2 : 1) / 40e3;
-    const double idle_us = (rounds - static_cast<double>(p.tiles) / grid) * tile_us;
-    if (idle_us > 1.5 && p.tiles <= kFewMaxTiles && grid <= kFewMaxCtas && ctx->few_parts) {
-        p.per = (p.tiles * p.chunks + grid - 1) / grid;
-        p.parts = static_cast<float *>(ctx->few_parts);
-        p.counters = reinterpret_cast<int *>(p.parts + static_cast<size_t>(2 * kFewMaxCtas) * kFewPart);
-        grid = (p.tiles * p.chunks + p.per - 1) / p.per;
-    } else {
-        p.per = rounds * p.chunks;
-        grid = (p.tiles + rounds - 1) / rounds;
-    }
-    void (*k)(FewParams) = c.gated ? dense_few_kernel<true> : dense_few_kernel<false>;
-    LBK_CUDA(launch_chained(k, dim3(static_cast<unsigned>(grid)), dim3(kFewThreads), smem, st, p));
+    p.xs_stride = static_cast<int>(c.w.pitch * 2 + 16);  // neighbouring token rows start in different bank groups
+    p.err_word = ctx->err_word;
+    LBK_TRY(encode_bytes_map(&p.w, c.w.w, c.w.pitch * 2, c.w.rows, c.w.pitch * 2, 128, deal.box_rows));
+    const size_t smem = static_cast<size_t>(few::rest_at(ntl)) + (c.pre.mode != kPreNone ? c.m * p.xs_stride : 0) + 1024;
+    const FewKernel k = few_kernel(c.gated, ntl, deal.box_rows > 16 ? 2 : 1);
+    LBK_CUDA(launch_chained(k, dim3(static_cast<unsigned>(deal.ctas)), dim3(kThreads), smem, st, p));
     LBK_CUDA(cudaGetLastError());
     ctx->launches++;
     return LBK_OK;
@@ -884,12 +806,10 @@ int launch_f32(Ctx *ctx, const DenseCall &c, cudaStream_t st) {
 }
 
 int dense_init(Ctx *ctx) {
-    constexpr size_t parts = static_cast<size_t>(2 * kFewMaxCtas) * kFewPart * sizeof(float) + kFewMaxTiles * sizeof(int);
-    LBK_CUDA(cudaMalloc(&ctx->few_parts, parts));
-    LBK_CUDA(cudaMemset(ctx->few_parts, 0, parts));
-    const int few_max = 2 * kFewWarps * 2 * 128 * 4 + static_cast<int>(kFewXSmem);
-    LBK_CUDA(cudaFuncSetAttribute(dense_few_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, few_max));
-    LBK_CUDA(cudaFuncSetAttribute(dense_few_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, few_max));
+    for (const bool gated : {false, true})
+        for (const int ntl : {1, 2})
+            for (const int mt : {1, 2})
+                LBK_CUDA(cudaFuncSetAttribute(few_kernel(gated, ntl, mt), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ctx->smem_optin) - 256));
     if (static_cast<size_t>(kGSmem) > ctx->smem_optin) return fail(LBK_ERR_UNSUPPORTED, "dense GEMM kernel needs %d B of shared memory", kGSmem);
     for (void (*k)(GemmParams) : {dense_gemm_kernel<0, false>, dense_gemm_kernel<kGated, false>, dense_gemm_kernel<kWide, false>,
                                   dense_gemm_kernel<kGated | kWide, false>, dense_gemm_kernel<0, true>, dense_gemm_kernel<kGated, true>})
@@ -907,7 +827,7 @@ int launch_dense(Ctx *ctx, const DenseCall &c, cudaStream_t st) {
     if (!c.w.w || (!c.x && c.pre.mode == kPreNone)) return fail(LBK_ERR_INVALID, "dense projection: null buffer");
     if (c.compute == LBK_COMPUTE_F32) return launch_f32(ctx, c, st);
     if (c.pre.mode != kPreNone && (!dense_pre_supported(c.m, c.w.cols) || c.experts)) return fail(LBK_ERR_INVALID, "dense projection: this call cannot run the norms itself");
-    if (c.m <= static_cast<size_t>(kFewTokens) && !c.experts) return launch_few(ctx, c, st);
+    if (c.m <= static_cast<size_t>(few::kMaxTokens) && !c.experts) return launch_few(ctx, c, st);
     return launch_gemm_tc(ctx, c, st);
 }
 

@@ -8,13 +8,17 @@
 //                    copied in expert order; the expert projections are then dense_gemm_kernel / dense_f32_kernel
 //                    calls over the sorted rows (lbk_dense.cu), and the norm behind the layer gathers, weights and sums
 //                    each token's rows (lbk_layernorm.cu).
-//   moe_few_up_kernel, moe_few_down_kernel   up to 16 tokens, bf16. Bound: HBM, the chosen experts' weights once.
-//                    A persistent CTA routes the tokens itself, takes (chosen expert, 16 rows) units, and folds
-//                    the routing weight into the activation. The down kernel owns 16 output rows and walks the
-//                    shared and all chosen experts' columns as one long K, so no partial sums leave the CTA and
-//                    the result does not depend on any order of arrival.
+//   moe_few_up_kernel, moe_few_down_kernel   up to 16 tokens, bf16. Bound: HBM, the chosen experts' weights once; the
+//                    streaming loop is lbk_few.cuh's. The up kernel routes the tokens itself and folds the routing weight into
+//                    the activation. In the down kernel a CTA owns output rows and walks the shared and all chosen
+//                    experts' columns as one long K, so the result does not depend on any order of arrival. Eight tokens,
+//                    6 of 64 experts of 2560 x 1408 each (about 35 chosen, 252 MB a projection): up 105 -> 46 us, down 147 ->
+//                    47 us against kernels whose lanes loaded their MMA fragments from global memory (5.5 TB/s now). For the
+//                    down kernel boxes of 18 rows count: with two boxes of 9 for the same rows it took 72 us, whatever
+//                    was in flight; a box costs its warp a wait, a refill and a chain of four MMAs.
 #include "lbk_dense.cuh"
 #include "lbk_dense_dev.cuh"
+#include "lbk_few.cuh"
 #include "lbk_ptx.cuh"
 
 namespace lbk {
@@ -133,51 +137,49 @@ __global__ void __launch_bounds__(128) moe_scatter_kernel(const int *ids, int to
 }
 
 // ---- few tokens -------------------------------------------------------------------------------------
-constexpr int kThreads = 512, kWarps = 16, kUnroll = 4;
+using few::kThreads;
+using few::kTiles;
+using few::kWarps;
 
 struct FewMoeParams {
+    alignas(64) CUtensorMap up;      // bytes [experts * ff][pitch * 2], box [16][128]
+    alignas(64) CUtensorMap down;    // bytes [experts * width][pitch * 2], box [box_rows][128]
+    alignas(64) CUtensorMap sdown;   // bytes [width][pitch * 2], box [box_rows][128]
     const uint16_t *n;
     long ldn;
     int m;
     const float *z;
     long ldz;
     int experts, top;
-    const uint16_t *up, *down, *sdown;
-    size_t up_pitch, down_pitch, sdown_pitch;
-    int up_chunks, down_chunks, sdown_chunks;
-    int ff, width, ff_tiles, width_tiles;
+    size_t down_pitch, sdown_pitch;
+    int up_chunks, down_chunks, sdown_chunks;  // of 64 columns
+    int ff, width, ff_tiles, box_rows, boxes;  // down: a CTA's rows are `boxes` times box_rows
     uint16_t *h;
     const uint16_t *hs;
     float *y;
     int *act;       // [0]: number of chosen experts, then (expert, 16 slots packed as bytes: 4 ints) each
+    int *err_word;
 };
 constexpr int kActInts = 5;
 
-// acc += W rows (r_lo, r_hi: this lane's two row pointers at its 8-column offset) x B rows, chunks of 32 columns
-template <int NTL>
-__device__ __forceinline__ void mma_chunk(float (&acc)[NTL][4], const uint4 &wl, const uint4 &wh, const uint4 (&b)[NTL]) {
-    const uint32_t a0[4] = {wl.x, wh.x, wl.y, wh.y};
-    const uint32_t a1[4] = {wl.z, wh.z, wl.w, wh.w};
-#pragma unroll
-    for (int j = 0; j < NTL; ++j) {
-        ptx::mma_bf16(acc[j], a0, b[j].x, b[j].y);
-        ptx::mma_bf16(acc[j], a1, b[j].z, b[j].w);
-    }
-}
-
+// The chosen experts' up projections: their tiles of 16 rows, one after the other, are dealt to the CTAs.
 template <int NTL, int R>
-__global__ void __launch_bounds__(kThreads, 1) moe_few_up_kernel(const FewMoeParams p) {
-    __shared__ float s_part[2][kWarps][NTL * 128];
+__global__ void __launch_bounds__(kThreads, 1) moe_few_up_kernel(const __grid_constant__ FewMoeParams p) {
+    extern __shared__ uint8_t moe_smem[];
     __shared__ int s_ids[LBK_GEMV_MAX_M][kMaxTop];
     __shared__ float s_wt[LBK_GEMV_MAX_M][kMaxTop];
     __shared__ unsigned s_mask[kMaxExperts];
     __shared__ short s_act[LBK_GEMV_MAX_M * kMaxTop];
     __shared__ int s_n;
-    ptx::pdl_trigger();
-    ptx::pdl_wait();
+    const uint32_t raw = ptx::smem_u32(moe_smem), base = (raw + 1023u) & ~1023u;
+    uint8_t *sm = moe_smem + (base - raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    few::Ring ring(sm, base, warp, 16);
+    ptx::pdl_trigger();
+    if (lane == 0) ring.init();
     for (int e = tid; e < p.experts; e += kThreads) s_mask[e] = 0u;
     __syncthreads();
+    ptx::pdl_wait();
     if (warp < p.m)
         route_token<R>(p.z + static_cast<size_t>(warp) * p.ldz, p.experts, p.top, lane, [&](int k, int e, float w) {
             if (lane == 0) {
@@ -205,7 +207,24 @@ __global__ void __launch_bounds__(kThreads, 1) moe_few_up_kernel(const FewMoePar
         while (k < p.top - 1 && s_ids[tk][k] != e) ++k;
         return k;
     };
-    if (blockIdx.x == 0) {  // the list for the down kernel
+    const int units = n_act * p.ff_tiles, cta = static_cast<int>(blockIdx.x), ctas = static_cast<int>(gridDim.x);
+    const int u0 = static_cast<int>(static_cast<long long>(units) * cta / ctas), u1 = static_cast<int>(static_cast<long long>(units) * (cta + 1) / ctas);
+    const int total = few::chunks_of(p.up_chunks, warp) * (u1 - u0);
+    struct Cursor {
+        int q, k, c;
+    } is{u0, 0, warp};
+    auto load = [&](int slot) {
+        const int u = is.q + is.k, a = u / p.ff_tiles;
+        ring.fetch(slot, &p.up, is.c * 128, s_act[a] * p.ff + (u - a * p.ff_tiles) * 16);
+        if (++is.k < min(kTiles, u1 - is.q)) return;
+        is.k = 0;
+        if ((is.c += kWarps) < p.up_chunks) return;
+        is.c = warp;
+        is.q += kTiles;
+    };
+    if (lane == 0)
+        for (int i = 0; i < min(ring.depth, total); ++i) load(i);
+    if (cta == 0) {  // the list for the down kernel
         if (tid == 0) p.act[0] = n_act;
         for (int a = tid; a < n_act; a += kThreads) {
             const int e = s_act[a];
@@ -217,76 +236,128 @@ __global__ void __launch_bounds__(kThreads, 1) moe_few_up_kernel(const FewMoePar
             }
         }
     }
-    const int c_per = (p.up_chunks + kWarps - 1) / kWarps;
-    const int c0 = min(p.up_chunks, warp * c_per), c1 = min(p.up_chunks, c0 + c_per);
-    int buf = 0;
-    for (int unit = blockIdx.x; unit < n_act * p.ff_tiles; unit += gridDim.x, buf ^= 1) {
-        const int a = unit / p.ff_tiles, tile = unit - a * p.ff_tiles, e = s_act[a];
-        const unsigned mask = s_mask[e];
-        float acc[NTL][4];
-#pragma unroll
-        for (int j = 0; j < NTL; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-        const size_t row0 = static_cast<size_t>(e) * p.ff;
-        const uint16_t *wl_p = p.up + (row0 + min(tile * 16 + g, p.ff - 1)) * p.up_pitch + t * 8;
-        const uint16_t *wh_p = p.up + (row0 + min(tile * 16 + g + 8, p.ff - 1)) * p.up_pitch + t * 8;
-        for (int c = c0; c < c1; c += kUnroll) {
-            uint4 wl[kUnroll], wh[kUnroll];
-#pragma unroll
-            for (int i = 0; i < kUnroll; ++i)
-                if (c + i < c1) {
-                    wl[i] = __ldcs(reinterpret_cast<const uint4 *>(wl_p + (c + i) * 32));
-                    wh[i] = __ldcs(reinterpret_cast<const uint4 *>(wh_p + (c + i) * 32));
-                }
-#pragma unroll
-            for (int i = 0; i < kUnroll; ++i)
-                if (c + i < c1) {
-                    uint4 b[NTL];
-#pragma unroll
-                    for (int j = 0; j < NTL; ++j) {
-                        b[j] = make_uint4(0u, 0u, 0u, 0u);
-                        if ((mask >> (j * 8 + g)) & 1u) b[j] = *reinterpret_cast<const uint4 *>(p.n + static_cast<size_t>(j * 8 + g) * p.ldn + (c + i) * 32 + t * 8);
-                    }
-                    mma_chunk<NTL>(acc, wl[i], wh[i], b);
-                }
-        }
-        float *part = s_part[buf][warp];
+    auto tokens = [&](few::Tokens<NTL> &x, int c) {
 #pragma unroll
         for (int j = 0; j < NTL; ++j) {
-            part[j * 128 + (2 * t) * 16 + g] = acc[j][0];
-            part[j * 128 + (2 * t + 1) * 16 + g] = acc[j][1];
-            part[j * 128 + (2 * t) * 16 + g + 8] = acc[j][2];
-            part[j * 128 + (2 * t + 1) * 16 + g + 8] = acc[j][3];
+            x.lo[j] = x.hi[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (j * 8 + g < p.m) {  // an expert meets every token; what it gives those that did not choose it is dropped
+                const uint16_t *r = p.n + static_cast<size_t>(j * 8 + g) * p.ldn + c * 64 + t * 16;
+                x.lo[j] = *reinterpret_cast<const uint4 *>(r);
+                x.hi[j] = *reinterpret_cast<const uint4 *>(r + 8);
+            }
         }
-        __syncthreads();
-        for (int o = tid; o < NTL * 128; o += kThreads) {
-            const int tk = o >> 4, r = tile * 16 + (o & 15);
-            const int k = slot_of(tk, e);
-            if (k < 0 || r >= p.ff) continue;
-            float v = 0.0f;
+    };
+    const few::Units place(lane);
+    float *red = reinterpret_cast<float *>(sm + few::red_at());
+    few::Tokens<NTL> x, x_next;
+    if (warp < p.up_chunks) tokens(x_next, warp);
+    int done = 0;
+    for (int q = u0; q < u1; q += kTiles) {
+        const int tiles = min(kTiles, u1 - q);
+        float acc[kTiles][NTL][4];
+        few::zero<NTL>(acc);
+        for (int c = warp; c < p.up_chunks; c += kWarps) {
+            x = x_next;
+            tokens(x_next, c + kWarps < p.up_chunks ? c + kWarps : warp);
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) v += s_part[buf][w][o];
-            p.h[(static_cast<size_t>(tk) * p.top + k) * p.down_pitch + r] = dense::f32_bf16(dense::relu2(v) * s_wt[tk][k]);
+            for (int k = 0; k < kTiles; ++k)
+                if (k < tiles) {
+                    few::box_mma<NTL, 1>(ring.wait(), place, x, acc + k);
+                    __syncwarp();
+                    if (lane == 0 && done + ring.depth < total) load(ring.s);
+                    ++done;
+                    ring.next();
+                }
+        }
+        if (q > u0) __syncthreads();  // the sums of the tiles before have been read
+        few::leave<NTL>(red + warp * few::red_floats(NTL), lane, tiles, acc);
+        __syncthreads();
+        for (int o = tid; o < tiles * NTL * 128; o += kThreads) {
+            const int k = o / (NTL * 128), f = o - k * (NTL * 128), tk = few::place_token(f);
+            const int a = (q + k) / p.ff_tiles, r = (q + k - a * p.ff_tiles) * 16 + few::place_row(f);
+            const int choice = slot_of(tk, s_act[a]);
+            if (choice < 0 || r >= p.ff) continue;
+            const float v = few::collect<NTL>(red, k, f);
+            p.h[(static_cast<size_t>(tk) * p.top + choice) * p.down_pitch + r] = dense::f32_bf16(dense::relu2(v) * s_wt[tk][choice]);
         }
     }
+    if (!ring.ok && lane == 0) atomicExch(p.err_word, 5);
 }
 
-template <int NTL>
-__global__ void __launch_bounds__(kThreads, 1) moe_few_down_kernel(const FewMoeParams p) {
-    __shared__ float s_part[2][kWarps][NTL * 128];
+// All down projections as one long K: the shared expert's columns (times its gate), then the chosen experts'.
+template <int NTL, int MT>
+__global__ void __launch_bounds__(kThreads, 1) moe_few_down_kernel(const __grid_constant__ FewMoeParams p) {
+    extern __shared__ uint8_t moe_smem[];
     __shared__ short s_e[LBK_GEMV_MAX_M * kMaxTop];
     __shared__ signed char s_slot[LBK_GEMV_MAX_M * kMaxTop][16];
-    ptx::pdl_trigger();
-    ptx::pdl_wait();
+    const uint32_t raw = ptx::smem_u32(moe_smem), base = (raw + 1023u) & ~1023u;
+    uint8_t *sm = moe_smem + (base - raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    few::Ring ring(sm, base, warp, p.box_rows);
+    constexpr int NB = kTiles / MT;  // boxes a warp carries at a time
+    ptx::pdl_trigger();
+    if (lane == 0) ring.init();
+    ptx::pdl_wait();
     const int n_act = p.act[0];
     for (int a = tid; a < n_act; a += kThreads) {
         s_e[a] = static_cast<short>(p.act[1 + a * kActInts]);
         for (int w = 0; w < 4; ++w) *reinterpret_cast<int *>(&s_slot[a][4 * w]) = p.act[2 + a * kActInts + w];
     }
     __syncthreads();
-    const int cs = p.hs ? p.sdown_chunks : 0, ce = p.down_chunks, total = cs + n_act * ce;
-    const int c_per = (total + kWarps - 1) / kWarps;
-    const int c0 = min(total, warp * c_per), c1 = min(total, c0 + c_per);
+    const int cs = p.hs ? p.sdown_chunks : 0, ce = p.down_chunks, chunks = cs + n_act * ce;
+    const int total = few::chunks_of(chunks, warp) * p.boxes;
+    const int row_base = static_cast<int>(blockIdx.x) * p.boxes * p.box_rows;
+    // chunk c of the long K: the shared expert's, or chunk kk of the s-th chosen expert; steps of kWarps chunks
+    struct Place {
+        int c, s, kk;
+    };
+    auto place_at = [&](int c) { return Place{c, c < cs ? 0 : (c - cs) / ce, c < cs ? 0 : (c - cs) % ce}; };
+    const Place start = place_at(warp);
+    auto on = [&](Place &u) {
+        const int before = u.c;
+        u.c += kWarps;
+        if (u.c >= chunks) {
+            u = start;
+            return true;
+        }
+        if (u.c >= cs) u.kk += before < cs ? u.c - cs : kWarps;
+        while (u.kk >= ce) {
+            u.kk -= ce;
+            ++u.s;
+        }
+        return false;
+    };
+    Place is = start;
+    int is_q = 0, is_k = 0;
+    auto load = [&](int slot) {
+        const int row = row_base + (is_q + is_k) * p.box_rows;
+        if (is.c < cs) ring.fetch(slot, &p.sdown, is.c * 128, row);
+        else ring.fetch(slot, &p.down, is.kk * 128, s_e[is.s] * p.width + row);
+        if (++is_k < min(NB, p.boxes - is_q)) return;
+        is_k = 0;
+        if (on(is)) is_q += NB;
+    };
+    if (lane == 0)
+        for (int i = 0; i < min(ring.depth, total); ++i) load(i);
+    auto tokens = [&](few::Tokens<NTL> &x, const Place &u) {
+        const int kk = u.c < cs ? u.c : u.kk;
+#pragma unroll
+        for (int j = 0; j < NTL; ++j) {
+            const int tk = j * 8 + g;
+            x.lo[j] = x.hi[j] = make_uint4(0u, 0u, 0u, 0u);
+            const uint16_t *r = nullptr;
+            if (u.c < cs) {
+                if (tk < p.m) r = p.hs + static_cast<size_t>(tk) * p.sdown_pitch;
+            } else {
+                const int choice = s_slot[u.s][tk];
+                if (choice >= 0) r = p.h + (static_cast<size_t>(tk) * p.top + choice) * p.down_pitch;
+            }
+            if (r) {
+                x.lo[j] = *reinterpret_cast<const uint4 *>(r + kk * 64 + t * 16);
+                x.hi[j] = *reinterpret_cast<const uint4 *>(r + kk * 64 + t * 16 + 8);
+            }
+        }
+    };
     float gate[NTL][2];
 #pragma unroll
     for (int j = 0; j < NTL; ++j)
@@ -295,74 +366,68 @@ __global__ void __launch_bounds__(kThreads, 1) moe_few_down_kernel(const FewMoeP
             const int tk = j * 8 + 2 * t + i;
             gate[j][i] = p.hs && tk < p.m ? dense::sigmoid(p.z[static_cast<size_t>(tk) * p.ldz + p.experts]) : 0.0f;
         }
-    int buf = 0;
-    for (int tile = blockIdx.x; tile < p.width_tiles; tile += gridDim.x, buf ^= 1) {
-        float acc[NTL][4], accs[NTL][4];
+    const few::Units place(lane);
+    float *red = reinterpret_cast<float *>(sm + few::red_at());
+    few::Tokens<NTL> x, x_next;
+    Place ahead = start;
+    if (warp < chunks) tokens(x_next, ahead);
+    int done = 0;
+    for (int q = 0; q < p.boxes; q += NB) {
+        const int boxes = min(NB, p.boxes - q);
+        float acc[kTiles][NTL][4];
+        few::zero<NTL>(acc);
+        auto shared_done = [&]() {  // what has been added up so far is the shared expert's
 #pragma unroll
-        for (int j = 0; j < NTL; ++j)
+            for (int k = 0; k < kTiles; ++k)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc[j][i] = accs[j][i] = 0.0f;
-        const int rl = min(tile * 16 + g, p.width - 1), rh = min(tile * 16 + g + 8, p.width - 1);
-        for (int c = c0; c < c1; c += kUnroll) {
-            uint4 wl[kUnroll], wh[kUnroll];
+                for (int j = 0; j < NTL; ++j)
 #pragma unroll
-            for (int i = 0; i < kUnroll; ++i)
-                if (c + i < c1) {
-                    const uint16_t *a, *b;
-                    if (c + i < cs) {
-                        a = p.sdown + static_cast<size_t>(rl) * p.sdown_pitch + (c + i) * 32;
-                        b = p.sdown + static_cast<size_t>(rh) * p.sdown_pitch + (c + i) * 32;
-                    } else {
-                        const int s = (c + i - cs) / ce, kk = c + i - cs - s * ce;
-                        const size_t row0 = static_cast<size_t>(s_e[s]) * p.width;
-                        a = p.down + (row0 + rl) * p.down_pitch + kk * 32;
-                        b = p.down + (row0 + rh) * p.down_pitch + kk * 32;
-                    }
-                    wl[i] = __ldcs(reinterpret_cast<const uint4 *>(a + t * 8));
-                    wh[i] = __ldcs(reinterpret_cast<const uint4 *>(b + t * 8));
-                }
+                    for (int i = 0; i < 4; ++i) acc[k][j][i] *= gate[j][i & 1];
+        };
+        for (int c = warp; c < chunks; c += kWarps) {
+            x = x_next;
+            on(ahead);
+            tokens(x_next, ahead);
+            if (c >= cs && c < cs + kWarps) shared_done();
 #pragma unroll
-            for (int i = 0; i < kUnroll; ++i)
-                if (c + i < c1) {
-                    uint4 b[NTL];
-                    if (c + i < cs) {
-#pragma unroll
-                        for (int j = 0; j < NTL; ++j) {
-                            b[j] = make_uint4(0u, 0u, 0u, 0u);
-                            if (j * 8 + g < p.m) b[j] = *reinterpret_cast<const uint4 *>(p.hs + static_cast<size_t>(j * 8 + g) * p.sdown_pitch + (c + i) * 32 + t * 8);
-                        }
-                        mma_chunk<NTL>(accs, wl[i], wh[i], b);
-                    } else {
-                        const int s = (c + i - cs) / ce, kk = c + i - cs - s * ce;
-#pragma unroll
-                        for (int j = 0; j < NTL; ++j) {
-                            b[j] = make_uint4(0u, 0u, 0u, 0u);
-                            const int k = s_slot[s][j * 8 + g];
-                            if (k >= 0) b[j] = *reinterpret_cast<const uint4 *>(p.h + (static_cast<size_t>(j * 8 + g) * p.top + k) * p.down_pitch + kk * 32 + t * 8);
-                        }
-                        mma_chunk<NTL>(acc, wl[i], wh[i], b);
-                    }
+            for (int k = 0; k < NB; ++k)
+                if (k < boxes) {
+                    few::box_mma<NTL, MT>(ring.wait(), place, x, acc + k * MT);
+                    __syncwarp();
+                    if (lane == 0 && done + ring.depth < total) load(ring.s);
+                    ++done;
+                    ring.next();
                 }
         }
-        float *part = s_part[buf][warp];
-#pragma unroll
-        for (int j = 0; j < NTL; ++j) {
-            part[j * 128 + (2 * t) * 16 + g] = acc[j][0] + gate[j][0] * accs[j][0];
-            part[j * 128 + (2 * t + 1) * 16 + g] = acc[j][1] + gate[j][1] * accs[j][1];
-            part[j * 128 + (2 * t) * 16 + g + 8] = acc[j][2] + gate[j][0] * accs[j][2];
-            part[j * 128 + (2 * t + 1) * 16 + g + 8] = acc[j][3] + gate[j][1] * accs[j][3];
-        }
+        if (cs + ((warp - cs) & (kWarps - 1)) >= chunks) shared_done();  // this warp has none of the experts' chunks
+        if (q) __syncthreads();  // the sums of the boxes before have been read
+        few::leave<NTL>(red + warp * few::red_floats(NTL), lane, boxes * MT, acc);
         __syncthreads();
-        for (int o = tid; o < NTL * 128; o += kThreads) {
-            const int tk = o >> 4, r = tile * 16 + (o & 15);
-            if (tk >= p.m || r >= p.width) continue;
-            float v = 0.0f;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) v += s_part[buf][w][o];
-            p.y[static_cast<size_t>(tk) * p.width + r] = v;
+        for (int o = tid; o < boxes * MT * NTL * 128; o += kThreads) {
+            const int tile = o / (NTL * 128), f = o - tile * (NTL * 128), in_box = (tile % MT) * 16 + few::place_row(f), tk = few::place_token(f);
+            const int r = row_base + (q + tile / MT) * p.box_rows + in_box;
+            if (in_box < p.box_rows && r < p.width && tk < p.m) p.y[static_cast<size_t>(tk) * p.width + r] = few::collect<NTL>(red, tile, f);
         }
     }
+    if (!ring.ok && lane == 0) atomicExch(p.err_word, 5);
 }
+
+using FewMoeKernel = void (*)(FewMoeParams);
+FewMoeKernel few_up(bool two, bool wide) {
+    return two ? (wide ? moe_few_up_kernel<2, 32> : moe_few_up_kernel<2, 8>) : (wide ? moe_few_up_kernel<1, 32> : moe_few_up_kernel<1, 8>);
+}
+FewMoeKernel few_down(bool two, int mt) {
+    if (two) return mt == 1 ? moe_few_down_kernel<2, 1> : moe_few_down_kernel<2, 2>;
+    return mt == 1 ? moe_few_down_kernel<1, 1> : moe_few_down_kernel<1, 2>;
+}
+
+int moe_init(Ctx *ctx) {
+    for (const bool two : {false, true})
+        for (FewMoeKernel k : {few_up(two, false), few_up(two, true), few_down(two, 1), few_down(two, 2)})
+            LBK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, few::rest_at(2) + 1024));
+    return LBK_OK;
+}
+const InitHook kInitMoe(moe_init);
 
 int check_route(size_t experts, size_t top) {
     if (experts == 0 || top == 0 || top > experts) return fail(LBK_ERR_INVALID, "routing %zu of %zu experts", top, experts);
@@ -415,33 +480,34 @@ int launch_moe_few(Ctx *ctx, const MoeFewCall &c, cudaStream_t st) {
     p.ldz = c.ldz;
     p.experts = c.experts;
     p.top = c.top;
-    p.up = c.up.w;
-    p.down = c.down.w;
-    p.up_pitch = c.up.pitch;
     p.down_pitch = c.down.pitch;
-    p.up_chunks = static_cast<int>(c.up.pitch / 32);
-    p.down_chunks = static_cast<int>(c.down.pitch / 32);
+    p.up_chunks = static_cast<int>(c.up.pitch / 64);
+    p.down_chunks = static_cast<int>(c.down.pitch / 64);
     p.ff = static_cast<int>(c.ff);
     p.width = static_cast<int>(c.width);
     p.ff_tiles = (p.ff + 15) / 16;
-    p.width_tiles = (p.width + 15) / 16;
     p.h = c.h;
     p.y = c.y;
     p.act = c.act;
+    p.err_word = ctx->err_word;
+    const few::Deal deal = few::deal_rows(c.width, ctx->sm_count);
+    p.box_rows = deal.box_rows;
+    p.boxes = deal.boxes;
+    LBK_TRY(encode_bytes_map(&p.up, c.up.w, c.up.pitch * 2, c.up.rows, c.up.pitch * 2, 128, 16));
+    LBK_TRY(encode_bytes_map(&p.down, c.down.w, c.down.pitch * 2, c.down.rows, c.down.pitch * 2, 128, deal.box_rows));
     if (c.hs) {
         p.hs = c.hs;
-        p.sdown = c.shared_down.w;
         p.sdown_pitch = c.shared_down.pitch;
-        p.sdown_chunks = static_cast<int>(c.shared_down.pitch / 32);
+        p.sdown_chunks = static_cast<int>(c.shared_down.pitch / 64);
+        LBK_TRY(encode_bytes_map(&p.sdown, c.shared_down.w, c.shared_down.pitch * 2, c.shared_down.rows, c.shared_down.pitch * 2, 128, deal.box_rows));
     }
     const size_t most = c.m * c.top < static_cast<size_t>(c.experts) ? c.m * c.top : static_cast<size_t>(c.experts);
     const size_t units = most * p.ff_tiles;
     const dim3 gu(static_cast<unsigned>(units < static_cast<size_t>(ctx->sm_count) ? units : ctx->sm_count));
-    const dim3 gd(static_cast<unsigned>(p.width_tiles < ctx->sm_count ? p.width_tiles : ctx->sm_count));
-    const bool two = c.m > 8, wide = c.experts > 256;
-    void (*up)(FewMoeParams) = two ? (wide ? moe_few_up_kernel<2, 32> : moe_few_up_kernel<2, 8>) : (wide ? moe_few_up_kernel<1, 32> : moe_few_up_kernel<1, 8>);
-    LBK_CUDA(launch_chained(up, gu, dim3(kThreads), 0, st, p));
-    LBK_CUDA(launch_chained(two ? moe_few_down_kernel<2> : moe_few_down_kernel<1>, gd, dim3(kThreads), 0, st, p));
+    const bool two = c.m > 8;
+    const size_t smem = static_cast<size_t>(few::rest_at(two ? 2 : 1)) + 1024;
+    LBK_CUDA(launch_chained(few_up(two, c.experts > 256), gu, dim3(kThreads), smem, st, p));
+    LBK_CUDA(launch_chained(few_down(two, deal.box_rows > 16 ? 2 : 1), dim3(static_cast<unsigned>(deal.ctas)), dim3(kThreads), smem, st, p));
     LBK_CUDA(cudaGetLastError());
     ctx->launches += 2;
     return LBK_OK;

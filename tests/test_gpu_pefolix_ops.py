@@ -67,6 +67,31 @@ def test_sandwich_norm(ctx, po, n):
 DENSE_SHAPES = [(40, 72), (1, 64), (130, 200), (640, 256), (384, 1088), (97, 40)]
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 64), (148 * 16, 72), (148 * 16 + 1, 1000), (148 * 32, 1096), (148 * 32 + 5, 640), (148 * 65 + 3, 1030)])
+def test_few_token_projection_boxes(ctx, po, rows, cols):
+    """Rows around which the few-token kernel's boxes change (16 and 32 rows of an SM, several boxes, a last CTA with little),
+    columns that leave some of the sixteen warps one chunk more or none; one to sixteen tokens; rows past the end untouched.
+    The tolerance: 32-bit sums of products that are exact in 32 bits, and half a unit in the last place of bf16."""
+    import torch
+    L, lib = _lib()
+    rng = np.random.default_rng(rows + cols)
+    for m in (1, 8, 9, 16):
+        x, xv = dev_rows(rng.standard_normal((m, cols)), BF16, pad64(cols))
+        for gated in (0, 1):
+            w, wv = dev_rows(rng.standard_normal((rows * (1 + gated), cols)) * cols ** -0.5, BF16, pad64(cols))
+            pitch = pad64(rows) + 64
+            out = torch.full((m, pitch), 7.0, dtype=torch.bfloat16 if gated else torch.float32, device="cuda")
+            L.check(lib.lbk_dense_linear(ctx.handle, BF16, x.data_ptr(), x.shape[1], m, w.data_ptr(), w.shape[1], w.shape[0], cols, gated, rows, 0, out.data_ptr(),
+                                         pitch, 1 - gated, None, 0, _st()))
+            v = xv @ wv.T
+            want = po.gelu_tanh(v[:, :rows]) * v[:, rows:] if gated else v
+            got = out.float().cpu().numpy()
+            tol = 2.0 ** -8 if gated else 1e-5
+            assert np.abs(got[:, :rows] - want).max() <= tol * max(1.0, np.abs(want).max()), (m, gated)
+            assert (got[:, rows:] == 7.0).all(), (m, gated)
+    ctx.check_device_error()
+
+
 @pytest.mark.parametrize("compute", [BF16, F32])
 @pytest.mark.parametrize("rows,cols", DENSE_SHAPES)
 def test_dense_linear(ctx, po, compute, rows, cols):
