@@ -377,6 +377,23 @@ int lbk_add_rms_norm(lbk_ctx *ctx, float *x_dev, const float *y_dev, const float
                      float eps, float *out_dev, void *stream);
 int lbk_relu2_mul_rms_norm(lbk_ctx *ctx, const float *g_dev, const float *u_dev, const float *w_dev, size_t rows,
                            size_t n, float eps, float *out_dev, void *stream);
+/* A decode step of a ternary decoder in one launch (model.rs:305-374 with one token per sequence): all layers from the embedded
+ * tokens to the rows of the final norm. linears: 7 per layer (q, k, v, o, gate, up, down), norms: 4 per layer (input,
+ * attention sub-norm, post-attention, feed-forward sub-norm), f32, 16-byte aligned, head_dim 128; the step borrows them all.
+ * lbk_step_supported: whether `b` sequences with caches of `cap` positions are served (up to 16, 4 query heads per KV head at most).
+ * lbk_step_run: x f32 [b, hidden]; caches bf16 [layers][b][kv_heads][cap][128], `layer_elems` elements a layer, in which the
+ * new rows are appended; cos/sin f32 [max_pos][128]; positions pos[i * pos_stride]; work: lbk_step_work_bytes bytes that
+ * are zero before the first run and belong to one stream; out f32 [b, hidden]. All buffers 16-byte aligned. The blocks of the
+ * launch wait on one another (a cooperative launch), each wait bounded: LBK_ERR_TIMEOUT from lbk_check_device_error. */
+typedef struct lbk_step lbk_step;
+int lbk_step_create(lbk_ctx *ctx, size_t layers, const lbk_weight *const *linears, const float *const *norms, const float *final_norm,
+                    size_t heads, size_t kv_heads, float eps, lbk_step **out);
+int lbk_step_free(lbk_step *step);
+int lbk_step_supported(const lbk_step *step, size_t b, size_t cap);
+size_t lbk_step_work_bytes(const lbk_step *step, size_t b, size_t cap);
+int lbk_step_run(const lbk_step *step, size_t b, size_t cap, const float *x_dev, uint16_t *kcache_dev, uint16_t *vcache_dev, size_t layer_elems,
+                 const float *cos_dev, const float *sin_dev, const int32_t *pos_dev, int pos_stride, void *work_dev, float *out_dev, void *stream);
+
 /* ternary_linear_n for 1..16 token rows with the element-wise work that precedes the projection in
  * the decoder step (model.rs:331-366) done inside the same kernel, on the registers that hold the
  * input row: `pre` = LBK_PRE_RMS (x' = rms_norm(x) * w), LBK_PRE_ADD_RMS (s = x + y, written to

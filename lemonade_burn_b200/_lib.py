@@ -64,6 +64,11 @@ SYMBOLS = [
     ("lbk_attn_decode_fused", _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _sz, _sz, _sz, _sz, _sz, _vp, _vp, _vp, _vp, _vp, _vp]),
     ("lbk_ternary_linear_pre_supported", _i, [_sz, _sz]),
     ("lbk_ternary_linear_pre", _i, [_vp, _i, _vp, _vp, _vp, _f, _vp, _sz, _pp, _sz, _pp, _pp, _vp]),
+    ("lbk_step_create", _i, [_vp, _sz, _vp, _vp, _vp, _sz, _sz, _f, _pp]),
+    ("lbk_step_free", _i, [_vp]),
+    ("lbk_step_supported", _i, [_vp, _sz, _sz]),
+    ("lbk_step_work_bytes", _sz, [_vp, _sz, _sz]),
+    ("lbk_step_run", _i, [_vp, _sz, _sz, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _vp, _vp, _vp]),
     ("lbk_argmax", _i, [_vp, _vp, _sz, _sz, _vp, _vp]),
     ("lbk_advance_pos", _i, [_vp, _vp, _vp]),
     ("lbk_tp_region_bytes", _sz, []),

@@ -17,7 +17,7 @@ OBJ = PKG / "_build"  # object files (git-ignored)
 RUNTIME = ["lbk_context.cu", "lbk_bf16.cu", "lbk_decoder.cu", "lbk_attn_tc.cu", "lbk_model.cu"]
 FAMILIES = {
     "": ["lbk_api.cu", "lbk_gemv.cu", "lbk_quant.cu", "lbk_plan.cu", "lbk_sweep.cu", "lbk_gemm.cu", "lbk_noalloc.cu", "lbk_tp.cu",
-         "lbk_bitnet.cu", "lbk_convert.cu", "lbk_probe.cu"],
+         "lbk_bitnet.cu", "lbk_step.cu", "lbk_convert.cu", "lbk_probe.cu"],
     "Pefolix": ["lbk_layernorm.cu", "lbk_dense.cu", "lbk_moe.cu", "lbk_attn_window.cu", "lbk_pefolix.cu"],
     "Dugulorn": ["lbk_layernorm.cu", "lbk_dense.cu", "lbk_attn_window.cu", "lbk_latent.cu", "lbk_recur.cu", "lbk_dugulorn.cu"],
 }

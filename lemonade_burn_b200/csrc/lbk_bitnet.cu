@@ -28,7 +28,9 @@ struct BitNetModel : Model {
     float *cos = nullptr, *sin = nullptr;
     uint16_t *embed = nullptr;  // bf16 [vocab][hidden], also the LM head (tied)
     std::vector<lbk_weight *> weights;
+    lbk_step *step = nullptr;  // the decode step in one launch; none for a tensor-parallel shard
     ~BitNetModel() override {
+        lbk_step_free(step);
         for (lbk_weight *w : weights) lbk_weight_free(w);
     }
     int make_cache(size_t batch, size_t capacity, std::unique_ptr<Cache> &out) override;
@@ -46,6 +48,7 @@ struct BitNetCache : Cache {
     int32_t *counters = nullptr;
     float *x = nullptr, *x2 = nullptr, *n = nullptr, *q = nullptr, *kk = nullptr, *vv = nullptr, *attn = nullptr, *o = nullptr, *g = nullptr,
           *u = nullptr, *d = nullptr, *act = nullptr, *scratch = nullptr;
+    void *step_work = nullptr;  // where one launch serves the step: its buffers (the ones above, but x and n, are not there then)
     int8_t *q8 = nullptr;  // quantised input rows of the next projection (batches of 9 and more)
     float *qscale = nullptr;
     int32_t *qsum = nullptr;
@@ -84,6 +87,11 @@ int BitNetModel::enqueue_step(Cache *cache, cudaStream_t st) {
     const size_t b = c->b, H = cfg.hidden_size, I = cfg.intermediate_size, nh = cfg.num_attention_heads, kvh = cfg.num_key_value_heads,
                  hd = m->head_dim, L = cfg.num_hidden_layers;
     const float eps = cfg.rms_norm_eps;
+    if (c->step_work) {
+        LBK_TRY(lbk_embed_bf16(h, m->embed, c->tokens, b, H, c->x, st));
+        LBK_TRY(lbk_step_run(m->step, b, c->cap, c->x, c->k, c->v, b * kvh * c->cap * hd, m->cos, m->sin, c->pos, 1, c->step_work, c->n, st));
+        return enqueue_head(c->n, b, c->logits, st);
+    }
     const bool pre_h = lbk_ternary_linear_pre_supported(b, H), pre_a = lbk_ternary_linear_pre_supported(b, nh * hd),
                pre_i = lbk_ternary_linear_pre_supported(b, I);
     const bool fused_norms = H % 4 == 0 && H <= 8192 && I % 4 == 0 && I <= 8192;
@@ -280,6 +288,15 @@ int BitNetModel::make_cache(size_t batch, size_t capacity, std::unique_ptr<Cache
     LBK_TRY(dev_alloc(c->device_allocs, kv_elems * 2, reinterpret_cast<void **>(&c->v)));
     LBK_CUDA(cudaMemset(c->k, 0, kv_elems * 2));
     LBK_CUDA(cudaMemset(c->v, 0, kv_elems * 2));
+    if (step && lbk_step_supported(step, batch, capacity)) {
+        struct { void **p; size_t bytes; } own[] = {{reinterpret_cast<void **>(&c->x), batch * H * 4}, {reinterpret_cast<void **>(&c->n), batch * H * 4},
+                                                    {&c->step_work, lbk_step_work_bytes(step, batch, capacity)}};
+        for (auto &bf : own) {
+            LBK_TRY(dev_alloc(c->device_allocs, bf.bytes, bf.p));
+            LBK_CUDA(cudaMemset(*bf.p, 0, bf.bytes));
+        }
+        return LBK_OK;
+    }
     struct { void **p; size_t bytes; } bufs[] = {
         {reinterpret_cast<void **>(&c->counters), batch * kvh * 4}, {reinterpret_cast<void **>(&c->x), batch * H * 4},
         {reinterpret_cast<void **>(&c->x2), batch * H * 4}, {reinterpret_cast<void **>(&c->n), batch * H * 4},
@@ -436,6 +453,15 @@ int load_bitnet(Ctx *ctx, const std::string &dir, const Json &cj, int compute, i
     LBK_CUDA(cudaStreamSynchronize(ctx->own_stream));  // also: `cs`, `sn` and the staging buffers go away now
     m->stats.bytes_read = sg.bytes_read;
     m->stats.bytes_to_device = sg.bytes_to_device;
+    if (world == 1) {
+        std::vector<const lbk_weight *> linears;
+        std::vector<const float *> gains;
+        for (const BitNetModel::Layer &l : m->layers) {
+            for (const lbk_weight *w : {l.q, l.k, l.v, l.o, l.gate, l.up, l.down}) linears.push_back(w);
+            for (const float *w : {l.input_norm, l.attn_sub_norm, l.post_attn_norm, l.ffn_sub_norm}) gains.push_back(w);
+        }
+        LBK_TRY(lbk_step_create(c, L, linears.data(), gains.data(), m->final_norm, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.rms_norm_eps, &m->step));
+    }
     return LBK_OK;
 }
 

@@ -134,6 +134,7 @@ class BitNet:
         cos, sin = rope_tables(cfg)
         self.cos, self.sin = torch.from_numpy(cos).to(dev), torch.from_numpy(sin).to(dev)
         self._bufs = {}
+        self._step = ops.DecodeStep(self.layers, self.final_norm, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.rms_norm_eps, self.ctx)
 
     # ---- checkpoint --------------------------------------------------------------------------
     @classmethod
@@ -175,6 +176,7 @@ class BitNet:
         if b != cache.b:
             raise ValueError("batch size differs from the cache's")
         cache.reserve(1)
+        one_launch = splits is None and self._step.supported(b, cache.cap)
         if splits is None:
             splits = attention_splits(cache.cap)
         H, I, nh, kvh, hd = cfg.hidden_size, cfg.intermediate_size, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim()
@@ -184,6 +186,13 @@ class BitNet:
         x = self._buf("x", (b, H))
         x2 = self._buf("x2", (b, H))
         n = self._buf("n", (b, H))
+        if one_launch:
+            _lib.check(lib.lbk_embed_bf16(h, P(self.lm_head), P(tokens), b, H, P(x), st))
+            self._step.run(x, cache.k, cache.v, self.cos, self.sin, cache.pos, 0, n)
+            logits = ops.bf16_linear(n, self.lm_head, self.ctx)
+            _lib.check(lib.lbk_advance_pos(h, P(cache.pos), st))
+            cache.host_len += 1
+            return logits
         attn = self._buf("attn", (b, nh * hd))
         act = self._buf("act", (b, I))
         scratch = self._buf("attn_part", (b * nh * splits * (hd + 4),))

@@ -162,6 +162,41 @@ def bf16_linear(x: torch.Tensor, w: torch.Tensor, ctx: Optional[Context] = None)
     return out
 
 
+class DecodeStep:
+    """A decode step of a ternary decoder in one launch (lbk_step_*, model.rs:305-374 with one token per sequence): from the
+    embedded tokens to the rows of the final norm. `layers`: dicts with the projections q, k, v, o, gate, up, down
+    (TernaryLinear) and the norms input_norm, attn_sub_norm, post_attn_norm, ffn_sub_norm (f32 CUDA)."""
+
+    def __init__(self, layers: Sequence[dict], final_norm: torch.Tensor, heads: int, kv_heads: int, eps: float, ctx: Optional[Context] = None):
+        self.ctx = ctx or default_context()
+        self._keep = (list(layers), final_norm)
+        self._work = {}
+        wp, _k1 = _lib.ptr_array([l[n].weight.handle.value for l in layers for n in ("q", "k", "v", "o", "gate", "up", "down")])
+        np_, _k2 = _lib.ptr_array([l[n].data_ptr() for l in layers for n in ("input_norm", "attn_sub_norm", "post_attn_norm", "ffn_sub_norm")])
+        self.handle = C.c_void_p()
+        _lib.check(self.ctx._lib.lbk_step_create(self.ctx.handle, len(layers), wp, np_, C.c_void_p(final_norm.data_ptr()), heads, kv_heads,
+                                                 C.c_float(eps), C.byref(self.handle)))
+
+    def supported(self, b: int, cap: int) -> bool:
+        return bool(self.ctx._lib.lbk_step_supported(self.handle, b, cap))
+
+    def run(self, x: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: torch.Tensor, pos_stride: int,
+            out: torch.Tensor) -> None:
+        """x, out f32 [b, hidden]; k, v bf16 [layers, b, kv_heads, cap, 128]. One stream at a time."""
+        b, cap = k.shape[1], k.shape[3]
+        if (b, cap) not in self._work:
+            self._work[b, cap] = torch.zeros(int(self.ctx._lib.lbk_step_work_bytes(self.handle, b, cap)), dtype=torch.uint8, device=x.device)
+        P = lambda t: C.c_void_p(t.data_ptr())
+        _lib.check(self.ctx._lib.lbk_step_run(self.handle, b, cap, P(x), P(k), P(v), k.stride(0), P(cos), P(sin), P(pos), pos_stride,
+                                              P(self._work[b, cap]), P(out), C.c_void_p(_stream_ptr())))
+
+    def __del__(self):
+        try:
+            self.ctx._lib.lbk_step_free(self.handle)
+        except Exception:
+            pass
+
+
 class Plan:
     """A recorded sequence of fused decode groups replayed with one call (lbk_plan_*)."""
 
