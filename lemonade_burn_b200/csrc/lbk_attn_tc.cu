@@ -224,23 +224,21 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prompt_tc_kernel(const __gri
                 *reinterpret_cast<uint4 *>(sm + (u >> 3) * kHalf + r * 128 + (((u & 7) ^ (r & 7)) << 4)) = a;
             }
         } else {
-        const float *qr = p.q + (static_cast<size_t>(row0 + (live ? r : 0)) * p.nh + head) * kHd;
-#pragma unroll 4
-        for (int u = (warp >> 2) * 8; u < (warp >> 2) * 8 + 8; ++u) {  // 16-byte unit u of the row: dimensions 8u .. 8u+7; a row's two threads take a half each
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-            if (live) {
-                a = *reinterpret_cast<const float4 *>(qr + 8 * u);
-                b = *reinterpret_cast<const float4 *>(qr + 8 * u + 4);
+            // a warp 16 rows, each as one 512-byte load: lane l takes dimensions 4l .. 4l + 3. (A thread a row, 16 bytes at a time, touched 32
+            // lines an instruction.)
+            const int half = lane >> 4, unit = (lane & 15) >> 1;
+#pragma unroll 8
+            for (int i = 0; i < 16; ++i) {
+                const int qrow = warp * 16 + i;
+                float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (qrow < rows_here && pos_ok) a = *reinterpret_cast<const float4 *>(p.q + (static_cast<size_t>(row0 + qrow) * p.nh + head) * kHd + lane * 4);
+                uint2 hi, lo;
+                split_pair(a.x * p.scaling, a.y * p.scaling, hi.x, lo.x);
+                split_pair(a.z * p.scaling, a.w * p.scaling, hi.y, lo.y);
+                uint8_t *dst = sm + half * kHalf + qrow * 128 + ((unit ^ (qrow & 7)) << 4) + (lane & 1) * 8;
+                *reinterpret_cast<uint2 *>(dst) = hi;
+                *reinterpret_cast<uint2 *>(dst + 2 * kHalf) = lo;
             }
-            const float x[8] = {a.x * p.scaling, a.y * p.scaling, a.z * p.scaling, a.w * p.scaling, b.x * p.scaling, b.y * p.scaling, b.z * p.scaling, b.w * p.scaling};
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) split_pair(x[2 * e], x[2 * e + 1], hi[e], lo[e]);
-            const int half = u >> 3, unit = u & 7;
-            uint8_t *dst = sm + half * kHalf + r * 128 + ((unit ^ (r & 7)) << 4);
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4 *>(dst + 2 * kHalf) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        }
         }
         ptx::fence_proxy_async();  // the tensor core reads these through the asynchronous proxy
     }
@@ -494,7 +492,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prompt_tc_kernel(const __gri
         if (ok && nb > 0) {
             float inv = 1.0f / lsum;
             if (TWO && p.gate && r < rows_here) inv *= dense::sigmoid(p.gate[static_cast<size_t>(row0 + r) * p.ldg + head]);
-            float *dst = WINDOW ? nullptr : p.out + (static_cast<size_t>(row0 + (r < rows_here ? r : 0)) * p.nh + head) * kHd + kh2 * 64;
+            // The rows leave through shared memory, whose operands have been read by now, so that a store instruction writes whole
+            // lines: 16 bytes from each of 32 rows at a time kept a CTA busy for microseconds after its last product. A warp has its own place
+            // (32 rows of this warp's 64 dimensions, a pitch of an odd number of 16-byte units).
+            constexpr int kPitch = WINDOW ? 144 : 272;
+            uint8_t *own = sm + warp * (32 * kPitch);
 #pragma unroll 1
             for (int c = 0; c < 2; ++c) {  // this warp's 64 dimensions of the row
                 if (WINDOW) {
@@ -512,7 +514,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prompt_tc_kernel(const __gri
                                     uint32_t w[4];
 #pragma unroll
                                     for (int e = 0; e < 4; ++e) w[e] = bf16_pair(__uint_as_float(v[i + 2 * e]) * inv, __uint_as_float(v[i + 2 * e + 1]) * inv);
-                                    *reinterpret_cast<uint4 *>(o + i) = make_uint4(w[0], w[1], w[2], w[3]);
+                                    *reinterpret_cast<uint4 *>(own + lane * kPitch + (c * 32 + i) * 2) = make_uint4(w[0], w[1], w[2], w[3]);
                                 }
                         } else {
 #pragma unroll
@@ -525,11 +527,27 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prompt_tc_kernel(const __gri
                 uint32_t v[32];
                 tmem_ld32(tmem_base + lane_field + kColO + kh2 * 64 + c * 32, v);
                 tmem_ld_wait();
-                if (r < rows_here) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4 *>(dst + c * 32 + i) = make_float4(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv,
-                                                                                    __uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
+                for (int i = 0; i < 32; i += 4)
+                    *reinterpret_cast<float4 *>(own + lane * kPitch + (c * 32 + i) * 4) = make_float4(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv,
+                                                                                                      __uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
+            }
+            __syncwarp();
+            if (!WINDOW) {
+#pragma unroll 4
+                for (int i = 0; i < 32; i += 2) {
+                    const int rr = i + (lane >> 4), row = quad * 32 + rr;
+                    if (row < rows_here)
+                        *reinterpret_cast<float4 *>(p.out + (static_cast<size_t>(row0 + row) * p.nh + head) * kHd + kh2 * 64 + (lane & 15) * 4) =
+                            *reinterpret_cast<const float4 *>(own + rr * kPitch + (lane & 15) * 16);
+                }
+            } else if ((p.vdim & 7) == 0) {
+#pragma unroll 4
+                for (int i = 0; i < 32; i += 4) {
+                    const int rr = i + (lane >> 3), row = quad * 32 + rr, d = kh2 * 64 + (lane & 7) * 8;
+                    if (row < rows_here && d < p.vdim)
+                        *reinterpret_cast<uint4 *>(p.out16 + static_cast<size_t>(row0 + row) * p.ldo + static_cast<size_t>(head) * p.vdim + d) =
+                            *reinterpret_cast<const uint4 *>(own + rr * kPitch + (lane & 7) * 16);
                 }
             }
             tc_fence_before();
