@@ -5,6 +5,7 @@ There is no fallback: if the library is missing or a call fails, an exception is
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from pathlib import Path
 
 _PKG = Path(__file__).resolve().parent
@@ -208,6 +209,12 @@ def load() -> C.CDLL:
 def check(status: int) -> None:
     if status != LBK_OK:
         raise LbkError(status, load().lbk_last_error().decode(errors="replace"))
+
+
+@functools.lru_cache(maxsize=None)
+def pointers(n: int):
+    """The type void*[n]: made once per n, and passed as it is where a void** is asked for."""
+    return C.c_void_p * n
 
 
 def ptr_array(ptrs):
