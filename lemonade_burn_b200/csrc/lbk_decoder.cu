@@ -475,6 +475,9 @@ __global__ void __launch_bounds__(256, 3) attn_fused_kernel(const float *__restr
 }
 
 // ---- prompt ingestion: n consecutive positions of ONE sequence at once -----------------------------
+// x * cos + other * sin (model.rs:298-302), `other` the rotated half. Which product the addition absorbs is written out: left to the
+// compiler it differed between the forms below, and so did the bits of a row with its alignment.
+__device__ __forceinline__ float turned(float x, float c, float other, float s) { return __fmaf_rn(x, c, __fmul_rn(other, s)); }
 // RoPE on the n query rows (in place) and the n new key rows, which are appended with the value
 // rows at positions pos0 .. pos0 + n - 1 of sequence `seq` (model.rs:298-302, 339-341).
 __global__ void __launch_bounds__(256) rope_append_rows_kernel(float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
@@ -497,8 +500,8 @@ __global__ void __launch_bounds__(256) rope_append_rows_kernel(float *__restrict
             const float4 c1 = ld(c + i), c2 = ld(c + i + half), s1 = ld(s + i), s2 = ld(s + i + half);
             const float *src = h < nh ? q + (static_cast<size_t>(row) * nh + h) * hd : k + (static_cast<size_t>(row) * kvh + h - nh) * hd;
             const float4 a = ld(src + i), b = ld(src + i + half);
-            const float4 lo = make_float4(a.x * c1.x + (-b.x) * s1.x, a.y * c1.y + (-b.y) * s1.y, a.z * c1.z + (-b.z) * s1.z, a.w * c1.w + (-b.w) * s1.w);
-            const float4 hi = make_float4(b.x * c2.x + a.x * s2.x, b.y * c2.y + a.y * s2.y, b.z * c2.z + a.z * s2.z, b.w * c2.w + a.w * s2.w);
+            const float4 lo = make_float4(turned(a.x, c1.x, -b.x, s1.x), turned(a.y, c1.y, -b.y, s1.y), turned(a.z, c1.z, -b.z, s1.z), turned(a.w, c1.w, -b.w, s1.w));
+            const float4 hi = make_float4(turned(b.x, c2.x, a.x, s2.x), turned(b.y, c2.y, a.y, s2.y), turned(b.z, c2.z, a.z, s2.z), turned(b.w, c2.w, a.w, s2.w));
             if (h < nh) {
                 float *dst = q + (static_cast<size_t>(row) * nh + h) * hd;
                 *reinterpret_cast<float4 *>(dst + i) = lo;
@@ -519,16 +522,16 @@ __global__ void __launch_bounds__(256) rope_append_rows_kernel(float *__restrict
         if (h < nh) {
             float *qh = q + (static_cast<size_t>(row) * nh + h) * hd;
             const float x1 = qh[i], x2 = qh[i + half];
-            qh[i] = x1 * c[i] + (-x2) * s[i];
-            qh[i + half] = x2 * c[i + half] + x1 * s[i + half];
+            qh[i] = turned(x1, c[i], -x2, s[i]);
+            qh[i + half] = turned(x2, c[i + half], x1, s[i + half]);
         } else {
             const int kh = h - nh;
             const float *kk = k + (static_cast<size_t>(row) * kvh + kh) * hd;
             const float *vv = v + (static_cast<size_t>(row) * kvh + kh) * hd;
             const size_t slot = ((static_cast<size_t>(seq) * kvh + kh) * cap + pos) * hd;
             const float x1 = kk[i], x2 = kk[i + half];
-            kcache[slot + i] = f32_to_bf16(x1 * c[i] + (-x2) * s[i]);
-            kcache[slot + i + half] = f32_to_bf16(x2 * c[i + half] + x1 * s[i + half]);
+            kcache[slot + i] = f32_to_bf16(turned(x1, c[i], -x2, s[i]));
+            kcache[slot + i + half] = f32_to_bf16(turned(x2, c[i + half], x1, s[i + half]));
             vcache[slot + i] = f32_to_bf16(vv[i]);
             vcache[slot + i + half] = f32_to_bf16(vv[i + half]);
         }
