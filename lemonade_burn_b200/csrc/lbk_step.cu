@@ -739,6 +739,7 @@ StepKernel pick(int nh, int ni) {
     if (nh == 2) return ni == 2 ? step_kernel<MT, SHARED, 2, 2> : ni == 4 ? step_kernel<MT, SHARED, 2, 4> : step_kernel<MT, SHARED, 2, 8>;
     return ni <= 4 ? step_kernel<MT, SHARED, 4, 4> : step_kernel<MT, SHARED, 4, 8>;
 }
+StepKernel kernel_of(size_t b, int nh, int ni) { return b == 1 ? pick<1, false>(nh, ni) : b <= 8 ? pick<1, true>(nh, ni) : pick<2, true>(nh, ni); }
 
 size_t round_up(size_t v) { return (v + 255) / 256 * 256; }
 
@@ -751,6 +752,7 @@ struct Step {
     const float *final_norm = nullptr;
     StepLayer *table = nullptr;  // device
     bool shapes_ok = false;
+    int nh = 0, ni = 0;          // float4 a thread holds of a row of the hidden and of the feed-forward width
     ~Step() {
         if (table) cudaFree(table);
     }
@@ -880,8 +882,14 @@ int lbk_step_create(lbk_ctx *c, size_t layers, const lbk_weight *const *linears,
         }
     }
     const size_t a = heads * kHead;
-    const int nh = float4s(s->hidden > a ? s->hidden : a);
-    s->shapes_ok = heads / kv_heads <= kGroup && s->hidden % 4 == 0 && s->inner % 4 == 0 && (nh == 2 || nh == 4) && float4s(s->inner) != 0 && (bits & 15) == 0;
+    s->nh = float4s(s->hidden > a ? s->hidden : a);
+    s->ni = float4s(s->inner);
+    s->shapes_ok = heads / kv_heads <= kGroup && s->hidden % 4 == 0 && s->inner % 4 == 0 && (s->nh == 2 || s->nh == 4) && s->ni != 0 && (bits & 15) == 0;
+    // One value for every model, once: the limit belongs to the kernel, and with a launch's own size set before each launch a model
+    // lowered it under another thread's larger launch.
+    if (s->shapes_ok)
+        for (const size_t b : {1, 8, 16})
+            LBK_CUDA(cudaFuncSetAttribute(kernel_of(b, s->nh, s->ni), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ctx->smem_optin)));
     LBK_CUDA(cudaMalloc(&s->table, layers * sizeof(StepLayer)));
     LBK_CUDA(cudaMemcpy(s->table, table.data(), layers * sizeof(StepLayer), cudaMemcpyHostToDevice));
     *out = reinterpret_cast<lbk_step *>(s.release());
@@ -934,11 +942,8 @@ int lbk_step_run(const lbk_step *h, size_t b, size_t cap, const float *x_dev, ui
     p.vcache = vcache_dev;
     p.layer_stride = layer_elems;
     p.err_word = ctx->err_word;
-    const size_t a = s->heads * kHead;
-    const int nh = float4s(s->hidden > a ? s->hidden : a), ni = float4s(s->inner);
-    const StepKernel kernel = b == 1 ? pick<1, false>(nh, ni) : b <= 8 ? pick<1, true>(nh, ni) : pick<2, true>(nh, ni);
+    const StepKernel kernel = kernel_of(b, s->nh, s->ni);
     const size_t smem = layout_of(p.ring, p.list, p.region, p.acc_ints).total + 1024;
-    LBK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     void *args[] = {&p};
     // cooperative: the CTAs wait on one another, so all of them have to be resident
     LBK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(static_cast<unsigned>(ctx->sm_count)), dim3(kThreads), args, smem,

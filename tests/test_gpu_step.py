@@ -59,3 +59,39 @@ def test_step_past_the_cache_reports_and_leaves_the_cache(ctx):
     out = net.forward(torch.tensor([1, 2], dtype=torch.int32, device="cuda"), c)  # and the next launch is a good one
     ctx.check_device_error()
     assert np.isfinite(out.cpu().numpy()).all()
+
+
+def test_steps_of_two_sizes_from_two_threads(ctx):
+    """Two models whose steps take the same kernel with unequal shared memory, each launched from a thread and on a stream of its own, with
+    nothing but the call in the loop: no launch fails, and both give what they give alone."""
+    import threading
+    import torch
+    from lemonade_burn_b200 import _lib, model
+    lib, cap, failed, jobs = _lib.load(), 64, [], []
+    for hidden, inner, heads, kv in ((512, 768, 4, 1), (1280, 3408, 10, 5)):
+        cfg = model.Config(hidden, inner, heads, kv, 1, 500, 1e-5, 500000.0, cap)
+        net = model.BitNet(cfg, model.random_checkpoint(cfg, hidden), ctx)
+        c, x, out, h = net.new_cache(1, cap), torch.randn(1, hidden, device="cuda"), torch.zeros(2, hidden, device="cuda"), net._step.handle
+        work = torch.zeros(int(lib.lbk_step_work_bytes(h, 1, cap)), dtype=torch.uint8, device="cuda")
+        ptrs = [t.data_ptr() for t in (x, c.k, c.v)], [t.data_ptr() for t in (net.cos, net.sin, c.pos)]
+        jobs.append((net, c, x, work, out, torch.cuda.Stream(), lambda row, stream, h=h, a=ptrs, e=c.k.stride(0), w=work, o=out:
+                     lib.lbk_step_run(h, 1, cap, *a[0], e, *a[1], 0, w.data_ptr(), o[row].data_ptr(), stream)))
+        _lib.check(jobs[-1][-1](0, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+
+    def steps(stream, call):
+        for _ in range(4000):
+            if call(1, stream) != 0:
+                failed.append(lib.lbk_last_error())
+                return
+
+    threads = [threading.Thread(target=steps, args=(j[5].cuda_stream, j[6])) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    for j in jobs:
+        assert torch.equal(j[4][0], j[4][1])
+    ctx.check_device_error()
