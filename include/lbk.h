@@ -381,6 +381,8 @@ int lbk_relu2_mul_rms_norm(lbk_ctx *ctx, const float *g_dev, const float *u_dev,
  * tokens to the rows of the final norm. linears: 7 per layer (q, k, v, o, gate, up, down), norms: 4 per layer (input,
  * attention sub-norm, post-attention, feed-forward sub-norm), f32, 16-byte aligned, head_dim 128; the step borrows them all.
  * lbk_step_supported: whether `b` sequences with caches of `cap` positions are served (up to 16, 4 query heads per KV head at most).
+ * lbk_step_stream_supported: whether the launch can be made on `stream`: not where the stream's green context has a part of the
+ * device's multiprocessors (lbk_step_run then returns LBK_ERR_UNSUPPORTED).
  * lbk_step_run: x f32 [b, hidden]; caches bf16 [layers][b][kv_heads][cap][128], `layer_elems` elements a layer, in which the
  * new rows are appended; cos/sin f32 [max_pos][128]; positions pos[i * pos_stride]; work: lbk_step_work_bytes bytes that
  * are zero before the first run and belong to one stream; out f32 [b, hidden]. All buffers 16-byte aligned. The blocks of the
@@ -390,6 +392,7 @@ int lbk_step_create(lbk_ctx *ctx, size_t layers, const lbk_weight *const *linear
                     size_t heads, size_t kv_heads, float eps, lbk_step **out);
 int lbk_step_free(lbk_step *step);
 int lbk_step_supported(const lbk_step *step, size_t b, size_t cap);
+int lbk_step_stream_supported(const lbk_step *step, void *stream);
 size_t lbk_step_work_bytes(const lbk_step *step, size_t b, size_t cap);
 int lbk_step_run(const lbk_step *step, size_t b, size_t cap, const float *x_dev, uint16_t *kcache_dev, uint16_t *vcache_dev, size_t layer_elems,
                  const float *cos_dev, const float *sin_dev, const int32_t *pos_dev, int pos_stride, void *work_dev, float *out_dev, void *stream);

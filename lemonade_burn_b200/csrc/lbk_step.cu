@@ -743,6 +743,21 @@ StepKernel kernel_of(size_t b, int nh, int ni) { return b == 1 ? pick<1, false>(
 
 size_t round_up(size_t v) { return (v + 255) / 256 * 256; }
 
+// Whether a stream may use every SM: one of a green context has a part of them, on which the grid cannot be resident as a whole.
+bool stream_has_all(const Ctx *ctx, cudaStream_t st) {
+    auto entry = [](const char *name) {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? f : nullptr;
+    };
+    static const auto green_of = reinterpret_cast<CUresult (*)(CUstream, CUgreenCtx *)>(entry("cuStreamGetGreenCtx"));
+    static const auto resource = reinterpret_cast<CUresult (*)(CUgreenCtx, CUdevResource *, CUdevResourceType)>(entry("cuGreenCtxGetDevResource"));
+    CUgreenCtx green = nullptr;
+    if (!green_of || !resource || green_of(st, &green) != CUDA_SUCCESS || !green) return true;
+    CUdevResource r{};
+    return resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS && r.sm.smCount >= static_cast<unsigned>(ctx->sm_count);
+}
+
 }  // namespace
 
 struct Step {
@@ -751,7 +766,7 @@ struct Step {
     float eps = 0.0f;
     const float *final_norm = nullptr;
     StepLayer *table = nullptr;  // device
-    bool shapes_ok = false;
+    bool served = false;
     int nh = 0, ni = 0;          // float4 a thread holds of a row of the hidden and of the feed-forward width
     ~Step() {
         if (table) cudaFree(table);
@@ -762,7 +777,7 @@ struct Step {
 
     // sizes, rings and teams for b sequences; pointers are left out
     bool plan(size_t b, size_t cap, StepParams &p) const {
-        if (!shapes_ok || b == 0 || b > static_cast<size_t>(kMaxM) || cap == 0) return false;
+        if (!served || b == 0 || b > static_cast<size_t>(kMaxM) || cap == 0) return false;
         p = StepParams{};
         p.layers = static_cast<int>(layers);
         p.m = static_cast<int>(b);
@@ -884,12 +899,20 @@ int lbk_step_create(lbk_ctx *c, size_t layers, const lbk_weight *const *linears,
     const size_t a = heads * kHead;
     s->nh = float4s(s->hidden > a ? s->hidden : a);
     s->ni = float4s(s->inner);
-    s->shapes_ok = heads / kv_heads <= kGroup && s->hidden % 4 == 0 && s->inner % 4 == 0 && (s->nh == 2 || s->nh == 4) && s->ni != 0 && (bits & 15) == 0;
+    s->served = heads / kv_heads <= kGroup && s->hidden % 4 == 0 && s->inner % 4 == 0 && (s->nh == 2 || s->nh == 4) && s->ni != 0 && (bits & 15) == 0;
     // One value for every model, once: the limit belongs to the kernel, and with a launch's own size set before each launch a model
     // lowered it under another thread's larger launch.
-    if (s->shapes_ok)
-        for (const size_t b : {1, 8, 16})
-            LBK_CUDA(cudaFuncSetAttribute(kernel_of(b, s->nh, s->ni), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ctx->smem_optin)));
+    if (s->served) {
+        int cooperative = 0, resident = 0;
+        LBK_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, ctx->device));
+        s->served = cooperative != 0;
+        for (const size_t b : {1, 8, 16}) {
+            const StepKernel kernel = kernel_of(b, s->nh, s->ni);
+            LBK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ctx->smem_optin)));
+            LBK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kThreads, ctx->smem_optin));
+            s->served = s->served && resident > 0;
+        }
+    }
     LBK_CUDA(cudaMalloc(&s->table, layers * sizeof(StepLayer)));
     LBK_CUDA(cudaMemcpy(s->table, table.data(), layers * sizeof(StepLayer), cudaMemcpyHostToDevice));
     *out = reinterpret_cast<lbk_step *>(s.release());
@@ -908,6 +931,12 @@ int lbk_step_free(lbk_step *h) {
 int lbk_step_supported(const lbk_step *h, size_t b, size_t cap) {
     StepParams p;
     return h && reinterpret_cast<const Step *>(h)->plan(b, cap, p) ? 1 : 0;
+}
+
+int lbk_step_stream_supported(const lbk_step *h, void *stream) {
+    const Step *s = reinterpret_cast<const Step *>(h);
+    if (!s || cudaSetDevice(s->ctx->device) != cudaSuccess) return 0;
+    return stream_has_all(s->ctx, static_cast<cudaStream_t>(stream)) ? 1 : 0;
 }
 
 size_t lbk_step_work_bytes(const lbk_step *h, size_t b, size_t cap) {
@@ -929,6 +958,8 @@ int lbk_step_run(const lbk_step *h, size_t b, size_t cap, const float *x_dev, ui
     if (layer_elems < b * s->kv_heads * cap * kHead || layer_elems % 4) return fail(LBK_ERR_SHAPE, "lbk_step_run: a layer's cache holds %zu elements", layer_elems);
     Ctx *ctx = s->ctx;
     LBK_CUDA(cudaSetDevice(ctx->device));
+    if (!stream_has_all(ctx, static_cast<cudaStream_t>(stream)))
+        return fail(LBK_ERR_UNSUPPORTED, "lbk_step_run: the stream has a part of the device's multiprocessors, the step needs them all");
     s->carve(p, static_cast<uint8_t *>(work_dev));
     p.table = s->table;
     p.final_norm = s->final_norm;

@@ -182,7 +182,8 @@ class DecodeStep:
                                                  C.c_float(eps), C.byref(self.handle)))
 
     def supported(self, b: int, cap: int) -> bool:
-        return bool(self.ctx._lib.lbk_step_supported(self.handle, b, cap))
+        """On the current stream: one of a green context with a part of the SMs cannot hold the launch."""
+        return bool(self.ctx._lib.lbk_step_supported(self.handle, b, cap)) and bool(self.ctx._lib.lbk_step_stream_supported(self.handle, _stream_ptr()))
 
     def run(self, x: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: torch.Tensor, pos_stride: int,
             out: torch.Tensor) -> None:

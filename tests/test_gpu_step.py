@@ -95,3 +95,37 @@ def test_steps_of_two_sizes_from_two_threads(ctx):
     for j in jobs:
         assert torch.equal(j[4][0], j[4][1])
     ctx.check_device_error()
+
+
+def test_stream_with_a_part_of_the_device(ctx, tmp_path):
+    """On a stream whose green context has some of the SMs the step cannot be resident as a whole: the models decode all the same, and the
+    refused launch leaves no error behind for the next call."""
+    import torch
+    from lemonade_burn_b200 import _lib, model
+    from torch.cuda import green_contexts
+    if not green_contexts.SUPPORTED:
+        pytest.skip("no green contexts")
+    cfg = model.Config(512, 768, 4, 1, 2, 1000, 1e-5, 500000.0, 64)
+    tensors = model.random_checkpoint(cfg, 3)
+    model.save_checkpoint(tmp_path, cfg, tensors)
+    net, nat = model.BitNet(cfg, tensors, ctx), model.NativeBitNet(tmp_path, ctx)
+    toks = torch.tensor([1, 2], dtype=torch.int32, device="cuda")
+    chain = net.forward(toks, net.new_cache(2, 64), splits=model.attention_splits(64))
+    step = net.forward(toks, net.new_cache(2, 64))
+    work = torch.zeros(int(_lib.load().lbk_step_work_bytes(net._step.handle, 2, 64)), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    part = green_contexts.GreenContext.create(32, 0)
+    with torch.cuda.stream(part.Stream()):
+        assert not net._step.supported(2, 64)
+        got, native = net.forward(toks, net.new_cache(2, 64)), nat.decode(toks, nat.new_cache(2, 64))[0]
+        c, x = net.new_cache(2, 64), torch.zeros(2, 512, device="cuda")
+        args = [t.data_ptr() for t in (x, c.k, c.v)], [t.data_ptr() for t in (net.cos, net.sin, c.pos)]
+        status = _lib.load().lbk_step_run(net._step.handle, 2, 64, *args[0], c.k.stride(0), *args[1], 0, work.data_ptr(), x.data_ptr(),
+                                          torch.cuda.current_stream().cuda_stream)
+        assert status != 0 and b"multiprocessors" in _lib.load().lbk_last_error()
+        again = net.forward(toks, net.new_cache(2, 64))
+    torch.cuda.synchronize()
+    assert torch.equal(got, chain) and torch.equal(again, chain) and torch.equal(native, step)
+    assert net._step.supported(2, 64)
+    ctx.check_device_error()
+    nat.close()
