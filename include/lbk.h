@@ -385,7 +385,8 @@ int lbk_relu2_mul_rms_norm(lbk_ctx *ctx, const float *g_dev, const float *u_dev,
  * device's multiprocessors (lbk_step_run then returns LBK_ERR_UNSUPPORTED).
  * lbk_step_run: x f32 [b, hidden]; caches bf16 [layers][b][kv_heads][cap][128], `layer_elems` elements a layer, in which the
  * new rows are appended; cos/sin f32 [max_pos][128]; positions pos[i * pos_stride]; work: lbk_step_work_bytes bytes that
- * are zero before the first run and belong to one stream; out f32 [b, hidden]. All buffers 16-byte aligned. The blocks of the
+ * are zero before the first run and shared only by launches that come one after another: they count the launches' arrivals, and after
+ * launches that overlapped they have to be made zeros again (one that gave up leaves them as a good one does); out f32 [b, hidden]. All buffers 16-byte aligned. The blocks of the
  * launch wait on one another (a cooperative launch), each wait bounded: LBK_ERR_TIMEOUT from lbk_check_device_error. */
 typedef struct lbk_step lbk_step;
 int lbk_step_create(lbk_ctx *ctx, size_t layers, const lbk_weight *const *linears, const float *const *norms, const float *final_norm,

@@ -84,6 +84,7 @@ class KvCache:
         self.pos = torch.zeros(1, dtype=torch.int32, device=device)  # cache.len, on the device
         self.b, self.cap = b, cap
         self.host_len = 0  # the same length on the host: `forward` refuses a step that would not fit
+        self.step_work = None  # (the model's step, what its launches on this cache work in)
 
     @property
     def len(self) -> int:
@@ -159,7 +160,14 @@ class BitNet:
 
     def new_cache(self, b: int = 1, cap: Optional[int] = None) -> KvCache:
         """model.rs:234-236. The capacity cannot exceed the RoPE tables (max_position_embeddings)."""
-        return KvCache(self.cfg, b, cap or self.cfg.max_position_embeddings, self.device)
+        cache = KvCache(self.cfg, b, cap or self.cfg.max_position_embeddings, self.device)
+        self._work_of(cache)
+        return cache
+
+    def _work_of(self, cache: KvCache) -> Optional[torch.Tensor]:
+        if cache.step_work is None or cache.step_work[0] is not self._step:
+            cache.step_work = (self._step, self._step.new_work(cache.b, cache.cap, self.device))
+        return cache.step_work[1]
 
     # ---- one decode step -------------------------------------------------------------------------
     def _buf(self, name, shape, dtype=torch.float32):
@@ -188,7 +196,7 @@ class BitNet:
         n = self._buf("n", (b, H))
         if one_launch:
             _lib.check(lib.lbk_embed_bf16(h, P(self.lm_head), P(tokens), b, H, P(x), st))
-            self._step.run(x, cache.k, cache.v, self.cos, self.sin, cache.pos, 0, n)
+            self._step.run(x, cache.k, cache.v, self.cos, self.sin, cache.pos, 0, n, self._work_of(cache))
             logits = ops.bf16_linear(n, self.lm_head, self.ctx)
             _lib.check(lib.lbk_advance_pos(h, P(cache.pos), st))
             cache.host_len += 1

@@ -174,7 +174,6 @@ class DecodeStep:
     def __init__(self, layers: Sequence[dict], final_norm: torch.Tensor, heads: int, kv_heads: int, eps: float, ctx: Optional[Context] = None):
         self.ctx = ctx or default_context()
         self._keep = (list(layers), final_norm)
-        self._work = {}
         wp, _k1 = _lib.ptr_array([l[n].weight.handle.value for l in layers for n in ("q", "k", "v", "o", "gate", "up", "down")])
         np_, _k2 = _lib.ptr_array([l[n].data_ptr() for l in layers for n in ("input_norm", "attn_sub_norm", "post_attn_norm", "ffn_sub_norm")])
         self.handle = C.c_void_p()
@@ -185,15 +184,18 @@ class DecodeStep:
         """On the current stream: one of a green context with a part of the SMs cannot hold the launch."""
         return bool(self.ctx._lib.lbk_step_supported(self.handle, b, cap)) and bool(self.ctx._lib.lbk_step_stream_supported(self.handle, _stream_ptr()))
 
+    def new_work(self, b: int, cap: int, device) -> Optional[torch.Tensor]:
+        """What `run` works in, None where it does not serve such a cache. It counts the launches' arrivals, so launches that share it come
+        one after another: a buffer for each cache."""
+        n = int(self.ctx._lib.lbk_step_work_bytes(self.handle, b, cap))
+        return torch.zeros(n, dtype=torch.uint8, device=device) if n else None
+
     def run(self, x: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: torch.Tensor, pos_stride: int,
-            out: torch.Tensor) -> None:
-        """x, out f32 [b, hidden]; k, v bf16 [layers, b, kv_heads, cap, 128]. One stream at a time."""
-        b, cap = k.shape[1], k.shape[3]
-        if (b, cap) not in self._work:
-            self._work[b, cap] = torch.zeros(int(self.ctx._lib.lbk_step_work_bytes(self.handle, b, cap)), dtype=torch.uint8, device=x.device)
+            out: torch.Tensor, work: torch.Tensor) -> None:
+        """x, out f32 [b, hidden]; k, v bf16 [layers, b, kv_heads, cap, 128]; work: new_work(b, cap)."""
         P = lambda t: C.c_void_p(t.data_ptr())
-        _lib.check(self.ctx._lib.lbk_step_run(self.handle, b, cap, P(x), P(k), P(v), k.stride(0), P(cos), P(sin), P(pos), pos_stride,
-                                              P(self._work[b, cap]), P(out), C.c_void_p(_stream_ptr())))
+        _lib.check(self.ctx._lib.lbk_step_run(self.handle, k.shape[1], k.shape[3], P(x), P(k), P(v), k.stride(0), P(cos), P(sin), P(pos), pos_stride,
+                                              P(work), P(out), C.c_void_p(_stream_ptr())))
 
     def __del__(self):
         try:

@@ -129,3 +129,45 @@ def test_stream_with_a_part_of_the_device(ctx, tmp_path):
     assert net._step.supported(2, 64)
     ctx.check_device_error()
     nat.close()
+
+
+def test_caches_of_one_shape_step_on_two_streams(ctx):
+    """Each cache has a work buffer of its own, which goes with it: the launches of two caches count their arrivals apart."""
+    import weakref
+    import torch
+    from lemonade_burn_b200 import model
+    cap, b = 48, 2
+    cfg = model.Config(1280, 3408, 10, 5, 2, 500, 1e-5, 500000.0, cap)
+    net = model.BitNet(cfg, model.random_checkpoint(cfg, 9), ctx)
+    a, c = net.new_cache(b, cap), net.new_cache(b, cap)
+    assert a.step_work[1].data_ptr() != c.step_work[1].data_ptr()
+    gone = weakref.ref(c.step_work[1])
+    del c
+    assert gone() is None
+    runs = []
+    for i in range(2):
+        g = torch.Generator(device="cuda").manual_seed(i)
+        cache, x, out = net.new_cache(b, cap), torch.randn(b, 1280, generator=g, device="cuda"), torch.zeros(cap, b, 1280, device="cuda")
+        runs.append((cache, x, out, torch.cuda.Stream()))
+    pos = torch.arange(cap, dtype=torch.int32, device="cuda")
+
+    def step(run, t):
+        cache, x, out, _ = run
+        net._step.run(x, cache.k, cache.v, net.cos, net.sin, pos[t:], 0, out[t], cache.step_work[1])
+
+    want = []
+    for run in runs:  # one after the other
+        for t in range(cap):
+            step(run, t)
+        want.append(run[2].clone())
+        run[0].k.zero_()
+        run[0].v.zero_()
+        run[2].zero_()
+    torch.cuda.synchronize()
+    for t in range(cap):  # in turn, nothing between the streams
+        for run in runs:
+            with torch.cuda.stream(run[3]):
+                step(run, t)
+    torch.cuda.synchronize()
+    assert all(torch.equal(run[2], w) for run, w in zip(runs, want))
+    ctx.check_device_error()
