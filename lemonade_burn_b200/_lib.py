@@ -12,6 +12,7 @@ _PKG = Path(__file__).resolve().parent
 LIB_PATH = _PKG / "liblbk.so"
 
 LBK_OK = 0
+LBK_ERR_SHAPE = 2
 STATUS_NAMES = {0: "OK", 1: "INVALID", 2: "SHAPE", 3: "CUDA", 4: "UNSUPPORTED", 5: "TIMEOUT", 6: "NOMEM"}
 MAX_GROUP = 4
 GEMV_MAX_M = 16

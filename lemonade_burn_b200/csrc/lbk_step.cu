@@ -899,7 +899,7 @@ int lbk_step_create(lbk_ctx *c, size_t layers, const lbk_weight *const *linears,
     const size_t a = heads * kHead;
     s->nh = float4s(s->hidden > a ? s->hidden : a);
     s->ni = float4s(s->inner);
-    s->served = heads / kv_heads <= kGroup && s->hidden % 4 == 0 && s->inner % 4 == 0 && (s->nh == 2 || s->nh == 4) && s->ni != 0 && (bits & 15) == 0;
+    s->served = heads / kv_heads <= kGroup && s->hidden && s->inner && s->hidden % 4 == 0 && s->inner % 4 == 0 && (s->nh == 2 || s->nh == 4) && s->ni != 0 && (bits & 15) == 0;
     // One value for every model, once: the limit belongs to the kernel, and with a launch's own size set before each launch a model
     // lowered it under another thread's larger launch.
     if (s->served) {

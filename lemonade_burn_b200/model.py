@@ -135,7 +135,19 @@ class BitNet:
         cos, sin = rope_tables(cfg)
         self.cos, self.sin = torch.from_numpy(cos).to(dev), torch.from_numpy(sin).to(dev)
         self._bufs = {}
-        self._step = ops.DecodeStep(self.layers, self.final_norm, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.rms_norm_eps, self.ctx)
+        self._step = self._make_step()
+
+    def _make_step(self) -> Optional[ops.DecodeStep]:
+        """The step in one launch; None for a model of a form that it does not take."""
+        cfg = self.cfg
+        if not cfg.num_hidden_layers or not cfg.intermediate_size or cfg.head_dim() != 128 or cfg.num_attention_heads % cfg.num_key_value_heads:
+            return None
+        try:
+            return ops.DecodeStep(self.layers, self.final_norm, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.rms_norm_eps, self.ctx)
+        except _lib.LbkError as e:
+            if e.status != _lib.LBK_ERR_SHAPE:
+                raise
+            return None
 
     # ---- checkpoint --------------------------------------------------------------------------
     @classmethod
@@ -166,7 +178,7 @@ class BitNet:
 
     def _work_of(self, cache: KvCache) -> Optional[torch.Tensor]:
         if cache.step_work is None or cache.step_work[0] is not self._step:
-            cache.step_work = (self._step, self._step.new_work(cache.b, cache.cap, self.device))
+            cache.step_work = (self._step, self._step.new_work(cache.b, cache.cap, self.device) if self._step else None)
         return cache.step_work[1]
 
     # ---- one decode step -------------------------------------------------------------------------
@@ -184,7 +196,7 @@ class BitNet:
         if b != cache.b:
             raise ValueError("batch size differs from the cache's")
         cache.reserve(1)
-        one_launch = splits is None and self._step.supported(b, cache.cap)
+        one_launch = splits is None and self._step is not None and self._step.supported(b, cache.cap)
         if splits is None:
             splits = attention_splits(cache.cap)
         H, I, nh, kvh, hd = cfg.hidden_size, cfg.intermediate_size, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim()

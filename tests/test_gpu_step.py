@@ -171,3 +171,25 @@ def test_caches_of_one_shape_step_on_two_streams(ctx):
     torch.cuda.synchronize()
     assert all(torch.equal(run[2], w) for run, w in zip(runs, want))
     ctx.check_device_error()
+
+
+def test_models_that_the_step_does_not_take(ctx):
+    """No layers, heads of another size, query heads that KV heads do not divide, a projection of other rows: such models are made as before, and
+    the one without layers runs."""
+    import torch
+    from lemonade_burn_b200 import model
+    for hidden, heads, kv, layers in ((256, 2, 1, 0), (256, 4, 2, 1), (384, 3, 2, 1)):
+        cfg = model.Config(hidden, 256, heads, kv, layers, 300, 1e-5, 500000.0, 16)
+        net = model.BitNet(cfg, model.random_checkpoint(cfg, 1), ctx)
+        assert net._step is None
+        if not layers:
+            toks = torch.tensor([3, 4], dtype=torch.int32, device="cuda")
+            x = net.lm_head[toks.long()].double()
+            want = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5) * net.final_norm.double() @ net.lm_head.double().T
+            got = net.forward(toks, net.new_cache(2, 16))
+            assert (got - want).abs().max() <= TOL * want.abs().max()
+    cfg = model.Config(256, 256, 2, 1, 1, 300, 1e-5, 500000.0, 16)
+    tensors = model.random_checkpoint(cfg, 1)
+    tensors["model.layers.0.self_attn.v_proj.qweight"] = tensors["model.layers.0.self_attn.v_proj.qweight"].repeat(2, 1)
+    assert model.BitNet(cfg, tensors, ctx)._step is None
+    ctx.check_device_error()
