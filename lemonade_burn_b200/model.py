@@ -196,6 +196,8 @@ class BitNet:
         if b != cache.b:
             raise ValueError("batch size differs from the cache's")
         cache.reserve(1)
+        if self._step is not None and not self._step.holds(self.layers, self.final_norm):  # somebody has put other weights in
+            self._step = self._make_step()
         one_launch = splits is None and self._step is not None and self._step.supported(b, cache.cap)
         if splits is None:
             splits = attention_splits(cache.cap)

@@ -169,16 +169,29 @@ def bf16_linear(x: torch.Tensor, w: torch.Tensor, ctx: Optional[Context] = None)
 class DecodeStep:
     """A decode step of a ternary decoder in one launch (lbk_step_*, model.rs:305-374 with one token per sequence): from the
     embedded tokens to the rows of the final norm. `layers`: dicts with the projections q, k, v, o, gate, up, down
-    (TernaryLinear) and the norms input_norm, attn_sub_norm, post_attn_norm, ffn_sub_norm (f32 CUDA)."""
+    (TernaryLinear) and the norms input_norm, attn_sub_norm, post_attn_norm, ffn_sub_norm (f32 CUDA). It holds on to them: the
+    kernel's table has their addresses."""
+    LINEARS = ("q", "k", "v", "o", "gate", "up", "down")
+    NORMS = ("input_norm", "attn_sub_norm", "post_attn_norm", "ffn_sub_norm")
 
     def __init__(self, layers: Sequence[dict], final_norm: torch.Tensor, heads: int, kv_heads: int, eps: float, ctx: Optional[Context] = None):
         self.ctx = ctx or default_context()
-        self._keep = (list(layers), final_norm)
-        wp, _k1 = _lib.ptr_array([l[n].weight.handle.value for l in layers for n in ("q", "k", "v", "o", "gate", "up", "down")])
-        np_, _k2 = _lib.ptr_array([l[n].data_ptr() for l in layers for n in ("input_norm", "attn_sub_norm", "post_attn_norm", "ffn_sub_norm")])
+        linears = [l[n] for l in layers for n in self.LINEARS]
+        self._weights = [(w.weight, w.packed) for w in linears]
+        self._norms = [l[n] for l in layers for n in self.NORMS] + [final_norm]
+        self._at = [t.data_ptr() for t in self._norms]
+        wp, _k1 = _lib.ptr_array([w.weight.handle.value for w in linears])
+        np_, _k2 = _lib.ptr_array(self._at[:-1])
         self.handle = C.c_void_p()
         _lib.check(self.ctx._lib.lbk_step_create(self.ctx.handle, len(layers), wp, np_, C.c_void_p(final_norm.data_ptr()), heads, kv_heads,
                                                  C.c_float(eps), C.byref(self.handle)))
+
+    def holds(self, layers: Sequence[dict], final_norm: torch.Tensor) -> bool:
+        """Whether these are the weights that the step was made from, where they were then."""
+        if [l[n].weight for l in layers for n in self.LINEARS] != [w for w, _ in self._weights]:
+            return False
+        norms = [l[n] for l in layers for n in self.NORMS] + [final_norm]
+        return len(norms) == len(self._norms) and all(a is b for a, b in zip(norms, self._norms)) and [t.data_ptr() for t in norms] == self._at
 
     def supported(self, b: int, cap: int) -> bool:
         """On the current stream: one of a green context with a part of the SMs cannot hold the launch."""

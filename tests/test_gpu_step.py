@@ -193,3 +193,32 @@ def test_models_that_the_step_does_not_take(ctx):
     tensors["model.layers.0.self_attn.v_proj.qweight"] = tensors["model.layers.0.self_attn.v_proj.qweight"].repeat(2, 1)
     assert model.BitNet(cfg, tensors, ctx)._step is None
     ctx.check_device_error()
+
+
+def test_step_follows_weights_that_are_put_in_later(ctx):
+    """`layers` and `final_norm` are read at every call: another projection, another norm, a norm's storage exchanged under it."""
+    import torch
+    from lemonade_burn_b200 import model
+    cfg = model.Config(512, 768, 4, 1, 2, 500, 1e-5, 500000.0, 24)
+    net, other = (model.BitNet(cfg, model.random_checkpoint(cfg, s), ctx) for s in (1, 2))
+    toks = torch.tensor([3, 4], dtype=torch.int32, device="cuda")
+    forward = lambda **kw: net.forward(toks, net.new_cache(2, 24), **kw)  # noqa: E731
+    old, kept = [forward()], []  # what is taken out stays alive, so that a step that missed the change reads old weights and not free memory
+
+    def check():
+        got, want = forward(), forward(splits=model.attention_splits(24))
+        assert (got - want).abs().max() <= TOL * want.abs().max()
+        assert (got - old[0]).abs().max() > 10 * TOL * want.abs().max()
+        old[0] = got
+
+    for layer, name in ((0, "gate"), (1, "attn_sub_norm")):
+        kept.append(net.layers[layer][name])
+        net.layers[layer][name] = other.layers[layer][name] if name == "gate" else 3.0 * kept[-1].flip(0)
+        check()
+    kept.append(net.final_norm)
+    net.final_norm = 2.0 * net.final_norm.flip(0)
+    check()
+    kept.append(net.layers[0]["ffn_sub_norm"].data)
+    net.layers[0]["ffn_sub_norm"].data = torch.linspace(-2.0, 2.0, 768, device="cuda")
+    check()
+    ctx.check_device_error()
