@@ -386,14 +386,17 @@ int lbk_relu2_mul_rms_norm(lbk_ctx *ctx, const float *g_dev, const float *u_dev,
  * lbk_step_run: x f32 [b, hidden]; caches bf16 [layers][b][kv_heads][cap][128], `layer_elems` elements a layer, in which the
  * new rows are appended; cos/sin f32 [max_pos][128]; positions pos[i * pos_stride]; work: lbk_step_work_bytes bytes that
  * are zero before the first run and shared only by launches that come one after another: they count the launches' arrivals, and after
- * launches that overlapped they have to be made zeros again (one that gave up leaves them as a good one does); out f32 [b, hidden]. All buffers 16-byte aligned. The blocks of the
- * launch wait on one another (a cooperative launch), each wait bounded: LBK_ERR_TIMEOUT from lbk_check_device_error. */
+ * launches that overlapped they have to be made zeros again (one that gave up leaves them as a good one does); out f32 [b, hidden].
+ * All buffers 16-byte aligned. The blocks of the launch wait on one another (a cooperative launch), each wait bounded:
+ * LBK_ERR_TIMEOUT from lbk_check_device_error.
+ * lbk_step_set_wait_limit: polls before such a wait gives up, for launches from now on (default 2^20, about a second). */
 typedef struct lbk_step lbk_step;
 int lbk_step_create(lbk_ctx *ctx, size_t layers, const lbk_weight *const *linears, const float *const *norms, const float *final_norm,
                     size_t heads, size_t kv_heads, float eps, lbk_step **out);
 int lbk_step_free(lbk_step *step);
 int lbk_step_supported(const lbk_step *step, size_t b, size_t cap);
 int lbk_step_stream_supported(const lbk_step *step, void *stream);
+int lbk_step_set_wait_limit(lbk_step *step, uint32_t polls);
 size_t lbk_step_work_bytes(const lbk_step *step, size_t b, size_t cap);
 int lbk_step_run(const lbk_step *step, size_t b, size_t cap, const float *x_dev, uint16_t *kcache_dev, uint16_t *vcache_dev, size_t layer_elems,
                  const float *cos_dev, const float *sin_dev, const int32_t *pos_dev, int pos_stride, void *work_dev, float *out_dev, void *stream);

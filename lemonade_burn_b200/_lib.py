@@ -70,6 +70,7 @@ SYMBOLS = [
     ("lbk_step_free", _i, [_vp]),
     ("lbk_step_supported", _i, [_vp, _sz, _sz]),
     ("lbk_step_stream_supported", _i, [_vp, _vp]),
+    ("lbk_step_set_wait_limit", _i, [_vp, C.c_uint32]),
     ("lbk_step_work_bytes", _sz, [_vp, _sz, _sz]),
     ("lbk_step_run", _i, [_vp, _sz, _sz, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _vp, _vp, _vp]),
     ("lbk_argmax", _i, [_vp, _vp, _sz, _sz, _vp, _vp]),

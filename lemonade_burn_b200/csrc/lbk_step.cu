@@ -43,7 +43,7 @@ constexpr int kMaxRing = 8;
 constexpr int kPositions = 8;       // positions a warp takes at a time
 constexpr int kRecord = kHead + 4;  // floats of a slice's or warp's partial result: 128 sums, maximum, weight, padding
 constexpr int kMaxSlices = 32;      // a lane each when they are added up
-constexpr uint32_t kPollLimit = 1u << 20;
+constexpr uint32_t kPollLimit = 1u << 20;  // polls of a count before a wait gives up, about a second (lbk_step_set_wait_limit)
 
 struct alignas(16) LayerInfo {
     const float *norm[4];  // input, attention sub-norm, post-attention, feed-forward sub-norm
@@ -81,6 +81,7 @@ struct StepParams {
     // of all launches so far: barriers, inputs of projections, arrivals at barriers, rows of codes; and the CTAs that have left this one
     uint32_t *number, *codes, *met, *q8_ready, *exit_count;
     int *err_word;
+    uint32_t poll_limit;
     Phase ph[kPhases];
 };
 
@@ -145,13 +146,13 @@ struct Cta {
 
 // Counts what this CTA wrote before its last barrier of threads; and waits for a count.
 __device__ __forceinline__ void count_up(uint32_t *at) { asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(at) : "memory"); }
-__device__ __forceinline__ void await(const Cta &c, const uint32_t *at, uint32_t want) {
+__device__ __forceinline__ void await(const Cta &c, const StepParams &p, const uint32_t *at, uint32_t want) {
     if (*c.gave_up()) return;
     uint32_t seen, polls = 0;
     for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(at) : "memory");
         if (static_cast<int>(seen - want) >= 0) return;
-        if (++polls >= kPollLimit) break;
+        if (++polls >= p.poll_limit) break;
         __nanosleep(40);  // polls slow the arrivals down
     }
     c.give_up();
@@ -162,7 +163,7 @@ __device__ __forceinline__ void arrive(const Cta &c, const StepParams &p) {
     if (c.tid == 0) count_up(p.met);
 }
 __device__ __forceinline__ void wait(const Cta &c, const StepParams &p, uint32_t number) {
-    if (c.tid == 0) await(c, p.met, number * gridDim.x);
+    if (c.tid == 0) await(c, p, p.met, number * gridDim.x);
     __syncthreads();
 }
 
@@ -288,7 +289,7 @@ __device__ __forceinline__ void input_phase(const Cta &c, const StepParams &p, i
         }
     }
     if (SHARED) {
-        if (c.tid == 0) await(c, p.q8_ready, codes * p.m);
+        if (c.tid == 0) await(c, p, p.q8_ready, codes * p.m);
         __syncthreads();
         if (c.tid < p.m) {
             s_scale[c.tid] = __ldcg(p.q8_scale + c.tid);
@@ -767,6 +768,7 @@ struct Step {
     const float *final_norm = nullptr;
     StepLayer *table = nullptr;  // device
     bool served = false;
+    uint32_t poll_limit = kPollLimit;
     int nh = 0, ni = 0;          // float4 a thread holds of a row of the hidden and of the feed-forward width
     ~Step() {
         if (table) cudaFree(table);
@@ -933,6 +935,13 @@ int lbk_step_supported(const lbk_step *h, size_t b, size_t cap) {
     return h && reinterpret_cast<const Step *>(h)->plan(b, cap, p) ? 1 : 0;
 }
 
+int lbk_step_set_wait_limit(lbk_step *h, uint32_t polls) {
+    if (!h) return fail(LBK_ERR_INVALID, "lbk_step_set_wait_limit: null argument");
+    if (polls == 0) return fail(LBK_ERR_INVALID, "a wait limit of 0 polls would give up before looking");
+    reinterpret_cast<Step *>(h)->poll_limit = polls;
+    return LBK_OK;
+}
+
 int lbk_step_stream_supported(const lbk_step *h, void *stream) {
     const Step *s = reinterpret_cast<const Step *>(h);
     if (!s || cudaSetDevice(s->ctx->device) != cudaSuccess) return 0;
@@ -973,6 +982,7 @@ int lbk_step_run(const lbk_step *h, size_t b, size_t cap, const float *x_dev, ui
     p.vcache = vcache_dev;
     p.layer_stride = layer_elems;
     p.err_word = ctx->err_word;
+    p.poll_limit = s->poll_limit;
     const StepKernel kernel = kernel_of(b, s->nh, s->ni);
     const size_t smem = layout_of(p.ring, p.list, p.region, p.acc_ints).total + 1024;
     void *args[] = {&p};

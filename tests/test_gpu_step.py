@@ -222,3 +222,31 @@ def test_step_follows_weights_that_are_put_in_later(ctx):
     net.layers[0]["ffn_sub_norm"].data = torch.linspace(-2.0, 2.0, 768, device="cuda")
     check()
     ctx.check_device_error()
+
+
+@pytest.mark.parametrize("b", [1, 3])
+def test_step_whose_waits_run_out(ctx, b):
+    """A count that nothing ever reaches: with a short limit every wait gives up, the launch ends, the status says so, and with the counts
+    made zeros again the same buffers give the right rows."""
+    import torch
+    from lemonade_burn_b200 import _lib, model
+    lib = _lib.load()
+    cfg = model.Config(512, 768, 4, 1, 2, 500, 1e-5, 500000.0, 300)
+    net = model.BitNet(cfg, model.random_checkpoint(cfg, 4), ctx)
+    c, toks = net.new_cache(b, 300), torch.arange(b, dtype=torch.int32, device="cuda")
+    want = net.forward(toks, c)
+    ctx.check_device_error()
+    assert lib.lbk_step_set_wait_limit(net._step.handle, 0) != 0
+    _lib.check(lib.lbk_step_set_wait_limit(net._step.handle, 2000))
+    c.step_work[1].zero_()
+    c.step_work[1].view(torch.int32)[0] = 1  # one barrier that no block has come to
+    c.pos.zero_()
+    net.forward(toks, c)
+    with pytest.raises(_lib.LbkError) as e:
+        ctx.check_device_error()
+    assert e.value.status == 5
+    c.step_work[1].zero_()
+    _lib.check(lib.lbk_step_set_wait_limit(net._step.handle, 1 << 20))
+    c.pos.zero_()
+    assert torch.equal(net.forward(toks, c), want)
+    ctx.check_device_error()
