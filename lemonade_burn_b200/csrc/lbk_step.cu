@@ -763,6 +763,7 @@ bool stream_has_all(const Ctx *ctx, cudaStream_t st) {
 
 struct Step {
     Ctx *ctx = nullptr;
+    int device = 0;              // of its own: the step may be freed after the context
     size_t layers = 0, hidden = 0, inner = 0, heads = 0, kv_heads = 0;
     float eps = 0.0f;
     const float *final_norm = nullptr;
@@ -868,6 +869,7 @@ int lbk_step_create(lbk_ctx *c, size_t layers, const lbk_weight *const *linears,
     LBK_CUDA(cudaSetDevice(ctx->device));
     std::unique_ptr<Step> s(new Step());
     s->ctx = ctx;
+    s->device = ctx->device;
     s->layers = layers;
     s->heads = heads;
     s->kv_heads = kv_heads;
@@ -924,7 +926,7 @@ int lbk_step_create(lbk_ctx *c, size_t layers, const lbk_weight *const *linears,
 int lbk_step_free(lbk_step *h) {
     Step *s = reinterpret_cast<Step *>(h);
     if (!s) return LBK_OK;
-    LBK_CUDA(cudaSetDevice(s->ctx->device));
+    LBK_CUDA(cudaSetDevice(s->device));
     LBK_CUDA(cudaDeviceSynchronize());
     delete s;
     return LBK_OK;

@@ -250,3 +250,18 @@ def test_step_whose_waits_run_out(ctx, b):
     c.pos.zero_()
     assert torch.equal(net.forward(toks, c), want)
     ctx.check_device_error()
+
+
+def test_step_is_freed_after_its_context():
+    """As a weight that borrows its memory can be: nothing of the context is looked at."""
+    import torch
+    from lemonade_burn_b200 import model, ternary
+    own = ternary.Context(0)
+    cfg = model.Config(512, 768, 4, 1, 1, 500, 1e-5, 500000.0, 24)
+    net = model.BitNet(cfg, model.random_checkpoint(cfg, 1), own)
+    net.forward(torch.tensor([3], dtype=torch.int32, device="cuda"), net.new_cache(1, 24))
+    own.check_device_error()
+    step, net._step = net._step, None
+    own.close()
+    assert step.ctx._lib.lbk_step_free(step.handle) == 0
+    step.handle = None
