@@ -28,7 +28,9 @@
 // A layer of one sequence: six barriers 18000 cycles, norms and quantisers 9000, products 11000, attention 7000.
 #include "lbk_gemv_core.cuh"
 
+#include <exception>
 #include <memory>
+#include <new>
 
 namespace lbk {
 
@@ -867,7 +869,8 @@ int lbk_step_create(lbk_ctx *c, size_t layers, const lbk_weight *const *linears,
     if (!heads || !kv_heads || heads % kv_heads) return fail(LBK_ERR_INVALID, "lbk_step_create: inconsistent head counts");
     Ctx *ctx = reinterpret_cast<Ctx *>(c);
     LBK_CUDA(cudaSetDevice(ctx->device));
-    std::unique_ptr<Step> s(new Step());
+    std::unique_ptr<Step> s(new (std::nothrow) Step());
+    if (!s) return fail(LBK_ERR_NOMEM, "out of host memory");
     s->ctx = ctx;
     s->device = ctx->device;
     s->layers = layers;
@@ -875,7 +878,12 @@ int lbk_step_create(lbk_ctx *c, size_t layers, const lbk_weight *const *linears,
     s->kv_heads = kv_heads;
     s->eps = eps;
     s->final_norm = final_norm;
-    std::vector<StepLayer> table(layers);
+    std::vector<StepLayer> table;
+    try {
+        table.resize(layers);
+    } catch (const std::exception &) {  // no exception leaves a C entry
+        return fail(LBK_ERR_NOMEM, "lbk_step_create: no host memory for %zu layers", layers);
+    }
     uintptr_t bits = reinterpret_cast<uintptr_t>(final_norm);
     for (size_t l = 0; l < layers; ++l) {
         const Weight *w[7];

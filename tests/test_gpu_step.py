@@ -265,3 +265,12 @@ def test_step_is_freed_after_its_context():
     own.close()
     assert step.ctx._lib.lbk_step_free(step.handle) == 0
     step.handle = None
+
+
+def test_step_of_more_layers_than_memory_is_refused(ctx):
+    """A status, and no C++ exception through the C entry."""
+    import ctypes as C
+    from lemonade_burn_b200 import _lib
+    out, one = C.c_void_p(), (C.c_void_p * 1)()
+    status = _lib.load().lbk_step_create(ctx.handle, 1 << 58, one, one, C.c_void_p(16), 4, 1, C.c_float(1e-5), C.byref(out))
+    assert status == 6 and not out.value
