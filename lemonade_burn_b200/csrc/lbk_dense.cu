@@ -8,7 +8,8 @@
 //                      step (cold weights, time until the next kernel can start), against the kernel that loaded MMA
 //                      fragments straight from global memory and cut tiles between CTAs: gate/up 2560 -> 6912 33 -> 18 us at
 //                      one token (with the norms), 31 -> 12 at eight; 6912 -> 2560 14.6 -> 7 and 53 -> 6; and against the tcgen05
-//                      kernel at 16 tokens: 2560 -> 6912 10.7 -> 7.4, 6912 -> 2560 13.7 -> 10.5, 2560 -> 10240 20 -> 12.
+//                      kernel at 16 tokens: 2560 -> 6912 10.7 -> 7.4, 6912 -> 2560 13.7 -> 10.5, 2560 -> 10240 20 -> 12. Wide gated
+//                      calls of 9 to 16 tokens stay with that one (few_serves).
 //   dense_gemm_kernel  more tokens: tcgen05 (kind::f16), 128 weight rows x up to 256 tokens a tile, both operands
 //                      by TMA (SWIZZLE_128B, 64 columns a stage), two accumulators in tensor memory so that the
 //                      epilogue of one tile runs under the MMAs of the next, one persistent CTA per SM. A gated
@@ -653,6 +654,19 @@ FewKernel few_kernel_of(int ntl, int mt) {
 }
 FewKernel few_kernel(bool gated, int ntl, int mt) { return gated ? few_kernel_of<true>(ntl, mt) : few_kernel_of<false>(ntl, mt); }
 
+// Up to 16 tokens without experts, but for gated calls of 9 to 16 with more than 32 weight rows an SM, whose tokens a warp reads again for every
+// pair of boxes: there the GEMM is faster (16 tokens, cold weights, this kernel / the GEMM: 2560 -> 2 x 6912 18.2 / 16.5 us, 4096 -> 2 x 14336
+// 49.8 / 45.1, 5120 -> 2 x 5120 25.8 / 24.1), unless its last round of tiles is less than three quarters full (5120 -> 2 x 20480 77 / 96,
+// 4096 -> 2 x 24576 74 / 80; with three quarters and more 4096 -> 2 x 28672 87 / 82, 2560 -> 2 x 37888 78 / 64). With up to 32 rows an SM this one:
+// 2560 -> 2 x 4736 10.9 / 13.7, 2048 -> 2 x 2048 6.9 / 19. Not gated, it is as fast or faster everywhere (2560 -> 128256 109 / 113, 2560 -> 2560 5.4 / 7.7).
+bool few_serves(const Ctx *ctx, const DenseCall &c) {
+    if (c.m > static_cast<size_t>(few::kMaxTokens) || c.experts) return false;
+    const size_t sms = static_cast<size_t>(ctx->sm_count);
+    if (!c.gated || c.m <= 8 || c.out_rows <= 32 * sms) return true;
+    const size_t tiles = (c.out_rows + kGRows - 1) / kGRows, rounds = (tiles + sms - 1) / sms;
+    return rounds > 1 && 4 * tiles < 3 * rounds * sms;
+}
+
 int launch_few(Ctx *ctx, const DenseCall &c, cudaStream_t st) {
     FewParams p{};
     const int ntl = c.m > 8 ? 2 : 1;
@@ -827,7 +841,7 @@ int launch_dense(Ctx *ctx, const DenseCall &c, cudaStream_t st) {
     if (!c.w.w || (!c.x && c.pre.mode == kPreNone)) return fail(LBK_ERR_INVALID, "dense projection: null buffer");
     if (c.compute == LBK_COMPUTE_F32) return launch_f32(ctx, c, st);
     if (c.pre.mode != kPreNone && (!dense_pre_supported(c.m, c.w.cols) || c.experts)) return fail(LBK_ERR_INVALID, "dense projection: this call cannot run the norms itself");
-    if (c.m <= static_cast<size_t>(few::kMaxTokens) && !c.experts) return launch_few(ctx, c, st);
+    if (few_serves(ctx, c)) return launch_few(ctx, c, st);
     return launch_gemm_tc(ctx, c, st);
 }
 

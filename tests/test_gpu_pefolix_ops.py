@@ -67,7 +67,8 @@ def test_sandwich_norm(ctx, po, n):
 DENSE_SHAPES = [(40, 72), (1, 64), (130, 200), (640, 256), (384, 1088), (97, 40)]
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 64), (148 * 16, 72), (148 * 16 + 1, 1000), (148 * 32, 1096), (148 * 32 + 5, 640), (148 * 65 + 3, 1030)])
+@pytest.mark.parametrize("rows,cols", [(1, 64), (148 * 16, 72), (148 * 16 + 1, 1000), (148 * 32, 1096), (148 * 32 + 5, 640), (148 * 65 + 3, 1030),
+                                       (148 * 128 + 1, 72)])  # gated, 9 and more tokens: a second round of the GEMM's tiles that is nearly empty
 def test_few_token_projection_boxes(ctx, po, rows, cols):
     """Rows around which the few-token kernel's boxes change (16 and 32 rows of an SM, several boxes, a last CTA with little),
     columns that leave some of the sixteen warps one chunk more or none; one to sixteen tokens; rows past the end untouched.
