@@ -140,7 +140,7 @@ class BitNet:
     def _make_step(self) -> Optional[ops.DecodeStep]:
         """The step in one launch; None for a model of a form that it does not take."""
         cfg = self.cfg
-        if not cfg.num_hidden_layers or not cfg.intermediate_size or cfg.head_dim() != 128 or cfg.num_attention_heads % cfg.num_key_value_heads:
+        if not self.layers or not cfg.intermediate_size or cfg.head_dim() != 128 or cfg.num_attention_heads % cfg.num_key_value_heads:
             return None
         try:
             return ops.DecodeStep(self.layers, self.final_norm, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.rms_norm_eps, self.ctx)

@@ -176,6 +176,7 @@ class DecodeStep:
 
     def __init__(self, layers: Sequence[dict], final_norm: torch.Tensor, heads: int, kv_heads: int, eps: float, ctx: Optional[Context] = None):
         self.ctx = ctx or default_context()
+        self.layers = len(layers)
         linears = [l[n] for l in layers for n in self.LINEARS]
         self._weights = [(w.weight, w.packed) for w in linears]
         self._norms = [l[n] for l in layers for n in self.NORMS] + [final_norm]
@@ -206,6 +207,8 @@ class DecodeStep:
     def run(self, x: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: torch.Tensor, pos_stride: int,
             out: torch.Tensor, work: torch.Tensor) -> None:
         """x, out f32 [b, hidden]; k, v bf16 [layers, b, kv_heads, cap, 128]; work: new_work(b, cap)."""
+        if min(k.shape[0], v.shape[0]) < self.layers:  # the kernel goes from layer to layer by itself
+            raise IndexError(f"the cache has {min(k.shape[0], v.shape[0])} layers, the model {self.layers}")
         P = lambda t: C.c_void_p(t.data_ptr())
         _lib.check(self.ctx._lib.lbk_step_run(self.handle, k.shape[1], k.shape[3], P(x), P(k), P(v), k.stride(0), P(cos), P(sin), P(pos), pos_stride,
                                               P(work), P(out), C.c_void_p(_stream_ptr())))

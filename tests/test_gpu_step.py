@@ -274,3 +274,22 @@ def test_step_of_more_layers_than_memory_is_refused(ctx):
     out, one = C.c_void_p(), (C.c_void_p * 1)()
     status = _lib.load().lbk_step_create(ctx.handle, 1 << 58, one, one, C.c_void_p(16), 4, 1, C.c_float(1e-5), C.byref(out))
     assert status == 6 and not out.value
+
+
+def test_cache_of_fewer_layers_is_refused(ctx):
+    """By both routes, before anything is launched; and a model that has lost its layers still runs."""
+    import torch
+    from lemonade_burn_b200 import model
+    cfg = model.Config(512, 768, 4, 1, 2, 500, 1e-5, 500000.0, 24)
+    net = model.BitNet(cfg, model.random_checkpoint(cfg, 1), ctx)
+    short = model.Config(512, 768, 4, 1, 1, 500, 1e-5, 500000.0, 24)
+    tok = torch.tensor([3], dtype=torch.int32, device="cuda")
+    for kw in ({}, {"splits": 1}):
+        with pytest.raises(IndexError):
+            net.forward(tok, model.KvCache(short, 1, 24, "cuda"), **kw)
+    net.layers = net.layers[:1]
+    got, want = net.forward(tok, net.new_cache(1, 24)), net.forward(tok, net.new_cache(1, 24), splits=1)
+    assert (got - want).abs().max() <= TOL * want.abs().max()
+    net.layers = []
+    assert torch.equal(net.forward(tok, net.new_cache(1, 24)), net.forward(tok, net.new_cache(1, 24), splits=1))
+    ctx.check_device_error()
