@@ -24,6 +24,12 @@ def _to_oracle_weights(cfg, tensors):
 
 
 def _run(cfg, b, steps, ctx, seed=1):
+    """By both routes: the step as the model chooses it, and a kernel per operation."""
+    from lemonade_burn_b200 import model
+    return max(_run_route(cfg, b, steps, ctx, seed, splits) for splits in (None, model.attention_splits(cfg.max_position_embeddings)))
+
+
+def _run_route(cfg, b, steps, ctx, seed, splits):
     import torch
     from lemonade_burn_b200 import model
     from oracle import decoder_oracle as D
@@ -39,7 +45,7 @@ def _run(cfg, b, steps, ctx, seed=1):
     toks = rng.integers(0, cfg.vocab_size, size=(steps, b)).astype(np.int32)
     worst = 0.0
     for s in range(steps):
-        logits = net.forward(torch.from_numpy(toks[s]).cuda(), cache)
+        logits = net.forward(torch.from_numpy(toks[s]).cuda(), cache, splits=splits)
         greedy = net.argmax(logits).cpu().numpy()
         got = logits.cpu().numpy()
         for bi in range(b):
@@ -70,6 +76,35 @@ def test_bitnet_width_two_layers(ctx):
     cfg = model.Config(2560, 6912, 20, 5, 2, 8000, 1e-5, 500000.0, 8)
     _run(cfg, b=1, steps=3, ctx=ctx, seed=2)
     _run(cfg, b=3, steps=2, ctx=ctx, seed=3)
+
+
+@pytest.mark.parametrize("b", [1, 3, 9])
+@pytest.mark.parametrize("heads,kv", [(8, 1), (16, 2), (12, 2)])
+def test_more_query_heads_than_the_step_takes(ctx, tmp_path, heads, kv, b):
+    """Six and eight query heads for a KV head: these models decode with a kernel per operation, in the Python model and in the native
+    runtime's recorded step, and both agree with the oracle."""
+    import torch
+    from lemonade_burn_b200 import model
+    from oracle import decoder_oracle as D
+    cap, steps = 12, 3
+    cfg = model.Config(128 * heads, 896, heads, kv, 2, 600, 1e-5, 500000.0, cap)
+    tensors = model.random_checkpoint(cfg, heads + b)
+    model.save_checkpoint(tmp_path, cfg, tensors)
+    py, nat = model.BitNet(cfg, tensors, ctx), model.NativeBitNet(tmp_path, ctx)
+    assert not py._step.supported(b, cap)
+    w, pc, nc = _to_oracle_weights(cfg, tensors), py.new_cache(b, cap), nat.new_cache(b, cap)
+    okc, ovc = ([[np.zeros((kv, cap, 128), np.float32) for _ in range(2)] for _ in range(b)] for _ in range(2))
+    toks = np.random.default_rng(b).integers(0, 600, size=(steps, b)).astype(np.int32)
+    for s in range(steps):
+        tok = torch.from_numpy(toks[s]).cuda()
+        lp, ln = py.forward(tok, pc), nat.decode(tok, nc)[0]
+        torch.cuda.synchronize()
+        assert torch.equal(lp, ln)
+        for i, got in enumerate(ln.cpu().numpy()):
+            ref = D.decode_step(cfg.__dict__, w, int(toks[s, i]), okc[i], ovc[i], s)
+            assert np.abs(got - ref).max() < TOL * np.abs(ref).max()
+    ctx.check_device_error()
+    nat.close()
 
 
 def test_checkpoint_roundtrip_and_format_check(ctx, tmp_path):
