@@ -84,7 +84,7 @@ class KvCache:
         self.pos = torch.zeros(1, dtype=torch.int32, device=device)  # cache.len, on the device
         self.b, self.cap = b, cap
         self.host_len = 0  # the same length on the host: `forward` refuses a step that would not fit
-        self.step_work = None  # (the model's step, what its launches on this cache work in)
+        self.step_work = None  # what the one-launch steps on this cache work in
 
     @property
     def len(self) -> int:
@@ -136,6 +136,7 @@ class BitNet:
         self.cos, self.sin = torch.from_numpy(cos).to(dev), torch.from_numpy(sin).to(dev)
         self._bufs = {}
         self._step = self._make_step()
+        self._old_steps = []  # their tables stay: a graph that somebody has captured reads them
 
     def _make_step(self) -> Optional[ops.DecodeStep]:
         """The step in one launch; None for a model of a form that it does not take."""
@@ -177,9 +178,10 @@ class BitNet:
         return cache
 
     def _work_of(self, cache: KvCache) -> Optional[torch.Tensor]:
-        if cache.step_work is None or cache.step_work[0] is not self._step:
-            cache.step_work = (self._step, self._step.new_work(cache.b, cache.cap, self.device) if self._step else None)
-        return cache.step_work[1]
+        need = self._step.work_bytes(cache.b, cache.cap) if self._step else 0
+        if need and (cache.step_work is None or cache.step_work.numel() != need):
+            cache.step_work = torch.zeros(need, dtype=torch.uint8, device=self.device)
+        return cache.step_work
 
     # ---- one decode step -------------------------------------------------------------------------
     def _buf(self, name, shape, dtype=torch.float32):
@@ -196,9 +198,11 @@ class BitNet:
         if b != cache.b:
             raise ValueError("batch size differs from the cache's")
         cache.reserve(1)
-        if self._step is not None and not self._step.holds(self.layers, self.final_norm):  # somebody has put other weights in
-            self._step = self._make_step()
-        one_launch = splits is None and self._step is not None and self._step.supported(b, cache.cap)
+        same = self._step is None or self._step.holds(self.layers, self.final_norm)
+        if not same and not torch.cuda.is_current_stream_capturing():  # other weights have been put in; a capture takes no new table
+            self._old_steps.append(self._step.retire())
+            self._step, same = self._make_step(), True
+        one_launch = splits is None and same and self._step is not None and self._step.supported(b, cache.cap)
         if splits is None:
             splits = attention_splits(cache.cap)
         H, I, nh, kvh, hd = cfg.hidden_size, cfg.intermediate_size, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim()

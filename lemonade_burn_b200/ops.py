@@ -198,15 +198,19 @@ class DecodeStep:
         """On the current stream: one of a green context with a part of the SMs cannot hold the launch."""
         return bool(self.ctx._lib.lbk_step_supported(self.handle, b, cap)) and bool(self.ctx._lib.lbk_step_stream_supported(self.handle, _stream_ptr()))
 
-    def new_work(self, b: int, cap: int, device) -> Optional[torch.Tensor]:
-        """What `run` works in, None where it does not serve such a cache. It counts the launches' arrivals, so launches that share it come
-        one after another: a buffer for each cache."""
-        n = int(self.ctx._lib.lbk_step_work_bytes(self.handle, b, cap))
-        return torch.zeros(n, dtype=torch.uint8, device=device) if n else None
+    def retire(self) -> "DecodeStep":
+        """Lets the weights go and keeps the kernel's table, which a captured graph may hold."""
+        self._weights, self._norms, self._at = [], [], []
+        return self
+
+    def work_bytes(self, b: int, cap: int) -> int:
+        """Size of what `run` works in, zeros at first, 0 where it does not serve such a cache. The buffer counts the launches' arrivals, so launches
+        that share it come one after another: one for each cache."""
+        return int(self.ctx._lib.lbk_step_work_bytes(self.handle, b, cap))
 
     def run(self, x: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: torch.Tensor, pos_stride: int,
             out: torch.Tensor, work: torch.Tensor) -> None:
-        """x, out f32 [b, hidden]; k, v bf16 [layers, b, kv_heads, cap, 128]; work: new_work(b, cap)."""
+        """x, out f32 [b, hidden]; k, v bf16 [layers, b, kv_heads, cap, 128]; work: work_bytes(b, cap) bytes."""
         if min(k.shape[0], v.shape[0]) < self.layers:  # the kernel goes from layer to layer by itself
             raise IndexError(f"the cache has {min(k.shape[0], v.shape[0])} layers, the model {self.layers}")
         P = lambda t: C.c_void_p(t.data_ptr())

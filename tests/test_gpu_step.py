@@ -169,8 +169,8 @@ def test_caches_of_one_shape_step_on_two_streams(ctx):
     cfg = model.Config(1280, 3408, 10, 5, 2, 500, 1e-5, 500000.0, cap)
     net = model.BitNet(cfg, model.random_checkpoint(cfg, 9), ctx)
     a, c = net.new_cache(b, cap), net.new_cache(b, cap)
-    assert a.step_work[1].data_ptr() != c.step_work[1].data_ptr()
-    gone = weakref.ref(c.step_work[1])
+    assert a.step_work.data_ptr() != c.step_work.data_ptr()
+    gone = weakref.ref(c.step_work)
     del c
     assert gone() is None
     runs = []
@@ -182,7 +182,7 @@ def test_caches_of_one_shape_step_on_two_streams(ctx):
 
     def step(run, t):
         cache, x, out, _ = run
-        net._step.run(x, cache.k, cache.v, net.cos, net.sin, pos[t:], 0, out[t], cache.step_work[1])
+        net._step.run(x, cache.k, cache.v, net.cos, net.sin, pos[t:], 0, out[t], cache.step_work)
 
     want = []
     for run in runs:  # one after the other
@@ -267,14 +267,14 @@ def test_step_whose_waits_run_out(ctx, b):
     ctx.check_device_error()
     assert lib.lbk_step_set_wait_limit(net._step.handle, 0) != 0
     _lib.check(lib.lbk_step_set_wait_limit(net._step.handle, 2000))
-    c.step_work[1].zero_()
-    c.step_work[1].view(torch.int32)[0] = 1  # one barrier that no block has come to
+    c.step_work.zero_()
+    c.step_work.view(torch.int32)[0] = 1  # one barrier that no block has come to
     c.pos.zero_()
     net.forward(toks, c)
     with pytest.raises(_lib.LbkError) as e:
         ctx.check_device_error()
     assert e.value.status == 5
-    c.step_work[1].zero_()
+    c.step_work.zero_()
     _lib.check(lib.lbk_step_set_wait_limit(net._step.handle, 1 << 20))
     c.pos.zero_()
     assert torch.equal(net.forward(toks, c), want)
@@ -320,7 +320,7 @@ def test_codes_on_a_rounding_boundary(ctx):
         c.pos.zero_()
         c.host_len = 0
         net.forward(toks, c)
-        got = c.step_work[1][768:768 + b * 2560 * 4].view(torch.float32).view(b, 2560)  # behind three counters' places of 256 bytes
+        got = c.step_work[768:768 + b * 2560 * 4].view(torch.float32).view(b, 2560)  # behind three counters' places of 256 bytes
         x = net.lm_head[toks.long()].float()
         n = torch.empty_like(x)
         _lib.check(lib.lbk_rms_norm(ctx.handle, x.data_ptr(), l["input_norm"].data_ptr(), b, 2560, 1e-5, n.data_ptr(), torch.cuda.current_stream().cuda_stream))
@@ -349,4 +349,39 @@ def test_cache_of_fewer_layers_is_refused(ctx):
     assert (got - want).abs().max() <= TOL * want.abs().max()
     net.layers = []
     assert torch.equal(net.forward(tok, net.new_cache(1, 24)), net.forward(tok, net.new_cache(1, 24), splits=1))
+    ctx.check_device_error()
+
+
+def test_captured_step_survives_other_weights(ctx):
+    """A graph that a program has captured goes on with the weights that it was captured with, also after the model has been given
+    others and has stepped with them on the same cache."""
+    import torch
+    from lemonade_burn_b200 import model
+    cfg = model.Config(512, 768, 4, 1, 2, 500, 1e-5, 500000.0, 24)
+    net = model.BitNet(cfg, model.random_checkpoint(cfg, 1), ctx)
+    c, tok = net.new_cache(1, 24), torch.tensor([3], dtype=torch.int32, device="cuda")
+    net.forward(tok, c)
+    net.forward(tok, net.new_cache(1, 24), splits=model.attention_splits(24))  # its buffers are there before anything is captured
+    torch.cuda.synchronize()
+    graph, kept = torch.cuda.CUDAGraph(), net.layers[0]["gate"]
+    with torch.cuda.graph(graph):
+        out = net.forward(tok, c)
+
+    def at_start(call):
+        c.pos.zero_()
+        c.host_len = 0
+        call()
+
+    at_start(graph.replay)
+    want = out.clone()
+    net.layers[0]["gate"] = net.layers[1]["gate"]
+    got = []
+    at_start(lambda: got.append(net.forward(tok, c)))
+    assert len(net._old_steps) == 1 and not torch.equal(got[0], want)
+    junk = [torch.full((4096,), 255, dtype=torch.uint8, device="cuda") for _ in range(200)]  # what was given back is used again
+    at_start(graph.replay)
+    assert torch.equal(out, want) and kept is not net.layers[0]["gate"] and junk
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):  # other weights during a capture: a kernel per operation
+        net.layers[0]["gate"] = kept
+        at_start(lambda: net.forward(tok, c))
     ctx.check_device_error()
