@@ -1,15 +1,15 @@
 // Few tokens (up to 16) against bf16 weights: the streaming loop shared by the projections (lbk_dense.cu) and the
 // experts (lbk_moe.cu). Bound: HBM, the weights once.
 //
-//   rows      a CTA owns a contiguous range of weight rows over the whole of K, cut into boxes of at most 32 rows whose
-//             size is chosen so that all SMs have the same number of rows (2560 rows: 18 each); nothing crosses CTAs. Cutting (tile, K) runs between CTAs instead was built twice: the partial sums' trip through
-//             L2 (store, fence, count, read back) cost 3 to 4 us of a 10 us kernel.
+//   rows      a CTA owns a contiguous range of weight rows over the whole of K, cut into boxes of at most 32 rows whose size is chosen so that
+//             all SMs have the same number of rows (2560 rows: 18 each); nothing crosses CTAs. Cutting (tile, K) runs between CTAs
+//             instead was built twice: the partial sums' trip through L2 (store, fence, count, read back) cost 3 to 4 us of a 10 us kernel.
 //   boxes     a box is up to 32 rows (two tiles of the product) x 64 columns, laid down by TMA with the 128-byte swizzle. The 16 warps take the
 //             64-column chunks of K in turn, so that what is in flight is neighbouring memory; a warp owns a ring of boxes
 //             and goes through its chunks for up to kTiles tiles at a time, so nothing in the loop crosses warps and a
 //             token's values are read once for all of these tiles. Whole 128-byte lines by TMA,
 //             and not 64-byte pieces by lanes, is what the rate comes from: lanes that load MMA fragments straight from
-//             global memory got 1.8 to 2.4 TB/s out of the same weights.
+//             global memory got 1.8 to 2.4 TB/s out of weights 2560 wide and 4.7 out of 4096 -> 2 x 14336.
 //   product   mma.sync m16n8k16, the tile's rows as M, tokens as N. Lane (g, t) takes 16-byte units 2t and 2t + 1 of rows
 //             g and g + 8: two units are two MMAs' operands each, because the contraction index may be permuted as
 //             long as weights and tokens are permuted alike. Conflict-free under the swizzle.
@@ -42,23 +42,18 @@ __host__ __device__ inline int ring_depth(int box_rows) {
     return d < kMaxBoxes ? d : kMaxBoxes;
 }
 
-// How `rows` weight rows are dealt to `sms` CTAs: `boxes` boxes of box_rows rows each, as many bytes in flight as the ring
-// allows, fewer and larger boxes among equals.
+// How `rows` weight rows are dealt to `sms` CTAs: `boxes` boxes of box_rows rows each, as few as there can be. A box costs its warp a wait, a refill
+// and a chain of MMAs whatever its rows, and fewer, larger ones leave fewer rows over, so fewer SMs idle. (Choosing the most bytes in flight instead took,
+// at one token: 4096 -> 16384 27.9 us in five boxes of 23 rows, 24.0 in four of 28; 4096 -> 2 x 9472 30.7 in three of 22, 26.6 in two of 32; 8192 -> 2 x
+// 28672 171 in thirteen of 15, 135 in seven of 28; nothing measured is slower.)
 struct Deal {
     int box_rows = 16, boxes = 1, ctas = 1;
 };
 inline Deal deal_rows(size_t rows, int sms) {
     Deal d;
     const int each = static_cast<int>((rows + sms - 1) / sms);
-    int best = 0;
-    for (int n = (each + 31) / 32; n <= (each + 15) / 16; ++n) {
-        const int r = (each + n - 1) / n, flight = ring_depth(r) * r;
-        if (flight > best) {
-            best = flight;
-            d.boxes = n;
-            d.box_rows = r;
-        }
-    }
+    d.boxes = (each + 31) / 32;
+    d.box_rows = (each + d.boxes - 1) / d.boxes;
     const size_t per = static_cast<size_t>(d.boxes) * d.box_rows;
     d.ctas = static_cast<int>((rows + per - 1) / per);
     return d;
