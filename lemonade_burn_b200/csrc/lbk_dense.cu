@@ -655,16 +655,16 @@ FewKernel few_kernel_of(int ntl, int mt) {
 FewKernel few_kernel(bool gated, int ntl, int mt) { return gated ? few_kernel_of<true>(ntl, mt) : few_kernel_of<false>(ntl, mt); }
 
 // Up to 16 tokens without experts, but for gated calls of 9 to 16 with more than 32 weight rows an SM, whose tokens a warp reads again for every
-// pair of boxes: there the GEMM is faster (16 tokens, cold weights, this kernel / the GEMM: 2560 -> 2 x 6912 18.2 / 16.5 us, 4096 -> 2 x 14336
-// 49.8 / 45.1, 5120 -> 2 x 5120 25.8 / 24.1), unless its last round of tiles is less than three quarters full (5120 -> 2 x 20480 77 / 96,
-// 4096 -> 2 x 24576 74 / 80; with three quarters and more 4096 -> 2 x 28672 87 / 82, 2560 -> 2 x 37888 78 / 64). With up to 32 rows an SM this one:
+// pair of boxes: there the GEMM is faster (16 tokens, cold weights, this kernel / the GEMM: 2560 -> 2 x 6912 18.2 / 16.6 us, 4096 -> 2 x 14336
+// 46.9 / 44.3, 5120 -> 2 x 5120 25.6 / 24.1, 2560 -> 2 x 37888 72 / 64), unless its last round of tiles leaves the rounds less than four fifths full
+// (5120 -> 2 x 20480 74 / 96, 4096 -> 2 x 24576 72 / 80, 4096 -> 2 x 28672 82 / 83, 8192 -> 2 x 28672 150 / 154). With up to 32 rows an SM this one:
 // 2560 -> 2 x 4736 10.9 / 13.7, 2048 -> 2 x 2048 6.9 / 19. Not gated, it is as fast or faster everywhere (2560 -> 128256 109 / 113, 2560 -> 2560 5.4 / 7.7).
 bool few_serves(const Ctx *ctx, const DenseCall &c) {
     if (c.m > static_cast<size_t>(few::kMaxTokens) || c.experts) return false;
     const size_t sms = static_cast<size_t>(ctx->sm_count);
     if (!c.gated || c.m <= 8 || c.out_rows <= 32 * sms) return true;
     const size_t tiles = (c.out_rows + kGRows - 1) / kGRows, rounds = (tiles + sms - 1) / sms;
-    return rounds > 1 && 4 * tiles < 3 * rounds * sms;
+    return rounds > 1 && 5 * tiles < 4 * rounds * sms;
 }
 
 int launch_few(Ctx *ctx, const DenseCall &c, cudaStream_t st) {
