@@ -12,20 +12,24 @@
 //                  of their own
 //   2 x 4 expander thread r owns weight row r = TMEM lane r: 32 packed bytes -> 32 words of u8
 //   warps          codes, word c = columns 4c..4c+3 = (packed word >> 2k) & 0x03030303; the two
-//                  sets of four warps take alternate K blocks (one set alone was the bottleneck)
+//                  sets of four warps take the groups of K blocks in turn
 //                  (pack.rs:10-13: no shuffles), written straight to TMEM with tcgen05.st.
-//                  The expanded tile never touches shared memory: expanding into shared memory
-//                  cost 112 KB of shared-memory traffic per 512 cycles of MMA and starved the
-//                  tensor pipe (measured 27 % of peak).
-//   MMA thread     4 x tcgen05.mma (A from TMEM, u8; B from shared memory, s8; K = 32 each);
-//                  tcgen05.commit frees the rings / publishes the accumulator
-//   4 epilogue     tcgen05.ld, dot = acc - sum(q) (codes are w+1: gemm.rs:6-9,306-308),
+//                  The expanded tile never touches shared memory: the MMAs' reads of the activations, the TMA's
+//                  writes of them and 16 KB of codes a block written and read would be more than
+//                  its 128 bytes a cycle.
+//   MMA warp       4 x tcgen05.mma a block (A from TMEM, u8; B from shared memory, s8; K = 32 each), issued by
+//                  one elected lane; tcgen05.commit frees the rings / publishes the accumulator
+//   8 epilogue     tcgen05.ld, dot = acc - sum(q) (codes are w+1: gemm.rs:6-9,306-308),
 //   warps          y = (float)dot * (1/(s_a*s_w)) (gemm.rs:158,178); a warp's 32 lanes are 32
-//                  consecutive weight rows, so every store instruction writes 128 contiguous bytes
+//                  consecutive weight rows, so every store instruction writes 128 contiguous bytes. Two warps a
+//                  quadrant of lanes, 16 token rows at a time: with one, what it computes and the stores it waits for came one after
+//                  the other, 9700 cycles a tile of 192 token rows and 2000 around them, more than the tile's products; now 4400.
 //
 // TMEM columns: two accumulators of NT columns (the epilogue of one tile overlaps the MMAs of the
-// next) + a ring of 32-column weight tiles, two hand-off groups deep (4 tiles at NT = 192, 8 at
-// NT = 64). Bound: int8 tensor pipe; 2*m*rows*cols ops.
+// next) + a ring of 32-column weight tiles, two hand-off groups deep at NT = 192 (4 tiles), three at NT = 64 (12).
+// Bound: int8 tensor pipe; 2*m*rows*cols ops. A block of 192 token rows is 384 cycles of MMAs and takes 417 without an epilogue, 475
+// beside one (585 when four epilogue warps and one-lane issue bounded it). Quantiser and GEMM, us, before -> now: 2560 -> 2 x 6912 at 17 / 333 / 2048 rows 10.4 -> 7.6,
+// 20.3 -> 17.3, 74.8 -> 61.9; 6912 -> 2560 at 333 rows 17.9 -> 13.8; 4096 -> 2 x 14336 at 17 / 400 rows 19.0 -> 13.8, 51.1 -> 42.7.
 #include "lbk_internal.cuh"
 #include "lbk_ptx.cuh"
 #include "lbk_tcgen05.cuh"
@@ -38,43 +42,43 @@ constexpr int kBMW = 128;          // weight rows per tile (MMA M, TMEM lanes)
 constexpr int kBK = 128;           // columns per stage = one packed block
 constexpr int kPackBlocks = 4;      // K-blocks per packed-weight stage: [128 rows][128 B] boxes
 constexpr int kPackBytes = kBMW * kBlockBytes * kPackBlocks;  // 16 KB, SWIZZLE_128B
-constexpr int kEpiWarps = 4, kExpWarps = 4, kExpSets = 2;
-// warps 0-3 epilogue, 4-7 and 8-11 expanders (warp % 4 = the TMEM lane quadrant a warp may touch)
-// warp 12 feeds the activation ring, warp 14 the packed-weight ring: two threads, so that the weight
+constexpr int kEpiWarps = 8, kExpWarps = 4, kExpSets = 2;
+constexpr int kEpiThreads = kEpiWarps * 32, kEpiSets = kEpiWarps / 4;
+constexpr int kEpiCols = 16;      // token rows an epilogue warp takes at a time
+// warps 0-7 epilogue, 8-11 and 12-15 expanders (warp % 4 = the TMEM lane quadrant a warp may touch)
+// warp 16 feeds the activation ring, warp 18 the packed-weight ring: two threads, so that the weight
 // stream from HBM runs ahead by its own ring's depth whatever the activation ring is waiting for
-constexpr int kExpWarp0 = 4, kTmaWarp = 12, kMmaWarp = 13, kPackWarp = 14;
-constexpr int kThreads = 15 * 32;
+constexpr int kExpWarp0 = kEpiWarps, kTmaWarp = kExpWarp0 + kExpWarps * kExpSets, kMmaWarp = kTmaWarp + 1, kPackWarp = kTmaWarp + 2;
+constexpr int kThreads = (kPackWarp + 1) * 32;
 constexpr uint32_t kTmemCols = 512;
+constexpr int kWide = 192;         // token rows of the wide form's tile at most
 
 template <int NT>  // capacity in token rows per tile (MMA N): 192 or 64; a launch uses nt <= NT
 struct Cfg {
     static constexpr int kActBytes = NT * kBK;                  // multiple of 1024 for NT = 192, 64
-    static constexpr int kLoadStages = NT == 192 ? 6 : 12;      // activation ring, in K blocks
-    static constexpr int kGroup = NT == 192 ? 2 : 4;            // K blocks per hand-off (see kBarFull below)
+    static constexpr int kLoadStages = NT == kWide ? 6 : 12;    // activation ring, in K blocks
+    static constexpr int kGroup = NT == kWide ? 2 : 4;          // K blocks per hand-off (see kBarFull below)
     static constexpr int kGroupStages = kLoadStages / kGroup;   // activation ring in hand-off units
-    static constexpr int kAStages = 2 * kGroup;                 // expanded weight tiles in TMEM (32 columns each): two groups
+    static constexpr int kAGroups = NT == kWide ? 2 : 3;        // groups of expanded weight tiles in TMEM (32 columns a tile)
     // Packed-weight ring, 16 KB a stage. With 64 token rows the weights come straight from HBM (no
     // other token tile shares them through L2) and the ring has to cover the memory latency.
-    static constexpr int kPackStages = NT == 192 ? 3 : 8;
+    static constexpr int kPackStages = NT == kWide ? 3 : 8;
     static constexpr uint32_t kPack0 = kLoadStages * kActBytes;
     static constexpr uint32_t kAcc0 = 0, kAcc1 = NT, kA0 = 2 * NT;  // TMEM column map: two accumulators, then the weight tiles
-    static_assert(2 * NT + kAStages * 32 <= 512, "TMEM budget");
-    static_assert(kGroup == 2 || kGroup == kPackBlocks, "a group is half a packed-weight stage or a whole one");
+    static_assert(2 * NT + kAGroups * kGroup * 32 <= 512, "TMEM budget");
+    static constexpr int kStageGroups = kPackBlocks / kGroup;  // groups of a packed-weight stage: the second set's is the second, or every other stage's
+    static_assert(kStageGroups == 1 || kStageGroups == kExpSets, "a group is half a packed-weight stage or a whole one");
     // instruction descriptor without N: D s32, A u8 (codes, TMEM), B s8 (activations), K-major, M=128
     static constexpr uint32_t kIdesc = (2u << 4) | (0u << 7) | (1u << 10) | ((kBMW >> 4) << 24);
     static constexpr uint32_t kBars = kPack0 + kPackStages * kPackBytes;
     static constexpr uint32_t kMisc = kBars + 48 * 8;
     static constexpr uint32_t kTok = kMisc + 64;              // per-token sum(q) and 1/(s_a*s_w): 2 x [2][NT]
     static constexpr uint32_t kTotal = kTok + 2 * 2 * NT * 4;
-    // Hand-off is by GROUPS of kGroup K blocks. Every barrier wait in the MMA thread drains the
-    // tensor pipe for a few hundred cycles whatever the MMA shape (measured: 4 MMAs + one wait per
-    // loop turn run at 590 cycles a turn, 8 MMAs + one wait at 900), so a wait has to buy as many
-    // MMAs as shared memory and TMEM allow: 2 blocks of 192 token rows, 4 blocks of 64. One "full"
-    // barrier per group collects both operands: the activation bytes of its blocks (TMA
-    // transaction count) and one arrival from each of the eight expander warps (set 0 expands the
-    // group's even blocks, set 1 its odd ones; a warp with no block at the ragged end of K arrives
-    // all the same). One "consumed" barrier per group (a single tcgen05.commit) releases the
-    // activation stages and, two groups later, the TMEM weight slots.
+    // Hand-off is by GROUPS of kGroup K blocks: a turn of the MMA warp (wait, issue, commit) takes some 330 cycles beside
+    // the MMAs, as much as those of one block, so a group is 2 blocks of 192 token rows (one block a turn: 555 cycles a block) or 4 of 64. One
+    // "full" barrier per group collects both operands: the activation bytes of its blocks (TMA transaction count) and one
+    // arrival from each of the four expander warps whose set the group is. One "consumed" barrier per group (a single
+    // tcgen05.commit) releases the activation stages and the TMEM weight slots.
     static constexpr int kBarFull = 0;                        // [group stages]
     static constexpr int kBarConsumed = kLoadStages;          // [group stages]
     static constexpr int kBarFullPack = 2 * kLoadStages;      // [PS] packed weights landed
@@ -83,7 +87,7 @@ struct Cfg {
     static constexpr int kBarAccEmpty = kBarAccFull + 2;      // [2]
     static_assert(kBarAccEmpty + 2 <= 48, "barrier area too small");
     static_assert(kTotal + 1024 <= 232448, "shared memory budget");
-    static_assert(2 < kGroupStages, "a consumed-barrier phase must still be observable two groups later");
+    static_assert(kAGroups <= kGroupStages, "a consumed-barrier phase must still be observable when its weight slots are filled again");
 };
 
 struct GemmParams {
@@ -93,7 +97,7 @@ struct GemmParams {
     int32_t *iout[LBK_MAX_GROUP];
     float wscale[LBK_MAX_GROUP];
     int rows[LBK_MAX_GROUP];
-    int tile_end[LBK_MAX_GROUP];        // running tile count up to and including matrix i
+    int row_end[LBK_MAX_GROUP];         // running count of 128-row tiles up to and including matrix i
     int n_mat, m, m_tiles, k_blocks, total_tiles;
     int nt;                             // token rows per tile in this launch (multiple of 16, <= capacity)
     int ksplit, kb_part;                // every tile's K blocks are cut into ksplit parts of kb_part blocks (a multiple of 4)
@@ -132,6 +136,15 @@ __device__ __forceinline__ void umma_i8_ts_block(uint32_t d_tmem, uint32_t a_tme
         "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate_first)
         : "memory");
 }
+// A wait of a whole warp, with one outcome for all its lanes (what follows needs them together)
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag));
+}
+__device__ __forceinline__ bool elect_one() {  // one lane of a converged warp
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
 // SC: matrix 0's int32 dots go to the token owners' buffers (GemmParams::scatter) instead of iout: an instantiation of its
 // own, so that the ordinary kernel's epilogue keeps its registers
 template <int NT, bool SC>
@@ -151,12 +164,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
 
     if (tid == 0) {
         for (int i = 0; i < PG; ++i) {
-            ptx::mbar_init(bar(C::kBarFull + i), 1 + kExpWarps * kExpSets);
+            ptx::mbar_init(bar(C::kBarFull + i), 1 + kExpWarps);
             ptx::mbar_init(bar(C::kBarConsumed + i), 1);
         }
         for (int i = 0; i < PS; ++i) {
             ptx::mbar_init(bar(C::kBarFullPack + i), 1);
-            ptx::mbar_init(bar(C::kBarEmptyPack + i), kExpWarps * kExpSets);
+            ptx::mbar_init(bar(C::kBarEmptyPack + i), kExpWarps * C::kStageGroups);
         }
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(bar(C::kBarAccFull + a), 1);
@@ -182,19 +195,26 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
 
     const int k_blocks = p.k_blocks;
     bool ok = true;
-    // tile -> (matrix, weight-row tile, token tile); token tiles vary fastest so that CTAs
-    // running side by side share the same packed weights in L2
+    // tile -> (matrix, weight-row tile, token tile); token tiles vary fastest so that CTAs running side by side share the same
+    // packed weights in L2; the shorter last token tiles of a ragged batch come after all others.
+    const int row_tiles = p.row_end[p.n_mat - 1], full = p.m / p.nt;
     auto decode_tile = [&](int tile, int &mat, int &m_tile, int &n_tile) {
+        if (tile < full * row_tiles) {
+            n_tile = tile / full;
+            m_tile = tile - n_tile * full;
+        } else {
+            n_tile = tile - full * row_tiles;
+            m_tile = full;
+        }
         mat = 0;
-        while (mat < p.n_mat - 1 && tile >= p.tile_end[mat]) ++mat;
-        const int local = tile - (mat ? p.tile_end[mat - 1] : 0);
-        m_tile = local % p.m_tiles;
-        n_tile = local / p.m_tiles;
+        while (mat < p.n_mat - 1 && n_tile >= p.row_end[mat]) ++mat;
+        if (mat) n_tile -= p.row_end[mat - 1];
     };
 
-    // A work item is one tile, or one of the ksplit equal parts of a tile's K blocks. All roles walk
-    // items blockIdx.x, blockIdx.x + gridDim.x, ...
-    const int total_items = p.total_tiles * p.ksplit;
+    // A work item is one tile, or one of the ksplit equal parts of a tile's K blocks. All roles walk the same items, every
+    // other round backwards: a CTA whose item of the round before last was a short one gets one of those that are left over.
+    const int total_items = p.total_tiles * p.ksplit, ctas = gridDim.x;
+    auto item_at = [&](int round) { return round * ctas + ((round & 1) ? ctas - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x)); };
     auto item_range = [&](int item, int &tile, int &kb0, int &kb1) {
         tile = item / p.ksplit;
         const int part = item - tile * p.ksplit;
@@ -206,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         // ================= TMA producer: packed weights =================
         if (lane == 0) {
             int pit = 0;
-            for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+            for (int turn = 0, item; (item = item_at(turn)) < total_items && ok; ++turn) {
                 int tile, kb0, kb1, mat, m_tile, n_tile;
                 item_range(item, tile, kb0, kb1);
                 decode_tile(tile, mat, m_tile, n_tile);
@@ -226,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
             int gr = 0;  // groups of activation blocks
-            for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+            for (int turn = 0, item; (item = item_at(turn)) < total_items && ok; ++turn) {
                 int tile, kb0, kb1, mat, m_tile, n_tile;
                 item_range(item, tile, kb0, kb1);
                 decode_tile(tile, mat, m_tile, n_tile);
@@ -245,120 +265,111 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         }
     } else if (warp >= kExpWarp0 && warp < kExpWarp0 + kExpWarps * kExpSets) {
         // ================= expanders: packed 2-bit -> u8 codes in TMEM =================
+        // The sets take the groups of K blocks in turn: the codes of two blocks are worked out in registers while the slots they go to are
+        // still being read, so what lies between a slot that is free again and its next "full" is one store and its wait. With
+        // a block of every group for each set, the set's own turn (waits, arrivals, a store of 250 cycles a block) bounded the kernel.
         const int quad = (warp - kExpWarp0) % kExpWarps, set = (warp - kExpWarp0) / kExpWarps;
         const int r = quad * 32 + lane;  // weight row of the tile = TMEM lane
-        const uint32_t lane_field = static_cast<uint32_t>(quad * 32) << 16;
-        // Ring positions are counters (no divisions in the loop): group `gr` uses barrier slot `sp`
-        // and the TMEM slots of parity gr & 1; (lg, lg_phase) follow group gr - 2, whose MMAs were
-        // the last readers of those TMEM slots; (ps, pphase) follow the packed-weight stage.
-        int gr = 0, sp = 0, lg = PG - 2, ps = -1;
-        uint32_t lg_phase = 1, pphase = 1;
-        for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+        const uint32_t a_dst = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + C::kA0;
+        const uint8_t *pk_row = sm + C::kPack0 + r * 128;  // row r of a [128][128 B] swizzled stage; block b's 32 bytes are units 2 b, 2 b + 1
+        const int x = r & 7;
+        int gr = 0, stage = 0;  // groups and packed-weight stages so far
+        for (int turn = 0, item; (item = item_at(turn)) < total_items && ok; ++turn) {
             int tile, kb0, kb1;
             item_range(item, tile, kb0, kb1);
-            for (int kb = kb0; kb < kb1; kb += G, ++gr) {
-                if ((kb % kPackBlocks) == 0) {
-                    if (++ps == PS) ps = 0;
-                    if (ps == 0) pphase ^= 1u;
-                    if (!wait_bar(bar(C::kBarFullPack + ps), pphase, s_abort)) {
-                        ok = false;
-                        break;
-                    }
+            for (int kb = kb0; kb < kb1; kb += kPackBlocks, ++stage) {
+                const int groups = C::kStageGroups == 1 || kb + G >= kb1 ? 1 : 2;  // of this stage
+                const int mine = C::kStageGroups == 1 ? gr : gr + set;               // the number of this set's
+                const bool have = C::kStageGroups == 1 ? (gr & 1) == set : set < groups;
+                gr += groups;
+                if (C::kStageGroups == 1 && !have) continue;
+                const int ps = stage % PS;
+                if (!warp_wait(bar(C::kBarFullPack + ps), (stage / PS) & 1, s_abort)) {
+                    ok = false;
+                    break;
                 }
-                bool wrote = false;
+                if (!have) {  // a last stage without a group of this set goes by
+                    if (lane == 0) ptx::mbar_arrive(bar(C::kBarEmptyPack + ps));
+                    continue;
+                }
+                const uint8_t *pk = pk_row + ps * kPackBytes;
 #pragma unroll
-                for (int b = set; b < G; b += kExpSets) {  // this warp's blocks of the group
-                    if (kb + b >= kb1) break;
-                    if (!wrote) {
-                        // the TMEM slots of this parity were last read by group gr - 2
-                        if (gr >= 2 && !wait_bar(bar(C::kBarConsumed + lg), lg_phase, s_abort)) {
+                for (int half = 0; half < G / 2; ++half) {
+                    const int u0 = 4 * (C::kStageGroups == 1 ? half : set);  // first of the two blocks' four units
+                    uint32_t v[64];  // word 32 b + 8 k + i = columns k * 32 + 4 i .. 4 i + 3 of block b (blocks behind the end are not read)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const uint4 w4 = *reinterpret_cast<const uint4 *>(pk + (((u0 + u) ^ x) << 4));  // packed bytes 16 (u % 2) .. of block u / 2
+                        const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) v[32 * (u / 2) + 8 * k + 4 * (u % 2) + i] = (w[i] >> (2 * k)) & 0x03030303u;
+                    }
+                    if (half == 0) {
+                        // these TMEM slots were last read by group mine - kAGroups
+                        const int last = mine - C::kAGroups;
+                        if (last >= 0 && !warp_wait(bar(C::kBarConsumed + last % PG), (last / PG) & 1, s_abort)) {
                             ok = false;
                             break;
                         }
                         tc_fence_after();
-                        wrote = true;
                     }
-                    // row r of the [128][128 B] swizzled stage; this block's 32 bytes are units 2*sub, 2*sub+1
-                    const int sub = ((kb + b) % kPackBlocks);
-                    const uint8_t *pk = sm + C::kPack0 + ps * kPackBytes + r * 128;
-                    const int x = r & 7;
-                    const uint4 w0 = *reinterpret_cast<const uint4 *>(pk + (((2 * sub) ^ x) << 4));      // packed bytes j = 0..15
-                    const uint4 w1 = *reinterpret_cast<const uint4 *>(pk + (((2 * sub + 1) ^ x) << 4));  // packed bytes j = 16..31
-                    const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-                    uint32_t v[32];  // word 8k + i = columns k*32 + 4i .. 4i+3
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[8 * k + i] = (w[i] >> (2 * k)) & 0x03030303u;
-                    tmem_st32(tmem_base + lane_field + C::kA0 + ((gr & 1) * G + b) * 32, v);
+                    tmem_st64(a_dst + ((mine % C::kAGroups) * G + 2 * half) * 32, v);
                 }
                 if (!ok) break;
-                // this warp's last read of the packed stage is behind it when the stage's last block is
-                if (((kb + G) % kPackBlocks) == 0 || kb + G >= kb1) {
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(bar(C::kBarEmptyPack + ps));
-                }
-                if (wrote) {
-                    tmem_st_wait();
-                    tc_fence_before();
-                }
+                // The stage is given back behind the stores: what they take has arrived from shared memory. Given back as soon as the loads were
+                // issued, it was filled again, once in some thousand tiles, before a load behind the epilogue's stores had read its first rows.
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar(C::kBarFull + sp));
-                if (++sp == PG) sp = 0;
-                if (++lg == PG) {
-                    lg = 0;
-                    lg_phase ^= 1u;
-                }
+                if (lane == 0) ptx::mbar_arrive(bar(C::kBarEmptyPack + ps));
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(C::kBarFull + mine % PG));
             }
         }
     } else if (warp == kMmaWarp) {
-        // ================= MMA issuer (one thread) =================
-        if (lane == 0) {
-            // Ring positions are kept as counters: this thread's instruction stream is the critical
-            // path of the whole CTA (one thread issues every MMA), so no divisions by the ring size here.
-            int tcount = 0, sp = 0;
-            uint32_t full_phase = 0, pa = 0;
-            const uint64_t bdesc0 = smem_desc_sw128(base);  // activation block stage 0; stage s adds s * kActBytes / 16
-            for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x, ++tcount) {
-                const int a = tcount & 1, around = tcount >> 1;
-                if (around > 0 && !wait_bar(bar(C::kBarAccEmpty + a), (around - 1) & 1, s_abort)) {
-                    ok = false;
-                    break;
-                }
+        // ================= MMA issuer =================
+        // The whole warp walks and waits, one elected lane issues. Under a branch of one lane a turn of a wait and four MMAs took
+        // 504 cycles whatever N (the MMAs of N = 192 take 384); so it takes 384, and four blocks of N = 64 in a turn 172 a block instead of 264.
+        int tcount = 0, sp = 0, as = 0;
+        uint32_t full_phase = 0;
+        const uint64_t bdesc0 = smem_desc_sw128(base);  // activation block stage 0; stage s adds s * kActBytes / 16
+        for (int item; (item = item_at(tcount)) < total_items; ++tcount) {
+            const int a = tcount & 1, around = tcount >> 1;
+            if (around > 0) ok = warp_wait(bar(C::kBarAccEmpty + a), (around - 1) & 1, s_abort) && ok;
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + (a ? C::kAcc1 : C::kAcc0);
+            // N of this tile: the launch's token tile, less for the last tile of a ragged batch
+            int tile, kb0, kb1, mat, m_tile, n_tile;
+            item_range(item, tile, kb0, kb1);
+            decode_tile(tile, mat, m_tile, n_tile);
+            const int left = p.m - m_tile * p.nt;
+            const int n_mma = left < p.nt ? (left + 15) & ~15 : p.nt;
+            const uint32_t idesc = C::kIdesc | (static_cast<uint32_t>(n_mma >> 3) << 17);
+            for (int kb = kb0; kb < kb1; kb += G) {
+                ok = warp_wait(bar(C::kBarFull + sp), full_phase, s_abort) && ok;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (a ? C::kAcc1 : C::kAcc0);
-                // N of this tile: the launch's token tile, less for the last tile of a ragged batch
-                int tile, kb0, kb1, mat, m_tile, n_tile;
-                item_range(item, tile, kb0, kb1);
-                decode_tile(tile, mat, m_tile, n_tile);
-                const int left = p.m - m_tile * p.nt;
-                const int n_mma = left < p.nt ? (left + 15) & ~15 : p.nt;
-                const uint32_t idesc = C::kIdesc | (static_cast<uint32_t>(n_mma >> 3) << 17);
-                for (int kb = kb0; kb < kb1; kb += G) {
-                    if (!wait_bar(bar(C::kBarFull + sp), full_phase, s_abort)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_tmem = tmem_base + C::kA0 + pa * (G * 32);
-                    const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(sp * G * (C::kActBytes >> 4));
+                const uint32_t a_tmem = tmem_base + C::kA0 + as * (G * 32);
+                const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(sp * G * (C::kActBytes >> 4));
+                if (elect_one() && ok) {
                     umma_i8_ts_block(d_tmem, a_tmem, bdesc, idesc, kb != kb0 ? 1u : 0u);
 #pragma unroll
                     for (int b = 1; b < G; ++b)
                         if (kb + b < kb1) umma_i8_ts_block(d_tmem, a_tmem + b * 32, bdesc + static_cast<uint64_t>(b * (C::kActBytes >> 4)), idesc, 1u);
                     umma_commit(bar(C::kBarConsumed + sp));  // both operands' slots are reusable once these MMAs retire
-                    if (++sp == PG) {
-                        sp = 0;
-                        full_phase ^= 1u;
-                    }
-                    pa ^= 1u;
+                    if (kb + G >= kb1) umma_commit(bar(C::kBarAccFull + a));  // accumulator complete
                 }
-                if (!ok) break;
-                umma_commit(bar(C::kBarAccFull + a));  // accumulator complete
+                __syncwarp();
+                if (++sp == PG) {
+                    sp = 0;
+                    full_phase ^= 1u;
+                }
+                if (++as == C::kAGroups) as = 0;
             }
         }
     } else if (warp < kEpiWarps) {
-        // ================= epilogue (warps 0..3 = TMEM lane quadrants 0..3) =================
+        // ================= epilogue (warp % 4 = TMEM lane quadrant) =================
         int *s_qs = reinterpret_cast<int *>(sm + C::kTok);
         float *s_inv = reinterpret_cast<float *>(sm + C::kTok + 2 * NT * 4);
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -366,7 +377,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         // fetched them 32 at a time in front of the tile held the accumulators for 5500 of the 14400 cycles a tile of 2560 columns took. Calls with
         // small tiles have one or two a CTA, their terms come during the products: warp 0 fetches them there (ahead it was 1 us slower at 333 rows).
         constexpr bool kAhead = NT > 128;
-        constexpr int kTerms = (NT + 127) / 128;
+        constexpr int kTerms = (NT + kEpiThreads - 1) / kEpiThreads;
+        const int quad = warp & 3;
         int term_q[kTerms];
         float term_s[kTerms];
         auto fetch_terms = [&](int item) {
@@ -376,21 +388,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
             decode_tile(tile, mat, m_tile, n_tile);
 #pragma unroll
             for (int e = 0; e < kTerms; ++e) {
-                const int i = tid + e * 128, tk = m_tile * p.nt + i;
+                const int i = tid + e * kEpiThreads, tk = m_tile * p.nt + i;
                 const bool in = i < p.nt && tk < p.m;
                 term_q[e] = in ? p.qsum[tk] : 0;
                 term_s[e] = in && p.qscale ? p.qscale[tk] : 0.0f;
             }
         };
-        if constexpr (kAhead) fetch_terms(blockIdx.x);
+        if constexpr (kAhead) fetch_terms(item_at(0));
         int tcount = 0;
-        for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x, ++tcount) {
+        for (int item; (item = item_at(tcount)) < total_items && ok; ++tcount) {
             const int a = tcount & 1, around = tcount >> 1;
             int tile, kb0, kb1, mat, m_tile, n_tile;
             item_range(item, tile, kb0, kb1);
             decode_tile(tile, mat, m_tile, n_tile);
             const int rows = p.rows[mat];
-            const int row = n_tile * kBMW + warp * 32 + lane;
+            const int row = n_tile * kBMW + quad * 32 + lane;
             const int nt = p.nt;
             const int tok0 = m_tile * nt;
             float *out = p.out[mat];
@@ -400,39 +412,39 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
             if constexpr (kAhead) {
 #pragma unroll
                 for (int e = 0; e < kTerms; ++e) {
-                    const int i = tid + e * 128, tk = tok0 + i;
+                    const int i = tid + e * kEpiThreads, tk = tok0 + i;
                     if (i < NT) {
                         qs[i] = term_q[e];
                         inv[i] = i < nt && tk < p.m && p.qscale ? __fdiv_rn(1.0f, __fmul_rn(term_s[e], p.wscale[mat])) : 0.0f;  // gemm.rs:158
                     }
                 }
-                fetch_terms(item + gridDim.x);
+                fetch_terms(item_at(tcount + 1));
             } else if (warp == 0) {
-                for (int i = lane; i < ((nt + 31) & ~31); i += 32) {
+                for (int i = lane; i < nt; i += 32) {
                     const int tk = tok0 + i;
                     qs[i] = tk < p.m ? p.qsum[tk] : 0;
                     inv[i] = (tk < p.m && p.qscale) ? __fdiv_rn(1.0f, __fmul_rn(p.qscale[tk], p.wscale[mat])) : 0.0f;  // gemm.rs:158
                 }
             }
-            asm volatile("bar.sync 2, 128;" ::: "memory");  // the four epilogue warps
-            if (!wait_bar(bar(C::kBarAccFull + a), around & 1, s_abort)) {
+            ptx::named_barrier(2, kEpiThreads);  // the epilogue warps
+            if (!warp_wait(bar(C::kBarAccFull + a), around & 1, s_abort)) {
                 ok = false;
                 break;
             }
             tc_fence_after();
             const int ntok = p.m - tok0 < nt ? p.m - tok0 : nt;
 #pragma unroll 1
-            for (int c = 0; c * 32 < ntok; ++c) {
-                uint32_t v[32];
-                tmem_ld32(tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + (a ? C::kAcc1 : C::kAcc0) + c * 32, v);
+            for (int c = warp >> 2; c * kEpiCols < ntok; c += kEpiSets) {
+                uint32_t v[kEpiCols];
+                tmem_ld16(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (a ? C::kAcc1 : C::kAcc0) + c * kEpiCols, v);
                 // per-token terms into registers first: the stores below may alias the shared
                 // arrays as far as the compiler knows, which would serialise load -> store pairs
-                int q[32];
-                float sc[32];
+                int q[kEpiCols];
+                float sc[kEpiCols];
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    const int4 q4 = *reinterpret_cast<const int4 *>(qs + c * 32 + i);
-                    const float4 s4 = *reinterpret_cast<const float4 *>(inv + c * 32 + i);
+                for (int i = 0; i < kEpiCols; i += 4) {
+                    const int4 q4 = *reinterpret_cast<const int4 *>(qs + c * kEpiCols + i);
+                    const float4 s4 = *reinterpret_cast<const float4 *>(inv + c * kEpiCols + i);
                     q[i] = q4.x; q[i + 1] = q4.y; q[i + 2] = q4.z; q[i + 3] = q4.w;
                     sc[i] = s4.x; sc[i + 1] = s4.y; sc[i + 2] = s4.z; sc[i + 3] = s4.w;
                 }
@@ -442,11 +454,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                     // into the buffer of the rank that owns the token (plain stores into peer memory, 128 consecutive
                     // bytes per warp instruction), while the MMAs of the next tile run.
                     if (row < rows) {
-                        const int tk = tok0 + c * 32;
+                        const int tk = tok0 + c * kEpiCols;
                         int o = tk / p.scatter_mt, lt = tk - o * p.scatter_mt;
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            if (c * 32 + i < ntok) p.scatter[o][static_cast<size_t>(lt) * rows + row] = static_cast<int>(v[i]) - q[i];
+                        for (int i = 0; i < kEpiCols; ++i) {
+                            if (c * kEpiCols + i < ntok) p.scatter[o][static_cast<size_t>(lt) * rows + row] = static_cast<int>(v[i]) - q[i];
                             if (++lt == p.scatter_mt) {
                                 lt = 0;
                                 ++o;
@@ -459,29 +471,29 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                     // one of several parts of this tile: add the sums into the zeroed int32 buffer
                     // (the part that starts at block 0 also takes off sum(q)); a small kernel scales later
                     if (row < rows) {
-                        int32_t *dst = p.acc[mat] + static_cast<size_t>(tok0 + c * 32) * rows + row;
+                        int32_t *dst = p.acc[mat] + static_cast<size_t>(tok0 + c * kEpiCols) * rows + row;
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (c * 32 + i < ntok) atomicAdd(dst + static_cast<size_t>(i) * rows, static_cast<int>(v[i]) - (kb0 == 0 ? q[i] : 0));
+                        for (int i = 0; i < kEpiCols; ++i)
+                            if (c * kEpiCols + i < ntok) atomicAdd(dst + static_cast<size_t>(i) * rows, static_cast<int>(v[i]) - (kb0 == 0 ? q[i] : 0));
                     }
                     continue;
                 }
                 if (row < rows) {
-                    const size_t o0 = static_cast<size_t>(tok0 + c * 32) * rows + row;
-                    if (c * 32 + 32 <= ntok) {
+                    const size_t o0 = static_cast<size_t>(tok0 + c * kEpiCols) * rows + row;
+                    if (c * kEpiCols + kEpiCols <= ntok) {
                         if (out) {
 #pragma unroll
-                            for (int i = 0; i < 32; ++i)
+                            for (int i = 0; i < kEpiCols; ++i)
                                 out[o0 + static_cast<size_t>(i) * rows] = __fmul_rn(__int2float_rn(static_cast<int>(v[i]) - q[i]), sc[i]);
                         }
                         if (iout) {
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) iout[o0 + static_cast<size_t>(i) * rows] = static_cast<int>(v[i]) - q[i];
+                            for (int i = 0; i < kEpiCols; ++i) iout[o0 + static_cast<size_t>(i) * rows] = static_cast<int>(v[i]) - q[i];
                         }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            if (c * 32 + i < ntok) {
+                        for (int i = 0; i < kEpiCols; ++i) {
+                            if (c * kEpiCols + i < ntok) {
                                 const int d = static_cast<int>(v[i]) - q[i];
                                 if (iout) iout[o0 + static_cast<size_t>(i) * rows] = d;
                                 if (out) out[o0 + static_cast<size_t>(i) * rows] = __fmul_rn(__int2float_rn(d), sc[i]);
@@ -491,7 +503,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                 }
             }
             tc_fence_before();
-            asm volatile("bar.sync 2, 128;" ::: "memory");  // all four warps are done with qs/inv of this parity
+            ptx::named_barrier(2, kEpiThreads);  // all epilogue warps are done with qs/inv of this parity
             if (lane == 0) ptx::mbar_arrive(bar(C::kBarAccEmpty + a));
         }
     }
@@ -517,7 +529,7 @@ static int init_one(Ctx *ctx) {
 }
 
 int gemm_init(Ctx *ctx) {
-    LBK_TRY(init_one<192>(ctx));
+    LBK_TRY(init_one<kWide>(ctx));
     LBK_TRY(init_one<64>(ctx));
     LBK_CUDA(cudaMalloc(&ctx->gemm_acc, kGemmAccBytes));
     LBK_CUDA(cudaMemset(ctx->gemm_acc, 0, kGemmAccBytes));  // kept zero between launches: the scaling kernel zeroes what it reads
@@ -551,25 +563,32 @@ static int choose_ksplit(int tiles, int k_blocks, int sms, int *kb_part) {
 }
 
 
-// Token rows per tile for a launch: the multiple of 16 (at most 192) whose tile count fills whole
-// rounds of the grid best. Per K block a tile costs the larger of the tensor-pipe time
-// (proportional to nt, about 400 cycles at nt = 192) and the issue thread's turn-around (about
-// 470 cycles whatever nt is: measured), plus the epilogue's share that the next tile cannot hide.
-static int choose_nt(size_t m, int row_tiles, int k_blocks, int sms) {
-    if (m <= 64) return static_cast<int>((m + 15) & ~static_cast<size_t>(15));
-    int best_nt = 192;
-    double best = 1e30;
-    for (int tiles_m = static_cast<int>((m + 191) / 192); tiles_m <= static_cast<int>((m + 63) / 64); ++tiles_m) {
-        const int nt = static_cast<int>(((m + tiles_m - 1) / tiles_m + 15) & ~static_cast<size_t>(15));
-        if (nt > 192 || nt < 64) continue;
-        const long long tiles = static_cast<long long>(row_tiles) * ((m + nt - 1) / nt);
-        const long long rounds = (tiles + sms - 1) / sms;
-        const double block = nt * (400.0 / 192.0) > 470.0 ? nt * (400.0 / 192.0) : 470.0;
-        const double cost = static_cast<double>(rounds) * (k_blocks * block + 12.0 * nt);
-        if (cost < best) {
+// Token rows per tile for a launch, a multiple of 16: the count with the least cost in cycles of the fullest CTA. Up to 64 the
+// narrow kernel runs, 250 cycles a K block; the wide one takes 365 at 96 token rows and 490 at 192 (launches of many
+// rounds, their epilogues beside the products; 341 and 416 in a single round). 35 cycles a token row are the last tile's
+// epilogue, 300 the start of a tile. Short tiles of a ragged batch come last (decode_tile in the kernel): what is left
+// over behind the full rounds are short ones, and with the order turned round every other time a CTA that has two of them
+// at the end takes less than a full tile longer than the others. Measured at 2560 -> 2 x 6912, us: 400 rows in tiles of 112 / 144 / 176
+// 15.5 / 15.8 / 14.8, 2048 rows in tiles of 64 / 128 / 160 / 192 69.4 / 59.0 / 56.0 / 54.7; 2560 -> 3840 at 96 rows in tiles of 48 / 96: 5.3 / 6.6.
+static int choose_nt(int m, int row_tiles, int k_blocks, int sms) {
+    auto block = [](int nt) { return nt <= 64 ? 250.0 : 240.0 + 1.3 * nt; };
+    int best_nt = 0;
+    double best = 0.0;
+    for (int nt = 16; nt <= kWide; nt += 16) {
+        const int full = m / nt, rest = m % nt;
+        const long long shorts = rest ? row_tiles : 0, tiles = static_cast<long long>(full) * row_tiles + shorts;
+        const long long whole = tiles / sms, left = tiles % sms;
+        const double part = full && rest ? (240.0 + 1.3 * rest) / block(nt) : 1.0, least = part < 1.0 ? part : 1.0;
+        double rounds = static_cast<double>(whole);
+        if (left > shorts) rounds += 1.0;
+        else if (left > 0 && 2 * left <= shorts && whole > 0) rounds += 2.0 * least > 1.0 ? 2.0 * least - 1.0 : 0.0;
+        else if (left > 0) rounds += least;
+        const double cost = rounds * (k_blocks * block(nt) + 300.0) + 35.0 * nt;
+        if (best_nt == 0 || cost < best) {
             best = cost;
             best_nt = nt;
         }
+        if (nt >= m) break;
     }
     return best_nt;
 }
@@ -582,13 +601,13 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
     const size_t kp = g.w[0]->kp;
     int row_tiles = 0;
     for (int i = 0; i < g.n; ++i) row_tiles += static_cast<int>((g.w[i]->rows + kBMW - 1) / kBMW);
-    const int nt = choose_nt(g.m, row_tiles, static_cast<int>(kp / kBK), ctx->sm_count);
+    const int nt = choose_nt(static_cast<int>(g.m), row_tiles, static_cast<int>(kp / kBK), ctx->sm_count);
     LBK_TRY(encode_act_map(&p.act, g.q, g.m, kp, nt));
     p.nt = nt;
     p.m = static_cast<int>(g.m);
     p.m_tiles = static_cast<int>((g.m + nt - 1) / nt);
     p.k_blocks = static_cast<int>(kp / kBK);
-    int tiles = 0;
+    row_tiles = 0;
     for (int i = 0; i < g.n; ++i) {
         const Weight *w = g.w[i];
         if (w->kp != kp) return fail(LBK_ERR_SHAPE, "inner dimension mismatch");
@@ -598,9 +617,10 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
         p.iout[i] = g.iout[i];
         p.wscale[i] = w->scale;
         p.rows[i] = static_cast<int>(w->rows);
-        tiles += p.m_tiles * static_cast<int>((w->rows + kBMW - 1) / kBMW);
-        p.tile_end[i] = tiles;
+        row_tiles += static_cast<int>((w->rows + kBMW - 1) / kBMW);
+        p.row_end[i] = row_tiles;
     }
+    const int tiles = row_tiles * p.m_tiles;
     p.n_mat = g.n;
     p.total_tiles = tiles;
     p.qscale = g.qscale;
@@ -653,9 +673,9 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     if (nt > 64) {
-        cfg.dynamicSmemBytes = Cfg<192>::kTotal + 1024;
-        if (p.scatter_world) LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<192, true>, p));
-        else LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<192, false>, p));
+        cfg.dynamicSmemBytes = Cfg<kWide>::kTotal + 1024;
+        if (p.scatter_world) LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<kWide, true>, p));
+        else LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<kWide, false>, p));
     } else {
         cfg.dynamicSmemBytes = Cfg<64>::kTotal + 1024;
         if (p.scatter_world) LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<64, true>, p));

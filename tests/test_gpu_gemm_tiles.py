@@ -1,0 +1,50 @@
+"""Prefill GEMM at the edges of its tiles: token rows around the narrow form's 64 and the wide form's 192, ragged last token tiles, K of one
+block to several packed-weight stages (last stages of one, two and three blocks, whose second half or whole is one set of expanders' or nobody's),
+row tiles of one to many, one to three matrices. Whole numbers: equality with the oracle. And launches close behind one another: the same rows every time."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def group(oracle, ctx, rows, cols, m, seed):
+    import torch
+    from lemonade_burn_b200 import ops
+    rng = np.random.default_rng(seed)
+    packed = [oracle.pack_matrix(rng.choice(np.array([-1, 0, 1], dtype=np.int8), size=(r, cols), p=[0.3, 0.4, 0.3])) for r in rows]
+    scales = [np.float32(50 + 3 * i) for i in range(len(rows))]
+    x = rng.standard_normal((m, cols)).astype(np.float32)
+    lins = [ops.TernaryLinear(torch.from_numpy(p).cuda(), float(s), cols, ctx) for p, s in zip(packed, scales)]
+    return packed, scales, x, torch.from_numpy(x).cuda(), lins
+
+
+@pytest.mark.parametrize("rows,cols", [([128], 128), ([300, 4], 640), ([256, 128, 77], 896), ([20000], 256)])
+@pytest.mark.parametrize("m", [17, 63, 64, 65, 95, 97, 192, 193, 400, 577])
+def test_tile_edges(oracle, ctx, rows, cols, m):
+    from lemonade_burn_b200 import ops
+    packed, scales, x, xd, lins = group(oracle, ctx, rows, cols, m, cols + m)
+    q, s, ssum = oracle.quantize_acts(x)
+    wf, wi = oracle.simd_gemm_multi(packed, scales, q, s, ssum, want_i32=True)
+    outs, iouts = ops.ternary_linear_multi(xd, lins, want_i32=True)
+    for got, goti, ef, ei in zip(outs, iouts, wf, wi):
+        assert np.array_equal(goti.cpu().numpy(), ei)
+        assert np.array_equal(got.cpu().numpy().view(np.uint32), ef.view(np.uint32))
+    outs = ops.ternary_linear_multi(xd, lins)  # without integer outputs K may be cut into parts
+    for got, ef in zip(outs, wf):
+        assert np.array_equal(got.cpu().numpy().view(np.uint32), ef.view(np.uint32))
+    ctx.check_device_error()
+
+
+@pytest.mark.parametrize("m", [333, 2011])
+def test_launches_behind_one_another_give_the_same_rows(oracle, ctx, m):
+    """Weights that are overwritten in the ring before they are read turn up as single rows of a tile, once in thousands: 2011 rows
+    of 2560 -> 2 x 6912, eight launches in a row with nothing between them, 40 times."""
+    import torch
+    from lemonade_burn_b200 import ops
+    _, _, _, xd, lins = group(oracle, ctx, [6912, 6912], 2560, m, 7)
+    want = [o.clone() for o in ops.ternary_linear_multi(xd, lins)]
+    for _ in range(40):
+        for outs in [ops.ternary_linear_multi(xd, lins) for _ in range(8)]:
+            for a, b in zip(outs, want):
+                assert torch.equal(a, b)
+    ctx.check_device_error()
