@@ -6,77 +6,79 @@
 // zero padded to padded_cols(k). The decode GEMV has its own fused copy of this; this
 // kernel feeds the prefill GEMM and the quantize_acts entry point.
 #include "lbk_internal.cuh"
+#include "lbk_ptx.cuh"
 
 namespace lbk {
 
 namespace {
-
-constexpr int kQThreads = 256;
 
 __device__ __forceinline__ int quant_one(float v, float scale) {
     int r = __float2int_rn(__fmul_rn(v, scale));  // NaN -> 0 like `NaN as i8` (quant.rs:115-118)
     return max(-128, min(127, r));
 }
 
+// One CTA of T threads per row. ROW: float4 a thread holds between the maximum and the rounding (rows of up to 4 T ROW values,
+// 16-byte aligned, are read once), 0: any row, read twice. A thread holds what the row needs and no more: with 8 for every row four
+// CTAs fit an SM instead of eight. Bound: HBM. 2048 rows of 2560 / 4096 / 6912: 8.4 -> 6.2, 9.8 -> 7.9, 12.1 -> 11.3 us (4.2 to 6.2 TB/s); of 14336, read
+// twice before, 35.1 -> 27.1 (5.4 TB/s). 512 threads for 6912 values took 13.7, 1024 18.3. It starts beside the end of the kernel in front (11 rows of 2560: 1.9 -> 1.6).
 // amax_in: per-row max|x| supplied by the caller (tensor-parallel: the maximum over all ranks'
 // column slices), or null to compute it here. amax_out: when non-null only the row maximum is
 // written and nothing is quantised.
-__global__ void __launch_bounds__(kQThreads) quantize_kernel(const float *__restrict__ x, int k,
+template <int T, int ROW>
+__global__ void __launch_bounds__(T) quantize_kernel(const float *x, int k,
                                                             int kp, int8_t *__restrict__ q,
                                                             float *__restrict__ scale,
                                                             int32_t *__restrict__ sum,
-                                                            const float *__restrict__ amax_in,
+                                                            const float *amax_in,
                                                             float *__restrict__ amax_out) {
-    __shared__ float s_f[kQThreads / 32];
-    __shared__ int s_i[kQThreads / 32];
+    __shared__ float s_f[T / 32];
+    __shared__ int s_i[T / 32];
     __shared__ float s_scale;
     // A kernel launched behind this one with programmatic stream serialisation (the prefill GEMM)
     // may start its prologue now; it waits for this grid's results with griddepcontrol.wait.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    ptx::pdl_trigger();
+    ptx::pdl_wait();  // x may come from the kernel in front, and the rows of codes may still be read by it
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float *xr = x + static_cast<size_t>(row) * k;
     int8_t *qr = q + static_cast<size_t>(row) * kp;
     const bool vec = (k & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
 
-    // Rows of up to kRowCache float4 per thread are read once and kept in registers between the
-    // maximum and the rounding (prefill feeds this kernel 2048 rows of 2560..6912 floats).
-    constexpr int kRowCache = 8;
-    float4 cache[kRowCache];
+    constexpr bool cached = ROW != 0;
+    float4 cache[cached ? ROW : 1];
     const int n4 = k >> 2;
-    const bool cached = vec && n4 <= kRowCache * kQThreads;
     float am = 0.0f;  // fmaxf drops a NaN operand, as f32::max does (quant.rs:101-104)
-    if (cached) {
+    if constexpr (cached) {
         const float4 *x4 = reinterpret_cast<const float4 *>(xr);
 #pragma unroll
-        for (int j = 0; j < kRowCache; ++j) {
-            const int i = tid + j * kQThreads;
-            cache[j] = i < n4 ? __ldg(x4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < ROW; ++j) {
+            const int i = tid + j * T;
+            cache[j] = i < n4 ? __ldcg(x4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if (amax_in == nullptr) {
 #pragma unroll
-            for (int j = 0; j < kRowCache; ++j)
+            for (int j = 0; j < ROW; ++j)
                 am = fmaxf(am, fmaxf(fmaxf(fabsf(cache[j].x), fabsf(cache[j].y)), fmaxf(fabsf(cache[j].z), fabsf(cache[j].w))));
         }
     }
     if (amax_in != nullptr) {
-        am = amax_in[row];
+        am = __ldcg(amax_in + row);
     } else if (cached) {
         // done above
     } else if (vec) {
         const float4 *x4 = reinterpret_cast<const float4 *>(xr);
-        for (int i = tid; i < (k >> 2); i += kQThreads) {
-            float4 v = __ldg(x4 + i);
+        for (int i = tid; i < (k >> 2); i += T) {
+            float4 v = __ldcg(x4 + i);
             am = fmaxf(am, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
         }
     } else {
-        for (int i = tid; i < k; i += kQThreads) am = fmaxf(am, fabsf(__ldg(xr + i)));
+        for (int i = tid; i < k; i += T) am = fmaxf(am, fabsf(__ldcg(xr + i)));
     }
     for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
     if (lane == 0) s_f[warp] = am;
     __syncthreads();
     if (tid == 0) {
         float a = 0.0f;
-        for (int w = 0; w < kQThreads / 32; ++w) a = fmaxf(a, s_f[w]);
+        for (int w = 0; w < T / 32; ++w) a = fmaxf(a, s_f[w]);
         if (amax_out != nullptr) amax_out[row] = a;
         s_scale = __fdiv_rn(127.0f, fmaxf(a, 1e-5f));
     }
@@ -84,10 +86,10 @@ __global__ void __launch_bounds__(kQThreads) quantize_kernel(const float *__rest
     if (amax_out != nullptr) return;
     const float sc = s_scale;
     int acc = 0;
-    if (cached) {
+    if constexpr (cached) {
 #pragma unroll
-        for (int j = 0; j < kRowCache; ++j) {
-            const int i = (tid + j * kQThreads) * 4;
+        for (int j = 0; j < ROW; ++j) {
+            const int i = (tid + j * T) * 4;
             if (i < kp) {  // columns past k hold zeros, which quantise to zero
                 const int q0 = quant_one(cache[j].x, sc), q1 = quant_one(cache[j].y, sc);
                 const int q2 = quant_one(cache[j].z, sc), q3 = quant_one(cache[j].w, sc);
@@ -96,19 +98,19 @@ __global__ void __launch_bounds__(kQThreads) quantize_kernel(const float *__rest
                                                         (static_cast<uint32_t>(q3 & 255) << 24);
             }
         }
-        for (int i = (tid + kRowCache * kQThreads) * 4; i < kp; i += kQThreads * 4) *reinterpret_cast<uint32_t *>(qr + i) = 0u;
+        for (int i = (tid + ROW * T) * 4; i < kp; i += T * 4) *reinterpret_cast<uint32_t *>(qr + i) = 0u;
     } else
-    for (int i = tid * 4; i < kp; i += kQThreads * 4) {
+    for (int i = tid * 4; i < kp; i += T * 4) {
         int q0 = 0, q1 = 0, q2 = 0, q3 = 0;
         if (vec && i + 3 < k) {
-            float4 v = __ldg(reinterpret_cast<const float4 *>(xr + i));
+            float4 v = __ldcg(reinterpret_cast<const float4 *>(xr + i));
             q0 = quant_one(v.x, sc); q1 = quant_one(v.y, sc);
             q2 = quant_one(v.z, sc); q3 = quant_one(v.w, sc);
         } else {
-            if (i < k) q0 = quant_one(__ldg(xr + i), sc);
-            if (i + 1 < k) q1 = quant_one(__ldg(xr + i + 1), sc);
-            if (i + 2 < k) q2 = quant_one(__ldg(xr + i + 2), sc);
-            if (i + 3 < k) q3 = quant_one(__ldg(xr + i + 3), sc);
+            if (i < k) q0 = quant_one(__ldcg(xr + i), sc);
+            if (i + 1 < k) q1 = quant_one(__ldcg(xr + i + 1), sc);
+            if (i + 2 < k) q2 = quant_one(__ldcg(xr + i + 2), sc);
+            if (i + 3 < k) q3 = quant_one(__ldcg(xr + i + 3), sc);
         }
         acc += q0 + q1 + q2 + q3;
         *reinterpret_cast<uint32_t *>(qr + i) = (q0 & 255) | ((q1 & 255) << 8) | ((q2 & 255) << 16) |
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(kQThreads) quantize_kernel(const float *__rest
     __syncthreads();
     if (tid == 0) {
         int s = 0;
-        for (int w = 0; w < kQThreads / 32; ++w) s += s_i[w];
+        for (int w = 0; w < T / 32; ++w) s += s_i[w];
         scale[row] = sc;
         sum[row] = s;
     }
@@ -199,9 +201,15 @@ int launch_scale_epilogue(Ctx *ctx, const int32_t *dots, const float *ascale, fl
 int launch_quantize_ex(Ctx *ctx, const float *x, size_t m, size_t k, int8_t *q, float *scale, int32_t *sum,
                        const float *amax_in, float *amax_out, cudaStream_t stream) {
     if (m == 0) return LBK_OK;
-    const size_t kp = lbk_padded_cols(k);
-    quantize_kernel<<<static_cast<unsigned>(m), kQThreads, 0, stream>>>(x, static_cast<int>(k), static_cast<int>(kp), q,
-                                                                        scale, sum, amax_in, amax_out);
+    const size_t kp = lbk_padded_cols(k), n4 = k / 4;
+    const bool vec = k % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    void (*kernel)(const float *, int, int, int8_t *, float *, int32_t *, const float *, float *) = quantize_kernel<256, 0>;
+    unsigned threads = 256;
+    if (vec && n4 <= 3 * 256) kernel = quantize_kernel<256, 3>;
+    else if (vec && n4 <= 4 * 256) kernel = quantize_kernel<256, 4>;
+    else if (vec && n4 <= 7 * 256) kernel = quantize_kernel<256, 7>;
+    else if (vec && n4 <= 8 * 512) kernel = quantize_kernel<512, 8>, threads = 512;
+    LBK_CUDA(launch_chained(kernel, dim3(static_cast<unsigned>(m)), dim3(threads), 0, stream, x, static_cast<int>(k), static_cast<int>(kp), q, scale, sum, amax_in, amax_out));
     LBK_CUDA(cudaGetLastError());
     ctx->launches++;
     return LBK_OK;
@@ -209,13 +217,7 @@ int launch_quantize_ex(Ctx *ctx, const float *x, size_t m, size_t k, int8_t *q, 
 
 int launch_quantize(Ctx *ctx, const float *x, size_t m, size_t k, int8_t *q, float *scale,
                     int32_t *sum, cudaStream_t stream) {
-    if (m == 0) return LBK_OK;
-    const size_t kp = lbk_padded_cols(k);
-    quantize_kernel<<<static_cast<unsigned>(m), kQThreads, 0, stream>>>(
-        x, static_cast<int>(k), static_cast<int>(kp), q, scale, sum, nullptr, nullptr);
-    LBK_CUDA(cudaGetLastError());
-    ctx->launches++;
-    return LBK_OK;
+    return launch_quantize_ex(ctx, x, m, k, q, scale, sum, nullptr, nullptr, stream);
 }
 
 }  // namespace lbk
