@@ -136,15 +136,6 @@ __device__ __forceinline__ void umma_i8_ts_block(uint32_t d_tmem, uint32_t a_tme
         "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate_first)
         : "memory");
 }
-// A wait of a whole warp, with one outcome for all its lanes (what follows needs them together)
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag));
-}
-__device__ __forceinline__ bool elect_one() {  // one lane of a converged warp
-    uint32_t one;
-    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-    return one != 0;
-}
 // SC: matrix 0's int32 dots go to the token owners' buffers (GemmParams::scatter) instead of iout: an instantiation of its
 // own, so that the ordinary kernel's epilogue keeps its registers
 template <int NT, bool SC>
@@ -330,8 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         }
     } else if (warp == kMmaWarp) {
         // ================= MMA issuer =================
-        // The whole warp walks and waits, one elected lane issues. Under a branch of one lane a turn of a wait and four MMAs took
-        // 504 cycles whatever N (the MMAs of N = 192 take 384); so it takes 384, and four blocks of N = 64 in a turn 172 a block instead of 264.
+        // The whole warp walks and waits, one elected lane issues.
         int tcount = 0, sp = 0, as = 0;
         uint32_t full_phase = 0;
         const uint64_t bdesc0 = smem_desc_sw128(base);  // activation block stage 0; stage s adds s * kActBytes / 16

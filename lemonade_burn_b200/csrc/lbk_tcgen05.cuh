@@ -96,6 +96,17 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
     return false;
 }
 
+// A wait of a whole warp, with one outcome for all its lanes, and the lane that issues. MMAs issued under a branch of one lane, which waits for
+// barriers in between, take 504 cycles a turn of a wait, four MMAs and a commit whatever their N (kind::i8, N = 192: 384 cycles of products); when the whole
+// warp walks and one elected lane issues, 384, and four such blocks of N = 64 in a turn 172 a block instead of 264.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag));
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
 
 }  // namespace tc
 }  // namespace lbk
