@@ -430,6 +430,10 @@ size_t attn_window_splits(size_t cap, const AttnMask &mask) {
 }
 size_t attn_window_scratch(size_t b, size_t heads, size_t vdimp, size_t splits) { return b * heads * splits * (vdimp + 4); }
 
+bool attn_window_tiled(const AttnCall &c) {
+    return c.compute == LBK_COMPUTE_BF16 && c.rows_of_seq >= 0 && c.n >= kTcMinRows && c.dimp <= 128 && c.vdimp <= 128;
+}
+
 int launch_attn_window(Ctx *ctx, const AttnCall &c, cudaStream_t st) {
     if (c.n == 0) return LBK_OK;
     if (!c.q || !c.kc || !c.vc || !c.pos || !c.out) return fail(LBK_ERR_INVALID, "windowed attention: null buffer");
@@ -462,7 +466,7 @@ int launch_attn_window(Ctx *ctx, const AttnCall &c, cudaStream_t st) {
     if (c.compute == LBK_COMPUTE_F32) return launch_generic<float>(ctx, p, st);
     const size_t dmax = c.dimp > c.vdimp ? c.dimp : c.vdimp;
     if (c.rows_of_seq >= 0) {
-        if (c.n >= kTcMinRows && dmax <= 128) return launch_attn_window_tc(ctx, c, st);
+        if (attn_window_tiled(c)) return launch_attn_window_tc(ctx, c, st);
         return launch_generic<uint16_t>(ctx, p, st);
     }
     if (dmax > 256) return launch_generic<uint16_t>(ctx, p, st);

@@ -36,7 +36,7 @@ struct BitNetModel : Model {
     int make_cache(size_t batch, size_t capacity, std::unique_ptr<Cache> &out) override;
     int make_prefill_buffers(Cache *c, size_t rows) override;
     int enqueue_step(Cache *c, cudaStream_t st) override;
-    int enqueue_rows(Cache *c, size_t seq, size_t n, cudaStream_t st) override;
+    int enqueue_rows(Cache *c, size_t seq, size_t n, size_t first, cudaStream_t st) override;
     int enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) override {
         return lbk_bf16_linear(reinterpret_cast<lbk_ctx *>(ctx), rows, n, embed, cfg.vocab_size, cfg.hidden_size, logits, st);
     }
@@ -210,7 +210,7 @@ int BitNetModel::make_prefill_buffers(Cache *cache, size_t rows) {
 
 // `n` consecutive tokens of sequence `seq` of the cache in one pass: the projections see n token rows (the
 // tcgen05 GEMM above 16 rows), attention is causal over the cache (model.rs:305-374 with m = n).
-int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, cudaStream_t st) {
+int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, size_t first, cudaStream_t st) {
     BitNetModel *m = this;
     BitNetCache *c = static_cast<BitNetCache *>(cache);
     lbk_ctx *h = reinterpret_cast<lbk_ctx *>(ctx);
@@ -218,16 +218,18 @@ int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, cudaStream_t s
                  L = cfg.num_hidden_layers;
     const float eps = cfg.rms_norm_eps;
     const bool fused_h = H % 4 == 0 && H <= 8192, fused_i = I % 4 == 0 && I <= 8192;
+    size_t kept = 0;  // rows in front of which the last layer's are left out; `n` counts those that are worked on
     auto add_norm = [&](float *x, const float *y, const float *w) -> int {  // x += y; pf_n = rms_norm(x) * w
-        if (fused_h) return lbk_add_rms_norm(h, x, y, w, n, H, eps, c->pf_n, st);
+        if (fused_h) return lbk_add_rms_norm(h, x, y, w, n, H, eps, c->pf_n + kept * H, st);
         LBK_TRY(lbk_add_inplace(h, x, y, n * H, st));
-        return lbk_rms_norm(h, x, w, n, H, eps, c->pf_n, st);
+        return lbk_rms_norm(h, x, w, n, H, eps, c->pf_n + kept * H, st);
     };
     const size_t layer_kv = c->b * kvh * c->cap * hd;
     // From 9 rows on every projection takes the GEMM path, whose input is the quantised rows: the norm
     // in front of a projection then writes those directly (lbk_norm_quant) and the f32 copy of the
     // normalised rows, with the quantise kernel that would read it back, goes away. Same bits.
-    const bool nq = n >= 9 && lbk_norm_quant_supported(H) && lbk_norm_quant_supported(I) && lbk_norm_quant_supported(nh * hd);
+    const bool can_nq = lbk_norm_quant_supported(H) && lbk_norm_quant_supported(I) && lbk_norm_quant_supported(nh * hd);
+    bool nq = n >= 9 && can_nq;
     auto norm_q = [&](int pre, float *x, const float *y, const float *w, size_t width) -> int {
         return lbk_norm_quant(h, pre, x, y, w, n, width, eps, c->pf_q8, c->pf_qscale, c->pf_qsum, st);
     };
@@ -245,17 +247,35 @@ int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, cudaStream_t s
         LBK_TRY(project(c->pf_n, qkv, 3, qkv_out));
         uint16_t *kc = c->k + li * layer_kv, *vc = c->v + li * layer_kv;
         LBK_TRY(lbk_rope_kv_append_rows(h, c->pf_q, c->pf_k, c->pf_v, m->cos, m->sin, c->pos + seq, n, nh, kvh, hd, c->cap, seq, kc, vc, st));
-        LBK_TRY(lbk_attn_prefill(h, c->pf_q, kc, vc, c->pos + seq, n, nh, kvh, hd, c->cap, seq, c->pf_attn, st));
-        if (nq) LBK_TRY(norm_q(LBK_PRE_RMS, c->pf_attn, nullptr, l.attn_sub_norm, nh * hd));
-        else LBK_TRY(lbk_rms_norm(h, c->pf_attn, l.attn_sub_norm, n, nh * hd, eps, c->pf_attn, st));
+        float *x = c->pf_x, *attn = c->pf_attn;
+        if (li + 1 == L && first > 0) {
+            if (first == n) return LBK_OK;
+            // attention of the 128-row tiles that hold wanted rows (the same tiles, the same bits), everything behind it for the wanted rows
+            const size_t left = n >= 64 && hd == 128 && nh <= 8 * kvh ? first / 128 * 128 : 0;
+            if (left > 0) {
+                LBK_TRY(later_rows(c, seq, left, st));
+                LBK_TRY(launch_attn_prompt_tc(ctx, c->pf_q + left * nh * hd, kc, vc, c->pos_first, n - left, nh, kvh, c->cap, seq, c->pf_attn + left * nh * hd, st));
+            } else {
+                LBK_TRY(lbk_attn_prefill(h, c->pf_q, kc, vc, c->pos + seq, n, nh, kvh, hd, c->cap, seq, c->pf_attn, st));
+            }
+            kept = first;
+            n -= first;
+            nq = n >= 9 && can_nq;
+            x += first * H;
+            attn += first * nh * hd;
+        } else {
+            LBK_TRY(lbk_attn_prefill(h, c->pf_q, kc, vc, c->pos + seq, n, nh, kvh, hd, c->cap, seq, c->pf_attn, st));
+        }
+        if (nq) LBK_TRY(norm_q(LBK_PRE_RMS, attn, nullptr, l.attn_sub_norm, nh * hd));
+        else LBK_TRY(lbk_rms_norm(h, attn, l.attn_sub_norm, n, nh * hd, eps, attn, st));
         const lbk_weight *ow[1] = {l.o};
         float *oo[1] = {c->pf_o};
-        LBK_TRY(project(c->pf_attn, ow, 1, oo));
-        if (nq) LBK_TRY(norm_q(LBK_PRE_ADD_RMS, c->pf_x, c->pf_o, l.post_attn_norm, H));
-        else LBK_TRY(add_norm(c->pf_x, c->pf_o, l.post_attn_norm));
+        LBK_TRY(project(attn, ow, 1, oo));
+        if (nq) LBK_TRY(norm_q(LBK_PRE_ADD_RMS, x, c->pf_o, l.post_attn_norm, H));
+        else LBK_TRY(add_norm(x, c->pf_o, l.post_attn_norm));
         const lbk_weight *gu[2] = {l.gate, l.up};
         float *guo[2] = {c->pf_g, c->pf_u};
-        LBK_TRY(project(c->pf_n, gu, 2, guo));
+        LBK_TRY(project(c->pf_n + kept * H, gu, 2, guo));
         if (nq) {
             LBK_TRY(norm_q(LBK_PRE_RELU2_MUL_RMS, c->pf_g, c->pf_u, l.ffn_sub_norm, I));
         } else if (fused_i) {
@@ -267,10 +287,10 @@ int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, cudaStream_t s
         const lbk_weight *dw[1] = {l.down};
         float *dout[1] = {c->pf_d};
         LBK_TRY(project(c->pf_act, dw, 1, dout));
-        if (nq && li + 1 < L) LBK_TRY(norm_q(LBK_PRE_ADD_RMS, c->pf_x, c->pf_d, m->layers[li + 1].input_norm, H));
-        else LBK_TRY(add_norm(c->pf_x, c->pf_d, li + 1 < L ? m->layers[li + 1].input_norm : m->final_norm));
+        if (nq && li + 1 < L) LBK_TRY(norm_q(LBK_PRE_ADD_RMS, x, c->pf_d, m->layers[li + 1].input_norm, H));
+        else LBK_TRY(add_norm(x, c->pf_d, li + 1 < L ? m->layers[li + 1].input_norm : m->final_norm));
     }
-    return LBK_OK;  // pf_n holds the final norm of every row
+    return LBK_OK;  // pf_n holds the final norm of every wanted row
 }
 
 int BitNetModel::make_cache(size_t batch, size_t capacity, std::unique_ptr<Cache> &out) {

@@ -102,6 +102,7 @@ struct AttnCall {
 size_t attn_window_scratch(size_t b, size_t heads, size_t vdimp, size_t splits);
 size_t attn_window_splits(size_t cap, const AttnMask &mask);
 int launch_attn_window(Ctx *ctx, const AttnCall &c, cudaStream_t st);
+bool attn_window_tiled(const AttnCall &c);  // the call goes to the tcgen05 form, 128 rows a tile
 // the tcgen05 form of it for prompt rows (lbk_attn_tc.cu); bf16, dim and vdim at most 128 (with k2: three pieces of 64)
 int launch_attn_window_tc(Ctx *ctx, const AttnCall &c, cudaStream_t st);
 

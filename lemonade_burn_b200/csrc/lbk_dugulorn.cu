@@ -72,12 +72,12 @@ struct DugulornModel : Model {
     int make_cache(size_t batch, size_t capacity, std::unique_ptr<Cache> &out) override;
     int make_prefill_buffers(Cache *c, size_t rows) override;
     int enqueue_step(Cache *c, cudaStream_t st) override;
-    int enqueue_rows(Cache *c, size_t seq, size_t n, cudaStream_t st) override;
+    int enqueue_rows(Cache *c, size_t seq, size_t n, size_t first, cudaStream_t st) override;
     int enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) override;
     struct Work;
     struct Pass;
     int make_work(std::vector<void *> &owner, Work &w, size_t rows, bool batch, size_t cap);
-    int enqueue_tokens(DugulornCache *c, Work &w, const int32_t *tokens, size_t m, int seq, float *final_rows, cudaStream_t st);
+    int enqueue_tokens(DugulornCache *c, Work &w, const int32_t *tokens, size_t m, size_t first, int seq, float *final_rows, cudaStream_t st);
     int enqueue_latent(const Pass &p, const DugulornLayer &l);
     int enqueue_recurrent(const Pass &p, const DugulornLayer &l, size_t li);
 };
@@ -117,7 +117,8 @@ struct DugulornModel::Pass {
     Work &w;
     size_t m;
     int seq;
-    const int *pos;
+    const int *pos;   // of row 0
+    size_t length;    // positions of the sequence behind the last row
     cudaStream_t st;
 };
 
@@ -273,7 +274,7 @@ int DugulornModel::enqueue_latent(const Pass &p, const DugulornLayer &l) {
     a.out = w.mid;
     a.ldo = static_cast<long>(l.o.pitch);
     if (p.seq >= 0 && expands(p.m)) {
-        a.length = p.c->lens[static_cast<size_t>(p.seq)] + p.m;
+        a.length = p.length;
         a.ek = p.c->ek;
         a.ev = p.c->ev;
         a.ecap = p.c->ecap;
@@ -374,10 +375,10 @@ int DugulornModel::enqueue_recurrent(const Pass &p, const DugulornLayer &l, size
 }
 
 // `m` tokens through all layers: consecutive positions of sequence `seq`, or (seq < 0) one token of each sequence.
-int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *tokens, size_t m, int seq, float *final_rows, cudaStream_t st) {
-    const bool fuse = compute == LBK_COMPUTE_BF16 && dense_pre_supported(m, width);  // sums and norms run inside the projection behind them
+int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *tokens, size_t m, size_t first, int seq, float *final_rows, cudaStream_t st) {
+    bool fuse = compute == LBK_COMPUTE_BF16 && dense_pre_supported(m, width);  // sums and norms run inside the projection behind them
     const long npitch = static_cast<long>(dense_pitch(width));
-    const Pass pass{c, w, m, seq, c->pos + (seq >= 0 ? seq : 0), st};
+    Pass pass{c, w, m, seq, c->pos + (seq >= 0 ? seq : 0), seq >= 0 ? c->lens[static_cast<size_t>(seq)] + m : 0, st};
     LBK_TRY(lbk_embed_bf16(reinterpret_cast<lbk_ctx *>(ctx), embed, tokens, m, width, w.x, st));
     float *x = w.x, *x2 = w.x2;
     // what the last sublayer still owes the residual: its output rows and the norm in front of the sum
@@ -438,8 +439,32 @@ int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *toke
     };
 
     LBK_TRY(norm_rows(embed_norm, w.n, x));
+    // the rows from number `by` on alone are worked on from here
+    auto leave_out = [&](size_t by) {
+        x += by * width;
+        if (y) y += by * width;
+        final_rows += by * width;
+        m -= by;
+        first -= by;
+        fuse = compute == LBK_COMPUTE_BF16 && dense_pre_supported(m, width);
+    };
     for (size_t li = 0; li < layers.size(); ++li) {
         const DugulornLayer &l = layers[li];
+        const char *mid = static_cast<const char *>(w.mid);
+        const bool last = li + 1 == layers.size() && first > 0;
+        if (last && l.type == Mixer::Latent && !l.own) {
+            // nothing of this layer is kept: only the rows of the 128-row tiles that hold wanted rows go through it
+            if (first == m) return LBK_OK;
+            size_t left = first / 128 * 128;
+            if (left > 0 && expands(m) && !expands(m - left)) left -= 128;  // the same form
+            if (left > 0) {
+                LBK_TRY(later_rows(c, static_cast<size_t>(seq), left, st));
+                leave_out(left);
+                pass.m = m;
+                pass.pos = c->pos_first;
+                if (!y) LBK_TRY(norm_rows(nullptr, w.n, nullptr));  // the rows as the projection reads them, from the front
+            }
+        }
         DenseCall d;
         d.w = l.in;
         d.out_rows = l.in.rows;
@@ -464,7 +489,12 @@ int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *toke
             LBK_TRY(project(d));
             LBK_TRY(enqueue_recurrent(pass, l, li));
         }
-        LBK_TRY(leave(w.mid, l.o, nullptr, l.norm1));
+        if (last && first > 0) {
+            if (first == m) return LBK_OK;
+            mid += first * l.o.pitch * elem();
+            leave_out(first);
+        }
+        LBK_TRY(leave(mid, l.o, nullptr, l.norm1));
         if (l.ff) {
             DenseCall u;
             u.w = l.up;
@@ -483,14 +513,14 @@ int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *toke
 
 int DugulornModel::enqueue_step(Cache *cache, cudaStream_t st) {
     DugulornCache *c = static_cast<DugulornCache *>(cache);
-    LBK_TRY(enqueue_tokens(c, c->step_work, c->tokens, c->b, -1, c->final_rows, st));
+    LBK_TRY(enqueue_tokens(c, c->step_work, c->tokens, c->b, 0, -1, c->final_rows, st));
     return enqueue_head(c->final_rows, c->b, c->logits, st);
 }
 
-int DugulornModel::enqueue_rows(Cache *cache, size_t seq, size_t n, cudaStream_t st) {
+int DugulornModel::enqueue_rows(Cache *cache, size_t seq, size_t n, size_t first, cudaStream_t st) {
     DugulornCache *c = static_cast<DugulornCache *>(cache);
     if (expands(n)) LBK_TRY(c->expand_room(this, c->lens[seq] + n));
-    return enqueue_tokens(c, c->rows_work, c->pf_tokens, n, static_cast<int>(seq), c->pf_n, st);
+    return enqueue_tokens(c, c->rows_work, c->pf_tokens, n, first, static_cast<int>(seq), c->pf_n, st);
 }
 
 int DugulornModel::enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) {

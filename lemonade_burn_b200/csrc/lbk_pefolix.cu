@@ -48,11 +48,11 @@ struct PefolixModel : Model {
     int make_cache(size_t batch, size_t capacity, std::unique_ptr<Cache> &out) override;
     int make_prefill_buffers(Cache *c, size_t rows) override;
     int enqueue_step(Cache *c, cudaStream_t st) override;
-    int enqueue_rows(Cache *c, size_t seq, size_t n, cudaStream_t st) override;
+    int enqueue_rows(Cache *c, size_t seq, size_t n, size_t first, cudaStream_t st) override;
     int enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) override;
     struct Work;
     int make_work(std::vector<void *> &owner, Work &w, size_t rows, size_t decode_b, size_t cap);
-    int enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens, size_t m, int seq, float *final_rows, cudaStream_t st);
+    int enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens, size_t m, size_t first, int seq, float *final_rows, cudaStream_t st);
 };
 
 // Buffers of one pass over `rows` tokens, sized for the largest layer. Rows of the compute type have a pitch of a
@@ -136,10 +136,10 @@ int PefolixModel::make_prefill_buffers(Cache *cache, size_t rows) {
 }
 
 // `m` tokens through all layers: consecutive positions of sequence `seq`, or (seq < 0) one token of each sequence.
-int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens, size_t m, int seq, float *final_rows, cudaStream_t st) {
+int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens, size_t m, size_t first, int seq, float *final_rows, cudaStream_t st) {
     const bool f32 = compute == LBK_COMPUTE_F32;
-    const bool few = m <= LBK_GEMV_MAX_M && !f32;
-    const bool fuse = !f32 && dense_pre_supported(m, width);  // the norms run inside the projection behind them
+    bool few = m <= LBK_GEMV_MAX_M && !f32;
+    bool fuse = !f32 && dense_pre_supported(m, width);  // the norms run inside the projection behind them
     const long npitch = static_cast<long>(dense_pitch(width));
     const int *pos = c->pos + (seq >= 0 ? seq : 0);
     LBK_TRY(lbk_embed_bf16(reinterpret_cast<lbk_ctx *>(ctx), embed, tokens, m, width, w.x, st));
@@ -207,6 +207,7 @@ int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens
 
     for (size_t li = 0; li < layers.size(); ++li) {
         const PefolixLayer &l = layers[li];
+        const char *attn = static_cast<const char *>(w.attn);
         {
             DenseCall d;
             d.w = l.qkv;
@@ -250,9 +251,31 @@ int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens
             a.scratch = w.scratch;
             a.out = w.attn;
             a.ldo = static_cast<long>(l.o.pitch);
-            LBK_TRY(launch_attn_window(ctx, a, st));
+            if (li + 1 < layers.size() || first == 0) {
+                LBK_TRY(launch_attn_window(ctx, a, st));
+            } else {
+                if (first == m) return LBK_OK;
+                // attention of the 128-row tiles that hold wanted rows, everything behind it for the wanted rows
+                const size_t left = attn_window_tiled(a) ? first / 128 * 128 : 0;
+                if (left > 0) {
+                    LBK_TRY(later_rows(c, static_cast<size_t>(seq), left, st));
+                    a.pos = c->pos_first;
+                    a.n = m - left;
+                    a.q = static_cast<const char *>(a.q) + left * l.heads * l.dimp * elem();
+                    a.out = static_cast<char *>(a.out) + left * l.o.pitch * elem();
+                    LBK_TRY(launch_attn_window_tc(ctx, a, st));
+                } else {
+                    LBK_TRY(launch_attn_window(ctx, a, st));
+                }
+                attn += first * l.o.pitch * elem();
+                x += first * width;
+                final_rows += first * width;
+                m -= first;
+                few = m <= LBK_GEMV_MAX_M && !f32;
+                fuse = !f32 && dense_pre_supported(m, width);
+            }
         }
-        LBK_TRY(rows_f32(w.attn, l.o, w.y));
+        LBK_TRY(rows_f32(attn, l.o, w.y));
         y = w.y;
         w_post = l.norm1b;
         if (l.kind == PefolixLayer::Dense) {
@@ -350,13 +373,13 @@ int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens
 
 int PefolixModel::enqueue_step(Cache *cache, cudaStream_t st) {
     PefolixCache *c = static_cast<PefolixCache *>(cache);
-    LBK_TRY(enqueue_tokens(c, c->step_work, c->tokens, c->b, -1, c->final_rows, st));
+    LBK_TRY(enqueue_tokens(c, c->step_work, c->tokens, c->b, 0, -1, c->final_rows, st));
     return enqueue_head(c->final_rows, c->b, c->logits, st);
 }
 
-int PefolixModel::enqueue_rows(Cache *cache, size_t seq, size_t n, cudaStream_t st) {
+int PefolixModel::enqueue_rows(Cache *cache, size_t seq, size_t n, size_t first, cudaStream_t st) {
     PefolixCache *c = static_cast<PefolixCache *>(cache);
-    return enqueue_tokens(c, c->rows_work, c->pf_tokens, n, static_cast<int>(seq), c->pf_n, st);
+    return enqueue_tokens(c, c->rows_work, c->pf_tokens, n, first, static_cast<int>(seq), c->pf_n, st);
 }
 
 int PefolixModel::enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) {

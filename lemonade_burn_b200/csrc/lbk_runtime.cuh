@@ -351,6 +351,7 @@ struct Cache {
     Model *model = nullptr;
     size_t b = 0, cap = 0;
     int32_t *pos = nullptr;               // [b] length of every sequence, on the device
+    int32_t *pos_first = nullptr;         // the position of the first row a last layer works on (later_rows)
     int32_t *active = nullptr;            // [b] 1: the sequence takes part in the step (its position advances)
     std::vector<size_t> lens;             // the lengths again, on the host
     int32_t *tokens = nullptr, *next = nullptr;
@@ -382,11 +383,15 @@ struct Model {
     virtual int make_prefill_buffers(Cache *c, size_t rows) = 0;
     // one token per sequence: c->tokens at c->pos -> c->logits (positions not advanced)
     virtual int enqueue_step(Cache *c, cudaStream_t st) = 0;
-    // c->pf_tokens[0 .. n) of sequence `seq` at its position -> c->pf_n (position not advanced)
-    virtual int enqueue_rows(Cache *c, size_t seq, size_t n, cudaStream_t st) = 0;
+    // c->pf_tokens[0 .. n) of sequence `seq` at its position -> rows first .. n - 1 of c->pf_n (position not advanced). Of the rows in front of
+    // `first` (at most n) the last layer has to leave what later tokens read, and no more.
+    virtual int enqueue_rows(Cache *c, size_t seq, size_t n, size_t first, cudaStream_t st) = 0;
     // rows of the final norm -> logits
     virtual int enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) = 0;
 };
+
+// c->pos_first = position of sequence `seq` + by
+int later_rows(Cache *c, size_t seq, size_t by, cudaStream_t st);
 
 // A family's loader: `config` is the parsed config.json of `dir`.
 using LoadFn = int (*)(Ctx *ctx, const std::string &dir, const Json &config, int compute, int rank, int world, std::unique_ptr<Model> &out);
