@@ -294,6 +294,11 @@ int lbk_ternary_gemm_dev(lbk_ctx *ctx, const lbk_weight *const *ws, size_t n, co
                          const float *scale_dev, const int32_t *sum_dev, size_t m,
                          float *const *outs_dev, int32_t *const *iouts_dev, void *stream);
 
+/* The feed-forward's first half on quantised rows (model.rs:361-363): out f32 [m][rows] = relu(gate)^2 * up, the bits of
+ * lbk_ternary_gemm_dev on both followed by lbk_relu2_mul. */
+int lbk_ternary_relu2_gemm_dev(lbk_ctx *ctx, const lbk_weight *gate, const lbk_weight *up, const int8_t *q_dev, const float *scale_dev,
+                               const int32_t *sum_dev, size_t m, float *out_dev, void *stream);
+
 /* bf16_linear (crates/lb-model/src/ops.rs:199-218): x f32 [m, cols] @ W^T, W bf16
  * [rows, cols] -> out f32 [m, rows], all device memory. */
 int lbk_bf16_linear(lbk_ctx *ctx, const float *x_dev, size_t m, const uint16_t *w_dev, size_t rows,

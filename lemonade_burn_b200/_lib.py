@@ -51,6 +51,7 @@ SYMBOLS = [
     ("lbk_quantize_acts_amax_dev", _i, [_vp, _vp, _sz, _sz, _vp, _vp, _vp, _vp, _vp]),
     ("lbk_scale_epilogue_dev", _i, [_vp, _vp, _vp, _f, _sz, _sz, _vp, _vp]),
     ("lbk_ternary_gemm_dev", _i, [_vp, _pp, _sz, _vp, _vp, _vp, _sz, _pp, _pp, _vp]),
+    ("lbk_ternary_relu2_gemm_dev", _i, [_vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
     ("lbk_bf16_linear", _i, [_vp, _vp, _sz, _vp, _sz, _sz, _vp, _vp]),
     ("lbk_embed_bf16", _i, [_vp, _vp, _vp, _sz, _sz, _vp, _vp]),
     ("lbk_rms_norm", _i, [_vp, _vp, _vp, _sz, _sz, _f, _vp, _vp]),

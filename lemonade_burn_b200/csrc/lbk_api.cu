@@ -320,6 +320,29 @@ int lbk_ternary_gemm_dev(lbk_ctx *c, const lbk_weight *const *ws, size_t n, cons
     return run_group(ctx, g, static_cast<cudaStream_t>(stream), nullptr, nullptr, nullptr);
 }
 
+int lbk_ternary_relu2_gemm_dev(lbk_ctx *c, const lbk_weight *gate, const lbk_weight *up, const int8_t *q_dev, const float *scale_dev, const int32_t *sum_dev,
+                               size_t m, float *out_dev, void *stream) {
+    if (!c) return fail(LBK_ERR_INVALID, "context is null");
+    Ctx *ctx = C_(c);
+    const lbk_weight *ws[2] = {gate, up};
+    LBK_TRY(check_group(ws, 2, ctx));
+    if (m && (!q_dev || !sum_dev || !scale_dev || !out_dev)) return fail(LBK_ERR_INVALID, "lbk_ternary_relu2_gemm_dev: null buffer");
+    if (W_(gate)->rows != W_(up)->rows) return fail(LBK_ERR_SHAPE, "gate and up have %zu and %zu rows", W_(gate)->rows, W_(up)->rows);
+    LBK_CUDA(cudaSetDevice(ctx->device));
+    if (m && W_(gate)->kp == 0) {  // no columns
+        if (W_(gate)->rows) LBK_CUDA(cudaMemsetAsync(out_dev, 0, m * W_(gate)->rows * sizeof(float), static_cast<cudaStream_t>(stream)));
+        return LBK_OK;
+    }
+    GroupArgs g;
+    float *outs[2] = {out_dev, out_dev};
+    LBK_TRY(fill_group(g, ws, 2, outs, nullptr, m));
+    g.gated = true;
+    g.q = q_dev;
+    g.qscale = scale_dev;
+    g.qsum = sum_dev;
+    return launch_gemm(ctx, g, static_cast<cudaStream_t>(stream));
+}
+
 // ---- host-pointer entry points -------------------------------------------------------
 
 int lbk_quantize_acts(lbk_ctx *c, const float *x, size_t m, size_t k, int8_t *q, float *scale, int32_t *sum) {

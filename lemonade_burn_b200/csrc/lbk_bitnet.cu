@@ -273,16 +273,19 @@ int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, size_t first, 
         LBK_TRY(project(attn, ow, 1, oo));
         if (nq) LBK_TRY(norm_q(LBK_PRE_ADD_RMS, x, c->pf_o, l.post_attn_norm, H));
         else LBK_TRY(add_norm(x, c->pf_o, l.post_attn_norm));
-        const lbk_weight *gu[2] = {l.gate, l.up};
-        float *guo[2] = {c->pf_g, c->pf_u};
-        LBK_TRY(project(c->pf_n + kept * H, gu, 2, guo));
-        if (nq) {
-            LBK_TRY(norm_q(LBK_PRE_RELU2_MUL_RMS, c->pf_g, c->pf_u, l.ffn_sub_norm, I));
-        } else if (fused_i) {
-            LBK_TRY(lbk_relu2_mul_rms_norm(h, c->pf_g, c->pf_u, l.ffn_sub_norm, n, I, eps, c->pf_act, st));
+        if (nq) {  // relu(gate)^2 * up leaves the GEMM as one row; same bits
+            LBK_TRY(lbk_ternary_relu2_gemm_dev(h, l.gate, l.up, c->pf_q8, c->pf_qscale, c->pf_qsum, n, c->pf_act, st));
+            LBK_TRY(norm_q(LBK_PRE_RMS, c->pf_act, nullptr, l.ffn_sub_norm, I));
         } else {
-            LBK_TRY(lbk_relu2_mul(h, c->pf_g, c->pf_u, n * I, c->pf_act, st));
-            LBK_TRY(lbk_rms_norm(h, c->pf_act, l.ffn_sub_norm, n, I, eps, c->pf_act, st));
+            const lbk_weight *gu[2] = {l.gate, l.up};
+            float *guo[2] = {c->pf_g, c->pf_u};
+            LBK_TRY(project(c->pf_n + kept * H, gu, 2, guo));
+            if (fused_i) {
+                LBK_TRY(lbk_relu2_mul_rms_norm(h, c->pf_g, c->pf_u, l.ffn_sub_norm, n, I, eps, c->pf_act, st));
+            } else {
+                LBK_TRY(lbk_relu2_mul(h, c->pf_g, c->pf_u, n * I, c->pf_act, st));
+                LBK_TRY(lbk_rms_norm(h, c->pf_act, l.ffn_sub_norm, n, I, eps, c->pf_act, st));
+            }
         }
         const lbk_weight *dw[1] = {l.down};
         float *dout[1] = {c->pf_d};

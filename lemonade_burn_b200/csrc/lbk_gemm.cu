@@ -52,6 +52,7 @@ constexpr int kExpWarp0 = kEpiWarps, kTmaWarp = kExpWarp0 + kExpWarps * kExpSets
 constexpr int kThreads = (kPackWarp + 1) * 32;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kWide = 192;         // token rows of the wide form's tile at most
+constexpr int kPlain = 0, kScatter = 1, kGated = 2;  // what the epilogue does with a tile
 
 template <int NT>  // capacity in token rows per tile (MMA N): 192 or 64; a launch uses nt <= NT
 struct Cfg {
@@ -72,8 +73,8 @@ struct Cfg {
     static constexpr uint32_t kIdesc = (2u << 4) | (0u << 7) | (1u << 10) | ((kBMW >> 4) << 24);
     static constexpr uint32_t kBars = kPack0 + kPackStages * kPackBytes;
     static constexpr uint32_t kMisc = kBars + 48 * 8;
-    static constexpr uint32_t kTok = kMisc + 64;              // per-token sum(q) and 1/(s_a*s_w): 2 x [2][NT]
-    static constexpr uint32_t kTotal = kTok + 2 * 2 * NT * 4;
+    static constexpr uint32_t kTok = kMisc + 64;              // per-token sum(q) and 1/(s_a*s_w), kGated: of gate and of up: 3 x [2][NT]
+    static constexpr uint32_t kTotal = kTok + 3 * 2 * NT * 4;
     // Hand-off is by GROUPS of kGroup K blocks: a turn of the MMA warp (wait, issue, commit) takes some 330 cycles beside
     // the MMAs, as much as those of one block, so a group is 2 blocks of 192 token rows (one block a turn: 555 cycles a block) or 4 of 64. One
     // "full" barrier per group collects both operands: the activation bytes of its blocks (TMA transaction count) and one
@@ -136,9 +137,12 @@ __device__ __forceinline__ void umma_i8_ts_block(uint32_t d_tmem, uint32_t a_tme
         "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate_first)
         : "memory");
 }
-// SC: matrix 0's int32 dots go to the token owners' buffers (GemmParams::scatter) instead of iout: an instantiation of its
-// own, so that the ordinary kernel's epilogue keeps its registers
-template <int NT, bool SC>
+// EPI, an instantiation of its own each, so that the ordinary kernel's epilogue keeps its registers:
+//   kScatter  matrix 0's int32 dots go to the token owners' buffers (GemmParams::scatter) instead of iout
+//   kGated    matrices 0 and 1 are gate and up of one feed-forward, out[0] gets relu(gate)^2 * up: a tile is 64 rows of each, 16 of gate and 16 of up in turn,
+//             so that a lane and the lane 16 further on hold the two factors. Half the bytes leave the kernel (2011 rows of 2560 -> 2 x 6912: 57 -> 54 us) and
+//             the norm behind it reads half as many (32 -> 17 us, both in a prompt's stream). Same bits as the two projections and lbk_relu2_mul.
+template <int NT, int EPI>
 __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant__ GemmParams p) {
     using C = Cfg<NT>;
     constexpr int G = C::kGroup, PG = C::kGroupStages, PS = C::kPackStages;
@@ -228,7 +232,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                         break;
                     }
                     ptx::mbar_arrive_expect_tx(bar(C::kBarFullPack + ps), kPackBytes);
-                    ptx::tma_load_2d(base + C::kPack0 + ps * kPackBytes, &p.wpk[mat], bar(C::kBarFullPack + ps), kb * kBlockBytes, n_tile * kBMW);
+                    if constexpr (EPI == kGated) {
+                        for (int i = 0; i < 8; ++i)
+                            ptx::tma_load_2d(base + C::kPack0 + ps * kPackBytes + i * 16 * 128, &p.wpk[i & 1], bar(C::kBarFullPack + ps), kb * kBlockBytes,
+                                             n_tile * (kBMW / 2) + (i >> 1) * 16);
+                    } else {
+                        ptx::tma_load_2d(base + C::kPack0 + ps * kPackBytes, &p.wpk[mat], bar(C::kBarFullPack + ps), kb * kBlockBytes, n_tile * kBMW);
+                    }
                 }
             }
         }
@@ -361,7 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
     } else if (warp < kEpiWarps) {
         // ================= epilogue (warp % 4 = TMEM lane quadrant) =================
         int *s_qs = reinterpret_cast<int *>(sm + C::kTok);
-        float *s_inv = reinterpret_cast<float *>(sm + C::kTok + 2 * NT * 4);
+        float *s_inv = reinterpret_cast<float *>(sm + C::kTok + 2 * NT * 4), *s_inv2 = s_inv + 2 * NT;
         asm volatile("griddepcontrol.wait;" ::: "memory");
         // Per-token terms of a tile: a thread asks for those of tokens tid and tid + 128 one tile ahead, before this tile's stores. One warp that
         // fetched them 32 at a time in front of the tile held the accumulators for 5500 of the 14400 cycles a tile of 2560 columns took. Calls with
@@ -392,13 +402,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
             item_range(item, tile, kb0, kb1);
             decode_tile(tile, mat, m_tile, n_tile);
             const int rows = p.rows[mat];
-            const int row = n_tile * kBMW + quad * 32 + lane;
+            const int row = EPI == kGated ? n_tile * (kBMW / 2) + quad * 16 + (lane & 15) : n_tile * kBMW + quad * 32 + lane;
             const int nt = p.nt;
             const int tok0 = m_tile * nt;
             float *out = p.out[mat];
             int32_t *iout = p.iout[mat];
             int *qs = s_qs + a * NT;  // reuse by accumulator parity is safe: see acc_empty below
-            float *inv = s_inv + a * NT;
+            float *inv = s_inv + a * NT, *inv2 = s_inv2 + a * NT;
             if constexpr (kAhead) {
 #pragma unroll
                 for (int e = 0; e < kTerms; ++e) {
@@ -406,6 +416,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                     if (i < NT) {
                         qs[i] = term_q[e];
                         inv[i] = i < nt && tk < p.m && p.qscale ? __fdiv_rn(1.0f, __fmul_rn(term_s[e], p.wscale[mat])) : 0.0f;  // gemm.rs:158
+                        if constexpr (EPI == kGated) inv2[i] = i < nt && tk < p.m ? __fdiv_rn(1.0f, __fmul_rn(term_s[e], p.wscale[1])) : 0.0f;
                     }
                 }
                 fetch_terms(item_at(tcount + 1));
@@ -414,6 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                     const int tk = tok0 + i;
                     qs[i] = tk < p.m ? p.qsum[tk] : 0;
                     inv[i] = (tk < p.m && p.qscale) ? __fdiv_rn(1.0f, __fmul_rn(p.qscale[tk], p.wscale[mat])) : 0.0f;  // gemm.rs:158
+                    if constexpr (EPI == kGated) inv2[i] = tk < p.m ? __fdiv_rn(1.0f, __fmul_rn(p.qscale[tk], p.wscale[1])) : 0.0f;
                 }
             }
             ptx::named_barrier(2, kEpiThreads);  // the epilogue warps
@@ -434,12 +446,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
 #pragma unroll
                 for (int i = 0; i < kEpiCols; i += 4) {
                     const int4 q4 = *reinterpret_cast<const int4 *>(qs + c * kEpiCols + i);
-                    const float4 s4 = *reinterpret_cast<const float4 *>(inv + c * kEpiCols + i);
+                    const float4 s4 = *reinterpret_cast<const float4 *>((EPI == kGated && lane >= 16 ? inv2 : inv) + c * kEpiCols + i);
                     q[i] = q4.x; q[i + 1] = q4.y; q[i + 2] = q4.z; q[i + 3] = q4.w;
                     sc[i] = s4.x; sc[i + 1] = s4.y; sc[i + 2] = s4.z; sc[i + 3] = s4.w;
                 }
                 tmem_ld_wait();
-                if constexpr (SC) {
+                if constexpr (EPI == kScatter) {
                     // The reduce-scatter of a row-parallel layer starts here: the int32 dots of a token go straight
                     // into the buffer of the rank that owns the token (plain stores into peer memory, 128 consecutive
                     // bytes per warp instruction), while the MMAs of the next tile run.
@@ -454,6 +466,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                                 ++o;
                             }
                         }
+                    }
+                    continue;
+                }
+                if constexpr (EPI == kGated) {
+                    // of two token rows in turn the lower half of the warp finishes the first and the upper half the second
+                    const bool up = lane >= 16;
+#pragma unroll
+                    for (int i = 0; i < kEpiCols; i += 2) {
+                        const float y0 = __fmul_rn(__int2float_rn(static_cast<int>(v[i]) - q[i]), sc[i]), y1 = __fmul_rn(__int2float_rn(static_cast<int>(v[i + 1]) - q[i + 1]), sc[i + 1]);
+                        const float other = __shfl_xor_sync(0xffffffffu, up ? y0 : y1, 16), gate = fmaxf(up ? other : y0, 0.0f), by = up ? y1 : other;
+                        const int tk = c * kEpiCols + i + (up ? 1 : 0);
+                        if (row < rows && tk < ntok) out[static_cast<size_t>(tok0 + tk) * rows + row] = __fmul_rn(__fmul_rn(gate, gate), by);
                     }
                     continue;
                 }
@@ -513,8 +537,8 @@ template <int NT>
 static int init_one(Ctx *ctx) {
     const size_t smem = Cfg<NT>::kTotal + 1024;
     if (smem > ctx->smem_optin) return fail(LBK_ERR_UNSUPPORTED, "gemm kernel needs %zu B of shared memory", smem);
-    LBK_CUDA(cudaFuncSetAttribute(gemm_kernel<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    LBK_CUDA(cudaFuncSetAttribute(gemm_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    for (void (*k)(GemmParams) : {gemm_kernel<NT, kPlain>, gemm_kernel<NT, kScatter>, gemm_kernel<NT, kGated>})
+        LBK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     return LBK_OK;
 }
 
@@ -590,7 +614,10 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
     GemmParams p{};
     const size_t kp = g.w[0]->kp;
     int row_tiles = 0;
+    if (g.gated && (g.n != 2 || g.w[0]->rows != g.w[1]->rows || g.iout[0] || g.iout[1] || g.scatter_world || !g.qscale || !g.out[0]))
+        return fail(LBK_ERR_INVALID, "gemm: a gated pair is two matrices of one shape with an f32 output");
     for (int i = 0; i < g.n; ++i) row_tiles += static_cast<int>((g.w[i]->rows + kBMW - 1) / kBMW);
+    if (g.gated) row_tiles = static_cast<int>((g.w[0]->rows + kBMW / 2 - 1) / (kBMW / 2));
     const int nt = choose_nt(static_cast<int>(g.m), row_tiles, static_cast<int>(kp / kBK), ctx->sm_count);
     LBK_TRY(encode_act_map(&p.act, g.q, g.m, kp, nt));
     p.nt = nt;
@@ -602,7 +629,7 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
         const Weight *w = g.w[i];
         if (w->kp != kp) return fail(LBK_ERR_SHAPE, "inner dimension mismatch");
         if (g.out[i] && !g.qscale) return fail(LBK_ERR_INVALID, "gemm: f32 outputs need the activation scales");
-        p.wpk[i] = w->tmap_gemm;
+        p.wpk[i] = g.gated ? w->tmap_gemv : w->tmap_gemm;  // boxes of 16 rows or of 128
         p.out[i] = g.out[i];
         p.iout[i] = g.iout[i];
         p.wscale[i] = w->scale;
@@ -610,14 +637,22 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
         row_tiles += static_cast<int>((w->rows + kBMW - 1) / kBMW);
         p.row_end[i] = row_tiles;
     }
-    const int tiles = row_tiles * p.m_tiles;
     p.n_mat = g.n;
+    if (g.gated) {  // one matrix of pairs
+        p.n_mat = 1;
+        p.row_end[0] = row_tiles = static_cast<int>((g.w[0]->rows + kBMW / 2 - 1) / (kBMW / 2));
+    }
+    const int tiles = row_tiles * p.m_tiles;
     p.total_tiles = tiles;
     p.qscale = g.qscale;
     p.qsum = g.qsum;
     p.err_word = ctx->err_word;
     if (tiles == 0 || p.k_blocks == 0) return LBK_OK;
     p.ksplit = choose_ksplit(tiles, p.k_blocks, ctx->sm_count, &p.kb_part);
+    if (g.gated) {  // the parts' sums would have to meet before the product
+        p.ksplit = 1;
+        p.kb_part = p.k_blocks;
+    }
     p.scatter_world = g.scatter_world;
     p.scatter_mt = g.scatter_mt;
     for (int i = 0; i < 8; ++i) p.scatter[i] = g.scatter_base[i];
@@ -662,15 +697,11 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    if (nt > 64) {
-        cfg.dynamicSmemBytes = Cfg<kWide>::kTotal + 1024;
-        if (p.scatter_world) LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<kWide, true>, p));
-        else LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<kWide, false>, p));
-    } else {
-        cfg.dynamicSmemBytes = Cfg<64>::kTotal + 1024;
-        if (p.scatter_world) LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<64, true>, p));
-        else LBK_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<64, false>, p));
-    }
+    cfg.dynamicSmemBytes = (nt > 64 ? Cfg<kWide>::kTotal : Cfg<64>::kTotal) + 1024;
+    void (*kernel)(GemmParams) = nt > 64 ? gemm_kernel<kWide, kPlain> : gemm_kernel<64, kPlain>;
+    if (p.scatter_world) kernel = nt > 64 ? gemm_kernel<kWide, kScatter> : gemm_kernel<64, kScatter>;
+    if (g.gated) kernel = nt > 64 ? gemm_kernel<kWide, kGated> : gemm_kernel<64, kGated>;
+    LBK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
     LBK_CUDA(cudaGetLastError());
     ctx->launches++;
     if (p.ksplit > 1) {  // one launch scales every matrix of the group (and zeroes the context's sums again)

@@ -93,6 +93,8 @@ struct GroupArgs {
     // t % scatter_mt instead of iout (the tensor-parallel layers: the bases are the token owners' buffers, peer memory)
     int scatter_world = 0, scatter_mt = 0;
     int32_t *scatter_base[8] = {};
+    // tcgen05 GEMM only: w[0] and w[1] are gate and up, out[0] gets relu(gate)^2 * up
+    bool gated = false;
     // exactly one of x (f32, quantised inside the kernel) or q/scale/sum is set
     const float *x = nullptr;
     const int8_t *q = nullptr;
