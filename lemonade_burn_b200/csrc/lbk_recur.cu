@@ -73,7 +73,7 @@ struct RecurParams {
     int *err_word;
     // recur_step_kernel
     const uint16_t *a2, *g2;
-    int a2_pitch, g2_pitch, a_at, g_at, a_rank, g_rank;
+    int a2_pitch, g2_pitch, a_at, g_at, a_rank, g_rank, state_at;  // state_at: floats of shared memory in front of a held state
     const float *norm_w;
     float eps;
     void *out;
@@ -523,80 +523,178 @@ __device__ __forceinline__ void low_rank(const uint16_t *w, int pitch, int rank,
 }
 
 // A warp takes eight columns of S at a time. Slot s of a lane holds column s XOR (lane / 4) of the eight.
-template <typename T, bool DELTA, int P>
-__global__ void __launch_bounds__(kStepThreads, 1) recur_step_kernel(const RecurParams p) {
+// FAST: delta rule with both low ranks inside, four taps, heads and ranks of at most 128 (launch_step): a thread has at most one value of q, k and v and one
+// row's quarter of either low rank, and asks for all it needs at once, weights before the kernel in front is known to be complete. As below, where the
+// loops' loads wait for one another, a block was a chain of some fifteen trips to L2: 16 sequences of 20 heads of 128 x 128 35 us, so 25.5.
+constexpr int kFastRank = 128;
+// HELD: the state comes to shared memory by a bulk copy (states of up to kHeldBytes) instead of into registers, so two blocks fit an SM and one's copies run beside
+// the other's arithmetic: a step of 16 sequences of four mixed layers of 2560, a plain and a delta-rule one with 20 heads of 128 x 128 each, 306 -> 299 us.
+constexpr size_t kHeldBytes = 64 * 1024;
+template <typename T, bool DELTA, int P, bool FAST, bool HELD>
+__global__ void __launch_bounds__(kStepThreads, HELD ? 2 : 1) recur_step_kernel(const RecurParams p) {
     extern __shared__ __align__(16) float rs_smem[];
     __shared__ float s_red[32], s_sum[4];
+    __shared__ __align__(8) uint64_t s_bar;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.x, seq = blockIdx.y;
     float *s_k = rs_smem, *s_q = s_k + 64 * P, *s_kg = s_q + 64 * P, *s_qg = s_kg + 64 * P, *s_g = s_qg + 64 * P, *s_v = s_g + 64 * P;
     float *s_o = s_v + p.vp, *s_gate = s_o + p.vp, *s_x = s_gate + p.vp;
+    float *s_state = rs_smem + p.state_at;
+    const int group = p.heads / p.kv_heads, kvh = h / group;
     ptx::pdl_trigger();
+    // FAST: this thread's value of q, k or v and its quarter of row `lr` of the low ranks
+    const int which = tid < 64 * P ? 0 : tid < 128 * P ? 1 : 2, vd = tid - which * 64 * P, lr = tid >> 2, part = tid & 3;
+    const bool mine = FAST && vd < (which < 2 ? p.dim : p.vdim);
+    const int at = (which == 0 ? p.q_at + kvh * p.dim : which == 1 ? p.k_at + kvh * p.dim : p.v_at + h * p.vdim) + vd, cc = at - p.q_at;
+    float tap[4], rate = 0.0f, bias = 0.0f, nw = 0.0f;
+    uint4 wa[4], wg4[4];
+    if constexpr (FAST) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) tap[b] = mine ? __ldg(p.conv + static_cast<size_t>(3 - b) * p.channels + cc) : 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int col = part * 8 + 32 * c;
+            wa[c] = lr < p.dim && col < p.a2_pitch ? __ldg(reinterpret_cast<const uint4 *>(p.a2 + static_cast<size_t>(h * p.dim + lr) * p.a2_pitch + col)) : make_uint4(0u, 0u, 0u, 0u);
+            wg4[c] = lr < p.vdim && col < p.g2_pitch ? __ldg(reinterpret_cast<const uint4 *>(p.g2 + static_cast<size_t>(h * p.vdim + lr) * p.g2_pitch + col)) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        rate = expf(__ldg(p.a_log + h));
+        bias = lr < p.dim ? __ldg(p.dt_bias + h * p.dim + lr) : 0.0f;
+        nw = tid < p.vdim ? __ldg(p.norm_w + tid) : 0.0f;
+    }
     ptx::pdl_wait();
     const int pos = p.pos[seq];
     if (pos < 0 || pos >= p.cap) {
         if (tid == 0) atomicExch(p.err_word, 7);
         return;
     }
-    const bool keep = !p.active || p.active[seq] != 0;
+    bool keep = !p.active || p.active[seq] != 0;
     float *st = p.state + static_cast<size_t>(seq * p.heads + h) * p.vdim * p.dp;
+    const uint32_t bar = ptx::smem_u32(&s_bar);
+    if (HELD && tid == 0) {
+        ptx::mbar_init(bar, 1);
+        ptx::fence_barrier_init();
+        if (pos > 0) {
+            const uint32_t bytes = static_cast<uint32_t>(p.vdim * p.dp) * 4;
+            ptx::mbar_arrive_expect_tx(bar, bytes);
+            for (uint32_t at = 0; at < bytes; at += 16384) bulk_load(ptx::smem_u32(s_state) + at, reinterpret_cast<const uint8_t *>(st) + at, min(bytes - at, 16384u), bar);
+        }
+    }
     const int cg = lane >> 2;
-    u64 S[8][P];
+    u64 S[HELD ? 1 : 8][P];
+    auto column = [&](const float *from, int col, u64 (&c)[P]) {
+#pragma unroll
+        for (int j = 0; j < P; ++j) c[j] = 0;
+        if (pos > 0 && col < p.vdim) share<P>(from + static_cast<size_t>(col) * p.dp, lane, c);
+    };
     auto load = [&](int col0) {
+        if constexpr (!HELD)
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
+            for (int s = 0; s < 8; ++s) column(st, col0 + (s ^ cg), S[s]);
+    };
+    // slot s of the eight columns: held in registers, or read again where it is needed
+    auto slot = [&](int col0, int s, u64 (&c)[P]) {
+        if constexpr (HELD) {
+            column(s_state, col0 + (s ^ cg), c);
+        } else {
 #pragma unroll
-            for (int j = 0; j < P; ++j) S[s][j] = 0;
-            if (pos > 0 && col0 + (s ^ cg) < p.vdim) share<P>(st + static_cast<size_t>(col0 + (s ^ cg)) * p.dp, lane, S[s]);
+            for (int j = 0; j < P; ++j) c[j] = S[s][j];
         }
     };
-    load(warp * 8);  // on its way while the token's vectors are worked out
+    if (!HELD) load(warp * 8);  // on its way while the token's vectors are worked out
     const T *x = static_cast<const T *>(p.x) + static_cast<size_t>(seq) * p.ldx;
-    const int group = p.heads / p.kv_heads, kvh = h / group;
-    for (int e = tid; e < 128 * P + p.vp; e += kStepThreads) {
-        const int which = e < 64 * P ? 0 : e < 128 * P ? 1 : 2, d = which == 0 ? e : which == 1 ? e - 64 * P : e - 128 * P;
-        float v = 0.0f;
-        if (d < (which < 2 ? p.dim : p.vdim)) {
-            const int at = (which == 0 ? p.q_at + kvh * p.dim : which == 1 ? p.k_at + kvh * p.dim : p.v_at + h * p.vdim) + d;
-            v = dense::get(x + at);
-            if (DELTA) {
-                const int cc = at - p.q_at;
-                T *ring = static_cast<T *>(p.ring) + static_cast<size_t>(seq) * p.taps * p.channels + cc;
-                float y = v * p.conv[static_cast<size_t>(p.taps - 1) * p.channels + cc];
-                for (int back = 1; back < p.taps; ++back)
-                    if (pos - back >= 0)
-                        y = fmaf(dense::get(ring + static_cast<size_t>((pos - back) % p.taps) * p.channels), p.conv[static_cast<size_t>(p.taps - 1 - back) * p.channels + cc], y);
-                // the place of this token is not one that is read now; q and k belong to the first head of their group
-                if (keep && (which == 2 || h % group == 0)) ring[static_cast<size_t>(pos % p.taps) * p.channels] = x[at];
-                v = act<T>(y);
-            }
-        }
-        (which == 0 ? s_q : which == 1 ? s_k : s_v)[d] = v;
-    }
-    if (DELTA) {
-        const float rate = expf(p.a_log[h]);
-        auto decay = [&](int d, float z) { s_g[d] = decay_of(rate, z + p.dt_bias[h * p.dim + d]); };
-        if (p.a2) {
-            low_rank(p.a2 + static_cast<size_t>(h) * p.dim * p.a2_pitch, p.a2_pitch, p.a_rank, x + p.a_at, p.dim, s_x, decay);
-            low_rank(p.g2 + static_cast<size_t>(h) * p.vdim * p.g2_pitch, p.g2_pitch, p.g_rank, x + p.g_at, p.vdim, s_x, [&](int d, float z) { s_gate[d] = dense::sigmoid(z); });
-        } else {
-            for (int d = tid; d < p.dim; d += kStepThreads) decay(d, p.a[static_cast<size_t>(seq) * p.lda + h * p.dim + d]);
-        }
-        for (int d = p.dim + tid; d < 64 * P; d += kStepThreads) s_g[d] = 1.0f;
-    } else {
-        for (int d = tid; d < 64 * P; d += kStepThreads) s_g[d] = p.decay[h];
-    }
-    __syncthreads();
-    if (warp < 3) {  // |q|^2, |k|^2, q . k
+    const float beta_logit = DELTA ? p.b[static_cast<size_t>(seq) * p.ldb + h] : 0.0f;
+    auto sums = [&] {  // |q|^2, |k|^2, q . k
+        if (warp >= 3) return;
         const float *l = warp == 1 ? s_k : s_q, *r = warp == 0 ? s_q : s_k;
         float t = 0.0f;
         for (int d = lane; d < 64 * P; d += 32) t = fmaf(l[d], r[d], t);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (lane == 0) s_sum[warp] = t;
+    };
+    if constexpr (FAST) {
+        float *s_x2 = s_x + kFastRank;
+        if (tid < 128 * P + p.vp) {
+            float v = 0.0f;
+            if (mine) {
+                T *ring = static_cast<T *>(p.ring) + static_cast<size_t>(seq) * 4 * p.channels + cc;
+                const T now = x[at];
+                float old[4];
+#pragma unroll
+                for (int b = 1; b < 4; ++b) old[b] = pos - b >= 0 ? dense::get(ring + static_cast<size_t>((pos - b) & 3) * p.channels) : 0.0f;
+                float y = dense::get(&now) * tap[0];
+#pragma unroll
+                for (int b = 1; b < 4; ++b)
+                    if (pos - b >= 0) y = fmaf(old[b], tap[b], y);
+                if (keep && (which == 2 || h % group == 0)) ring[static_cast<size_t>(pos & 3) * p.channels] = now;  // not a place that is read now
+                v = act<T>(y);
+            }
+            (which == 0 ? s_q : which == 1 ? s_k : s_v)[vd] = v;
+        }
+        for (int i = kStepThreads - 1 - tid; i < 2 * kFastRank; i += kStepThreads)  // threads without a value first
+            s_x[i] = i < kFastRank ? (i < p.a_rank ? dense::get(x + p.a_at + i) : 0.0f) : (i - kFastRank < p.g_rank ? dense::get(x + p.g_at + i - kFastRank) : 0.0f);
+        __syncthreads();
+        float da = 0.0f, dg = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const uint32_t va[4] = {wa[c].x, wa[c].y, wa[c].z, wa[c].w}, vg[4] = {wg4[c].x, wg4[c].y, wg4[c].z, wg4[c].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int col = part * 8 + 32 * c + 2 * i;
+                da = fmaf(__uint_as_float(va[i] << 16), s_x[col], da);
+                da = fmaf(__uint_as_float(va[i] & 0xffff0000u), s_x[col + 1], da);
+                dg = fmaf(__uint_as_float(vg[i] << 16), s_x2[col], dg);
+                dg = fmaf(__uint_as_float(vg[i] & 0xffff0000u), s_x2[col + 1], dg);
+            }
+        }
+        da += __shfl_xor_sync(0xffffffffu, da, 1);
+        da += __shfl_xor_sync(0xffffffffu, da, 2);
+        dg += __shfl_xor_sync(0xffffffffu, dg, 1);
+        dg += __shfl_xor_sync(0xffffffffu, dg, 2);
+        if (part == 0) {
+            if (lr < 64 * P) s_g[lr] = lr < p.dim ? decay_of(rate, da + bias) : 1.0f;
+            if (lr < p.vdim) s_gate[lr] = dense::sigmoid(dg);
+        }
+        sums();
+    } else {
+        for (int e = tid; e < 128 * P + p.vp; e += kStepThreads) {
+            const int which = e < 64 * P ? 0 : e < 128 * P ? 1 : 2, d = which == 0 ? e : which == 1 ? e - 64 * P : e - 128 * P;
+            float v = 0.0f;
+            if (d < (which < 2 ? p.dim : p.vdim)) {
+                const int at = (which == 0 ? p.q_at + kvh * p.dim : which == 1 ? p.k_at + kvh * p.dim : p.v_at + h * p.vdim) + d;
+                v = dense::get(x + at);
+                if (DELTA) {
+                    const int cc = at - p.q_at;
+                    T *ring = static_cast<T *>(p.ring) + static_cast<size_t>(seq) * p.taps * p.channels + cc;
+                    float y = v * p.conv[static_cast<size_t>(p.taps - 1) * p.channels + cc];
+                    for (int back = 1; back < p.taps; ++back)
+                        if (pos - back >= 0)
+                            y = fmaf(dense::get(ring + static_cast<size_t>((pos - back) % p.taps) * p.channels), p.conv[static_cast<size_t>(p.taps - 1 - back) * p.channels + cc], y);
+                    // the place of this token is not one that is read now; q and k belong to the first head of their group
+                    if (keep && (which == 2 || h % group == 0)) ring[static_cast<size_t>(pos % p.taps) * p.channels] = x[at];
+                    v = act<T>(y);
+                }
+            }
+            (which == 0 ? s_q : which == 1 ? s_k : s_v)[d] = v;
+        }
+        if (DELTA) {
+            const float rate = expf(p.a_log[h]);
+            auto decay = [&](int d, float z) { s_g[d] = decay_of(rate, z + p.dt_bias[h * p.dim + d]); };
+            if (p.a2) {
+                low_rank(p.a2 + static_cast<size_t>(h) * p.dim * p.a2_pitch, p.a2_pitch, p.a_rank, x + p.a_at, p.dim, s_x, decay);
+                low_rank(p.g2 + static_cast<size_t>(h) * p.vdim * p.g2_pitch, p.g2_pitch, p.g_rank, x + p.g_at, p.vdim, s_x, [&](int d, float z) { s_gate[d] = dense::sigmoid(z); });
+            } else {
+                for (int d = tid; d < p.dim; d += kStepThreads) decay(d, p.a[static_cast<size_t>(seq) * p.lda + h * p.dim + d]);
+            }
+            for (int d = p.dim + tid; d < 64 * P; d += kStepThreads) s_g[d] = 1.0f;
+        } else {
+            for (int d = tid; d < 64 * P; d += kStepThreads) s_g[d] = p.decay[h];
+        }
+        __syncthreads();
+        sums();
     }
     __syncthreads();
     const float fq = DELTA ? 1.0f / sqrtf(static_cast<float>(p.dim)) / sqrtf(s_sum[0] + 1e-6f) : 1.0f, fk = DELTA ? 1.0f / sqrtf(s_sum[1] + 1e-6f) : 1.0f;
-    const float qk = s_sum[2] * fq * fk, beta = DELTA ? dense::sigmoid(p.b[static_cast<size_t>(seq) * p.ldb + h]) : 1.0f;
+    const float qk = s_sum[2] * fq * fk, beta = DELTA ? dense::sigmoid(beta_logit) : 1.0f;
     for (int d = tid; d < 64 * P; d += kStepThreads) {
         const float k = s_k[d] * fk, g = s_g[d];
         s_k[d] = k;
@@ -610,18 +708,28 @@ __global__ void __launch_bounds__(kStepThreads, 1) recur_step_kernel(const Recur
     share<P>(up ? s_kg : s_qg, lane, wg);
     share<P>(s_g, lane, g);
     share<P>(s_k, lane, kk);
+    if (HELD && pos > 0 && !__all_sync(0xffffffffu, ptx::mbar_wait(bar, 0, kWaitLimit))) {  // every thread has passed a barrier behind its set-up
+        if (lane == 0) atomicExch(p.err_word, 5);
+        keep = false;
+    }
     for (int col0 = warp * 8; col0 < p.vdim; col0 += kStepWarps * 8) {
         if (col0 != warp * 8) load(col0);
         float r[8];
         if (DELTA) {
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
-                r[s] = dot<P>(w, S[s]);
-                r[s] += __shfl_xor_sync(0xffffffffu, dot<P>(wg, S[s]), 2);
+                u64 c[P];
+                slot(col0, s, c);
+                r[s] = dot<P>(w, c);
+                r[s] += __shfl_xor_sync(0xffffffffu, dot<P>(wg, c), 2);
             }
         } else {
 #pragma unroll
-            for (int s = 0; s < 8; ++s) r[s] = dot<P>(up ? w : wg, S[s]);
+            for (int s = 0; s < 8; ++s) {
+                u64 c[P];
+                slot(col0, s, c);
+                r[s] = dot<P>(up ? w : wg, c);
+            }
         }
 #pragma unroll
         for (int c = 4; c >= 1; c >>= 1)
@@ -644,9 +752,11 @@ __global__ void __launch_bounds__(kStepThreads, 1) recur_step_kernel(const Recur
             for (int s = 0; s < 8; ++s) {
                 const float us = s ? __shfl_xor_sync(0xffffffffu, u, 4 * s) : u;
                 const u64 uu = pack2(us, us);
+                u64 c[P];
+                slot(col0, s, c);
 #pragma unroll
-                for (int j = 0; j < P; ++j) S[s][j] = fma2(kk[j], uu, mul2(g[j], S[s][j]));
-                if (col0 + (s ^ cg) < p.vdim) unshare<P>(st + static_cast<size_t>(col0 + (s ^ cg)) * p.dp, lane, S[s]);
+                for (int j = 0; j < P; ++j) c[j] = fma2(kk[j], uu, mul2(g[j], c[j]));
+                if (col0 + (s ^ cg) < p.vdim) unshare<P>(st + static_cast<size_t>(col0 + (s ^ cg)) * p.dp, lane, c);
             }
         }
     }
@@ -656,7 +766,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) recur_step_kernel(const Recur
         for (int c = tid; c < p.vdim; c += kStepThreads) ss = fmaf(s_o[c], s_o[c], ss);
         const float r = 1.0f / sqrtf(dense::block_sum<kStepThreads>(ss, s_red) / static_cast<float>(p.vdim) + p.eps);
         T *out = static_cast<T *>(p.out) + static_cast<size_t>(seq) * p.ldo + static_cast<size_t>(h) * p.vdim;
-        for (int c = tid; c < p.vdim; c += kStepThreads) dense::put(out + c, s_o[c] * r * p.norm_w[c] * s_gate[c]);
+        for (int c = tid; c < p.vdim; c += kStepThreads) dense::put(out + c, s_o[c] * r * (FAST ? nw : p.norm_w[c]) * s_gate[c]);
     } else {
         for (int c = tid; c < p.vdim; c += kStepThreads) p.o[(static_cast<size_t>(seq) * p.heads + h) * p.vdim + c] = s_o[c];
     }
@@ -761,6 +871,8 @@ template <typename T, bool DELTA>
 int recur_init_kind() {
     for (void (*k)(RecurParams) : {recur_walk_kernel<T, DELTA, 1>, recur_walk_kernel<T, DELTA, 2>, recur_walk_kernel<T, DELTA, 4>})
         LBK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRingBytes)));
+    for (void (*k)(RecurParams) : {recur_step_kernel<T, DELTA, 1, DELTA, true>, recur_step_kernel<T, DELTA, 2, DELTA, true>})
+        LBK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kHeldBytes + 48 * 1024)));
     return LBK_OK;
 }
 int recur_init(Ctx *) {
@@ -797,9 +909,18 @@ int launch_walk(Ctx *ctx, RecurParams &p, cudaStream_t st) {
 template <typename T, bool DELTA>
 int launch_step(Ctx *ctx, RecurParams &p, cudaStream_t st) {
     const int x = p.a2_pitch > p.g2_pitch ? p.a2_pitch : p.g2_pitch;
-    const size_t smem = (5 * static_cast<size_t>(p.dp) + 3 * static_cast<size_t>(p.vp) + static_cast<size_t>(x)) * sizeof(float);
+    const bool fast = DELTA && p.a2 && p.taps == 4 && p.dp <= 128 && p.vp <= 128 && p.a2_pitch <= kFastRank && p.g2_pitch <= kFastRank && (reinterpret_cast<uintptr_t>(p.state) & 15) == 0;
+    const size_t held = static_cast<size_t>(p.vdim) * p.dp * 4;
+    const bool hold = fast || (!DELTA && held <= kHeldBytes && p.dp <= 128 && (reinterpret_cast<uintptr_t>(p.state) & 15) == 0);
+    size_t smem = (5 * static_cast<size_t>(p.dp) + 3 * static_cast<size_t>(p.vp) + static_cast<size_t>(fast ? 2 * kFastRank : x)) * sizeof(float);
     if (smem > 48 * 1024) return fail(LBK_ERR_UNSUPPORTED, "recurrence: the low ranks are too large");
-    void (*k)(RecurParams) = p.dp == 64 ? recur_step_kernel<T, DELTA, 1> : p.dp == 128 ? recur_step_kernel<T, DELTA, 2> : recur_step_kernel<T, DELTA, 4>;
+    if (hold) {
+        smem = (smem + 15) / 16 * 16;
+        p.state_at = static_cast<int>(smem / 4);
+        smem += held;
+    }
+    void (*k)(RecurParams) = p.dp == 64 ? recur_step_kernel<T, DELTA, 1, false, false> : p.dp == 128 ? recur_step_kernel<T, DELTA, 2, false, false> : recur_step_kernel<T, DELTA, 4, false, false>;
+    if (hold) k = p.dp == 64 ? recur_step_kernel<T, DELTA, 1, DELTA, true> : recur_step_kernel<T, DELTA, 2, DELTA, true>;
     LBK_CUDA(launch_chained(k, dim3(static_cast<unsigned>(p.heads), static_cast<unsigned>(p.n)), dim3(kStepThreads), smem, st, p));
     LBK_CUDA(cudaGetLastError());
     ctx->launches++;
