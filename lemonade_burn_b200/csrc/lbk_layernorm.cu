@@ -124,9 +124,20 @@ __global__ void __launch_bounds__(NT) sandwich_norm_kernel(const NormParams p) {
 }
 
 // The same with four neighbouring values a thread (rows of whole 16-byte units): the usual case.
-template <int NV, typename T>
+// EARLY, for at most a row an SM: the weights are asked for before the kernel in front is known to be complete, and held. Behind each reduction they
+// are another trip to L2 (with latent_prep_kernel's loads done the same way a step of 16 sequences of four mixed layers of 2560 took 299 us instead of 311); with many rows the registers would cost warps instead.
+template <int NV, typename T, bool EARLY>
 __global__ void __launch_bounds__(256) sandwich_norm_vec_kernel(const NormParams p) {
     ptx::pdl_trigger();
+    float4 post[EARLY ? NV : 1], gain[EARLY ? NV : 1];
+    if constexpr (EARLY) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int i = threadIdx.x + j * 256;
+            post[j] = p.w_post && i < p.n >> 2 ? __ldg(reinterpret_cast<const float4 *>(p.w_post) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            gain[j] = p.w && i < p.n >> 2 ? __ldg(reinterpret_cast<const float4 *>(p.w) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
     ptx::pdl_wait();
     __shared__ float s_red[32];
     const int n = p.n, n4 = n >> 2;
@@ -191,7 +202,7 @@ __global__ void __launch_bounds__(256) sandwich_norm_vec_kernel(const NormParams
         for (int j = 0; j < NV; ++j) {
             const int i = threadIdx.x + j * 256;
             if (i < n4) {
-                const float4 g = __ldg(reinterpret_cast<const float4 *>(p.w_post) + i);
+                const float4 g = EARLY ? post[EARLY ? j : 0] : __ldg(reinterpret_cast<const float4 *>(p.w_post) + i);
                 v[j] = make_float4(u[j].x + v[j].x * r * g.x, u[j].y + v[j].y * r * g.y, u[j].z + v[j].z * r * g.z, u[j].w + v[j].w * r * g.w);
                 xr[i] = v[j];
             }
@@ -230,7 +241,7 @@ __global__ void __launch_bounds__(256) sandwich_norm_vec_kernel(const NormParams
     for (int j = 0; j < NV; ++j) {
         const int i = threadIdx.x + j * 256;
         if (i < n4) {
-            const float4 g = __ldg(reinterpret_cast<const float4 *>(p.w) + i);
+            const float4 g = EARLY ? gain[EARLY ? j : 0] : __ldg(reinterpret_cast<const float4 *>(p.w) + i);
             const float4 o = make_float4(v[j].x * r * g.x, v[j].y * r * g.y, v[j].z * r * g.z, v[j].w * r * g.w);
             if (p.out_f) reinterpret_cast<float4 *>(p.out_f + row * n)[i] = o;
             if (p.out_e) dense::put4(static_cast<T *>(p.out_e) + row * p.lde + 4 * i, o);
@@ -264,9 +275,11 @@ int norm_impl(Ctx *ctx, const NormCall &c, cudaStream_t st) {
         vec = vec && c.moe->ld % 4 == 0;
     }
     if (vec && (bits & 15) == 0) {
-        if (c.n <= 1024) LBK_CUDA(launch_chained(sandwich_norm_vec_kernel<1, T>, grid, dim3(256), 0, st, p));
-        else if (c.n <= 4096) LBK_CUDA(launch_chained(sandwich_norm_vec_kernel<4, T>, grid, dim3(256), 0, st, p));
-        else LBK_CUDA(launch_chained(sandwich_norm_vec_kernel<8, T>, grid, dim3(256), 0, st, p));
+        const bool early = c.rows <= static_cast<size_t>(ctx->sm_count);
+        void (*k)(NormParams) = early ? sandwich_norm_vec_kernel<8, T, true> : sandwich_norm_vec_kernel<8, T, false>;
+        if (c.n <= 1024) k = early ? sandwich_norm_vec_kernel<1, T, true> : sandwich_norm_vec_kernel<1, T, false>;
+        else if (c.n <= 4096) k = early ? sandwich_norm_vec_kernel<4, T, true> : sandwich_norm_vec_kernel<4, T, false>;
+        LBK_CUDA(launch_chained(k, grid, dim3(256), 0, st, p));
     } else if (c.n <= 8192) {
         LBK_CUDA(launch_chained(sandwich_norm_kernel<256, 32, T>, grid, dim3(256), 0, st, p));
     } else if (c.n <= 32768) {
