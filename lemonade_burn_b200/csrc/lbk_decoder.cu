@@ -49,7 +49,17 @@ __global__ void embed_kernel(const uint16_t *__restrict__ table, const int *__re
 
     const int b = blockIdx.x;
     const uint16_t *row = table + static_cast<size_t>(tokens[b]) * hidden;
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) out[static_cast<size_t>(b) * hidden + i] = bf16_to_f32(row[i]);
+    float *o = out + static_cast<size_t>(b) * hidden;
+    if ((hidden & 7) == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+        // eight values a thread in one load: value by value a row of 2560 was ten trips through two bytes each (a step's one row 8 -> 2.5 us, 2011 rows 12.5 -> 7.6)
+        for (int i = threadIdx.x; i < (hidden >> 3); i += blockDim.x) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row) + i);
+            reinterpret_cast<float4 *>(o)[2 * i] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+            reinterpret_cast<float4 *>(o)[2 * i + 1] = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u), __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < hidden; i += blockDim.x) o[i] = bf16_to_f32(row[i]);
 }
 
 __global__ void __launch_bounds__(256) rms_norm_kernel(const float *x, const float *__restrict__ w, int n,
