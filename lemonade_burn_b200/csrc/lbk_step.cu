@@ -307,7 +307,8 @@ __device__ __forceinline__ void input_phase(const Cta &c, const StepParams &p, i
     }
 }
 
-template <int MT>
+// ROW: one sequence, on the integer pipes (consume_stage_row)
+template <int MT, bool ROW>
 __device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p, int phase, const float *ws, Stream &st, uint64_t policy) {
     const Phase &ph = p.ph[phase];
     const int g = c.lane >> 2, t = c.lane & 3, m = p.m;
@@ -327,6 +328,7 @@ __device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p,
         tok = tok < m ? tok : m - 1;  // lanes past the last row read it again; what they get is dropped
         xrow[mt] = s_xq + static_cast<size_t>(tok) * stride + t * 16;
     }
+    int sums[2][4] = {};
     int acc[MT][2][4][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
@@ -339,7 +341,8 @@ __device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p,
     int tile = run.x, chunk = run.y;
     for (int item = 0; item < run.z; ++item) {
         if (!ptx::mbar_wait(st.bars + st.s * 8, st.phase, kWaitLimit)) st.ok = false;
-        consume_stage<MT>(st.ptr + st.s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
+        if constexpr (ROW) consume_stage_row(st.ptr + st.s * kStageBytes, off, xrow[0], static_cast<uint32_t>(chunk) * kChunkCols, sums);
+        else consume_stage<MT>(st.ptr + st.s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
         __syncwarp();  // every lane has read the stage before it is refilled
         if (c.lane == 0) st.issue(p, st.s, policy);
         if (++st.s == st.depth) {
@@ -349,6 +352,12 @@ __device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p,
         const bool done = ++chunk == ph.chunks;
         if (done || item + 1 == run.z) {
             int *rec = s_acc + (tile - cta.x) * m * kTileRows;
+            if constexpr (ROW) {
+                const int lo = sum_row(sums[0]), hi = sum_row(sums[1]);
+                if (t < 2) atomicAdd(rec + g + 8 * t, t ? hi : lo);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) sums[0][kk] = sums[1][kk] = 0;
+            } else
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -684,7 +693,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
 #pragma unroll 1
         for (int ph = 0; ph < kPhases; ++ph) {
             input_phase<NI, NH, SHARED>(c, p, ph, from, number, ++codes, info.norm[ph], x);
-            product_phase<MT>(c, p, ph, info.wscale, st, policy);
+            product_phase<MT, !SHARED>(c, p, ph, info.wscale, st, policy);
             meet();
             from = p.ph[ph].out[0];
             if (ph != 0) continue;

@@ -219,8 +219,8 @@ __global__ void __launch_bounds__(kThreads, 1) sweep_kernel(const SweepParams p)
 
     // ---- consume cursor ----------------------------------------------------------------
     const LaneOffsets off = lane_offsets(lane);
-    const uint8_t *xrow[1] = {s_xq + t * 16};
-    int acc[1][2][4][4];  // written by the first stage of every tile
+    const uint8_t *xrow = s_xq + t * 16;
+    int acc[2][4];  // written by the first stage of every tile
 
     int cg = run.z - 1;  // forces the first group set-up
     SweepGroup cgrp{};
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 1) sweep_kernel(const SweepParams p)
     bool ok = true;
 
     // dot = acc - sum(q), y = (float)dot * (1/(s_a*s_w)) for the 16 rows of `tile`; v_lo / v_hi are
-    // the complete sums of rows g and g + 8 (meaningful on lanes with t == 0).
+    // the complete sums of rows g and g + 8.
     auto write_tile = [&](int v_lo, int v_hi) {
         const int local = tile - cgrp.tile0;
         if (cmat < 0 || local >= mat_tile_end) {
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) sweep_kernel(const SweepParams p)
             inv = __fdiv_rn(1.0f, __fmul_rn(a_scale, __ldg(&mt->wscale)));  // gemm.rs:141
         }
         const int row0 = (local - mat_tile_base) * kTileRows;
-        if (t == 0) {  // token 0 lives in column 0 of the tile
+        if (t == 0) {  // all four lanes of a row have its sum
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int row = row0 + g + h * 8;
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) sweep_kernel(const SweepParams p)
                 cgrp = load_group(p.groups + ++cg, keep);
             } while (tile >= cgrp.tile0 + cgrp.tiles);
             const int slot = cg - slot_g0;
-            xrow[0] = s_xq + static_cast<size_t>(slot) * p.xq_bytes + t * 16;
+            xrow = s_xq + static_cast<size_t>(slot) * p.xq_bytes + t * 16;
             a_scale = s_scale[slot];
             a_sum = s_sum[slot];
             cmat = -1;
@@ -309,8 +309,8 @@ __global__ void __launch_bounds__(kThreads, 1) sweep_kernel(const SweepParams p)
                 ok = false;
                 break;
             }
-            if (chunk == c0) consume_stage<1, true>(stage_ptr + s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
-            else consume_stage<1, false>(stage_ptr + s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
+            if (chunk == c0) consume_stage_row<true>(stage_ptr + s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
+            else consume_stage_row<false>(stage_ptr + s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
             __syncwarp();  // every lane has read the stage before it is refilled
             if (lane == 0 && issued < n_stages) issue(s);
             if (++s == kSweepStages) {
@@ -319,8 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1) sweep_kernel(const SweepParams p)
             }
         }
         if (!ok) break;
-        // columns 1..7 of the MMA tile repeat token 0 and are never read
-        const int v_lo = read_acc<1>(acc, 0, 0), v_hi = read_acc<1>(acc, 0, 2);
+        const int v_lo = sum_row(acc[0]), v_hi = sum_row(acc[1]);
         if (c0 > 0) share_tile(gw, true, v_lo, v_hi);             // the previous warp holds the first columns
         else if (c1 < cgrp.chunks) share_tile(gw + 1, false, v_lo, v_hi);  // the next warp holds the rest
         else write_tile(v_lo, v_hi);
