@@ -10,9 +10,13 @@
 //   projections gemv_kernel's arithmetic (lbk_gemv_core.cuh): a CTA owns a contiguous range of 16-row tiles, its 16 warps share the
 //               (tile, chunk) stages, and meet in shared memory; same integers, same scale product. Gate and up tiles lie
 //               side by side, so relu(gate)^2 * up leaves as one row;
-//   barriers    between dependent parts all CTAs meet on a counter in L2, 6 times a layer, 2500 to 3500 cycles each. The thread that
-//               arrives is the one that polls: polls of other warps held the arriving thread's release up by 10000 cycles.
-//               Norm weights and cached rows are asked for between arriving and waiting;
+//   meetings    between dependent parts all CTAs meet on a counter in L2, 6 times a layer. The thread that arrives is the one that
+//               polls: polls of other warps held the arriving thread's release up by 10000 cycles. Norm weights and cached rows are
+//               asked for between arriving and waiting. A barrier, whose count is ordered behind the CTA's values, costs 2500 to 3500
+//               cycles, a third of it until the values are known to be in L2. With one sequence five of the six are loose: the count
+//               goes out beside the values, and a reader tells by the words themselves whether they are there (Place). A step of
+//               30 layers of 2560 at 2000 positions 868 -> 822 us, of 12 layers at 100 positions 319 -> 302. With more
+//               sequences, whose rows one CTA each reads, all six stay barriers: loose ones took 392 us for 388 with sixteen;
 //   inputs      with one sequence every CTA normalises and quantises the row itself. With more, one CTA per row does and leaves
 //               the codes and a flag for all: reading b f32 rows in 148 places costs more than the extra step. The
 //               residual stream stays in the registers of the CTA that needs it;
@@ -20,13 +24,12 @@
 //               positions at a time, a lane four dimensions, and the first keys and values are in registers before
 //               the barrier in front. Slices are added up by one CTA or warp per head.
 //
-// Handing values on as 64-bit words with a number, polled by whoever needs them, was built too: a store and a load instead of a
-// barrier, but with 148 CTAs polling the lines that others write a step took 1.5 times as long. So did a flag per CTA.
+// Polling the values instead of a count (64-bit words with a number, or a flag per CTA): with 148 CTAs polling the lines that others write
+// a step took 1.5 times as long.
 //
 // Measured, a whole step with head and argmax, a kernel per operation -> this: one sequence at 2000 positions, 30 layers of 2560,
-// vocabulary 128256 1309 -> 916 us (of it 130 the head); sixteen sequences at 400 positions, 8 layers, vocabulary 32000 547 -> 394 us. At other widths,
+// vocabulary 128256 1309 -> 822 us (of it 110 the head); sixteen sequences at 400 positions, 8 layers, vocabulary 32000 547 -> 383 us. At other widths,
 // 512 to 8192, with 1 to 16 sequences at 100 and 2000 positions, 1.14 to 2.8 times as fast as a kernel per operation, rings of two stages included.
-// A layer of one sequence: six barriers 18000 cycles, norms and quantisers 9000, products 11000, attention 7000.
 #include "lbk_gemv_core.cuh"
 
 #include <exception>
@@ -82,7 +85,7 @@ struct StepParams {
     float *q8_scale;
     int32_t *q8_sum;
     // of all launches so far: barriers, inputs of projections, arrivals at barriers, rows of codes; and the CTAs that have left this one
-    uint32_t *number, *codes, *met, *q8_ready, *exit_count;
+    uint32_t *number, *codes, *turn, *met, *q8_ready, *exit_count;
     int *err_word;
     uint32_t poll_limit;
     Phase ph[kPhases];
@@ -126,6 +129,61 @@ __device__ __forceinline__ float4 shfl_xor4(float4 v, int o) {
     return make_float4(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o), __shfl_xor_sync(0xffffffffu, v.z, o),
                        __shfl_xor_sync(0xffffffffu, v.w, o));
 }
+// How values go from one part to the next.
+// LOOSE: behind a count that is not ordered after them. A float travels as its complement, so that a word of zeros means "not there yet" (the
+// value it would stand for, a NaN that no arithmetic leaves, goes as another NaN), and every reader looks again until all words are there.
+// There are two places for each value, taken in turn by the layers: whoever writes one clears the other. At that time all CTAs have met
+// at this layer's barrier, behind their last look at the other, and they meet at the next before they look at it again.
+// Otherwise as they are, behind a barrier.
+template <bool LOOSE>
+struct Place {
+    float *at;
+    ptrdiff_t other;  // floats from a place to the other
+    static __device__ __forceinline__ uint32_t word(float v) {  // as it travels
+        const uint32_t u = __float_as_uint(v);
+        return !LOOSE ? u : u == ~0u ? ~0x7fffffffu : ~u;
+    }
+    static __device__ __forceinline__ float value(uint32_t u) { return __uint_as_float(LOOSE ? ~u : u); }
+    static __device__ __forceinline__ uint4 words(float4 v) { return make_uint4(word(v.x), word(v.y), word(v.z), word(v.w)); }
+    static __device__ __forceinline__ float4 values(uint4 u) { return make_float4(value(u.x), value(u.y), value(u.z), value(u.w)); }
+    __device__ __forceinline__ void put(size_t i, float v) const {
+        if constexpr (!LOOSE) {
+            at[i] = v;
+        } else {
+            asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(at + i), "r"(word(v)) : "memory");
+            asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(at + i + other), "r"(0u) : "memory");
+        }
+    }
+    __device__ __forceinline__ void put2(size_t i, float2 v) const {
+        if constexpr (!LOOSE) {
+            *reinterpret_cast<float2 *>(at + i) = v;
+        } else {
+            asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(at + i), "r"(word(v.x)), "r"(word(v.y)) : "memory");
+            asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %1};" ::"l"(at + i + other), "r"(0u) : "memory");
+        }
+    }
+    __device__ __forceinline__ void put4(size_t i, float4 v) const {
+        if constexpr (!LOOSE) {
+            *reinterpret_cast<float4 *>(at + i) = v;
+        } else {
+            const uint4 u = words(v);
+            asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(at + i), "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w) : "memory");
+            asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %1, %1, %1};" ::"l"(at + i + other), "r"(0u) : "memory");
+        }
+    }
+    static __device__ __forceinline__ uint4 look4(const float *from) {
+        if (!LOOSE) return __ldcg(reinterpret_cast<const uint4 *>(from));
+        uint4 u;
+        asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(from) : "memory");
+        return u;
+    }
+    static __device__ __forceinline__ uint2 look2(const float *from) {
+        if (!LOOSE) return __ldcg(reinterpret_cast<const uint2 *>(from));
+        uint2 u;
+        asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(u.x), "=r"(u.y) : "l"(from) : "memory");
+        return u;
+    }
+};
 __device__ __forceinline__ float4 ldcg4(const float *at) { return __ldcg(reinterpret_cast<const float4 *>(at)); }
 
 // What a CTA carries through the step.
@@ -165,18 +223,55 @@ __device__ __forceinline__ void arrive(const Cta &c, const StepParams &p) {
     __syncthreads();
     if (c.tid == 0) count_up(p.met);
 }
+// The same behind a part that hands its values on by Place<LOOSE>. LOOSE: the count only says when it is worth looking, and is not held up until the
+// values have reached L2.
+template <bool LOOSE>
+__device__ __forceinline__ void arrive_behind(const Cta &c, const StepParams &p) {
+    if (!LOOSE) return arrive(c, p);
+    __syncthreads();
+    if (c.tid == 0) asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(p.met) : "memory");
+}
 __device__ __forceinline__ void wait(const Cta &c, const StepParams &p, uint32_t number) {
     if (c.tid == 0) await(c, p, p.met, number * gridDim.x);
     __syncthreads();
 }
 
+// What look4() or look2() got, once it is there.
+template <bool LOOSE>
+__device__ __forceinline__ float4 settle(const Cta &c, const StepParams &p, const float *from, uint4 u) {
+    if (LOOSE)
+        for (uint32_t polls = 0; !u.x || !u.y || !u.z || !u.w; u = Place<true>::look4(from))
+            if (*c.gave_up() || ++polls >= p.poll_limit) {
+                c.give_up();
+                break;
+            }
+    return Place<LOOSE>::values(u);
+}
+template <bool LOOSE>
+__device__ __forceinline__ float2 settle(const Cta &c, const StepParams &p, const float *from, uint2 u) {
+    if (LOOSE)
+        for (uint32_t polls = 0; !u.x || !u.y; u = Place<true>::look2(from))
+            if (*c.gave_up() || ++polls >= p.poll_limit) {
+                c.give_up();
+                break;
+            }
+    return make_float2(Place<LOOSE>::value(u.x), Place<LOOSE>::value(u.y));
+}
+
+// r of a row whose squares sum to ss; the scale of its codes from that sum and max|y|
+__device__ __forceinline__ float norm_factor(float ss, int k, float eps) { return 1.0f / sqrtf(ss / static_cast<float>(k) + eps); }
+__device__ __forceinline__ float scale_of(float2 row, int k, float eps) {
+    return __fdiv_rn(127.0f, fmaxf(row.y * norm_factor(row.x, k, eps), 1e-5f));  // quant.rs:105
+}
 // A row through the norm and the quantiser, by the whole CTA: v holds it in float4 tid + 512 j, w the norm's weights. With
 // y = x w and r the norm's factor the codes are round(y r 127 / max|y r|) = round(y 127 / max|y|): r only enters the scale, so the sum
-// of squares and the maximum are reduced together. (The norm and quantise kernels round (x r w) (127 / max|x r w|): the same but for a code
-// that lies on a rounding boundary to within a few units in the last place, a row of 2560 in some hundreds.) Leaves the codes (fragment order, zeros up to kfill) at dst and their sum
-// in shared memory; returns the scale (quant.rs:101-118, model.rs:267-272).
+// of squares and the maximum are reduced together, and the codes do not wait for r, whose two divisions and root took 500 of the 1800
+// cycles: returned are the sum and the maximum, from which one thread has the scale (scale_of) beside or behind the codes. (The norm and
+// quantise kernels round (x r w) (127 / max|x r w|): the same but for a code that lies on a rounding boundary to within a few units in
+// the last place, a row of 2560 in some hundreds.) Leaves the codes (fragment order, zeros up to kfill) at dst and their sum
+// in shared memory (quant.rs:101-118, model.rs:267-272).
 template <int NJ>
-__device__ __forceinline__ float norm_quant_row(const Cta &c, float4 (&v)[NJ], const float4 (&w)[NJ], int k, int kfill, float eps, uint8_t *dst) {
+__device__ __forceinline__ float2 norm_quant_row(const Cta &c, float4 (&v)[NJ], const float4 (&w)[NJ], int k, int kfill, float eps, uint8_t *dst) {
     float *s_ss = reinterpret_cast<float *>(c.sm + c.L.part), *s_max = s_ss + kWarps;
     int *s_sum = reinterpret_cast<int *>(s_max + kWarps);
     if (c.tid == 0) *s_sum = 0;
@@ -202,9 +297,11 @@ __device__ __forceinline__ float norm_quant_row(const Cta &c, float4 (&v)[NJ], c
         ss += (f.x + f.y) + (f.z + f.w);
         am = fmaxf(am, fmaxf(fmaxf(g.x, g.y), fmaxf(g.z, g.w)));
     }
-    const float r = 1.0f / sqrtf(ss / static_cast<float>(k) + eps), top = am * r;
-    const float sc = __fdiv_rn(127.0f, fmaxf(top, 1e-5f));             // quant.rs:105
-    const float mult = top >= 1e-5f ? __fdiv_rn(127.0f, am) : r * sc;  // of y; a NaN factor takes the second way
+    float mult = __fdiv_rn(127.0f, am);  // of y, unless max|y r| < 1e-5 or no number: an estimate of it tells, at half the bound or closer the value itself
+    if (!(am * rsqrtf(__fdividef(ss, static_cast<float>(k)) + eps) >= 2e-5f)) {
+        const float r = norm_factor(ss, k, eps);
+        if (!(am * r >= 1e-5f)) mult = r * scale_of(make_float2(ss, am), k, eps);
+    }
     int total = 0;
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
@@ -217,17 +314,30 @@ __device__ __forceinline__ float norm_quant_row(const Cta &c, float4 (&v)[NJ], c
     }
     total = __reduce_add_sync(0xffffffffu, total);
     if (c.lane == 0) atomicAdd(s_sum, total);
-    return sc;
+    return make_float2(ss, am);
 }
 
-// This thread's part of row `row` of what the part in front left into v, added to the residual row x where `add` says so.
-template <int NJ, int NX>
-__device__ __forceinline__ void get_row(const Cta &c, int row, int k, const float *from, bool add, float4 (&x)[NX], float4 (&v)[NJ]) {
+// This thread's part of row `row` of what the part in front left into v, added to the residual row x where `add` says so. The embedded tokens
+// come as they are, everything else as Place<LOOSE> hands it on.
+template <bool LOOSE, int NJ, int NX>
+__device__ __forceinline__ void get_row(const Cta &c, const StepParams &p, int row, int k, const float *from, bool add, float4 (&x)[NX], float4 (&v)[NJ]) {
     const float *src = from + static_cast<size_t>(row) * k;
+    const int n = k >> 2;
+    if (!LOOSE || from == p.x) {
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-        const int i = c.tid + j * kThreads;
-        v[j] = i < (k >> 2) ? ldcg4(src + i * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < NJ; ++j) {
+            const int i = c.tid + j * kThreads;
+            v[j] = i < n ? ldcg4(src + i * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    } else {
+        uint4 u[NJ];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const int i = c.tid + j * kThreads;
+            u[j] = i < n ? Place<LOOSE>::look4(src + i * 4) : Place<LOOSE>::words(make_float4(0.f, 0.f, 0.f, 0.f));
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) v[j] = settle<LOOSE>(c, p, src + (c.tid + j * kThreads) * 4, u[j]);
     }
     if (add) {
 #pragma unroll
@@ -278,16 +388,16 @@ __device__ __forceinline__ void input_phase(const Cta &c, const StepParams &p, i
             wv[j] = i < (k >> 2) ? __ldg(reinterpret_cast<const float4 *>(w) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         wait(c, p, number);
-        get_row(c, row, k, from, (phase & 1) == 0, x, v);
-        const float sc = norm_quant_row<NJ>(c, v, wv, k, kfill, p.eps, SHARED ? p.q8 + static_cast<size_t>(row) * stride : s_xq);
+        get_row<!SHARED>(c, p, row, k, from, (phase & 1) == 0, x, v);
+        const float2 sum_top = norm_quant_row<NJ>(c, v, wv, k, kfill, p.eps, SHARED ? p.q8 + static_cast<size_t>(row) * stride : s_xq);
+        if (SHARED && c.tid == kThreads - 1) p.q8_scale[row] = scale_of(sum_top, k, p.eps);  // beside the other warps' codes
         __syncthreads();
         if (c.tid == 0) {
             if (SHARED) {
-                p.q8_scale[row] = sc;
                 p.q8_sum[row] = *s_codes;
                 count_up(p.q8_ready);
             } else {  // read behind the barrier after the products
-                s_scale[0] = sc;
+                s_scale[0] = scale_of(sum_top, k, p.eps);
                 s_sum[0] = *s_codes;
             }
         }
@@ -295,13 +405,13 @@ __device__ __forceinline__ void input_phase(const Cta &c, const StepParams &p, i
     if (SHARED) {
         if (c.tid == 0) await(c, p, p.q8_ready, codes * p.m);
         __syncthreads();
+        const uint32_t dst = ptx::smem_u32(s_xq);
+        for (int i = c.tid; i < p.m * (stride >> 4); i += kThreads) ptx::cp_async_16(dst + i * 16, p.q8 + static_cast<size_t>(i) * 16);
+        ptx::cp_async_commit();
         if (c.tid < p.m) {
             s_scale[c.tid] = __ldcg(p.q8_scale + c.tid);
             s_sum[c.tid] = __ldcg(p.q8_sum + c.tid);
         }
-        const uint32_t dst = ptx::smem_u32(s_xq);
-        for (int i = c.tid; i < p.m * (stride >> 4); i += kThreads) ptx::cp_async_16(dst + i * 16, p.q8 + static_cast<size_t>(i) * 16);
-        ptx::cp_async_commit();
         ptx::cp_async_wait<0>();
         __syncthreads();
     }
@@ -309,7 +419,7 @@ __device__ __forceinline__ void input_phase(const Cta &c, const StepParams &p, i
 
 // ROW: one sequence, on the integer pipes (consume_stage_row)
 template <int MT, bool ROW>
-__device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p, int phase, const float *ws, Stream &st, uint64_t policy) {
+__device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p, int phase, const float *ws, const Place<ROW> &to, Stream &st, uint64_t policy) {
     const Phase &ph = p.ph[phase];
     const int g = c.lane >> 2, t = c.lane & 3, m = p.m;
     const LaneOffsets off = lane_offsets(c.lane);
@@ -382,7 +492,7 @@ __device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p,
             const int row = ((cta.x >> 1) + tl) * kTileRows + (rest & 15);
             if (row < ph.rows[0]) {
                 const float a = fmaxf(scaled(*gate, tok, wscale[0]), 0.f);
-                ph.out[0][static_cast<size_t>(tok) * ph.rows[0] + row] = a * a * scaled(*up, tok, wscale[1]);
+                to.put(static_cast<size_t>(tok) * ph.rows[0] + row, a * a * scaled(*up, tok, wscale[1]));
             }
             *gate = *up = 0;
         }
@@ -394,8 +504,12 @@ __device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p,
         int mat = 0;
         while (mat < ph.n_mat - 1 && tile_id >= ph.tile_end[mat]) ++mat;
         const int row = (tile_id - (mat ? ph.tile_end[mat - 1] : 0)) * kTileRows + (rest & 15);
-        if (row < ph.rows[mat])
-            ph.out[mat][static_cast<size_t>(tok) * ph.rows[mat] + row] = scaled(s_acc[e], tok, wscale[mat]);
+        if (row < ph.rows[mat]) {
+            const size_t at = static_cast<size_t>(tok) * ph.rows[mat] + row;
+            const float v = scaled(s_acc[e], tok, wscale[mat]);
+            if (phase == 0) ph.out[mat][at] = v;
+            else to.put(at, v);
+        }
         s_acc[e] = 0;
     }
 }
@@ -422,22 +536,31 @@ __device__ __forceinline__ float4 merge_records(const float *from, int n, int st
 // Adds up the slices of every head of every sequence. Up to four slices: a warp per head, a lane four dimensions. More: a warp per eight
 // dimensions of a head, a lane a slice (16 such warps on one SM took 4900 cycles, spread over the SMs 1500). Either way all that a warp
 // needs is asked for at once.
-__device__ __forceinline__ void merge_slices(const Cta &c, const StepParams &p) {
+template <bool LOOSE>
+__device__ __forceinline__ void merge_slices(const Cta &c, const StepParams &p, const float *part_at, const Place<LOOSE> &to) {
+    using At = Place<LOOSE>;
     const int group = p.heads / p.kv_heads, heads = p.m * p.heads, S = p.slices;
     const bool per_warp = S <= 4;
     const int units = per_warp ? heads : heads * (kHead / 8);
     for (int unit = c.warp * gridDim.x + blockIdx.x; unit < units; unit += gridDim.x * kWarps) {
         const int u = per_warp ? unit : unit / (kHead / 8), part = per_warp ? 0 : unit % (kHead / 8);
         const int b = u / p.heads, h = u - b * p.heads, kh = h / group;
-        const float *rec = p.part + (static_cast<size_t>(b * p.kv_heads + kh) * kGroup + (h - kh * group)) * S * kRecord;
-        float *dst = p.attn + static_cast<size_t>(u) * kHead;
+        const float *rec = part_at + (static_cast<size_t>(b * p.kv_heads + kh) * kGroup + (h - kh * group)) * S * kRecord;
+        const size_t dst = static_cast<size_t>(u) * kHead;
         if (per_warp) {
             float2 ml[4];
             float4 v[4];
+            uint2 ml_u[4];
+            uint4 v_u[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                ml[i] = i < S ? __ldcg(reinterpret_cast<const float2 *>(rec + i * kRecord + kHead)) : make_float2(-INFINITY, 0.0f);
-                v[i] = i < S ? ldcg4(rec + i * kRecord + c.lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                ml_u[i] = i < S ? At::look2(rec + i * kRecord + kHead) : make_uint2(At::word(-INFINITY), At::word(0.f));
+                v_u[i] = i < S ? At::look4(rec + i * kRecord + c.lane * 4) : At::words(make_float4(0.f, 0.f, 0.f, 0.f));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                ml[i] = settle<LOOSE>(c, p, rec + i * kRecord + kHead, ml_u[i]);
+                v[i] = settle<LOOSE>(c, p, rec + i * kRecord + c.lane * 4, v_u[i]);
             }
             const float gm = fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x));
             float gs = 0.0f;
@@ -449,12 +572,15 @@ __device__ __forceinline__ void merge_slices(const Cta &c, const StepParams &p) 
                 o.x += f * v[i].x; o.y += f * v[i].y; o.z += f * v[i].z; o.w += f * v[i].w;
             }
             const float inv = 1.0f / gs;
-            reinterpret_cast<float4 *>(dst)[c.lane] = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+            to.put4(dst + c.lane * 4, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv));
         } else {
             const float *r = rec + c.lane * kRecord;
             const bool in = c.lane < S;
-            const float2 ml = in ? __ldcg(reinterpret_cast<const float2 *>(r + kHead)) : make_float2(-INFINITY, 0.0f);
-            const float4 a = in ? ldcg4(r + part * 8) : make_float4(0.f, 0.f, 0.f, 0.f), e = in ? ldcg4(r + part * 8 + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const uint4 none = At::words(make_float4(0.f, 0.f, 0.f, 0.f));
+            const uint2 ml_u = in ? At::look2(r + kHead) : make_uint2(At::word(-INFINITY), At::word(0.f));
+            const uint4 a_u = in ? At::look4(r + part * 8) : none, e_u = in ? At::look4(r + part * 8 + 4) : none;
+            const float2 ml = settle<LOOSE>(c, p, r + kHead, ml_u);
+            const float4 a = settle<LOOSE>(c, p, r + part * 8, a_u), e = settle<LOOSE>(c, p, r + part * 8 + 4, e_u);
             const float gm = warp_max(ml.x), f = ml.x == -INFINITY ? 0.0f : __expf(ml.x - gm);
             float d[9] = {f * a.x, f * a.y, f * a.z, f * a.w, f * e.x, f * e.y, f * e.z, f * e.w, f * ml.y};
 #pragma unroll
@@ -462,14 +588,15 @@ __device__ __forceinline__ void merge_slices(const Cta &c, const StepParams &p) 
 #pragma unroll
                 for (int i = 0; i < 9; ++i) d[i] += __shfl_xor_sync(0xffffffffu, d[i], o);
             const float inv = 1.0f / d[8];
-            if (c.lane == 0) reinterpret_cast<float4 *>(dst)[part * 2] = make_float4(d[0] * inv, d[1] * inv, d[2] * inv, d[3] * inv);
-            if (c.lane == 1) reinterpret_cast<float4 *>(dst)[part * 2 + 1] = make_float4(d[4] * inv, d[5] * inv, d[6] * inv, d[7] * inv);
+            if (c.lane == 0) to.put4(dst + part * 8, make_float4(d[0] * inv, d[1] * inv, d[2] * inv, d[3] * inv));
+            if (c.lane == 1) to.put4(dst + part * 8 + 4, make_float4(d[4] * inv, d[5] * inv, d[6] * inv, d[7] * inv));
         }
     }
 }
 
 // Attention of the step's tokens over the cache (model.rs:334-357), f32 on bf16 keys and values.
-__device__ __forceinline__ void attention_phase(const Cta &c, const StepParams &p, int layer, uint32_t number) {
+template <bool LOOSE>
+__device__ __forceinline__ void attention_phase(const Cta &c, const StepParams &p, int layer, uint32_t number, const Place<LOOSE> &attn, const Place<LOOSE> &part) {
     const int TW = p.team_warps, teams = kWarps / TW, team = c.warp / TW, wt = c.warp % TW, ttid = c.tid - team * TW * 32;
     const int group = p.heads / p.kv_heads, units = p.m * p.kv_heads * p.slices, bar = 1 + team, tthreads = TW * 32;
     const int *s_pos = reinterpret_cast<const int *>(c.sm + c.L.pos);
@@ -507,6 +634,14 @@ __device__ __forceinline__ void attention_phase(const Cta &c, const StepParams &
         }
         if (!valid) {
             if (have && ttid == 0) atomicExch(p.err_word, 7);
+            if (LOOSE && have && wt < group) {  // whoever reads on waits for something
+                if (p.slices == 1) attn.put4((static_cast<size_t>(b) * p.heads + kh * group + wt) * kHead + c.lane * 4, make_float4(0.f, 0.f, 0.f, 0.f));
+                else {
+                    const size_t dst = ((static_cast<size_t>(pair) * kGroup + wt) * p.slices + slice) * kRecord;
+                    part.put4(dst + c.lane * 4, make_float4(0.f, 0.f, 0.f, 0.f));
+                    if (c.lane == 0) part.put2(dst + kHead, make_float2(-INFINITY, 0.f));
+                }
+            }
             continue;
         }
         // x * cos + rotate_half(x) * sin (model.rs:298-302); lane and lane ^ 16 hold the two halves
@@ -603,12 +738,11 @@ __device__ __forceinline__ void attention_phase(const Cta &c, const StepParams &
             const float4 o = merge_records(s_rec + wt * kRecord, TW, kGroup * kRecord, c.lane, gm, gs);
             if (p.slices == 1) {
                 const float inv = 1.0f / gs;
-                reinterpret_cast<float4 *>(p.attn + (static_cast<size_t>(b) * p.heads + kh * group + wt) * kHead)[c.lane] =
-                    make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+                attn.put4((static_cast<size_t>(b) * p.heads + kh * group + wt) * kHead + c.lane * 4, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv));
             } else {
-                float *dst = p.part + ((static_cast<size_t>(pair) * kGroup + wt) * p.slices + slice) * kRecord;
-                reinterpret_cast<float4 *>(dst)[c.lane] = o;
-                if (c.lane == 0) *reinterpret_cast<float2 *>(dst + kHead) = make_float2(gm, gs);
+                const size_t dst = ((static_cast<size_t>(pair) * kGroup + wt) * p.slices + slice) * kRecord;
+                part.put4(dst + c.lane * 4, o);
+                if (c.lane == 0) part.put2(dst + kHead, make_float2(gm, gs));
             }
         }
         ptx::named_barrier(bar, tthreads);  // the records are free again
@@ -675,11 +809,15 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
     }
     __syncthreads();
 
-    const uint32_t number0 = *p.number;
-    uint32_t number = number0, codes = *p.codes;  // barriers and inputs so far
+    constexpr bool LOOSE = !SHARED;
+    uint32_t number = *p.number, codes = *p.codes, turn = *p.turn;  // meetings, inputs and layers so far
     auto meet = [&] {
-        arrive(c, p);
+        arrive_behind<LOOSE>(c, p);
         ++number;
+    };
+    auto place = [&](float *two, size_t floats) {  // this layer's of the two
+        const ptrdiff_t n = static_cast<ptrdiff_t>(floats);
+        return LOOSE && (turn & 1) ? Place<LOOSE>{two + n, -n} : Place<LOOSE>{two, n};
     };
     float4 x[NH];  // the residual row: of the one sequence, or of the sequence that this CTA serves
 #pragma unroll
@@ -693,19 +831,27 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
 #pragma unroll 1
         for (int ph = 0; ph < kPhases; ++ph) {
             input_phase<NI, NH, SHARED>(c, p, ph, from, number, ++codes, info.norm[ph], x);
-            product_phase<MT, !SHARED>(c, p, ph, info.wscale, st, policy);
-            meet();
-            from = p.ph[ph].out[0];
-            if (ph != 0) continue;
-            attention_phase(c, p, l, number);
+            const Place<LOOSE> to = place(p.ph[ph].out[0], static_cast<size_t>(p.m) * p.ph[ph].rows[0]);
+            product_phase<MT, !SHARED>(c, p, ph, info.wscale, to, st, policy);
+            if (ph != 0) {
+                meet();
+                from = to.at;
+                continue;
+            }
+            arrive(c, p);  // the one barrier of the layer: keys, values and queries go on as they are, and the places of the layer before are free
+            ++number;
+            const Place<LOOSE> attn = place(p.attn, static_cast<size_t>(p.m) * p.heads * kHead);
+            const Place<LOOSE> part = place(p.part, static_cast<size_t>(p.m) * p.kv_heads * kGroup * p.slices * kRecord);
+            attention_phase(c, p, l, number, attn, part);
             meet();
             if (p.slices > 1) {
                 wait(c, p, number);
-                merge_slices(c, p);
+                merge_slices(c, p, part.at, attn);
                 meet();
             }
-            from = p.attn;
+            from = attn.at;
         }
+        ++turn;
     }
     wait(c, p, number);
     // the model's last norm, a CTA per row
@@ -713,7 +859,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
         const int k = p.ph[0].k, row = row_cta(blockIdx.x);
         float *s_ss = reinterpret_cast<float *>(c.sm + c.L.part);
         float4 v[NH];
-        get_row(c, row, k, p.ph[3].out[0], true, x, v);
+        get_row<!SHARED>(c, p, row, k, from, true, x, v);
         float ss = 0.0f;
 #pragma unroll
         for (int j = 0; j < NH; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
@@ -737,6 +883,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
     if (c.tid == 0 && atomicAdd(p.exit_count, 1u) == gridDim.x - 1) {  // all have taken the number: the next launch goes on from here
         *p.number = number;
         *p.codes = codes;
+        *p.turn = turn;
         *p.exit_count = 0;
     }
 }
@@ -850,15 +997,16 @@ struct Step {
         };
         auto floats = [&](size_t n) { return reinterpret_cast<float *>(take(n * sizeof(float))); };
         const size_t b = p.m;
-        p.number = reinterpret_cast<uint32_t *>(take(4));
+        p.number = reinterpret_cast<uint32_t *>(take(16));
         p.codes = p.number + 1;
         p.exit_count = p.number + 2;
+        p.turn = p.number + 3;
         p.met = reinterpret_cast<uint32_t *>(take(4));
         p.q8_ready = reinterpret_cast<uint32_t *>(take(4));
         for (int i = 0; i < kPhases; ++i)
-            for (int j = 0; j < (i == 2 ? 1 : p.ph[i].n_mat); ++j) p.ph[i].out[j] = floats(b * p.ph[i].rows[j]);
-        p.attn = floats(b * heads * kHead);
-        p.part = floats(b * kv_heads * kGroup * p.slices * kRecord);
+            for (int j = 0; j < (i == 2 ? 1 : p.ph[i].n_mat); ++j) p.ph[i].out[j] = floats((i ? 2 : 1) * b * p.ph[i].rows[j]);
+        p.attn = floats(2 * b * heads * kHead);
+        p.part = floats(2 * b * kv_heads * kGroup * p.slices * kRecord);
         int chunks = 0;
         for (const Phase &f : p.ph) chunks = f.chunks > chunks ? f.chunks : chunks;
         p.q8 = take(b * row_stride(chunks));
