@@ -28,7 +28,7 @@
 // a step took 1.5 times as long.
 //
 // Measured, a whole step with head and argmax, a kernel per operation -> this: one sequence at 2000 positions, 30 layers of 2560,
-// vocabulary 128256 1309 -> 822 us (of it 110 the head); sixteen sequences at 400 positions, 8 layers, vocabulary 32000 547 -> 383 us. At other widths,
+// vocabulary 128256 1309 -> 787 us (of it 110 the head); sixteen sequences at 400 positions, 8 layers, vocabulary 32000 547 -> 378 us. At other widths,
 // 512 to 8192, with 1 to 16 sequences at 100 and 2000 positions, 1.14 to 2.8 times as fast as a kernel per operation, rings of two stages included.
 #include "lbk_gemv_core.cuh"
 
@@ -598,6 +598,24 @@ __device__ __forceinline__ void merge_slices(const Cta &c, const StepParams &p, 
     }
 }
 
+// Asks for the keys and values that this CTA takes in `layer`'s attention to come to L2, a layer ahead: asked for behind the q/k/v products they
+// queued behind the weights of the next projections, which every SM fetches at that time, and the slowest slice was twice the usual one. 30 layers of 2560
+// at 2000 positions 799 -> 787 us a step, 16 sequences at 400, eight layers 385 -> 378.
+__device__ __forceinline__ void call_cache(const Cta &c, const StepParams &p, int layer) {
+    const int TW = p.team_warps, teams = kWarps / TW, team = c.warp / TW, units = p.m * p.kv_heads * p.slices;
+    if (c.tid - team * TW * 32 != 0) return;
+    const int *s_pos = reinterpret_cast<const int *>(c.sm + c.L.pos);
+    for (int unit = blockIdx.x * teams + team; unit < units; unit += gridDim.x * teams) {
+        const int pair = unit / p.slices, slice = unit - pair * p.slices, b = pair / p.kv_heads, kh = pair - b * p.kv_heads, pos = s_pos[b];
+        const int per = (pos + p.slices) / p.slices, p0 = slice * per, p1 = min(min(pos, p.cap), p0 + per);  // rows of earlier tokens
+        if (p1 <= p0) continue;
+        const size_t at = static_cast<size_t>(layer) * p.layer_stride + ((static_cast<size_t>(b) * p.kv_heads + kh) * p.cap + p0) * kHead;
+        const uint32_t bytes = static_cast<uint32_t>(p1 - p0) * kHead * 2;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.kcache + at), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.vcache + at), "r"(bytes) : "memory");
+    }
+}
+
 // Attention of the step's tokens over the cache (model.rs:334-357), f32 on bf16 keys and values.
 template <bool LOOSE>
 __device__ __forceinline__ void attention_phase(const Cta &c, const StepParams &p, int layer, uint32_t number, const Place<LOOSE> &attn, const Place<LOOSE> &part) {
@@ -827,6 +845,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
 #pragma unroll
     for (int j = 0; j < NH; ++j) x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     const float *from = p.x;
+    call_cache(c, p, 0);
     // One copy of each part's code for all layers and projections: instructions that are fetched once a layer come from L2 otherwise.
 #pragma unroll 1
     for (int l = 0; l < p.layers; ++l) {
@@ -854,6 +873,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
                 meet();
             }
             from = attn.at;
+            if (l + 1 < p.layers) call_cache(c, p, l + 1);
         }
         ++turn;
     }
