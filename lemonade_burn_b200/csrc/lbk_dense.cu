@@ -44,6 +44,12 @@ using few::kWarps;
 constexpr int kFewPreMax = 2;               // tokens whose norms run in the prologue
 constexpr int kFewPrefetch = 8;             // boxes beyond its ring that a warp asks L2 for ahead of the kernel in front
 
+// Bytes of the next projections' weights that a call asks L2 for when its own are all on their way: between two projections of a step, in their first
+// and last trips, the norms, attention or a recurrence, HBM would idle. More of them are in the way of what those kernels read themselves. Steps of
+// one sequence / eight with experts / sixteen of the mixed family, none asked for: 225 / 226 / 301 us; 8 MB 220 / 224 / 296, 12 219 / 223 / 290, 16 218 / 222 / 288,
+// 24 218 / 224 / 290, 48 230 / 226 / 306. Up to 24 or 36 in front of attention alone: 219 / 224 / 293.
+constexpr size_t kFewAhead = 16u << 20;
+
 struct FewParams {
     alignas(64) CUtensorMap w;              // bytes [rows][pitch * 2], box [box_rows][128]
     int out_rows, up_row, chunks, m;        // chunks of 64 columns
@@ -52,6 +58,8 @@ struct FewParams {
     long ldx;
     DenseEpi epi;
     DensePre pre;
+    const uint8_t *ahead[2];                // the next projections' weights
+    uint32_t ahead_bytes[2];                // of them, multiples of 128
     int n, xs_stride;                       // columns of the normed row; bytes between such rows in shared memory
     int *err_word;
 };
@@ -175,6 +183,14 @@ __global__ void __launch_bounds__(kThreads, 1) dense_few_kernel(const __grid_con
         ring.fetch(slot, &p.w, is.c * 128, row_of(is));
         step(is);
     };
+    // behind this warp's last box: its share of the next projections' weights
+    auto call_ahead = [&] {
+        const uint32_t all = gridDim.x * kWarps, who = blockIdx.x * kWarps + warp;
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t bytes = p.ahead_bytes[i], piece = ((bytes + all - 1) / all + 127) & ~127u;
+            if (static_cast<uint64_t>(piece) * who < bytes) ptx::prefetch_l2(p.ahead[i] + static_cast<size_t>(piece) * who, min(piece, bytes - piece * who));
+        }
+    };
     // The weights are constants: this warp's first boxes are on their way, and more of them asked into L2, while the kernel
     // in front finishes.
     if (lane == 0) {
@@ -185,6 +201,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_few_kernel(const __grid_con
             few::prefetch_box(&p.w, ahead.c * 128, row_of(ahead));
             step(ahead);
         }
+        if (total <= ring.depth) call_ahead();
     }
     FewGains gains;
     if (p.pre.mode != kPreNone) gains.load(p);
@@ -227,7 +244,10 @@ __global__ void __launch_bounds__(kThreads, 1) dense_few_kernel(const __grid_con
                 if (k < boxes * NA) {
                     few::box_mma<NTL, MT>(ring.wait(), units, x, acc + k * MT);
                     __syncwarp();           // every lane has read the box before it is refilled
-                    if (lane == 0 && done + ring.depth < total) load(ring.s);
+                    if (lane == 0 && done + ring.depth < total) {
+                        load(ring.s);
+                        if (done + ring.depth + 1 == total) call_ahead();
+                    }
                     ++done;
                     ring.next();
                 }
@@ -681,6 +701,14 @@ int launch_few(Ctx *ctx, const DenseCall &c, cudaStream_t st) {
     p.ldx = c.ldx;
     p.epi = c.epi;
     p.pre = c.pre;
+    size_t left = kFewAhead;
+    for (int i = 0; i < 2; ++i) {
+        const bool asked = c.ahead[i].w && (reinterpret_cast<uintptr_t>(c.ahead[i].w) & 15) == 0;
+        const size_t bytes = asked ? std::min(left, c.ahead[i].rows * c.ahead[i].pitch * 2) / 128 * 128 : 0;
+        p.ahead[i] = reinterpret_cast<const uint8_t *>(c.ahead[i].w);
+        p.ahead_bytes[i] = static_cast<uint32_t>(bytes);
+        left -= bytes;
+    }
     p.n = static_cast<int>(c.w.cols);
     p.xs_stride = static_cast<int>(c.w.pitch * 2 + 16);  // neighbouring token rows start in different bank groups
     p.err_word = ctx->err_word;

@@ -64,6 +64,7 @@ struct DenseCall {
     size_t up_row = 0, out_rows = 0;
     DenseEpi epi;
     DensePre pre;
+    DenseWeight ahead[2];  // what the next projections read: a call of up to 16 tokens asks for its first bytes to come to L2
     // experts: w holds `experts` matrices stacked group_rows apart; tokens sorted by expert, expert e's are
     // x rows offs[e] .. offs[e+1]-1 (device) and so are its output rows
     int experts = 0;

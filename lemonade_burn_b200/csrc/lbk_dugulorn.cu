@@ -254,6 +254,8 @@ int DugulornModel::enqueue_latent(const Pass &p, const DugulornLayer &l) {
     d.epi.dimp = static_cast<int>(s.qp());
     d.epi.q_split = static_cast<int>(s.dim);
     d.epi.q_gap = static_cast<int>(s.dp() - s.dim);
+    d.ahead[0] = l.o;
+    d.ahead[1] = l.up;
     LBK_TRY(launch_dense(ctx, d, p.st));
     LatentAttnCall a;
     a.compute = compute;
@@ -421,8 +423,10 @@ int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *toke
         return launch_dense(ctx, d, st);
     };
     // the last projection of a sublayer: its rows wait for their norm
-    auto leave = [&](const void *in, const DenseWeight &wt, const float *bias, const float *norm) -> int {
+    auto leave = [&](const void *in, const DenseWeight &wt, const float *bias, const float *norm, const DenseWeight &next, const DenseWeight &then) -> int {
         DenseCall d;
+        d.ahead[0] = next;
+        d.ahead[1] = then;
         d.compute = compute;
         d.m = m;
         d.x = in;
@@ -465,9 +469,12 @@ int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *toke
                 if (!y) LBK_TRY(norm_rows(nullptr, w.n, nullptr));  // the rows as the projection reads them, from the front
             }
         }
+        const DenseWeight none, &next = li + 1 < layers.size() ? layers[li + 1].in : head;  // behind this layer
         DenseCall d;
         d.w = l.in;
         d.out_rows = l.in.rows;
+        d.ahead[0] = l.type == Mixer::Latent ? l.uq : l.o;
+        d.ahead[1] = l.type == Mixer::Latent ? l.o : l.ff ? l.up : none;
         if (l.type == Mixer::Latent) {
             d.epi.kind = kEpiF32;
             d.epi.out = w.z;
@@ -494,10 +501,12 @@ int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *toke
             mid += first * l.o.pitch * elem();
             leave_out(first);
         }
-        LBK_TRY(leave(mid, l.o, nullptr, l.norm1));
+        LBK_TRY(leave(mid, l.o, nullptr, l.norm1, l.ff ? l.up : next, l.ff ? l.down : none));
         if (l.ff) {
             DenseCall u;
             u.w = l.up;
+            u.ahead[0] = l.down;
+            u.ahead[1] = next;
             u.out_rows = l.ff;
             u.epi.kind = kEpiElem;
             u.epi.act = kActRelu2;
@@ -505,7 +514,7 @@ int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *toke
             u.epi.out = w.h;
             u.epi.ld = static_cast<long>(l.down.pitch);
             LBK_TRY(project(u));
-            LBK_TRY(leave(w.h, l.down, l.down_bias, l.norm2));
+            LBK_TRY(leave(w.h, l.down, l.down_bias, l.norm2, next, none));
         }
     }
     return norm_rows(final_norm, nullptr, final_rows);

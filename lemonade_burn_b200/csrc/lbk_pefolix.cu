@@ -191,8 +191,10 @@ int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens
         have_moe = false;
         return LBK_OK;
     };
-    auto rows_f32 = [&](const void *in, const DenseWeight &wt, float *out) -> int {
+    auto rows_f32 = [&](const void *in, const DenseWeight &wt, float *out, const DenseWeight &next, const DenseWeight &then) -> int {
         DenseCall d;
+        d.ahead[0] = next;
+        d.ahead[1] = then;
         d.compute = compute;
         d.m = m;
         d.x = in;
@@ -208,9 +210,14 @@ int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens
     for (size_t li = 0; li < layers.size(); ++li) {
         const PefolixLayer &l = layers[li];
         const char *attn = static_cast<const char *>(w.attn);
+        const bool ends = li + 1 == layers.size();
+        const DenseWeight none, &next = ends ? head : layers[li + 1].qkv, &then = ends ? none : layers[li + 1].o;  // behind this layer
+        const DenseWeight &mid = l.kind == PefolixLayer::Dense ? l.gate_up : l.kind == PefolixLayer::Moe ? l.in : next;  // behind its attention
         {
             DenseCall d;
             d.w = l.qkv;
+            d.ahead[0] = l.o;
+            d.ahead[1] = mid;
             d.out_rows = l.qkv.rows;
             d.epi.kind = kEpiQkv;
             d.epi.out = w.q;
@@ -275,19 +282,21 @@ int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens
                 fuse = !f32 && dense_pre_supported(m, width);
             }
         }
-        LBK_TRY(rows_f32(attn, l.o, w.y));
+        LBK_TRY(rows_f32(attn, l.o, w.y, mid, l.kind == PefolixLayer::Dense ? l.down : none));
         y = w.y;
         w_post = l.norm1b;
         if (l.kind == PefolixLayer::Dense) {
             DenseCall d;
             d.w = l.gate_up;
+            d.ahead[0] = l.down;
+            d.ahead[1] = next;
             d.gated = true;
             d.up_row = d.out_rows = l.ff;
             d.epi.kind = kEpiElem;
             d.epi.out = w.h;
             d.epi.ld = static_cast<long>(l.down.pitch);
             LBK_TRY(project(d, l.norm2, false));
-            LBK_TRY(rows_f32(w.h, l.down, w.y));
+            LBK_TRY(rows_f32(w.h, l.down, w.y, next, then));
             y = w.y;
             w_post = l.norm2b;
         } else if (l.kind == PefolixLayer::Moe) {
@@ -353,7 +362,7 @@ int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens
                 dn.epi.out = w.eo;
                 dn.epi.ld = npitch;
                 LBK_TRY(launch_dense(ctx, dn, st));
-                if (l.sff) LBK_TRY(rows_f32(w.hs, l.sdown, w.ys));
+                if (l.sff) LBK_TRY(rows_f32(w.hs, l.sdown, w.ys, none, none));
                 moe = MoeOut{};
                 if (f32) moe.rows32 = static_cast<const float *>(w.eo);
                 else moe.rows16 = static_cast<const uint16_t *>(w.eo);

@@ -138,6 +138,11 @@ __device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, 
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// asks for `bytes` (a multiple of 16, as the address) to come to L2
+__device__ __forceinline__ void prefetch_l2(const void *at, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"(bytes) : "memory");
+}
+
 // 16 bytes global -> shared without passing through registers; completion by groups
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");

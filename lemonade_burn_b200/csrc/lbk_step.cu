@@ -611,8 +611,8 @@ __device__ __forceinline__ void call_cache(const Cta &c, const StepParams &p, in
         if (p1 <= p0) continue;
         const size_t at = static_cast<size_t>(layer) * p.layer_stride + ((static_cast<size_t>(b) * p.kv_heads + kh) * p.cap + p0) * kHead;
         const uint32_t bytes = static_cast<uint32_t>(p1 - p0) * kHead * 2;
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.kcache + at), "r"(bytes) : "memory");
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.vcache + at), "r"(bytes) : "memory");
+        ptx::prefetch_l2(p.kcache + at, bytes);
+        ptx::prefetch_l2(p.vcache + at, bytes);
     }
 }
 
