@@ -347,6 +347,12 @@ bool json_positive(const Json *j, size_t *out);
 struct Model;
 
 // The sequences ("slots") a model serves together. The family's class adds its K/V rows and work buffers.
+// Where a caller wants the results of the step that is being launched; null: nowhere.
+struct StepOut {
+    float *logits = nullptr;
+    int32_t *next = nullptr;
+};
+
 struct Cache {
     Model *model = nullptr;
     size_t b = 0, cap = 0;
@@ -356,6 +362,10 @@ struct Cache {
     std::vector<size_t> lens;             // the lengths again, on the host
     int32_t *tokens = nullptr, *next = nullptr;
     float *logits = nullptr;              // [b][vocab] of the last decode step
+    float *part_v = nullptr;              // what the step's last kernel works with (pick_kernel); zeros between launches: parts_done, out
+    int *part_i = nullptr;
+    unsigned *parts_done = nullptr;
+    StepOut *out = nullptr;
     cudaGraphExec_t step = nullptr;       // the recorded decode step
     uint64_t step_launches = 0;           // kernels in it
     std::vector<void *> device_allocs;
