@@ -603,7 +603,7 @@ __device__ __forceinline__ void merge_slices(const Cta &c, const StepParams &p, 
 // at 2000 positions 799 -> 787 us a step, 16 sequences at 400, eight layers 385 -> 378.
 __device__ __forceinline__ void call_cache(const Cta &c, const StepParams &p, int layer) {
     const int TW = p.team_warps, teams = kWarps / TW, team = c.warp / TW, units = p.m * p.kv_heads * p.slices;
-    if (c.tid - team * TW * 32 != 0) return;
+    if (c.tid - team * TW * 32 != 0 || p.layer_stride % 8) return;  // a bulk prefetch starts on 16 bytes; the loads themselves need 8
     const int *s_pos = reinterpret_cast<const int *>(c.sm + c.L.pos);
     for (int unit = blockIdx.x * teams + team; unit < units; unit += gridDim.x * teams) {
         const int pair = unit / p.slices, slice = unit - pair * p.slices, b = pair / p.kv_heads, kh = pair - b * p.kv_heads, pos = s_pos[b];
