@@ -389,9 +389,10 @@ int lbk_relu2_mul_rms_norm(lbk_ctx *ctx, const float *g_dev, const float *u_dev,
  * lbk_step_stream_supported: whether the launch can be made on `stream`: not where the stream's green context has a part of the
  * device's multiprocessors (lbk_step_run then returns LBK_ERR_UNSUPPORTED).
  * lbk_step_run: x f32 [b, hidden]; caches bf16 [layers][b][kv_heads][cap][128], `layer_elems` elements a layer, in which the
- * new rows are appended; cos/sin f32 [max_pos][128]; positions pos[i * pos_stride]; work: lbk_step_work_bytes bytes that
- * are zero before the first run and shared only by launches that come one after another: they count the launches' arrivals, and after
- * launches that overlapped they have to be made zeros again (one that gave up leaves them as a good one does); out f32 [b, hidden].
+ * new rows are appended; cos/sin f32 [max_pos][128]; positions pos[i * pos_stride]; work: lbk_step_work_bytes bytes or more that
+ * are zero before the first run and shared only by launches that come one after another, of whatever steps, numbers of sequences and
+ * capacities: they count the launches' arrivals, and after launches that overlapped they have to be made zeros again (one that gave up leaves
+ * them as a good one does); out f32 [b, hidden].
  * All buffers 16-byte aligned. The blocks of the launch wait on one another (a cooperative launch), each wait bounded:
  * LBK_ERR_TIMEOUT from lbk_check_device_error.
  * lbk_step_set_wait_limit: polls before such a wait gives up, for launches from now on (default 2^20, about a second). */

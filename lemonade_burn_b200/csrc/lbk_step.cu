@@ -84,8 +84,11 @@ struct StepParams {
     uint8_t *q8;                // [m][row] codes in fragment order
     float *q8_scale;
     int32_t *q8_sum;
-    // of all launches so far: barriers, inputs of projections, arrivals at barriers, rows of codes; and the CTAs that have left this one
+    // of all launches so far: meetings, rows of codes, layers; arrivals at meetings, rows of codes that are there; and the CTAs that have left this one
     uint32_t *number, *codes, *turn, *met, *q8_ready, *exit_count;
+    uint64_t layout, *held;     // the sizes that the places lie by, in this launch and in the one before it on this buffer
+    uint4 *places;              // all that Place stands for: behind the q/k/v rows, up to the codes
+    uint32_t place_words;       // 16 bytes each
     int *err_word;
     uint32_t poll_limit;
     Phase ph[kPhases];
@@ -370,7 +373,7 @@ struct Stream {
     }
 };
 
-// From the barrier in front (the number-th) to codes (the codes-th of every row), scales and sums of all rows in shared memory.
+// From the barrier in front (the number-th) to codes, scales and sums of all rows in shared memory (SHARED: the last of `codes` rows so far).
 template <int NJ, int NX, bool SHARED>
 __device__ __forceinline__ float2 input_phase(const Cta &c, const StepParams &p, int phase, const float *from, uint32_t number, uint32_t codes, const float *w, float4 (&x)[NX]) {
     const Phase &ph = p.ph[phase];
@@ -403,7 +406,7 @@ __device__ __forceinline__ float2 input_phase(const Cta &c, const StepParams &p,
         }
     }
     if (SHARED) {
-        if (c.tid == 0) await(c, p, p.q8_ready, codes * p.m);
+        if (c.tid == 0) await(c, p, p.q8_ready, codes);
         __syncthreads();
         const uint32_t dst = ptx::smem_u32(s_xq);
         for (int i = c.tid; i < p.m * (stride >> 4); i += kThreads) ptx::cp_async_16(dst + i * 16, p.q8 + static_cast<size_t>(i) * 16);
@@ -832,7 +835,11 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
     __syncthreads();
 
     constexpr bool LOOSE = !SHARED;
-    uint32_t number = *p.number, codes = *p.codes, turn = *p.turn;  // meetings, inputs and layers so far
+    uint32_t number = *p.number, codes = *p.codes, turn = *p.turn;  // meetings, rows of codes and layers so far
+    // A launch of other sizes has left its values where this one's places lie: they are cleared, by all, in front of the first barrier, behind which
+    // the first place is written or looked at. (With several sequences values do not tell whether they are there.)
+    if (LOOSE && *p.held != p.layout)
+        for (uint32_t i = blockIdx.x * kThreads + c.tid; i < p.place_words; i += gridDim.x * kThreads) p.places[i] = make_uint4(0u, 0u, 0u, 0u);
     auto meet = [&] {
         arrive_behind<LOOSE>(c, p);
         ++number;
@@ -853,7 +860,8 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
         if (l + 1 < p.layers) c.fetch_info(p.table, l + 1);
 #pragma unroll 1
         for (int ph = 0; ph < kPhases; ++ph) {
-            const float2 row = input_phase<NI, NH, SHARED>(c, p, ph, from, number, ++codes, info.norm[ph], x);
+            if (SHARED) codes += p.m;
+            const float2 row = input_phase<NI, NH, SHARED>(c, p, ph, from, number, codes, info.norm[ph], x);
             const Place<LOOSE> to = place(p.ph[ph].out[0], static_cast<size_t>(p.m) * p.ph[ph].rows[0]);
             product_phase<MT, !SHARED>(c, p, ph, row, info.wscale, to, st, policy);
             if (ph != 0) {
@@ -908,6 +916,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
         *p.number = number;
         *p.codes = codes;
         *p.turn = turn;
+        *p.held = p.layout;
         *p.exit_count = 0;
     }
 }
@@ -1011,7 +1020,7 @@ struct Step {
         if (p.slices > kMaxSlices) p.slices = kMaxSlices;
         return true;
     }
-    // places in the work buffer, all of which has to start as zeros
+    // places in the work buffer, which has to start as zeros
     size_t carve(StepParams &p, uint8_t *base) const {
         size_t at = 0;
         auto take = [&](size_t bytes) {
@@ -1021,16 +1030,22 @@ struct Step {
         };
         auto floats = [&](size_t n) { return reinterpret_cast<float *>(take(n * sizeof(float))); };
         const size_t b = p.m;
-        p.number = reinterpret_cast<uint32_t *>(take(16));
+        p.number = reinterpret_cast<uint32_t *>(take(24));
         p.codes = p.number + 1;
         p.exit_count = p.number + 2;
         p.turn = p.number + 3;
+        p.held = reinterpret_cast<uint64_t *>(p.number + 4);
         p.met = reinterpret_cast<uint32_t *>(take(4));
         p.q8_ready = reinterpret_cast<uint32_t *>(take(4));
         for (int i = 0; i < kPhases; ++i)
             for (int j = 0; j < (i == 2 ? 1 : p.ph[i].n_mat); ++j) p.ph[i].out[j] = floats((i ? 2 : 1) * b * p.ph[i].rows[j]);
         p.attn = floats(2 * b * heads * kHead);
         p.part = floats(2 * b * kv_heads * kGroup * p.slices * kRecord);
+        p.places = reinterpret_cast<uint4 *>(p.ph[1].out[0]);
+        p.place_words = static_cast<uint32_t>((base + at - reinterpret_cast<uint8_t *>(p.places)) / 16);
+        // every size that `take` saw so far, none of them 0: hidden and inner are multiples of 4 and at most 8192 and 16384, heads at most 64
+        p.layout = static_cast<uint64_t>(b) | static_cast<uint64_t>(p.slices) << 8 | static_cast<uint64_t>(heads) << 16 | static_cast<uint64_t>(kv_heads) << 24 |
+                   static_cast<uint64_t>(hidden) << 32 | static_cast<uint64_t>(inner) << 48;
         int chunks = 0;
         for (const Phase &f : p.ph) chunks = f.chunks > chunks ? f.chunks : chunks;
         p.q8 = take(b * row_stride(chunks));

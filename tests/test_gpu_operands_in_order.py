@@ -1,0 +1,59 @@
+"""Weights that a kernel of this library writes right in front of the call that reads them. The kernels start beside the end of the one in front
+(programmatic launches, each lets the next start at once), so a call that read its weights ahead would get what they were before: a head
+of many rows keeps the writer waiting for some hundred microseconds, time enough for the reader to be there. Equality: the same call once all is settled."""
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+class Front:
+    """Keeps the device busy: a launch whose end what follows on the stream has to wait for."""
+
+    def __init__(self, ctx):
+        import torch
+        self.ctx, self.w = ctx, torch.zeros(160000, 2560, dtype=torch.bfloat16, device="cuda")
+        self.x, self.out = torch.ones(1, 2560, device="cuda"), torch.empty(1, 160000, device="cuda")
+
+    def launch(self, st):
+        from lemonade_burn_b200 import _lib
+        _lib.check(_lib.load().lbk_bf16_linear(self.ctx.handle, self.x.data_ptr(), 1, self.w.data_ptr(), 160000, 2560, self.out.data_ptr(), st))
+
+    def vector(self, src, dst, st):
+        """dst = src by a kernel: x += y on zeros."""
+        from lemonade_burn_b200 import _lib
+        _lib.check(_lib.load().lbk_add_inplace(self.ctx.handle, dst.data_ptr(), src.data_ptr(), src.numel(), st))
+
+
+@pytest.fixture(scope="module")
+def front(ctx):
+    return Front(ctx)
+
+
+@pytest.mark.parametrize("kv,cap", [(1, 1), (2, 64), (8, 512)])
+def test_head_over_rows_just_appended(ctx, front, kv, cap):
+    """lbk_bf16_linear of one row over cache rows that lbk_rope_kv_append writes."""
+    import torch
+    from lemonade_burn_b200 import _lib
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(kv + cap)
+    table = torch.randn(kv * cap, 128, generator=g, device="cuda").to(torch.bfloat16)
+    other = torch.zeros_like(table)
+    q, k, v = (torch.randn(1, n * 128, generator=g, device="cuda") for n in (kv, kv, kv))
+    cos, sin = torch.ones(cap, 128, device="cuda"), torch.zeros(cap, 128, device="cuda")
+    pos, x = torch.tensor([cap - 1], dtype=torch.int32, device="cuda"), torch.randn(1, 128, generator=g, device="cuda")
+    got, want = torch.empty(1, kv * cap, device="cuda"), torch.empty(1, kv * cap, device="cuda")
+    head = lambda out: _lib.check(lib.lbk_bf16_linear(ctx.handle, x.data_ptr(), 1, table.data_ptr(), kv * cap, 128, out.data_ptr(), st))  # noqa: E731
+    for _ in range(5):
+        table[cap - 1::cap] = 0  # the rows that are appended
+        torch.cuda.synchronize()
+        front.launch(st)
+        _lib.check(lib.lbk_rope_kv_append(ctx.handle, q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), 1, kv, kv, 128, cap,
+                                          table.data_ptr(), other.data_ptr(), st))
+        head(got)
+        torch.cuda.synchronize()
+        head(want)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and bool((want[0, cap - 1::cap] != 0).all())
+    ctx.check_device_error()
