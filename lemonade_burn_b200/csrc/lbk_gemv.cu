@@ -359,8 +359,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
             break;
         }
         consume_stage<MT>(stage_ptr + s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
-        __syncwarp();  // every lane has read the stage before it is refilled
-        if (lane == 0 && item + kStages < n_items) issue(s);
+        const bool free = stage_read<MT>(acc);
+        if (free && lane == 0 && item + kStages < n_items) issue(s);
         if (++s == kStages) {
             s = 0;
             phase ^= 1;

@@ -259,6 +259,13 @@ __device__ __forceinline__ void consume_stage_row(const uint8_t *st, LaneOffsets
         }
     }
 }
+// Whether a stage whose words went into `acc` may be filled again: yes, once it answers. A load that has been issued may still be on its way when a bulk copy
+// issued behind it lands, so the copy has to hang on what became of the loads, in every lane: no sum is INT_MIN apart from another (a k-group of
+// factor 1 is at most 384 times the columns), which the compiler does not know.
+__device__ __forceinline__ bool stage_read(int low, int high) { return __all_sync(0xffffffffu, (low ^ high) != static_cast<int>(0x80000000u)); }
+__device__ __forceinline__ bool stage_read(const int (&acc)[2][4]) { return stage_read(acc[0][0], acc[1][0]); }  // rows g and g + 8 of the stage
+template <int MT>
+__device__ __forceinline__ bool stage_read(const int (&acc)[MT][2][4][4]) { return stage_read(acc[0][0][0][0], acc[0][0][0][2]); }
 // the complete sum of a row of the tile: over the k-groups, undoing the 4^k scaling as take_acc does, and over the four lanes of the row
 __device__ __forceinline__ int sum_row(const int (&acc)[4]) {
     int v = acc[0] + (acc[1] >> 2) + (acc[2] >> 4) + (acc[3] >> 6);

@@ -455,10 +455,15 @@ __device__ __forceinline__ void product_phase(const Cta &c, const StepParams &p,
     int tile = run.x, chunk = run.y;
     for (int item = 0; item < run.z; ++item) {
         if (!ptx::mbar_wait(st.bars + st.s * 8, st.phase, kWaitLimit)) st.ok = false;
-        if constexpr (ROW) consume_stage_row(st.ptr + st.s * kStageBytes, off, xrow[0], static_cast<uint32_t>(chunk) * kChunkCols, sums);
-        else consume_stage<MT>(st.ptr + st.s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
-        __syncwarp();  // every lane has read the stage before it is refilled
-        if (c.lane == 0) st.issue(p, st.s, policy);
+        bool free;
+        if constexpr (ROW) {
+            consume_stage_row(st.ptr + st.s * kStageBytes, off, xrow[0], static_cast<uint32_t>(chunk) * kChunkCols, sums);
+            free = stage_read(sums);
+        } else {
+            consume_stage<MT>(st.ptr + st.s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
+            free = stage_read<MT>(acc);
+        }
+        if (free && c.lane == 0) st.issue(p, st.s, policy);
         if (++st.s == st.depth) {
             st.s = 0;
             st.phase ^= 1;

@@ -311,8 +311,8 @@ __global__ void __launch_bounds__(kThreads, 1) sweep_kernel(const SweepParams p)
             }
             if (chunk == c0) consume_stage_row<true>(stage_ptr + s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
             else consume_stage_row<false>(stage_ptr + s * kStageBytes, off, xrow, static_cast<uint32_t>(chunk) * kChunkCols, acc);
-            __syncwarp();  // every lane has read the stage before it is refilled
-            if (lane == 0 && issued < n_stages) issue(s);
+            const bool free = stage_read(acc);
+            if (free && lane == 0 && issued < n_stages) issue(s);
             if (++s == kSweepStages) {
                 s = 0;
                 phase ^= 1;
