@@ -300,7 +300,10 @@ int lbk_ternary_relu2_gemm_dev(lbk_ctx *ctx, const lbk_weight *gate, const lbk_w
                                const int32_t *sum_dev, size_t m, float *out_dev, void *stream);
 
 /* bf16_linear (crates/lb-model/src/ops.rs:199-218): x f32 [m, cols] @ W^T, W bf16
- * [rows, cols] -> out f32 [m, rows], all device memory. */
+ * [rows, cols] -> out f32 [m, rows], all device memory. Kernels of this library start beside the end of the one in front of
+ * them on the stream and wait for it before they touch what it may write or read, with one exception: weight matrices are read
+ * ahead by lbk_bf16_linear of two and more rows (w), lbk_dense_linear and lbk_dense_linear_act (w) and lbk_latent_attn (ukv), so
+ * whatever wrote those has to be complete when the call is made. */
 int lbk_bf16_linear(lbk_ctx *ctx, const float *x_dev, size_t m, const uint16_t *w_dev, size_t rows,
                     size_t cols, float *out_dev, void *stream);
 

@@ -81,11 +81,11 @@ __global__ void __launch_bounds__(kThreads) bf16_linear_kernel(const float *__re
 }
 
 // One token row, whole 16-byte units: a warp takes two table rows at a time, U units of each a lane in flight together, and the first
-// ones are on their way before the kernel in front is known to be complete. Bound: HBM, rows * cols * 2 bytes. The kernel above, one row a
+// ones are on their way before the kernel in front is known to be complete where the caller vouches that no such kernel writes the table (`settled`). Bound: HBM, rows * cols * 2 bytes. The kernel above, one row a
 // warp with four units in flight, reads the table at 3.8 to 4.8 TB/s, this one at 6.4 to 7.0: 128256 x 2560 144 -> 96 us, 32000 x 2560 42.6 -> 25.6,
 // 32000 x 4096 58.9 -> 41.0, 32000 x 1000 26.2 -> 10.9. Same order of every sum, same bits.
 template <int U>
-__global__ void __launch_bounds__(kThreads, 3) bf16_row_kernel(const float *x, const uint16_t *__restrict__ w, int rows, int cols, float *out) {
+__global__ void __launch_bounds__(kThreads, 3) bf16_row_kernel(const float *x, const uint16_t *w, int rows, int cols, float *out, int settled) {
     extern __shared__ float s_x[];
     const int tid = threadIdx.x, lane = tid & 31, step = 2 * static_cast<int>(gridDim.x) * (kThreads / 32), units = cols >> 3;
     int r = 2 * (static_cast<int>(blockIdx.x) * (kThreads / 32) + (tid >> 5));
@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(kThreads, 3) bf16_row_kernel(const float *x, c
             b[j] = i < units ? __ldcs(wb + i) : make_uint4(0u, 0u, 0u, 0u);
         }
     };
+    if (!settled) ptx::pdl_wait();
     if (r < rows) load(r, 0);
     ptx::pdl_trigger();
     ptx::pdl_wait();
@@ -403,7 +404,7 @@ static int launch_bf16_head_tc(Ctx *ctx, const float *x, size_t m, const uint16_
 }
 
 int launch_bf16_linear(Ctx *ctx, const float *x, size_t m, const uint16_t *w, size_t rows,
-                       size_t cols, float *out, cudaStream_t stream) {
+                       size_t cols, float *out, cudaStream_t stream, bool settled) {
     if (m == 0 || rows == 0) return LBK_OK;
     if (m >= 2 && (cols & 7) == 0 && cols <= kTcMaxCols && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (reinterpret_cast<uintptr_t>(x) & 7) == 0)
         return launch_bf16_head_tc(ctx, x, m, w, rows, cols, out, stream);
@@ -413,9 +414,9 @@ int launch_bf16_linear(Ctx *ctx, const float *x, size_t m, const uint16_t *w, si
     if (m == 1 && cols != 0 && (cols & 7) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && smem1 <= 64 * 1024) {
         // as many units in flight as divide a row's: 5 at 2560 columns, else 4
         const size_t per = (cols / 8 + 31) / 32;
-        void (*k)(const float *, const uint16_t *, int, int, float *) = per % 5 == 0 ? bf16_row_kernel<5> : bf16_row_kernel<4>;
+        void (*k)(const float *, const uint16_t *, int, int, float *, int) = per % 5 == 0 ? bf16_row_kernel<5> : bf16_row_kernel<4>;
         if (smem1 > 48 * 1024) LBK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        LBK_CUDA(launch_chained(k, dim3(static_cast<unsigned>(ctx->sm_count * 3)), dim3(kThreads), smem1, stream, x, w, static_cast<int>(rows), static_cast<int>(cols), out));
+        LBK_CUDA(launch_chained(k, dim3(static_cast<unsigned>(ctx->sm_count * 3)), dim3(kThreads), smem1, stream, x, w, static_cast<int>(rows), static_cast<int>(cols), out, settled ? 1 : 0));
         LBK_CUDA(cudaGetLastError());
         ctx->launches++;
         return LBK_OK;

@@ -38,7 +38,7 @@ struct BitNetModel : Model {
     int enqueue_step(Cache *c, cudaStream_t st) override;
     int enqueue_rows(Cache *c, size_t seq, size_t n, size_t first, cudaStream_t st) override;
     int enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) override {
-        return lbk_bf16_linear(reinterpret_cast<lbk_ctx *>(ctx), rows, n, embed, cfg.vocab_size, cfg.hidden_size, logits, st);
+        return launch_bf16_linear(ctx, rows, n, embed, cfg.vocab_size, cfg.hidden_size, logits, st, true);
     }
 };
 

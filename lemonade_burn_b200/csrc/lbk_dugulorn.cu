@@ -533,7 +533,7 @@ int DugulornModel::enqueue_rows(Cache *cache, size_t seq, size_t n, size_t first
 }
 
 int DugulornModel::enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) {
-    if (compute == LBK_COMPUTE_BF16) return lbk_bf16_linear(reinterpret_cast<lbk_ctx *>(ctx), rows, n, head.w, head.rows, head.cols, logits, st);
+    if (compute == LBK_COMPUTE_BF16) return launch_bf16_linear(ctx, rows, n, head.w, head.rows, head.cols, logits, st, true);
     DenseCall d;
     d.compute = compute;
     d.x = rows;

@@ -162,7 +162,8 @@ int bf16_init(Ctx *ctx);
 int attn_tc_init(Ctx *ctx);
 int launch_attn_prompt_tc(Ctx *ctx, const float *q, const uint16_t *kc, const uint16_t *vc, const int32_t *pos_dev, size_t n, size_t nh, size_t kvh,
                           size_t cap, size_t seq, float *out, cudaStream_t stream);
+// settled: no kernel in front of this one on the stream writes w, so that its first rows may be read beside that kernel
 int launch_bf16_linear(Ctx *ctx, const float *x, size_t m, const uint16_t *w, size_t rows,
-                       size_t cols, float *out, cudaStream_t stream);
+                       size_t cols, float *out, cudaStream_t stream, bool settled = false);
 
 }  // namespace lbk
