@@ -123,6 +123,7 @@ struct MoeOut {
 struct NormCall {
     int compute = LBK_COMPUTE_BF16;
     bool rms = false;
+    bool settled = false;  // no kernel in front of this one on the stream writes w or w_post: they may be read beside it
     float *x = nullptr;
     const float *y = nullptr, *w_post = nullptr, *w = nullptr;
     const MoeOut *moe = nullptr;

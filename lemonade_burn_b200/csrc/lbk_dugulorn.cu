@@ -388,6 +388,7 @@ int DugulornModel::enqueue_tokens(DugulornCache *c, Work &w, const int32_t *toke
 
     auto norm_rows = [&](const float *w_next, void *out_e, float *out_f) -> int {
         NormCall n;
+        n.settled = true;
         n.compute = compute;
         n.rms = true;
         n.x = x;

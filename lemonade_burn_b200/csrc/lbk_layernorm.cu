@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(NT) sandwich_norm_kernel(const NormParams p) {
 }
 
 // The same with four neighbouring values a thread (rows of whole 16-byte units): the usual case.
-// EARLY, for at most a row an SM: the weights are asked for before the kernel in front is known to be complete, and held. Behind each reduction they
+// EARLY, for settled weights and at most a row an SM: the weights are asked for before the kernel in front is known to be complete, and held. Behind each reduction they
 // are another trip to L2 (with latent_prep_kernel's loads done the same way a step of 16 sequences of four mixed layers of 2560 took 299 us instead of 311); with many rows the registers would cost warps instead.
 template <int NV, typename T, bool EARLY>
 __global__ void __launch_bounds__(256) sandwich_norm_vec_kernel(const NormParams p) {
@@ -275,7 +275,7 @@ int norm_impl(Ctx *ctx, const NormCall &c, cudaStream_t st) {
         vec = vec && c.moe->ld % 4 == 0;
     }
     if (vec && (bits & 15) == 0) {
-        const bool early = c.rows <= static_cast<size_t>(ctx->sm_count);
+        const bool early = c.settled && c.rows <= static_cast<size_t>(ctx->sm_count);
         void (*k)(NormParams) = early ? sandwich_norm_vec_kernel<8, T, true> : sandwich_norm_vec_kernel<8, T, false>;
         if (c.n <= 1024) k = early ? sandwich_norm_vec_kernel<1, T, true> : sandwich_norm_vec_kernel<1, T, false>;
         else if (c.n <= 4096) k = early ? sandwich_norm_vec_kernel<4, T, true> : sandwich_norm_vec_kernel<4, T, false>;

@@ -151,6 +151,7 @@ int PefolixModel::enqueue_tokens(PefolixCache *c, Work &w, const int32_t *tokens
 
     auto norm_rows = [&](const float *w_next, void *out_e, float *out_f) -> int {
         NormCall n;
+        n.settled = true;
         n.compute = compute;
         n.x = x;
         n.y = have_moe ? nullptr : y;

@@ -57,3 +57,34 @@ def test_head_over_rows_just_appended(ctx, front, kv, cap):
         torch.cuda.synchronize()
         assert torch.equal(got, want) and bool((want[0, cap - 1::cap] != 0).all())
     ctx.check_device_error()
+
+
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,n", [(1, 512), (3, 2560), (148, 8192)])
+def test_norm_with_weights_just_written(ctx, front, rows, n, rms):
+    import torch
+    from lemonade_burn_b200 import _lib
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(rows + n)
+    x0, y, *src = (torch.randn(s, generator=g, device="cuda") for s in ((rows, n), (rows, n), (n,), (n,)))
+    w, w_post = torch.empty(n, device="cuda"), torch.empty(n, device="cuda")
+
+    def norm():
+        x, out = x0.clone(), torch.empty(rows, n, device="cuda")
+        call = lib.lbk_sandwich_rms_norm if rms else lib.lbk_sandwich_norm
+        return x, out, lambda: _lib.check(call(ctx.handle, x.data_ptr(), y.data_ptr(), w_post.data_ptr(), w.data_ptr(), rows, n, C.c_float(1e-6), out.data_ptr(), None, 0, st))
+
+    for late, early in ((w, w_post), (w_post, w)):
+        late.zero_()
+        early.copy_(src[late is w])
+        x, got, call = norm()
+        torch.cuda.synchronize()
+        front.launch(st)
+        front.vector(src[late is w_post], late, st)
+        call()
+        torch.cuda.synchronize()
+        xw, want, call = norm()
+        call()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and torch.equal(x, xw) and bool((got != 0).any())
+    ctx.check_device_error()
