@@ -238,6 +238,7 @@ int DugulornModel::enqueue_latent(const Pass &p, const DugulornLayer &l) {
     pc.cq = w.cq;
     pc.ldq = static_cast<long>(l.uq.pitch);
     pc.cache = l.own ? p.c->latent[l.source] : nullptr;
+    pc.settled = true;
     LBK_TRY(launch_latent_prep(ctx, pc, p.st));
     DenseCall d;
     d.compute = compute;

@@ -51,6 +51,7 @@ struct LatentPrepCall {
     void *cq = nullptr;
     long ldq = 0;
     void *cache = nullptr;  // [seq][cap][pitch]
+    bool settled = false;   // no kernel in front of this one on the stream writes q_norm or kv_norm: they may be read beside it
 };
 int launch_latent_prep(Ctx *ctx, const LatentPrepCall &c, cudaStream_t st);
 

@@ -88,3 +88,40 @@ def test_norm_with_weights_just_written(ctx, front, rows, n, rms):
         torch.cuda.synchronize()
         assert torch.equal(got, want) and torch.equal(x, xw) and bool((got != 0).any())
     ctx.check_device_error()
+
+
+@pytest.mark.parametrize("compute", [0, 1])
+@pytest.mark.parametrize("rows", [1, 16])
+def test_latents_with_weights_just_written(ctx, front, rows, compute):
+    import torch
+    from lemonade_burn_b200 import _lib, mixers
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    q_rank, kv_rank, rot, cap = 1536, 512, 64, 40
+    f, m = mixers.rotation_frequencies(rot, 1e4, None)
+    freq = torch.from_numpy(f).cuda()
+    d = mixers.LatentDesc(4, 128, rot, 128, kv_rank, q_rank, freq.data_ptr(), m)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    z = torch.randn(rows, q_rank + kv_rank + rot, generator=g, device="cuda")
+    pos, kind = torch.arange(rows, dtype=torch.int32, device="cuda"), torch.float32 if compute else torch.bfloat16
+    src = torch.randn(q_rank, generator=g, device="cuda"), torch.randn(kv_rank, generator=g, device="cuda")
+    w = torch.empty(q_rank, device="cuda"), torch.empty(kv_rank, device="cuda")
+
+    def prep():
+        cq, cache = torch.zeros(rows, q_rank, dtype=kind, device="cuda"), torch.zeros(rows, cap, lib.lbk_latent_pitch(C.byref(d)), dtype=kind, device="cuda")
+        return cq, cache, lambda: _lib.check(lib.lbk_latent_prep(ctx.handle, compute, C.byref(d), z.data_ptr(), z.shape[1], rows, -1, pos.data_ptr(), cap, w[0].data_ptr(),
+                                                                 w[1].data_ptr(), C.c_float(1e-6), cq.data_ptr(), q_rank, cache.data_ptr(), st))
+
+    for late in (0, 1):
+        w[late].zero_()
+        w[1 - late].copy_(src[1 - late])
+        cq, cache, call = prep()
+        torch.cuda.synchronize()
+        front.launch(st)
+        front.vector(src[late], w[late], st)
+        call()
+        torch.cuda.synchronize()
+        cqw, want, call = prep()
+        call()
+        torch.cuda.synchronize()
+        assert torch.equal(cq, cqw) and torch.equal(cache, want) and bool((cq != 0).any())
+    ctx.check_device_error()
