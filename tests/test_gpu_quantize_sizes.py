@@ -28,3 +28,26 @@ def test_row_lengths(oracle, ctx, k, shift):
     assert np.array_equal(s.cpu().numpy().view(np.uint32), np.asarray(ws, dtype=np.float32).view(np.uint32))
     assert np.array_equal(t.cpu().numpy(), np.asarray(wt))
     ctx.check_device_error()
+
+
+@pytest.mark.parametrize("m", [1, 700])
+@pytest.mark.parametrize("k", [7172, 8192, 8196, 12288, 12292, 20000, 21004, 28673])
+def test_long_rows(oracle, ctx, m, k):
+    """Where one form ends and the next begins, and rows that are read twice, whole units and not, few and more than the SMs hold."""
+    import torch
+    from lemonade_burn_b200 import _lib
+    rng = np.random.default_rng(k + m)
+    x = (rng.standard_normal((m, k)) * np.exp(rng.standard_normal((m, 1)))).astype(np.float32)
+    if m > 1:
+        x[3] = 0
+        x[5, k - 1] = 1e6  # the maximum in the last column
+    xd, kp = torch.from_numpy(x).cuda(), -(-k // 128) * 128
+    q = torch.full((m, kp), 77, dtype=torch.int8, device="cuda")
+    s, t = torch.empty(m, device="cuda"), torch.empty(m, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.load().lbk_quantize_acts_dev(ctx.handle, xd.data_ptr(), m, k, q.data_ptr(), s.data_ptr(), t.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    rows = slice(None) if m == 1 else slice(0, 9)
+    qw, sw, tw = oracle.quantize_acts(x[rows])
+    assert np.array_equal(q[rows, :k].cpu().numpy(), np.asarray(qw)[:, :k]) and np.array_equal(t[rows].cpu().numpy(), tw)
+    assert np.array_equal(s[rows].cpu().numpy().view(np.uint32), np.asarray(sw, dtype=np.float32).view(np.uint32))
+    assert not bool(q[:, k:].any()) and torch.equal(q.int().sum(1, dtype=torch.int32), t)
+    ctx.check_device_error()
