@@ -42,20 +42,19 @@ __device__ __forceinline__ float block_sum(float v, float *s_red) {
     return t;
 }
 
+// units: rows in units of four values, one to a thread and trip
 __global__ void embed_kernel(const uint16_t *__restrict__ table, const int *__restrict__ tokens, int hidden,
-                             float *__restrict__ out) {
+                             float *__restrict__ out, bool units) {
     ptx::pdl_trigger();  // the next kernel of the step may be scheduled now
     ptx::pdl_wait();     // everything this kernel reads or overwrites is settled from here on
 
     const int b = blockIdx.x;
     const uint16_t *row = table + static_cast<size_t>(tokens[b]) * hidden;
     float *o = out + static_cast<size_t>(b) * hidden;
-    if ((hidden & 7) == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
-        // eight values a thread in one load: value by value a row of 2560 was ten trips through two bytes each (a step's one row 8 -> 2.5 us, 2011 rows 12.5 -> 7.6)
-        for (int i = threadIdx.x; i < (hidden >> 3); i += blockDim.x) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row) + i);
-            reinterpret_cast<float4 *>(o)[2 * i] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
-            reinterpret_cast<float4 *>(o)[2 * i + 1] = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u), __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
+    if (units) {
+        for (int i = threadIdx.x; i < (hidden >> 2); i += blockDim.x) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(row) + i);
+            reinterpret_cast<float4 *>(o)[i] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
         }
         return;
     }
@@ -1268,7 +1267,13 @@ int lbk_embed_bf16(lbk_ctx *c, const uint16_t *table_dev, const int32_t *tokens_
     LBK_DEC_PRE("lbk_embed_bf16");
     if (b == 0) return LBK_OK;
     if (!table_dev || !tokens_dev || !out_dev) return fail(LBK_ERR_INVALID, "lbk_embed_bf16: null buffer");
-    LBK_CUDA(launch_chained(embed_kernel, dim3(static_cast<unsigned>(b)), dim3(256), 0, st, table_dev, tokens_dev, static_cast<int>(hidden), out_dev));
+    // Rows of 512 values and more in units of four: their loads and stores are whole lines (of eight values a thread the stores are every other 16
+    // bytes). Many rows by 128 threads each, up to three an SM by 512, whose trips are fewer. us, value by value / units of eight by 256 threads / so: 1 row
+    // of 2560 2.8 / 1.7 / 1.6, 2048 rows of 2560 from HBM 12.9 / 8.0 / 5.7, from L2 6.3 / 7.1 / 4.8, of 4096 17.5 / 11.0 / 7.8. Shorter rows are one trip or
+    // two for a value each: 16 rows of 64 1.2 / 1.3 / 1.2.
+    const bool units = hidden >= 512 && hidden % 4 == 0 && (reinterpret_cast<uintptr_t>(table_dev) & 7) == 0 && (reinterpret_cast<uintptr_t>(out_dev) & 15) == 0;
+    const unsigned threads = !units ? 256 : b <= 3 * static_cast<size_t>(ctx->sm_count) ? 512 : 128;
+    LBK_CUDA(launch_chained(embed_kernel, dim3(static_cast<unsigned>(b)), dim3(threads), 0, st, table_dev, tokens_dev, static_cast<int>(hidden), out_dev, units));
     LBK_DEC_POST();
 }
 
