@@ -19,12 +19,11 @@
 //   recur_prep_kernel   one block per (eight tokens, head): q, k, v as they are or, for delta, short convolution + silu, unit
 //                       vectors, decays and step sizes; writes one record per (eight tokens, head) with the vectors
 //                       and numbers above. Every token block is independent of every other.
-//   recur_walk_kernel   one block per (head, slice of value columns) walks the records in order. A warp holds two columns
+//   recur_walk_kernel   one block per (head, slice of value columns) walks the records in order. A warp holds two or four columns
 //                       of S in registers, dim / 32 values of each a lane (packed pairs for the two-wide FMA), so a vector
-//                       read from shared memory serves two columns. With four a vector was read half as often, but an SM had four or
-//                       five warps, and what a record takes is the chain dots, sums, system, update: 2048 rows of 20 heads of 128 x 128,
-//                       prep included, 257 -> 235 us (plain) and 454 -> 391 (delta); of 32 heads 439 -> 415 and 764 -> 647. The dots over the 32 lanes meet by
-//                       transposing shuffles: lane l ends up with those of column l / 16 and token l % 8. Every lane keeps its
+//                       read from shared memory serves them all. With four it is read half as often, with two an SM has twice the warps to hide
+//                       the chain of a record (dots, sums, system, update), which is longer in the delta rule (walk_cols). The dots over the 32 lanes meet by
+//                       transposing shuffles: lane l ends up with those of column l / 16 (l / 8) and token l % 8. Every lane keeps its
 //                       partial dots in an order of its own, slot s holding dot s XOR l, so that each step of the
 //                       transposition adds a received value to a register without choosing. A producer lane brings the
 //                       records into a ring of shared memory with bulk copies.
@@ -47,8 +46,12 @@ namespace {
 constexpr int kTok = 8;             // tokens per record
 constexpr int kPrepThreads = 128;
 constexpr int kScal = 2 * kTok * kTok;  // numbers of a record: T, then p, eight by eight
-constexpr int kMaxWarps = 16;       // warps of a walk's block that hold columns
-constexpr int kCols = 2;            // columns of a warp
+// Columns of a walk's warp, by rule and packed pairs a lane (dp / 64). us for 2048 rows, two / four columns, prep included: delta 20 heads of 128 x 128
+// 383 / 420, 64 of 64 x 128 1067 / 1288, 16 of 256 x 256 762 / 619; plain 64 of 64 x 128 515 / 431, 16 of 256 x 256 462 / 601. Plain heads of 128 lie
+// between: alone 20 heads take 238 / 240 (64 rows 18 / 15), 32 heads 409 / 394, sixteen prompts of a mixed model 0.5 % less with two.
+__host__ __device__ constexpr int walk_cols(bool delta, int pairs) { return (delta ? pairs <= 2 : pairs >= 2) ? 2 : 4; }
+// warps of a walk's block that hold columns at most
+__host__ __device__ constexpr int max_warps(int cols) { return 32 / cols; }
 constexpr int kMaxStages = 12;
 constexpr uint32_t kWaitLimit = 1u << 22;
 
@@ -356,9 +359,10 @@ __device__ __forceinline__ float dot(const u64 (&a)[P], const u64 (&b)[P]) {
     return sum2(t);
 }
 
-// P: packed pairs of a column per lane (dp = 64 P). Slot s of a lane holds column s XOR (lane / kLanes) of the warp's two.
+// P: packed pairs of a column per lane (dp = 64 P). Slot s of a lane holds column s XOR (lane / kLanes) of the warp's.
 template <typename T, bool DELTA, int P>
-__global__ void __launch_bounds__((kMaxWarps + 1) * 32) recur_walk_kernel(const RecurParams p) {
+__global__ void __launch_bounds__((max_warps(walk_cols(DELTA, P)) + 1) * 32) recur_walk_kernel(const RecurParams p) {
+    constexpr int COLS = walk_cols(DELTA, P);
     extern __shared__ __align__(16) uint8_t rc_smem[];
     __shared__ __align__(8) uint64_t s_bar[2 * kMaxStages];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -392,12 +396,12 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32) recur_walk_kernel(const 
             }
         }
     } else {
-        constexpr int kLanes = 32 / kCols;  // lanes that end up with a column's sums
-        const int cg = lane / kLanes, col0 = (slice * p.warps + warp) * kCols, col = col0 + cg, tk = lane & 7;  // the lane's own column and token
+        constexpr int kLanes = 32 / COLS;  // lanes that end up with a column's sums
+        const int cg = lane / kLanes, col0 = (slice * p.warps + warp) * COLS, col = col0 + cg, tk = lane & 7;  // the lane's own column and token
         float *st = p.state + static_cast<size_t>(seq * p.heads + h) * p.vdim * p.dp;
-        u64 S[kCols][P];
+        u64 S[COLS][P];
 #pragma unroll
-        for (int s = 0; s < kCols; ++s) {
+        for (int s = 0; s < COLS; ++s) {
 #pragma unroll
             for (int j = 0; j < P; ++j) S[s][j] = 0;
             if (pos_first + p.row0 > 0 && col0 + (s ^ cg) < p.vdim) share<P>(st + static_cast<size_t>(col0 + (s ^ cg)) * p.dp, lane, S[s]);
@@ -411,20 +415,27 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32) recur_walk_kernel(const 
             }
             const float *rec = reinterpret_cast<const float *>(rc_smem + static_cast<size_t>(s) * bytes);
             const float *rk = rec, *rq = rec + (DELTA ? kTok : 0) * 64 * P, *rh = rq + kTok * 64 * P, *rg = rh + kTok * 64 * P, *rs = rg + 64 * P, *rv = rs + kScal;
-            // dots of eight tokens' vectors with the two columns; the lane's own token and column
+            // dots of eight tokens' vectors with the warp's columns; the lane's own token and column
             auto dots = [&](const float *rows) -> float {
                 float r[kTok];
 #pragma unroll
                 for (int e = 0; e < kTok; ++e) {
                     u64 w[P];
                     share<P>(rows + (e ^ tk) * 64 * P, lane, w);
-                    r[e] = dot<P>(w, S[0]) + __shfl_xor_sync(0xffffffffu, dot<P>(w, S[1]), kLanes);
+                    float v[COLS];
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) v[c] = dot<P>(w, S[c]);
+#pragma unroll
+                    for (int c = COLS / 2; c >= 1; c >>= 1)
+#pragma unroll
+                        for (int k = 0; k < c; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k + c], kLanes * c);
+                    r[e] = v[0];
                 }
 #pragma unroll
                 for (int w = kTok / 2; w >= 1; w >>= 1)
 #pragma unroll
                     for (int e = 0; e < w; ++e) r[e] += __shfl_xor_sync(0xffffffffu, r[e + w], w);
-                return r[0] + __shfl_xor_sync(0xffffffffu, r[0], kTok);
+                return COLS == 2 ? r[0] + __shfl_xor_sync(0xffffffffu, r[0], kTok) : r[0];
             };
             auto times = [&](const float *row, const float (&v)[kTok]) -> float {  // eight numbers of shared memory . v
                 const float4 a = *reinterpret_cast<const float4 *>(row), c = *reinterpret_cast<const float4 *>(row + 4);
@@ -449,7 +460,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32) recur_walk_kernel(const 
             u64 g[P];
             share<P>(rg, lane, g);
 #pragma unroll
-            for (int c = 0; c < kCols; ++c)
+            for (int c = 0; c < COLS; ++c)
 #pragma unroll
                 for (int j = 0; j < P; ++j) S[c][j] = mul2(g[j], S[c][j]);
 #pragma unroll
@@ -457,7 +468,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32) recur_walk_kernel(const 
                 u64 w[P];
                 share<P>(rh + i * 64 * P, lane, w);
 #pragma unroll
-                for (int c = 0; c < kCols; ++c) {
+                for (int c = 0; c < COLS; ++c) {
                     const float uc = c ? __shfl_xor_sync(0xffffffffu, u[i], kLanes * c) : u[i];
                     const u64 uu = pack2(uc, uc);
 #pragma unroll
@@ -474,7 +485,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32) recur_walk_kernel(const 
         if (!ok && lane == 0) atomicExch(p.err_word, 5);
         if (ok && fits) {
 #pragma unroll
-            for (int c = 0; c < kCols; ++c)
+            for (int c = 0; c < COLS; ++c)
                 if (col0 + (c ^ cg) < p.vdim) unshare<P>(st + static_cast<size_t>(col0 + (c ^ cg)) * p.dp, lane, S[c]);
             if (DELTA && slice == 0 && p.last && p.taps > 1) {
                 // the inputs later tokens will convolve with: the last taps - 1 of this pass, this head's channels
@@ -890,16 +901,17 @@ int launch_walk(Ctx *ctx, RecurParams &p, cudaStream_t st) {
     p.stages = static_cast<int>(stages < 2 ? 2 : stages > kMaxStages ? kMaxStages : stages);
     if (p.blocks < p.stages) p.stages = p.blocks;
     // warps a block: the number that leaves the fullest SM the fewest
+    const int cols = walk_cols(DELTA, p.dp / 64);
     int best = 1 << 30;
-    for (int w = kMaxWarps / 2; w <= kMaxWarps; ++w) {
-        const int blocks = (p.vdim + kCols * w - 1) / (kCols * w) * p.heads, most = (blocks + ctx->sm_count - 1) / ctx->sm_count * w;
+    for (int w = max_warps(cols) / 2; w <= max_warps(cols); ++w) {
+        const int blocks = (p.vdim + cols * w - 1) / (cols * w) * p.heads, most = (blocks + ctx->sm_count - 1) / ctx->sm_count * w;
         if (most < best) {
             best = most;
             p.warps = w;
         }
     }
     void (*k)(RecurParams) = p.dp == 64 ? recur_walk_kernel<T, DELTA, 1> : p.dp == 128 ? recur_walk_kernel<T, DELTA, 2> : recur_walk_kernel<T, DELTA, 4>;
-    LBK_CUDA(launch_chained(k, dim3(static_cast<unsigned>((p.vdim + kCols * p.warps - 1) / (kCols * p.warps)), static_cast<unsigned>(p.heads)),
+    LBK_CUDA(launch_chained(k, dim3(static_cast<unsigned>((p.vdim + cols * p.warps - 1) / (cols * p.warps)), static_cast<unsigned>(p.heads)),
                             dim3(static_cast<unsigned>(p.warps + 1) * 32), rec * p.stages, st, p));
     LBK_CUDA(cudaGetLastError());
     ctx->launches++;
