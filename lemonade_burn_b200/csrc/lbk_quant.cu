@@ -228,8 +228,10 @@ int launch_quantize_ex(Ctx *ctx, const float *x, size_t m, size_t k, int8_t *q, 
     if (vec && n4 <= 3 * 256) kernel = quantize_kernel<256, 3>;
     else if (vec && n4 <= 4 * 256) kernel = quantize_kernel<256, 4>;
     else if (vec && n4 <= 7 * 256) kernel = quantize_kernel<256, 7>;
-    else if (vec && n4 <= 8 * 256) kernel = quantize_kernel<256, 8>;    // 2048 rows of 8192 by 512 threads, half of what they hold empty: 11.2 -> 17.6 us
-    else if (vec && n4 <= 12 * 256) kernel = quantize_kernel<256, 12>;  // of 8640 / 12288: 12.7 / 20.9, by 512 threads 18.6 / 25.2
+    // 2048 rows of 8192 / 8640 / 12288 by 512 threads, half of what they hold empty, 17.6 / 18.6 / 25.2 us, by 256 11.2 / 12.7 / 20.9; one or two rows an SM in
+    // front of a GEMM are done sooner by 512 (128 rows of 8192 -> 8192 14.5 us with the GEMM, by 256 15.0)
+    else if (vec && n4 <= 8 * 256 && m > 2 * static_cast<size_t>(ctx->sm_count)) kernel = quantize_kernel<256, 8>;
+    else if (vec && n4 <= 12 * 256 && m > 2 * static_cast<size_t>(ctx->sm_count)) kernel = quantize_kernel<256, 12>;
     else if (vec && n4 <= 8 * 512) kernel = quantize_kernel<512, 8>, threads = 512;
     // Rows read twice that together do not fit in L2 with eight CTAs an SM (135 MB of 28672 values) come in fours: shared memory that nobody uses.
     const size_t smem = k > 21000 && m > 4 * static_cast<size_t>(ctx->sm_count) ? 47 * 1024 : 0;
