@@ -554,20 +554,22 @@ static const InitHook kInitGemm(gemm_init);
 // Parts to cut every tile's K blocks into. A launch with few tiles against the SM count (small
 // token batches, tensor-parallel shards) or with a ragged last round leaves SMs idle; parts add
 // their int32 sums into a zeroed buffer and a small kernel scales them afterwards. Cost model in
-// K-block times of one CTA (about 500 cycles); the parts' atomic adds, the scaling launch and its
-// traffic are charged as 30 (14 was tried once the zeroing launches were gone: the 70B-shaped gate/up
-// projection at 64 token rows then split in two and took twice as long, 14.7 MB of sums added twice).
-static int choose_ksplit(int tiles, int k_blocks, int sms, int *kb_part) {
+// K-block times of one CTA (250 cycles in the narrow kernel to 490 in the wide one); the parts' atomic adds, the scaling launch and its
+// traffic are charged as 30 of them (14 was tried when a block took 500 cycles: the 70B-shaped gate/up
+// projection at 64 token rows then split in two and took twice as long, 14.7 MB of sums added twice). Uncut, the fullest CTA
+// has `rounds` tiles (choose_nt): counted as whole rounds, a launch whose last round are short tiles of a ragged batch looked twice as long as it
+// is and was cut in eight, at 777 rows of 8192 -> 2 x 2048 75 us instead of 31.
+static int choose_ksplit(int tiles, double rounds, int k_blocks, int sms, int *kb_part) {
     int best = 1;
-    long long best_cost = static_cast<long long>((tiles + sms - 1) / sms) * k_blocks;
+    double best_cost = rounds * k_blocks;
     *kb_part = k_blocks;
     for (int s = 2; s <= 8; ++s) {
         const int per = ((k_blocks + s - 1) / s + kPackBlocks - 1) / kPackBlocks * kPackBlocks;
         if (per < 2 * kPackBlocks) break;
         const int parts = (k_blocks + per - 1) / per;
         if (parts != s) continue;  // rounding made fewer parts: that count is or was tried as itself
-        const long long cost = static_cast<long long>((static_cast<long long>(tiles) * s + sms - 1) / sms) * per + 30;
-        if (cost * 100 < best_cost * 85) {
+        const double cost = static_cast<double>((static_cast<long long>(tiles) * s + sms - 1) / sms) * per + 30.0;
+        if (cost * 100.0 < best_cost * 85.0) {
             best_cost = cost;
             best = s;
             *kb_part = per;
@@ -579,12 +581,14 @@ static int choose_ksplit(int tiles, int k_blocks, int sms, int *kb_part) {
 
 // Token rows per tile for a launch, a multiple of 16: the count with the least cost in cycles of the fullest CTA. Up to 64 the
 // narrow kernel runs, 250 cycles a K block; the wide one takes 365 at 96 token rows and 490 at 192 (launches of many
-// rounds, their epilogues beside the products; 341 and 416 in a single round). 35 cycles a token row are the last tile's
-// epilogue, 300 the start of a tile. Short tiles of a ragged batch come last (decode_tile in the kernel): what is left
+// rounds, their epilogues beside the products; 341 and 416 in a single round). 15 cycles a token row are the last tile's
+// epilogue, 300 the start of a tile: with 35, fitted when four warps did an epilogue, matrices of few columns went in narrow tiles, 2048 rows
+// of 512 -> 2 x 1376 16.7 us instead of 11.9, 256 of 1000 -> 2 x 2700 9.6 instead of 7.4. Short tiles of a ragged batch come last (decode_tile in the kernel): what is left
 // over behind the full rounds are short ones, and with the order turned round every other time a CTA that has two of them
 // at the end takes less than a full tile longer than the others. Measured at 2560 -> 2 x 6912, us: 400 rows in tiles of 112 / 144 / 176
 // 15.5 / 15.8 / 14.8, 2048 rows in tiles of 64 / 128 / 160 / 192 69.4 / 59.0 / 56.0 / 54.7; 2560 -> 3840 at 96 rows in tiles of 48 / 96: 5.3 / 6.6.
-static int choose_nt(int m, int row_tiles, int k_blocks, int sms) {
+// Over 28 groups of 512 to 14336 columns at 20 sizes the choice is 2 % slower than the best tile (geometric mean).
+static int choose_nt(int m, int row_tiles, int k_blocks, int sms, double *rounds_out) {
     auto block = [](int nt) { return nt <= 64 ? 250.0 : 240.0 + 1.3 * nt; };
     int best_nt = 0;
     double best = 0.0;
@@ -597,10 +601,11 @@ static int choose_nt(int m, int row_tiles, int k_blocks, int sms) {
         if (left > shorts) rounds += 1.0;
         else if (left > 0 && 2 * left <= shorts && whole > 0) rounds += 2.0 * least > 1.0 ? 2.0 * least - 1.0 : 0.0;
         else if (left > 0) rounds += least;
-        const double cost = rounds * (k_blocks * block(nt) + 300.0) + 35.0 * nt;
+        const double cost = rounds * (k_blocks * block(nt) + 300.0) + 15.0 * nt;
         if (best_nt == 0 || cost < best) {
             best = cost;
             best_nt = nt;
+            *rounds_out = rounds;
         }
         if (nt >= m) break;
     }
@@ -618,7 +623,8 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
         return fail(LBK_ERR_INVALID, "gemm: a gated pair is two matrices of one shape with an f32 output");
     for (int i = 0; i < g.n; ++i) row_tiles += static_cast<int>((g.w[i]->rows + kBMW - 1) / kBMW);
     if (g.gated) row_tiles = static_cast<int>((g.w[0]->rows + kBMW / 2 - 1) / (kBMW / 2));
-    const int nt = choose_nt(static_cast<int>(g.m), row_tiles, static_cast<int>(kp / kBK), ctx->sm_count);
+    double rounds = 1.0;
+    const int nt = choose_nt(static_cast<int>(g.m), row_tiles, static_cast<int>(kp / kBK), ctx->sm_count, &rounds);
     LBK_TRY(encode_act_map(&p.act, g.q, g.m, kp, nt));
     p.nt = nt;
     p.m = static_cast<int>(g.m);
@@ -648,7 +654,7 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
     p.qsum = g.qsum;
     p.err_word = ctx->err_word;
     if (tiles == 0 || p.k_blocks == 0) return LBK_OK;
-    p.ksplit = choose_ksplit(tiles, p.k_blocks, ctx->sm_count, &p.kb_part);
+    p.ksplit = choose_ksplit(tiles, rounds, p.k_blocks, ctx->sm_count, &p.kb_part);
     if (g.gated) {  // the parts' sums would have to meet before the product
         p.ksplit = 1;
         p.kb_part = p.k_blocks;

@@ -48,3 +48,21 @@ def test_launches_behind_one_another_give_the_same_rows(oracle, ctx, m):
             for a, b in zip(outs, want):
                 assert torch.equal(a, b)
     ctx.check_device_error()
+
+
+@pytest.mark.parametrize("cols,rows,m", [(8192, [2048, 2048], 777), (8640, [3200], 1024), (512, [1376, 1376], 2048), (1000, [2700, 2700], 256), (14336, [4096], 17)])
+def test_one_batch_or_portions(ctx, cols, rows, m):
+    """Launches whose last round are short tiles, matrices of few columns, long columns in few tiles: whatever tile and cut are chosen for all rows at once, the
+    bits are those of the rows in portions of 64 and fewer, which go by other tiles. Equality: the same integers and products of scales."""
+    import torch
+    from lemonade_burn_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(cols + m)
+    lins = [ops.TernaryLinear(torch.randint(0, 3, (r, -(-cols // 128) * 32), generator=g, device="cuda", dtype=torch.uint8) * 21, 50.0 + i, cols, ctx) for i, r in enumerate(rows)]
+    x = torch.randn(m, cols, generator=g, device="cuda")
+    whole, ints = ops.ternary_linear_multi(x, lins, want_i32=True)
+    for r0 in range(0, m, 64):
+        part = ops.ternary_linear_multi(x[r0:r0 + 64], lins)
+        for w, p in zip(whole, part):
+            assert torch.equal(w[r0:r0 + 64], p)
+    assert all(bool((i != 0).any()) for i in ints)
+    ctx.check_device_error()
