@@ -35,6 +35,11 @@ struct BitNetModel : Model {
     }
     int make_cache(size_t batch, size_t capacity, std::unique_ptr<Cache> &out) override;
     int make_prefill_buffers(Cache *c, size_t rows) override;
+    // From kQuantisedRows rows on every projection takes the GEMM path; where its norms can leave quantised rows, gate and up leave it as one
+    static constexpr size_t kQuantisedRows = 9;
+    bool quantised_norms() const {
+        return lbk_norm_quant_supported(cfg.hidden_size) && lbk_norm_quant_supported(cfg.intermediate_size) && lbk_norm_quant_supported(cfg.num_attention_heads * head_dim);
+    }
     int enqueue_step(Cache *c, cudaStream_t st) override;
     int enqueue_rows(Cache *c, size_t seq, size_t n, size_t first, cudaStream_t st) override;
     int enqueue_head(const float *rows, size_t n, float *logits, cudaStream_t st) override {
@@ -192,15 +197,17 @@ int BitNetModel::enqueue_step(Cache *cache, cudaStream_t st) {
     return enqueue_head(c->n, b, c->logits, st);
 }
 
-// About 150 KB per row at 2B4T shapes.
+// About 90 KB per row at 2B4T shapes. Gate and up rows by themselves are written for few rows only where the sizes let the others leave the GEMM
+// as one row (enqueue_rows): room for all of them would be 226 MB of 4096 rows of 6912.
 int BitNetModel::make_prefill_buffers(Cache *cache, size_t rows) {
     BitNetCache *c = static_cast<BitNetCache *>(cache);
     const size_t H = cfg.hidden_size, I = cfg.intermediate_size, nh = cfg.num_attention_heads, kvh = cfg.num_key_value_heads, hd = head_dim;
+    const size_t apart = quantised_norms() ? std::min(rows, kQuantisedRows - 1) : rows;
     struct { void **p; size_t bytes; } bufs[] = {
         {reinterpret_cast<void **>(&c->pf_x), rows * H * 4}, {reinterpret_cast<void **>(&c->pf_q), rows * nh * hd * 4},
         {reinterpret_cast<void **>(&c->pf_k), rows * kvh * hd * 4}, {reinterpret_cast<void **>(&c->pf_v), rows * kvh * hd * 4},
         {reinterpret_cast<void **>(&c->pf_attn), rows * nh * hd * 4}, {reinterpret_cast<void **>(&c->pf_o), rows * H * 4},
-        {reinterpret_cast<void **>(&c->pf_g), rows * I * 4}, {reinterpret_cast<void **>(&c->pf_u), rows * I * 4},
+        {reinterpret_cast<void **>(&c->pf_g), apart * I * 4}, {reinterpret_cast<void **>(&c->pf_u), apart * I * 4},
         {reinterpret_cast<void **>(&c->pf_act), rows * I * 4}, {reinterpret_cast<void **>(&c->pf_d), rows * H * 4},
         {reinterpret_cast<void **>(&c->pf_q8), rows * (std::max(std::max(H, I), nh * hd) + 127) / 128 * 128},
         {reinterpret_cast<void **>(&c->pf_qscale), rows * 4}, {reinterpret_cast<void **>(&c->pf_qsum), rows * 4}};
@@ -228,8 +235,7 @@ int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, size_t first, 
     // From 9 rows on every projection takes the GEMM path, whose input is the quantised rows: the norm
     // in front of a projection then writes those directly (lbk_norm_quant) and the f32 copy of the
     // normalised rows, with the quantise kernel that would read it back, goes away. Same bits.
-    const bool can_nq = lbk_norm_quant_supported(H) && lbk_norm_quant_supported(I) && lbk_norm_quant_supported(nh * hd);
-    bool nq = n >= 9 && can_nq;
+    bool nq = n >= kQuantisedRows && quantised_norms();
     auto norm_q = [&](int pre, float *x, const float *y, const float *w, size_t width) -> int {
         return lbk_norm_quant(h, pre, x, y, w, n, width, eps, c->pf_q8, c->pf_qscale, c->pf_qsum, st);
     };
@@ -260,7 +266,7 @@ int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, size_t first, 
             }
             kept = first;
             n -= first;
-            nq = n >= 9 && can_nq;
+            nq = n >= kQuantisedRows && quantised_norms();
             x += first * H;
             attn += first * nh * hd;
         } else {

@@ -55,3 +55,34 @@ def test_wanted_rows(models, ctx, family, n, want):
     logits = [net.decode(step, c)[0] for c in caches]
     assert float((logits[0] - logits[1]).abs().max()) <= 1e-6 * spread
     ctx.check_device_error()
+
+
+@pytest.mark.parametrize("inner", [6912, 8196])
+def test_memory_of_a_prompt(ctx, tmp_path, inner):
+    """What a prompt's first pass allocates: one row of the feed-forward width for each token where gate and up leave the GEMM as one, three where the width
+    is beyond what the norm quantises (8192), and the rest; and short prompts, which go by other kernels, behind long ones and in front of them."""
+    import torch
+    from lemonade_burn_b200 import model
+    n, hidden = 4096, 512
+    cfg = model.Config(hidden, inner, 4, 1, 2, VOCAB, 1e-5, 500000.0, 4200)
+    model.save_checkpoint(tmp_path, cfg, model.random_checkpoint(cfg, 3))
+    net = model.NativeBitNet(tmp_path, ctx)
+    cache = net.new_cache(2, 4200)
+    tokens = np.random.default_rng(1).integers(0, VOCAB, n + 30).astype(np.uint32)
+    early = net.forward_rows(tokens[:7], cache, [6], seq=1)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    net.forward_rows(tokens[:n], cache, [n - 1])
+    torch.cuda.synchronize()
+    taken = before - torch.cuda.mem_get_info()[0]
+    rows = 3 if inner > 8192 else 1
+    assert taken <= n * (rows * inner * 4 + 7 * hidden * 4 + inner) + (64 << 20), taken
+    for k in (8, 9, 10):  # the last layer's rows alone, on both sides of the line
+        net.reset_cache(cache)
+        few = net.forward_rows(tokens[:30], cache, list(range(30 - k, 30)))
+        net.reset_cache(cache)
+        full = net.forward_rows(tokens[:30], cache, list(range(30)))
+        assert np.abs(few - full[30 - k:]).max() <= 1e-2 * np.abs(full).max()
+    net.reset_cache(cache)
+    assert np.array_equal(net.forward_rows(tokens[:7], cache, [6], seq=1), early)
+    ctx.check_device_error()
