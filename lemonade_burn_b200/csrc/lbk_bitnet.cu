@@ -257,7 +257,7 @@ int BitNetModel::enqueue_rows(Cache *cache, size_t seq, size_t n, size_t first, 
         if (li + 1 == L && first > 0) {
             if (first == n) return LBK_OK;
             // attention of the 128-row tiles that hold wanted rows (the same tiles, the same bits), everything behind it for the wanted rows
-            const size_t left = n >= 64 && hd == 128 && nh <= 8 * kvh ? first / 128 * 128 : 0;
+            const size_t left = attn_prompt_tiled(n, nh, kvh, hd) ? first / 128 * 128 : 0;
             if (left > 0) {
                 LBK_TRY(later_rows(c, seq, left, st));
                 LBK_TRY(launch_attn_prompt_tc(ctx, c->pf_q + left * nh * hd, kc, vc, c->pos_first, n - left, nh, kvh, c->cap, seq, c->pf_attn + left * nh * hd, st));

@@ -160,6 +160,9 @@ int bf16_init(Ctx *ctx);
 
 // causal attention of a prompt pass on tcgen05 (head_dim 128)
 int attn_tc_init(Ctx *ctx);
+// lbk_attn_prefill takes that form, 128 rows a tile: from 64 rows on (fewer: 16-row tiles on mma.sync, a 128-row tile would be mostly padding). Its limits are
+// those of the call: head_dim 128, 1 to 8 query heads per key head, at most 65535 rows.
+inline bool attn_prompt_tiled(size_t n, size_t nh, size_t kvh, size_t hd) { return n >= 64 && n <= 65535 && hd == 128 && kvh && nh % kvh == 0 && nh <= 8 * kvh; }
 int launch_attn_prompt_tc(Ctx *ctx, const float *q, const uint16_t *kc, const uint16_t *vc, const int32_t *pos_dev, size_t n, size_t nh, size_t kvh,
                           size_t cap, size_t seq, float *out, cudaStream_t stream);
 // settled: no kernel in front of this one on the stream writes w, so that its first rows may be read beside that kernel
