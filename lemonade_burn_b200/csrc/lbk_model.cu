@@ -125,15 +125,27 @@ __global__ void __launch_bounds__(256) pick_kernel(const PickParams p) {
     }
 }
 
-// Whether a kernel on the context's device may go through a caller's pointer: aligned and in this device's own memory. Any other is left to a copy.
-bool reachable(const Ctx *ctx, const void *p) {
+// Whether a kernel on the context's device may go through a caller's pointer to `bytes` bytes: aligned, in this device's own memory and inside one
+// allocation. Any other is left to a copy, which knows more kinds of memory and refuses what does not fit.
+bool reachable(const Ctx *ctx, const void *p, size_t bytes) {
     if (!p) return true;
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return (reinterpret_cast<uintptr_t>(p) & 3) == 0 && a.type == cudaMemoryTypeDevice && a.device == ctx->device;
+    static const auto attributes = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool found = cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+        return reinterpret_cast<CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr)>(found ? f : nullptr);
+    }();
+    if (!attributes || (reinterpret_cast<uintptr_t>(p) & 3) != 0) return false;
+    unsigned kind = 0, managed = 1;
+    int device = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *values[] = {&kind, &managed, &device, &start, &size};
+    if (attributes(5, which, values, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return false;
+    const size_t at = reinterpret_cast<CUdeviceptr>(p) - start;
+    return kind == CU_MEMORYTYPE_DEVICE && !managed && device == ctx->device && at <= size && bytes <= size - at;
 }
 }  // namespace
 
@@ -620,18 +632,21 @@ int lbk_model_decode(lbk_model *mp, lbk_kv_cache *cp, const int32_t *tokens_dev,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // The caller's buffers are reached by a kernel in front of the recorded step and by its last: three copies took 11 us of a step, each a
     // gap of 2 to 3 us and 2 us of copying.
-    const bool in = reachable(m->ctx, tokens_dev), results = reachable(m->ctx, logits_dev) && reachable(m->ctx, next_dev);
+    const size_t logit_bytes = c->b * m->cfg.vocab_size * 4;
+    const bool in = reachable(m->ctx, tokens_dev, c->b * 4), results = reachable(m->ctx, logits_dev, logit_bytes) && reachable(m->ctx, next_dev, c->b * 4);
     const StepOut to = results ? StepOut{logits_dev, next_dev} : StepOut{};
-    take_in_kernel<<<1, 32, 0, st>>>(tokens_dev, c->tokens, in ? static_cast<int>(c->b) : 0, to, c->out);
-    LBK_CUDA(cudaGetLastError());
-    m->ctx->launches++;
-    if (!in) LBK_CUDA(cudaMemcpyAsync(c->tokens, tokens_dev, c->b * 4, cudaMemcpyDeviceToDevice, st));
+    if (!in) LBK_CUDA(cudaMemcpyAsync(c->tokens, tokens_dev, c->b * 4, cudaMemcpyDeviceToDevice, st));  // first: a refused one leaves no pointers behind
+    if (in || to.logits || to.next) {
+        take_in_kernel<<<1, 32, 0, st>>>(tokens_dev, c->tokens, in ? static_cast<int>(c->b) : 0, to, c->out);
+        LBK_CUDA(cudaGetLastError());
+        m->ctx->launches++;
+    }
     const cudaError_t launched = cudaGraphLaunch(c->step, st);
     if (launched != cudaSuccess) cudaMemsetAsync(c->out, 0, sizeof(StepOut), st);  // nobody takes the pointers up
     LBK_CUDA(launched);
     m->ctx->launches += c->step_launches;
     if (!results) {
-        if (logits_dev) LBK_CUDA(cudaMemcpyAsync(logits_dev, c->logits, c->b * m->cfg.vocab_size * 4, cudaMemcpyDeviceToDevice, st));
+        if (logits_dev) LBK_CUDA(cudaMemcpyAsync(logits_dev, c->logits, logit_bytes, cudaMemcpyDeviceToDevice, st));
         if (next_dev) LBK_CUDA(cudaMemcpyAsync(next_dev, c->next, c->b * 4, cudaMemcpyDeviceToDevice, st));
     }
     for (size_t &l : c->lens) l += 1;

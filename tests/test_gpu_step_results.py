@@ -54,3 +54,66 @@ def test_results_reach_the_caller(ctx, tmp_path, vocab, b):
         net.forward(np.array([2 % vocab], np.uint32), cache)
         assert torch.equal(kept, before)
     ctx.check_device_error()
+
+
+class Device:
+    """An allocation of its own of so many bytes (512 lie behind any: nothing else is there to be hit)."""
+
+    def __init__(self, size, managed=False):
+        self.lib, self.at = C.CDLL("libcuda.so.1"), C.c_uint64()
+        status = self.lib.cuMemAllocManaged(C.byref(self.at), C.c_size_t(size), C.c_uint(1)) if managed else self.lib.cuMemAlloc_v2(C.byref(self.at), C.c_size_t(size))
+        assert status == 0
+        self.size = size
+
+    def tensor(self, dtype, n, offset=0):
+        import torch
+        raw = torch.empty(n * 4, dtype=torch.uint8, device="cuda")
+        assert self.lib.cuMemcpyDtoD_v2(C.c_uint64(raw.data_ptr()), C.c_uint64(self.at.value + offset), C.c_size_t(n * 4)) == 0
+        return raw.view(dtype)
+
+    def free(self):
+        self.lib.cuMemFree_v2(self.at)
+
+
+def _decode(net, cache, tokens, logits, nxt):
+    import torch
+    from lemonade_burn_b200 import _lib
+    return _lib.load().lbk_model_decode(net.handle, cache, C.c_void_p(tokens), C.c_void_p(logits), C.c_void_p(nxt), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+
+
+@pytest.mark.parametrize("b", [1, 5])
+def test_memory_of_other_kinds(ctx, tmp_path, b):
+    """Results and tokens in managed memory, and in allocations that end with them."""
+    import torch
+    net, vocab = _net(ctx, tmp_path, 100), 100
+    toks = torch.arange(b, dtype=torch.int32, device="cuda")
+    want, nxt = torch.zeros(b, vocab, device="cuda"), torch.zeros(b, dtype=torch.int32, device="cuda")
+    assert _decode(net, net.new_cache(b, 8), toks.data_ptr(), want.data_ptr(), nxt.data_ptr()) == 0
+    for managed in (True, False):
+        t, l, n = Device(b * 4, managed), Device(b * vocab * 4, managed), Device(b * 4, managed)
+        assert t.lib.cuMemcpyDtoD_v2(t.at, C.c_uint64(toks.data_ptr()), C.c_size_t(b * 4)) == 0
+        torch.cuda.synchronize()
+        assert _decode(net, net.new_cache(b, 8), t.at.value, l.at.value, n.at.value) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(l.tensor(torch.float32, b * vocab).view(b, vocab), want) and torch.equal(n.tensor(torch.int32, b), nxt)
+        for d in (t, l, n):
+            d.free()
+    ctx.check_device_error()
+
+
+def test_memory_that_does_not_hold_the_call_is_refused(ctx, tmp_path):
+    """By a status, as a copy refuses it; and a step that was refused for its tokens leaves nothing behind for the next one to write to."""
+    import torch
+    net, vocab = _net(ctx, tmp_path, 100), 100
+    toks = torch.zeros(1, dtype=torch.int32, device="cuda")
+    small, few = Device(vocab * 4 - 256), Device(4)
+    assert _decode(net, net.new_cache(1, 8), toks.data_ptr(), small.at.value, None) != 0
+    logits, cache = torch.zeros(5, vocab, device="cuda"), net.new_cache(5, 8)
+    assert _decode(net, cache, few.at.value, logits.data_ptr(), None) != 0
+    good = torch.zeros(5, dtype=torch.int32, device="cuda")
+    assert _decode(net, cache, good.data_ptr(), None, None) == 0
+    torch.cuda.synchronize()
+    assert not bool(logits.any())
+    small.free()
+    few.free()
+    ctx.check_device_error()
