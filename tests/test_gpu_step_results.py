@@ -117,3 +117,65 @@ def test_memory_that_does_not_hold_the_call_is_refused(ctx, tmp_path):
     small.free()
     few.free()
     ctx.check_device_error()
+
+
+def _greedy(row):
+    """sample.rs:17-25: the first index whose value is above all in front of it; comparisons with a NaN do not hold."""
+    best, at = row[0], 0
+    for i, v in enumerate(row):
+        if v > best:
+            best, at = v, i
+    return at
+
+
+@pytest.mark.parametrize("vocab", [257, 5003])
+def test_greedy_token_of_unusual_rows(ctx, tmp_path, vocab):
+    """A NaN in front, NaNs inside, rows of -inf but for one, equal maxima in two parts of a row, the maximum at either end."""
+    import torch
+    from lemonade_burn_b200 import _lib, dugulorn
+    cfg, token = dugulorn.make_config(vocab, 256, [dugulorn.delta_layer(2, 2, 64, 64, 4, 192)]), 7
+    tensors = dugulorn.random_checkpoint(cfg, 5, 16)
+    name = next(k for k, v in tensors.items() if v.shape == (vocab, 256))
+    table = torch.from_numpy(tensors[name].view(np.int16)).view(torch.bfloat16)
+
+    def step(change):
+        t = table.clone()
+        change(t)
+        folder = tmp_path / f"m{step.count}"
+        step.count += 1
+        folder.mkdir()
+        dugulorn.save_checkpoint(folder, cfg, {**tensors, name: t.view(torch.int16).numpy().view(np.uint16)})
+        net = dugulorn.NativeDugulorn(folder, ctx, "float32")
+        logits, nxt = torch.zeros(2, vocab, device="cuda"), torch.full((2,), -1, dtype=torch.int32, device="cuda")
+        toks = torch.tensor([token, token], dtype=torch.int32, device="cuda")
+        assert _decode(net, net.new_cache(2, 8), toks.data_ptr(), logits.data_ptr(), nxt.data_ptr()) == 0
+        argmax = torch.empty_like(nxt)
+        _lib.check(_lib.load().lbk_argmax(ctx.handle, logits.data_ptr(), 2, vocab, argmax.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        rows = logits.cpu().numpy()
+        assert nxt.tolist() == [_greedy(r) for r in rows] and torch.equal(nxt, argmax)
+        return rows[0], int(nxt[0])
+
+    step.count = 0
+    plain, top = step(lambda t: None)
+    assert top == int(plain.argmax())
+    along = torch.sign(torch.from_numpy(plain[top:top + 1])) * table[top].float()  # a row whose logit is positive
+
+    def rows_are(places, value):
+        def change(t):
+            for i in places:
+                t[i] = value
+        return change
+
+    assert step(rows_are([0], float("nan")))[1] == 0
+    row, at = step(rows_are([9, 64, vocab - 1], float("nan")))
+    assert np.isnan(row[[9, 64, vocab - 1]]).all() and at == int(np.nanargmax(row))
+    for places in ([100, vocab - 3], [0, vocab - 1], [vocab - 1], [79, 80]):
+        row, at = step(rows_are(places, (along * 64).to(torch.bfloat16)))
+        assert at == places[0] and (row[places] == row[at]).all()
+    low = torch.zeros(256)
+    low[int(along.abs().argmax())] = -torch.sign(along[int(along.abs().argmax())]) * float("inf")
+    others = [i for i in range(vocab) if i != token]
+    row, at = step(rows_are(others, low.to(torch.bfloat16)))
+    if not np.isnan(row).any():
+        assert at == (token if row[others[0]] == -np.inf else 0)
+    ctx.check_device_error()
