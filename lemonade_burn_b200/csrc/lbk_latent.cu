@@ -61,13 +61,13 @@ struct PrepParams {
     float eps;
     Angles rot;
     void *cq, *cache;
-    bool settled;
     int *err_word;
 };
 
 // What a thread needs is asked for at once, settled weights before the kernel in front is known to be complete: loaded where they are used they were a chain of six
 // trips to L2 (16 rows with a cache of their own 7.2 us; with the norms' weights asked for as early, a step of four mixed layers of 2560 took 299 us instead of 311).
-template <typename T>
+// SETTLED is compiled apart: behind a branch the compiler moves the loads of the weights back to where they are used.
+template <typename T, bool SETTLED>
 __global__ void __launch_bounds__(256) latent_prep_kernel(const PrepParams p) {
     ptx::pdl_trigger();
     __shared__ float2 s_red[8];
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) latent_prep_kernel(const PrepParams p) {
     constexpr int kHeld = 8, kHeldKv = 2;                  // the first values of a thread stay in registers
     float held[kHeld], held_kv[kHeldKv], wq[kHeld], wkv[kHeldKv];
     const int half = p.rot_dim / 2;
-    if (!p.settled) ptx::pdl_wait();
+    if (!SETTLED) ptx::pdl_wait();
 #pragma unroll
     for (int j = 0; j < kHeld; ++j) wq[j] = tid + 256 * j < p.q_rank ? __ldg(p.q_norm + tid + 256 * j) : 0.0f;
 #pragma unroll
@@ -928,9 +928,10 @@ int launch_latent_prep(Ctx *ctx, const LatentPrepCall &c, cudaStream_t st) {
     p.rot = angles(c.rot);
     p.cq = c.cq;
     p.cache = c.cache;
-    p.settled = c.settled;
     p.err_word = ctx->err_word;
-    LBK_CUDA(launch_chained(c.compute == LBK_COMPUTE_F32 ? latent_prep_kernel<float> : latent_prep_kernel<uint16_t>, dim3(static_cast<unsigned>(c.rows)), dim3(256), 0, st, p));
+    void (*k)(PrepParams) = c.settled ? latent_prep_kernel<uint16_t, true> : latent_prep_kernel<uint16_t, false>;
+    if (c.compute == LBK_COMPUTE_F32) k = c.settled ? latent_prep_kernel<float, true> : latent_prep_kernel<float, false>;
+    LBK_CUDA(launch_chained(k, dim3(static_cast<unsigned>(c.rows)), dim3(256), 0, st, p));
     LBK_CUDA(cudaGetLastError());
     ctx->launches++;
     return LBK_OK;
