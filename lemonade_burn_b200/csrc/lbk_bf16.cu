@@ -81,9 +81,10 @@ __global__ void __launch_bounds__(kThreads) bf16_linear_kernel(const float *__re
 }
 
 // One token row, whole 16-byte units: a warp takes two table rows at a time, U units of each a lane in flight together, and the first
-// ones are on their way before the kernel in front is known to be complete where the caller vouches that no such kernel writes the table (`settled`). Bound: HBM, rows * cols * 2 bytes. The kernel above, one row a
-// warp with four units in flight, reads the table at 3.8 to 4.8 TB/s, this one at 6.4 to 7.0: 128256 x 2560 144 -> 96 us, 32000 x 2560 42.6 -> 25.6,
-// 32000 x 4096 58.9 -> 41.0, 32000 x 1000 26.2 -> 10.9. Same order of every sum, same bits.
+// ones are on their way before the kernel in front is known to be complete where the caller vouches that no such kernel writes the table (`settled`). Bound: HBM, rows * cols * 2 bytes. Against the kernel above, one row a
+// warp with four units in flight, calls behind one another, so that up to 126 MB of a table are in L2: 128256 x 2560 150 -> 95 us = 4.4 -> 6.9 TB/s,
+// 32000 x 4096 69 -> 41 = 3.8 -> 6.4, 32000 x 2560 43 -> 26 = 3.8 -> 6.4, 32000 x 1000 (64 MB) 25 -> 10 = 2.6 -> 6.4. One call on a cold table, launch
+// included: 128256 x 2560 109 us = 6.0 TB/s. Same order of every sum, same bits.
 template <int U>
 __global__ void __launch_bounds__(kThreads, 3) bf16_row_kernel(const float *x, const uint16_t *w, int rows, int cols, float *out, int settled) {
     extern __shared__ float s_x[];

@@ -48,7 +48,7 @@ constexpr int kPrepThreads = 128;
 constexpr int kScal = 2 * kTok * kTok;  // numbers of a record: T, then p, eight by eight
 // Columns of a walk's warp, by rule and packed pairs a lane (dp / 64). us for 2048 rows, two / four columns, prep included: delta 20 heads of 128 x 128
 // 383 / 420, 64 of 64 x 128 1067 / 1288, 16 of 256 x 256 762 / 619; plain 64 of 64 x 128 515 / 431, 16 of 256 x 256 462 / 601. Plain heads of 128 lie
-// between: alone 20 heads take 238 / 240 (64 rows 18 / 15), 32 heads 409 / 394, sixteen prompts of a mixed model 0.5 % less with two.
+// between: alone 20 heads take 238 / 240 (64 rows 18 / 15), 32 heads 409 / 394, sixteen prompts and 48 steps of a mixed model 0.2 % less with two.
 __host__ __device__ constexpr int walk_cols(bool delta, int pairs) { return (delta ? pairs <= 2 : pairs >= 2) ? 2 : 4; }
 // warps of a walk's block that hold columns at most
 __host__ __device__ constexpr int max_warps(int cols) { return 32 / cols; }

@@ -346,13 +346,13 @@ bool json_positive(const Json *j, size_t *out);
 // ---- the base classes ---------------------------------------------------------------------------
 struct Model;
 
-// The sequences ("slots") a model serves together. The family's class adds its K/V rows and work buffers.
 // Where a caller wants the results of the step that is being launched; null: nowhere.
 struct StepOut {
     float *logits = nullptr;
     int32_t *next = nullptr;
 };
 
+// The sequences ("slots") a model serves together. The family's class adds its K/V rows and work buffers.
 struct Cache {
     Model *model = nullptr;
     size_t b = 0, cap = 0;

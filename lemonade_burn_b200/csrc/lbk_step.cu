@@ -28,7 +28,7 @@
 // a step took 1.5 times as long.
 //
 // Measured, a whole step with head and argmax, a kernel per operation -> this: one sequence at 2000 positions, 30 layers of 2560,
-// vocabulary 128256 1309 -> 787 us (of it 110 the head); sixteen sequences at 400 positions, 8 layers, vocabulary 32000 547 -> 378 us. At other widths,
+// vocabulary 128256 1309 -> 787 us (of it 110 the head); sixteen sequences at 400 positions, 8 layers, vocabulary 32000 547 -> 370 us. At other widths,
 // 512 to 8192, with 1 to 16 sequences at 100 and 2000 positions, 1.14 to 2.8 times as fast as a kernel per operation, rings of two stages included.
 #include "lbk_gemv_core.cuh"
 
@@ -608,7 +608,7 @@ __device__ __forceinline__ void merge_slices(const Cta &c, const StepParams &p, 
 
 // Asks for the keys and values that this CTA takes in `layer`'s attention to come to L2, a layer ahead: asked for behind the q/k/v products they
 // queued behind the weights of the next projections, which every SM fetches at that time, and the slowest slice was twice the usual one. 30 layers of 2560
-// at 2000 positions 799 -> 787 us a step, 16 sequences at 400, eight layers 385 -> 378.
+// at 2000 positions 799 -> 787 us a step, 16 sequences at 400, eight layers 385 -> 378 (with the step's last kernel as it was then).
 __device__ __forceinline__ void call_cache(const Cta &c, const StepParams &p, int layer) {
     const int TW = p.team_warps, teams = kWarps / TW, team = c.warp / TW, units = p.m * p.kv_heads * p.slices;
     if (c.tid - team * TW * 32 != 0 || p.layer_stride % 8) return;  // a bulk prefetch starts on 16 bytes; the loads themselves need 8
