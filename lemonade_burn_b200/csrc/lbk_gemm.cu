@@ -551,47 +551,25 @@ int gemm_init(Ctx *ctx) {
 }
 static const InitHook kInitGemm(gemm_init);
 
-// Parts to cut every tile's K blocks into. A launch with few tiles against the SM count (small
-// token batches, tensor-parallel shards) or with a ragged last round leaves SMs idle; parts add
-// their int32 sums into a zeroed buffer and a small kernel scales them afterwards. Cost model in
-// K-block times of one CTA (250 cycles in the narrow kernel to 490 in the wide one); the parts' atomic adds, the scaling launch and its
-// traffic are charged as 30 of them (14 was tried when a block took 500 cycles: the 70B-shaped gate/up
-// projection at 64 token rows then split in two and took twice as long, 14.7 MB of sums added twice). Uncut, the fullest CTA
-// has `rounds` tiles (choose_nt): counted as whole rounds, a launch whose last round are short tiles of a ragged batch looked twice as long as it
-// is and was cut in eight, at 777 rows of 8192 -> 2 x 2048 75 us instead of 31.
-static int choose_ksplit(int tiles, double rounds, int k_blocks, int sms, int *kb_part) {
-    int best = 1;
-    double best_cost = rounds * k_blocks;
-    *kb_part = k_blocks;
-    for (int s = 2; s <= 8; ++s) {
-        const int per = ((k_blocks + s - 1) / s + kPackBlocks - 1) / kPackBlocks * kPackBlocks;
-        if (per < 2 * kPackBlocks) break;
-        const int parts = (k_blocks + per - 1) / per;
-        if (parts != s) continue;  // rounding made fewer parts: that count is or was tried as itself
-        const double cost = static_cast<double>((static_cast<long long>(tiles) * s + sms - 1) / sms) * per + 30.0;
-        if (cost * 100.0 < best_cost * 85.0) {
-            best_cost = cost;
-            best = s;
-            *kb_part = per;
-        }
-    }
-    return best;
-}
-
-
-// Token rows per tile for a launch, a multiple of 16: the count with the least cost in cycles of the fullest CTA. Up to 64 the
-// narrow kernel runs, 250 cycles a K block; the wide one takes 365 at 96 token rows and 490 at 192 (launches of many
+// Token rows per tile for a launch, a multiple of 16, and parts to cut every tile's K blocks into: the pair with the least cost in cycles of the fullest CTA.
+// A K block takes 250 cycles in the narrow kernel, which runs up to 64 token rows; in the wide one 365 at 96 and 490 at 192 (launches of many
 // rounds, their epilogues beside the products; 341 and 416 in a single round). 15 cycles a token row are the last tile's
-// epilogue, 300 the start of a tile: with 35, fitted when four warps did an epilogue, matrices of few columns went in narrow tiles, 2048 rows
-// of 512 -> 2 x 1376 16.7 us instead of 11.9, 256 of 1000 -> 2 x 2700 9.6 instead of 7.4. Short tiles of a ragged batch come last (decode_tile in the kernel): what is left
+// epilogue, 300 the start of a tile. Short tiles of a ragged batch come last (decode_tile in the kernel): what is left
 // over behind the full rounds are short ones, and with the order turned round every other time a CTA that has two of them
-// at the end takes less than a full tile longer than the others. Measured at 2560 -> 2 x 6912, us: 400 rows in tiles of 112 / 144 / 176
-// 15.5 / 15.8 / 14.8, 2048 rows in tiles of 64 / 128 / 160 / 192 69.4 / 59.0 / 56.0 / 54.7; 2560 -> 3840 at 96 rows in tiles of 48 / 96: 5.3 / 6.6.
-// Over 28 groups of 512 to 14336 columns at 20 sizes the choice is 2 % slower than the best tile (geometric mean).
-static int choose_nt(int m, int row_tiles, int k_blocks, int sms, double *rounds_out) {
+// at the end takes less than a full tile longer than the others.
+// A launch with few tiles against the SM count (small token batches, tensor-parallel shards) leaves SMs idle: parts add
+// their int32 sums into a zeroed buffer, 60 cycles a token row and tile, and a small kernel scales them afterwards, 6000 cycles, and 0.004 for each sum
+// and each time it is added, read and zeroed. A cut has to be 7 % better.
+// The constants are fitted to every tile and cut of 14 groups of 512 to 28672 columns at 15 sizes: the choice is 1.4 % slower than the best pair (geometric mean). Tile first
+// and cut afterwards (3.3 %), with an epilogue as four warps did it and rounds counted as whole ones, had us, chosen then / now: 777 rows of 8192 -> 2 x 2048 75 / 31, 2048 of
+// 512 -> 2 x 1376 16.7 / 11.9, 24 of 14336 -> 4096 17.0 / 12.4, 150 of 20480 -> 1000 20.1 / 14.9.
+struct TileChoice {
+    int nt = 0, ksplit = 1, kb_part = 0;
+};
+static TileChoice choose_tile(int m, int row_tiles, size_t rows, int k_blocks, int sms, bool may_cut) {
     auto block = [](int nt) { return nt <= 64 ? 250.0 : 240.0 + 1.3 * nt; };
-    int best_nt = 0;
-    double best = 0.0;
+    TileChoice best;
+    double best_cost = 0.0;
     for (int nt = 16; nt <= kWide; nt += 16) {
         const int full = m / nt, rest = m % nt;
         const long long shorts = rest ? row_tiles : 0, tiles = static_cast<long long>(full) * row_tiles + shorts;
@@ -601,15 +579,25 @@ static int choose_nt(int m, int row_tiles, int k_blocks, int sms, double *rounds
         if (left > shorts) rounds += 1.0;
         else if (left > 0 && 2 * left <= shorts && whole > 0) rounds += 2.0 * least > 1.0 ? 2.0 * least - 1.0 : 0.0;
         else if (left > 0) rounds += least;
-        const double cost = rounds * (k_blocks * block(nt) + 300.0) + 15.0 * nt;
-        if (best_nt == 0 || cost < best) {
-            best = cost;
-            best_nt = nt;
-            *rounds_out = rounds;
+        const double last = 15.0 * nt, uncut = rounds * (k_blocks * block(nt) + 300.0) + last;
+        if (best.nt == 0 || uncut < best_cost) {
+            best_cost = uncut;
+            best = {nt, 1, k_blocks};
+        }
+        for (int s = 2; may_cut && s <= 8; ++s) {
+            const int per = ((k_blocks + s - 1) / s + kPackBlocks - 1) / kPackBlocks * kPackBlocks;
+            if (per < 2 * kPackBlocks) break;
+            if ((k_blocks + per - 1) / per != s) continue;  // rounding made fewer parts: that count is or was tried as itself
+            const double cost = static_cast<double>((tiles * s + sms - 1) / sms) * (per * block(nt) + 300.0 + 60.0 * nt) + last + 6000.0 +
+                                0.004 * m * static_cast<double>(rows) * (s + 2);
+            if (cost < 0.93 * best_cost) {
+                best_cost = cost;
+                best = {nt, s, per};
+            }
         }
         if (nt >= m) break;
     }
-    return best_nt;
+    return best;
 }
 
 int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
@@ -623,8 +611,15 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
         return fail(LBK_ERR_INVALID, "gemm: a gated pair is two matrices of one shape with an f32 output");
     for (int i = 0; i < g.n; ++i) row_tiles += static_cast<int>((g.w[i]->rows + kBMW - 1) / kBMW);
     if (g.gated) row_tiles = static_cast<int>((g.w[0]->rows + kBMW / 2 - 1) / (kBMW / 2));
-    double rounds = 1.0;
-    const int nt = choose_nt(static_cast<int>(g.m), row_tiles, static_cast<int>(kp / kBK), ctx->sm_count, &rounds);
+    // A cut tile's parts meet in the caller's integer outputs where they are given, else in slices of the context's buffer. Not before a gated pair's product, and
+    // not in peer memory.
+    size_t rows = 0, need = 0;
+    for (int i = 0; i < g.n; ++i) {
+        rows += g.w[i]->rows;
+        if (!g.iout[i]) need += (g.m * g.w[i]->rows * sizeof(int32_t) + 255) / 256 * 256;
+    }
+    const TileChoice choice = choose_tile(static_cast<int>(g.m), row_tiles, rows, static_cast<int>(kp / kBK), ctx->sm_count, !g.gated && !g.scatter_world && need <= kGemmAccBytes);
+    const int nt = choice.nt;
     LBK_TRY(encode_act_map(&p.act, g.q, g.m, kp, nt));
     p.nt = nt;
     p.m = static_cast<int>(g.m);
@@ -654,39 +649,25 @@ int launch_gemm(Ctx *ctx, const GroupArgs &g, cudaStream_t stream) {
     p.qsum = g.qsum;
     p.err_word = ctx->err_word;
     if (tiles == 0 || p.k_blocks == 0) return LBK_OK;
-    p.ksplit = choose_ksplit(tiles, rounds, p.k_blocks, ctx->sm_count, &p.kb_part);
-    if (g.gated) {  // the parts' sums would have to meet before the product
-        p.ksplit = 1;
-        p.kb_part = p.k_blocks;
-    }
+    p.ksplit = choice.ksplit;
+    p.kb_part = choice.kb_part;
     p.scatter_world = g.scatter_world;
     p.scatter_mt = g.scatter_mt;
     for (int i = 0; i < 8; ++i) p.scatter[i] = g.scatter_base[i];
     if (g.scatter_world) {
         if (g.n != 1 || g.scatter_mt < 1) return fail(LBK_ERR_INVALID, "gemm: scattered outputs take one matrix");
-        p.ksplit = 1;  // parts of a tile would have to add into peer memory
-        p.kb_part = p.k_blocks;
     }
     if (p.ksplit > 1) {
-        // int32 targets: the caller's integer outputs where given, else slices of the context's buffer
-        size_t need = 0;
-        for (int i = 0; i < g.n; ++i)
-            if (!g.iout[i]) need += (g.m * g.w[i]->rows * sizeof(int32_t) + 255) / 256 * 256;
-        if (need > kGemmAccBytes) {
-            p.ksplit = 1;
-            p.kb_part = p.k_blocks;
-        } else {
-            size_t off = 0;
-            for (int i = 0; i < g.n; ++i) {
-                const size_t bytes = g.m * g.w[i]->rows * sizeof(int32_t);
-                if (g.iout[i]) {
-                    p.acc[i] = g.iout[i];
-                    LBK_CUDA(cudaMemsetAsync(p.acc[i], 0, bytes, stream));  // the caller's buffer holds whatever it held
-                } else {
-                    // the context's buffer is zero at rest (launch_scale_epilogue_group zeroes what it reads)
-                    p.acc[i] = reinterpret_cast<int32_t *>(reinterpret_cast<char *>(ctx->gemm_acc) + off);
-                    off += (bytes + 255) / 256 * 256;
-                }
+        size_t off = 0;
+        for (int i = 0; i < g.n; ++i) {
+            const size_t bytes = g.m * g.w[i]->rows * sizeof(int32_t);
+            if (g.iout[i]) {
+                p.acc[i] = g.iout[i];
+                LBK_CUDA(cudaMemsetAsync(p.acc[i], 0, bytes, stream));  // the caller's buffer holds whatever it held
+            } else {
+                // the context's buffer is zero at rest (launch_scale_epilogue_group zeroes what it reads)
+                p.acc[i] = reinterpret_cast<int32_t *>(reinterpret_cast<char *>(ctx->gemm_acc) + off);
+                off += (bytes + 255) / 256 * 256;
             }
         }
     }

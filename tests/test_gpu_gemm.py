@@ -45,7 +45,7 @@ def random_case(rows, cols, m, seed, oracle):
 def test_config2_shapes(oracle, ctx, rows, cols, m):
     """Both BitNet-2B prefill projections at every token count of the benchmark configuration, every
     output element against the oracle: int32 sums and f32 bits. K = 6912 at the larger token counts is
-    where the GEMM cuts K into parts that add their sums (`choose_ksplit`); the host-buffer entry
+    where the GEMM cuts K into parts that add their sums (`choose_tile`); the host-buffer entry
     point and the device-resident one are both driven."""
     import torch
     from lemonade_burn_b200 import ops

@@ -50,7 +50,8 @@ def test_launches_behind_one_another_give_the_same_rows(oracle, ctx, m):
     ctx.check_device_error()
 
 
-@pytest.mark.parametrize("cols,rows,m", [(8192, [2048, 2048], 777), (8640, [3200], 1024), (512, [1376, 1376], 2048), (1000, [2700, 2700], 256), (14336, [4096], 17)])
+@pytest.mark.parametrize("cols,rows,m", [(8192, [2048, 2048], 777), (8640, [3200], 1024), (512, [1376, 1376], 2048), (1000, [2700, 2700], 256), (14336, [4096], 17), (14336, [4096], 61),
+                                         (8192, [2048, 2048], 25), (20480, [1000], 150)])
 def test_one_batch_or_portions(ctx, cols, rows, m):
     """Launches whose last round are short tiles, matrices of few columns, long columns in few tiles: whatever tile and cut are chosen for all rows at once, the
     bits are those of the rows in portions of 64 and fewer, which go by other tiles. Equality: the same integers and products of scales."""
